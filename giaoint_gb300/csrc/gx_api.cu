@@ -218,6 +218,8 @@ struct gx_context {
     std::vector<cudaStream_t> aux;
     std::vector<cudaEvent_t> aux_done;
     cudaEvent_t fork = nullptr;
+    cudaEvent_t exec_done = nullptr;  // end of the last asynchronous plan execution
+    bool exec_pending = false;
     std::shared_ptr<SharedTables> t;  // shared immutable tables of the device
     DeviceBuffer status;
     std::mutex mu;
@@ -339,6 +341,7 @@ struct gx_basis {
     int64_t nao = 0;
     // segmented shells: shell s, contraction x -> seg_first[s] + x
     int nseg = 0;
+    bool one_site = true;  // all shells on one centre
     std::vector<int> seg_first, seg_l, seg_nprim, seg_primoff, seg_raw, seg_orig;
     std::vector<double> seg_center, seg_exps, seg_coefs;
     DeviceBuffer d_center, d_l, d_nprim, d_primoff, d_exps, d_coefs, d_raw, d_sp_off;
@@ -401,6 +404,8 @@ void build_segments(gx_basis* b) {
     upload(b->d_exps, b->seg_exps, s);
     upload(b->d_coefs, b->seg_coefs, s);
     upload(b->d_raw, b->seg_raw, s);
+    for (int sh = 1; sh < b->ns; ++sh)
+        for (int k = 0; k < 3; ++k) b->one_site = b->one_site && b->center[3 * sh + k] == b->center[k];
     // every ordered segmented shell pair, primitive pairs pa-major
     const int ns = b->nseg;
     std::map<std::pair<int, int>, int> cls;
@@ -553,7 +558,7 @@ struct ClassConf {
     int minb = 0;       // generic kernel: register-budget variant (2 or 4 resident blocks; 0 = 2)
     int nostage = 0;    // generic kernel: 1 = read E~ records and class tables from global memory
     int stream = 0;     // generic kernel: 1 = per-entry recurrences into a two-column buffer (stream mode)
-    int nolane = 0;     // 1 = the generic kernel also takes the FP32 entries (no FP32 lane kernel)
+    int nolane = 0;     // 1 = the generic kernel takes the class (not the lane-dense kernel)
 };
 
 // Configuration of a class before any tuning, from the autotuner's choices on
@@ -590,7 +595,6 @@ ClassConf default_conf(const std::array<int, 4>& k) {
 struct GroupSet {
     DeviceBuffer dev;
     std::vector<std::pair<size_t, size_t>> range;  // per class: first group, count
-    std::vector<std::pair<size_t, size_t>> lane;   // per class: groups of the FP32 lane kernel (count 0: none)
 };
 
 struct PlanData {
@@ -598,6 +602,7 @@ struct PlanData {
     GroupSet base;                  // default configuration
     std::vector<PlanClass> classes;
     std::vector<int> task_kk;       // per task (class order): Kab << 16 | Kcd, for regrouping
+    std::vector<uint8_t> task_site; // per task: 2 when the bra shells share a centre, + 1 when the ket shells do
     std::vector<int> task_part;     // per task: its part (request) of a packed plan; empty for one part
     bool stable = false;            // launch configuration independent of the plan's size (see launch_class)
     std::vector<ClassConf> defconf; // per class: the configuration used before any tuning
@@ -607,6 +612,14 @@ struct PlanData {
                                     // sized for the classes of the whole list
     int64_t ntask = 0, primitive_quartets = 0;
     double model_flops = 0.0;
+    // units of the small and lane-dense classes, cut on the device at every
+    // execution; per class its FP64 and FP32 index there (-1: none), its unit
+    // count, unit weight and shell dimensions
+    DeviceBuffer unit_mem;
+    gx::UnitPlan units{};
+    std::vector<gx::UnitClass> unit_first;
+    std::vector<int> unit_class, unit_class32, unit_grid, unit_dims;
+    std::vector<int64_t> unit_target;
     // autotuned configuration per precision mode (GX_PRECISION_*)
     struct Tuned {
         bool valid = false;
@@ -687,17 +700,20 @@ void record_tuning(const gx_context* ctx, const gx_basis* b, int precision, cons
     for (size_t ci = 0; ci < plan.classes.size(); ++ci) db[plan.classes[ci].key] = conf[ci];
 }
 
-// Warp work units of class ci: runs of tasks with equal primitive counts
-// (Kab, Kcd).  Small classes (one lane per primitive quartet) take up to
-// `per_group` (default 1024) primitive quartets and 128 tasks per unit; the
-// generic kernel about `per_group` (default 32) primitive quartets and at
-// most 1024 tasks per unit, fewer tasks when the class is too small to give
-// every SM eight warps.
-std::vector<int2> make_groups(const gx_context* ctx, const PlanData& plan, size_t ci, const ClassConf& conf,
-                              bool lane_units = false) {
+// The class runs in the lane-dense kernel (unless it is pinned to the
+// class-generic one).
+bool runs_dense(const PlanClass& pc, const ClassConf& conf) {
+    return !conf.nolane && gx::dense_class(pc.key[0], pc.key[1], pc.key[2], pc.key[3]);
+}
+
+// Warp work units of class ci in the class-generic kernel: runs of tasks with
+// equal primitive counts (Kab, Kcd) and the same sides on one centre, about
+// `per_group` (default 32) primitive quartets and at most 1024 tasks per unit,
+// fewer tasks when the class is too small to give every SM eight warps.
+std::vector<int2> make_groups(const gx_context* ctx, const PlanData& plan, size_t ci, const ClassConf& conf) {
     const PlanClass& pc = plan.classes[ci];
-    const bool small = lane_units || gx::small_class(pc.key[0], pc.key[1], pc.key[2], pc.key[3]);
-    const int per = lane_units ? 1024 : (conf.per_group > 0 ? conf.per_group : (small ? 1024 : 32));
+    if (gx::small_class(pc.key[0], pc.key[1], pc.key[2], pc.key[3]) || runs_dense(pc, conf)) return {};
+    const int per = conf.per_group > 0 ? conf.per_group : 32;
     const size_t count = pc.count * (size_t)std::max(plan.spread_parts, 1);
     const int spread = std::max<int>(1, (int)(count / (size_t)(8 * std::max(ctx->sm_count, 1))));
     std::vector<int2> groups;
@@ -706,22 +722,16 @@ std::vector<int2> make_groups(const gx_context* ctx, const PlanData& plan, size_
     while (i < end) {
         const int kk_code = plan.task_kk[i];
         const int kk = (kk_code >> 16) * (kk_code & 0xffff);
-        // one lane per primitive quartet: up to `per` of them and 128 tasks per
-        // unit, but at least ~4 units per SM when the class is small (a
-        // Cholesky column plan holds a few dozen tasks per class); a stable
-        // plan keeps its units independent of the class size
-        int want = small ? std::max(1, std::min(128, per / kk))
-                         : std::max(1, std::min({1024, (per + kk - 1) / kk, spread}));
-        if (small && !plan.stable)
-            want = std::max(1, std::min<int>(want, (int)(count / (size_t)(4 * std::max(ctx->sm_count, 1)))));
+        const int want = std::max(1, std::min({1024, (per + kk - 1) / kk, spread}));
         size_t j = i + 1;
         if (plan.task_part.empty()) {
-            while (j < end && (int)(j - i) < want && plan.task_kk[j] == kk_code) ++j;
+            while (j < end && (int)(j - i) < want && plan.task_kk[j] == kk_code && plan.task_site[j] == plan.task_site[i])
+                ++j;
         } else {
             // a packed plan: units never mix requests, so that every request's
             // units (and its results, bit for bit) are those of its plan alone
             while (j < end && (int)(j - i) < want && plan.task_kk[j] == kk_code &&
-                   plan.task_part[j] == plan.task_part[i])
+                   plan.task_site[j] == plan.task_site[i] && plan.task_part[j] == plan.task_part[i])
                 ++j;
         }
         groups.push_back(make_int2((int)(i - pc.first), (int)(j - i)));
@@ -730,29 +740,87 @@ std::vector<int2> make_groups(const gx_context* ctx, const PlanData& plan, size_
     return groups;
 }
 
-bool lane_class(const PlanClass& pc) { return gx::lane32_class(pc.key[0], pc.key[1], pc.key[2], pc.key[3]); }
+// Work units of the small and lane-dense classes.  A unit holds about 256
+// surviving primitive quartets (eight batches of 32) in classes that have at
+// least eight such units per SM before screening, else 128, 64 or 32 (16 and 8
+// were measured too: the half-empty batches cost small plans with f shells
+// more than their shorter units gave); a few less, because a unit ends with a
+// whole task and should not spill into a batch of its own.  Classes with few tasks have no
+// entry in the unit arrays: their blocks cut the units themselves.
+void make_units(gx_context* ctx, PlanData& plan) {
+    std::vector<gx::UnitClass> cls;
+    const size_t nc = plan.classes.size();
+    plan.unit_class.assign(nc, -1);
+    plan.unit_class32.assign(nc, -1);
+    plan.unit_grid.assign(nc, 0);
+    plan.unit_target.assign(nc, 0);
+    plan.unit_dims.assign(nc, 0);
+    int64_t vtask = 0, nunit = 0, vtask64 = 0, nunit64 = 0;
+    for (int fp32 = 0; fp32 < 2; ++fp32) {
+        for (size_t ci = 0; ci < nc; ++ci) {
+            const PlanClass& pc = plan.classes[ci];
+            const bool small = gx::small_class(pc.key[0], pc.key[1], pc.key[2], pc.key[3]);
+            if (!gx::dense_class(pc.key[0], pc.key[1], pc.key[2], pc.key[3]) && !(small && !fp32)) continue;
+            const int64_t full = 8 * (int64_t)std::max(ctx->sm_count, 1);
+            const int64_t all = pc.primitive_quartets * std::max(plan.spread_parts, 1);
+            int entries = 256;
+            while (entries > 32 && all / entries < full) entries /= 2;
+            const int64_t mean = pc.primitive_quartets / std::max<int64_t>((int64_t)pc.count, 1);
+            const int64_t target = 64 * (entries - std::min<int64_t>(entries / 16, mean / 4));
+            // as many units as an execution without screening has
+            const int64_t grid = (64 * pc.primitive_quartets + (int64_t)pc.count) / target + 1;
+            int dims = 0;
+            for (int x = 0; x < 4; ++x) dims |= std::min(255, gx::ncart(pc.key[x])) << (8 * x);
+            plan.unit_grid[ci] = (int)grid;
+            plan.unit_target[ci] = target;
+            plan.unit_dims[ci] = dims;
+            if (pc.count < (size_t)gx::kUnitMinTasks) continue;
+            (fp32 ? plan.unit_class32 : plan.unit_class)[ci] = (int)cls.size();
+            cls.push_back(gx::UnitClass{vtask, (long long)pc.first, nunit, target, fp32 ? 1 : (small ? 2 : 0), dims});
+            vtask += (int64_t)pc.count;
+            nunit += grid + 1;
+        }
+        if (!fp32) {
+            vtask64 = vtask;
+            nunit64 = nunit;
+        }
+    }
+    plan.units = gx::UnitPlan{};
+    plan.unit_first = cls;
+    if (cls.empty()) return;
+    const int64_t tiles = gx::unit_tiles(vtask);
+    auto align = [](int64_t x) { return (x + 15) / 16 * 16; };
+    const int64_t o_cls = 16, o_prefix = align(o_cls + (int64_t)(cls.size() * sizeof(gx::UnitClass))),
+                  o_tile = o_prefix + 8 * vtask, o_count = o_tile + 8 * tiles, o_start = o_count + 4 * vtask;
+    plan.unit_mem.reserve((size_t)(o_start + 4 * nunit));
+    char* base = plan.unit_mem.as<char>();
+    GX_CUDA(cudaMemsetAsync(base, 0, 16, ctx->stream));
+    GX_CUDA(cudaMemcpyAsync(base + o_cls, cls.data(), cls.size() * sizeof(gx::UnitClass), cudaMemcpyHostToDevice,
+                            ctx->stream));
+    plan.units = gx::UnitPlan{reinterpret_cast<gx::UnitClass*>(base + o_cls),
+                              (int)cls.size(),
+                              vtask,
+                              nunit,
+                              vtask64,
+                              nunit64,
+                              reinterpret_cast<int*>(base + o_count),
+                              reinterpret_cast<long long*>(base + o_prefix),
+                              reinterpret_cast<long long*>(base + o_tile),
+                              reinterpret_cast<int*>(base + o_start),
+                              reinterpret_cast<unsigned*>(base)};
+}
 
-// Work units of every class, and for the classes with an FP32 lane kernel its
-// units (one lane per primitive quartet: up to 1024 primitive quartets and 128
-// tasks per warp), in one device array.
+// Generic-kernel work units of every class in one device array.
 void make_group_set(gx_context* ctx, const PlanData& plan, const std::vector<ClassConf>& conf, GroupSet& out) {
     const size_t nc = plan.classes.size();
-    std::vector<std::vector<int2>> g(nc), lg(nc);
+    std::vector<std::vector<int2>> g(nc);
 #pragma omp parallel for schedule(dynamic)
-    for (long long ci = 0; ci < (long long)nc; ++ci) {
-        g[ci] = make_groups(ctx, plan, ci, conf[ci]);
-        if (lane_class(plan.classes[ci])) lg[ci] = make_groups(ctx, plan, ci, conf[ci], true);
-    }
+    for (long long ci = 0; ci < (long long)nc; ++ci) g[ci] = make_groups(ctx, plan, ci, conf[ci]);
     std::vector<int2> all;
     out.range.clear();
-    out.lane.clear();
     for (size_t ci = 0; ci < nc; ++ci) {
         out.range.push_back({all.size(), g[ci].size()});
         all.insert(all.end(), g[ci].begin(), g[ci].end());
-    }
-    for (size_t ci = 0; ci < nc; ++ci) {
-        out.lane.push_back({all.size(), lg[ci].size()});
-        all.insert(all.end(), lg[ci].begin(), lg[ci].end());
     }
     upload(out.dev, all, ctx->stream);
 }
@@ -787,8 +855,9 @@ struct PlanPart {
 
 // Class-sorted task list of the parts' blocks: one task per segmented shell
 // quartet (general contractions split), ordered by class (la, lb, lc, ld),
-// then by decreasing bra and ket primitive counts, then by part and request
-// order -- a parallel counting sort over (class, Kab, Kcd) buckets: per-chunk
+// then by decreasing bra and ket primitive counts, then by which sides share a
+// centre, then by part and request
+// order -- a parallel counting sort over those buckets: per-chunk
 // bucket histograms, one prefix over (bucket, chunk), and a scatter pass.
 void build_plan_parts(gx_context* ctx, const std::vector<PlanPart>& parts, PlanData& plan) {
     // shell codes: distinct (l, nprim) of the segmented shells of all parts
@@ -801,11 +870,17 @@ void build_plan_parts(gx_context* ctx, const std::vector<PlanPart>& parts, PlanD
         codes.push_back(kv.first);
     }
     const int nsc = (int)codes.size();
-    std::vector<std::vector<int>> part_code(parts.size());
+    std::vector<std::vector<int>> part_code(parts.size()), part_site(parts.size());
     for (size_t pi = 0; pi < parts.size(); ++pi) {
         const gx_basis* b = parts[pi].b;
         part_code[pi].resize(b->nseg);
-        for (int s = 0; s < b->nseg; ++s) part_code[pi][s] = code_of[{b->seg_l[s], b->seg_nprim[s]}];
+        part_site[pi].resize(b->nseg);
+        std::map<std::array<double, 3>, int> site_of;
+        for (int s = 0; s < b->nseg; ++s) {
+            part_code[pi][s] = code_of[{b->seg_l[s], b->seg_nprim[s]}];
+            const std::array<double, 3> r{b->seg_center[3 * s], b->seg_center[3 * s + 1], b->seg_center[3 * s + 2]};
+            part_site[pi][s] = site_of.emplace(r, (int)site_of.size()).first->second;
+        }
     }
     const int64_t ntuple = (int64_t)nsc * nsc * nsc * nsc;
     if (ntuple > (int64_t)1 << 24) raise(GX_EINVAL, "too many distinct (l, primitive count) shells in one plan");
@@ -821,10 +896,13 @@ void build_plan_parts(gx_context* ctx, const std::vector<PlanPart>& parts, PlanD
     std::vector<BKey> bkeys(tkey);
     std::sort(bkeys.begin(), bkeys.end());
     bkeys.erase(std::unique(bkeys.begin(), bkeys.end()), bkeys.end());
-    const int nb = (int)bkeys.size();
+    // each (class, Kab, Kcd) bucket in four: by whether the bra and the ket
+    // shells share a centre, so that the batches of the kernels with real
+    // arithmetic for such pairs rarely mix the kinds
+    const int nb = 4 * (int)bkeys.size();
     std::vector<int> bucket_of(ntuple);
     for (int64_t t = 0; t < ntuple; ++t)
-        bucket_of[t] = (int)(std::lower_bound(bkeys.begin(), bkeys.end(), tkey[t]) - bkeys.begin());
+        bucket_of[t] = 4 * (int)(std::lower_bound(bkeys.begin(), bkeys.end(), tkey[t]) - bkeys.begin());
     // chunks of requests, never across parts: (part, first, end)
     constexpr int64_t kChunk = 1 << 15;
     struct Chunk {
@@ -846,9 +924,10 @@ void build_plan_parts(gx_context* ctx, const std::vector<PlanPart>& parts, PlanD
         if (parts.empty()) continue;
         const PlanPart& pt = parts[chunks[c].part];
         const gx_basis* b = pt.b;
-        const std::vector<int>& seg_code = part_code[chunks[c].part];
-        auto tuple_of = [&](int a, int bb, int cc, int d) {
-            return ((int64_t)(seg_code[a] * nsc + seg_code[bb]) * nsc + seg_code[cc]) * nsc + seg_code[d];
+        const std::vector<int>&seg_code = part_code[chunks[c].part], &site = part_site[chunks[c].part];
+        auto bucket = [&](int a, int bb, int cc, int d) {
+            const int64_t t = ((int64_t)(seg_code[a] * nsc + seg_code[bb]) * nsc + seg_code[cc]) * nsc + seg_code[d];
+            return bucket_of[t] + (site[a] == site[bb] ? 2 : 0) + (site[cc] == site[d] ? 1 : 0);
         };
         for (int64_t i = chunks[c].first; i < chunks[c].end; ++i) {
             const auto& r = (*pt.req)[i];
@@ -856,8 +935,8 @@ void build_plan_parts(gx_context* ctx, const std::vector<PlanPart>& parts, PlanD
                 for (int xb = 0; xb < b->ncontr[r.b]; ++xb)
                     for (int xc = 0; xc < b->ncontr[r.c]; ++xc)
                         for (int xd = 0; xd < b->ncontr[r.d]; ++xd)
-                            ++h[bucket_of[tuple_of(b->seg_first[r.a] + xa, b->seg_first[r.b] + xb,
-                                                   b->seg_first[r.c] + xc, b->seg_first[r.d] + xd)]];
+                            ++h[bucket(b->seg_first[r.a] + xa, b->seg_first[r.b] + xb, b->seg_first[r.c] + xc,
+                                       b->seg_first[r.d] + xd)];
         }
     }
     // prefix over (bucket, chunk): the first position of each chunk's run
@@ -871,10 +950,11 @@ void build_plan_parts(gx_context* ctx, const std::vector<PlanPart>& parts, PlanD
             btotal[bk] += n;
         }
     for (int bk = 0; bk < nb; ++bk)
-        if (btotal[bk] && bkeys[bk][0] + bkeys[bk][1] + bkeys[bk][2] + bkeys[bk][3] > 32)
+        if (btotal[bk] && bkeys[bk / 4][0] + bkeys[bk / 4][1] + bkeys[bk / 4][2] + bkeys[bk / 4][3] > 32)
             raise(GX_EINVAL, "electron repulsion supports combined angular order through 32");
     std::unique_ptr<gx::Task[]> all(new gx::Task[std::max<int64_t>(T, 1)]);
     plan.task_kk.resize(T);
+    plan.task_site.resize(T);
     plan.task_part.assign(parts.size() > 1 ? T : 0, 0);
     // pass 2: scatter
 #pragma omp parallel for schedule(static)
@@ -884,9 +964,10 @@ void build_plan_parts(gx_context* ctx, const std::vector<PlanPart>& parts, PlanD
         const int pidx = chunks[c].part;
         const PlanPart& pt = parts[pidx];
         const gx_basis* b = pt.b;
-        const std::vector<int>& seg_code = part_code[pidx];
-        auto tuple_of = [&](int a, int bb, int cc, int d) {
-            return ((int64_t)(seg_code[a] * nsc + seg_code[bb]) * nsc + seg_code[cc]) * nsc + seg_code[d];
+        const std::vector<int>&seg_code = part_code[pidx], &site = part_site[pidx];
+        auto bucket = [&](int a, int bb, int cc, int d) {
+            const int64_t t = ((int64_t)(seg_code[a] * nsc + seg_code[bb]) * nsc + seg_code[cc]) * nsc + seg_code[d];
+            return bucket_of[t] + (site[a] == site[bb] ? 2 : 0) + (site[cc] == site[d] ? 1 : 0);
         };
         for (int64_t i = chunks[c].first; i < chunks[c].end; ++i) {
             const auto& r = (*pt.req)[i];
@@ -917,8 +998,10 @@ void build_plan_parts(gx_context* ctx, const std::vector<PlanPart>& parts, PlanD
                             t.st[3] = 1;
                             t.pab = pt.pair_base + b->sp_off[(size_t)ga * b->nseg + gb];
                             t.pcd = pt.pair_base + b->sp_off[(size_t)gc * b->nseg + gd];
-                            const int64_t pos = cur[bucket_of[tuple_of(ga, gb, gc, gd)]]++;
+                            const int bk = bucket(ga, gb, gc, gd);
+                            const int64_t pos = cur[bk]++;
                             all[pos] = t;
+                            plan.task_site[pos] = (uint8_t)(bk & 3);
                             plan.task_kk[pos] = (b->seg_nprim[ga] * b->seg_nprim[gb]) << 16 |
                                                 (b->seg_nprim[gc] * b->seg_nprim[gd]);
                             if (!plan.task_part.empty()) plan.task_part[pos] = pidx;
@@ -931,15 +1014,14 @@ void build_plan_parts(gx_context* ctx, const std::vector<PlanPart>& parts, PlanD
     plan.model_flops = 0.0;
     size_t first = 0;
     for (int bk = 0; bk < nb;) {
-        const std::array<int, 4> key{bkeys[bk][0], bkeys[bk][1], bkeys[bk][2], bkeys[bk][3]};
+        const BKey& first_key = bkeys[bk / 4];
+        const std::array<int, 4> key{first_key[0], first_key[1], first_key[2], first_key[3]};
         size_t count = 0;
         int64_t np = 0;
         int e = bk;
-        for (; e < nb && bkeys[e][0] == key[0] && bkeys[e][1] == key[1] && bkeys[e][2] == key[2] &&
-               bkeys[e][3] == key[3];
-             ++e) {
+        for (; e < nb && std::equal(key.begin(), key.end(), bkeys[e / 4].begin()); ++e) {
             count += btotal[e];
-            np += btotal[e] * (int64_t)bkeys[e][4] * bkeys[e][5];  // (-Kab)(-Kcd)
+            np += btotal[e] * (int64_t)bkeys[e / 4][4] * bkeys[e / 4][5];  // (-Kab)(-Kcd)
         }
         if (count) {
             const double fl = model_flops(key[0], key[1], key[2], key[3]);
@@ -964,6 +1046,7 @@ void build_plan_parts(gx_context* ctx, const std::vector<PlanPart>& parts, PlanD
                (double)c.primitive_quartets * c.flops_per_primitive_quartet;
     });
     make_group_set(ctx, plan, plan.defconf, plan.base);
+    make_units(ctx, plan);
     // (a copy from pageable memory is staged before cudaMemcpyAsync returns,
     // so the host task array may be freed now)
 }
@@ -986,6 +1069,7 @@ gx::EriDev make_dev(gx_context* ctx, gx_basis* b, FieldPairs& fp, double2* out, 
     const bool mixed = precision == GX_PRECISION_MIXED;
     dev.skip_cut = (float)(mixed ? kSkipMixed : (precision == GX_PRECISION_FP64_EXACT ? 0.0 : kSkipFP64));
     dev.fp32_cut = (float)(mixed ? std::max(mixed_cutoff, kSkipMixed) : 0.0);
+    dev.all_real = (fp.B[0] == 0.0 && fp.B[1] == 0.0 && fp.B[2] == 0.0) || b->one_site ? 1 : 0;
     dev.basis = b->dev();
     dev.pairs = pair_view(b, fp);
     dev.boys = ctx->boys();
@@ -1003,27 +1087,51 @@ gx::EriDev make_dev(gx_context* ctx, gx_basis* b, FieldPairs& fp, double2* out, 
 // optional pointers.
 void launch_class(gx_context* ctx, gx::EriDev dev, const PlanData& plan, size_t ci, const ClassConf& conf,
                   const int2* groups, int ngroup, unsigned long long* counters, cudaStream_t s, int* used_b1 = nullptr,
-                  int* used_wpb = nullptr, int* used_tiles = nullptr, const int2* lane_groups = nullptr,
-                  int nlane = 0) {
+                  int* used_wpb = nullptr, int* used_tiles = nullptr) {
     const auto& pc = plan.classes[ci];
     const auto& k = pc.key;
     dev.counters = counters ? counters + 2 * ci : nullptr;
-    if (gx::small_class(k[0], k[1], k[2], k[3])) {
-        gx::QuartetClass qc{};
-        qc.L = k[0] + k[1] + k[2] + k[3];
-        qc.ntask = (int)pc.count;
-        qc.tasks = plan.tasks.as<gx::Task>() + pc.first;
-        qc.ngroup = ngroup;
-        qc.groups = groups;
-        GX_CUDA(gx::launch_small(k[0], k[1], k[2], k[3], dev, qc, s));
+    gx::QuartetClass qc{};
+    qc.L = k[0] + k[1] + k[2] + k[3];
+    qc.ntask = (int)pc.count;
+    qc.tasks = plan.tasks.as<gx::Task>() + pc.first;
+    const bool small = gx::small_class(k[0], k[1], k[2], k[3]);
+    if (small || runs_dense(pc, conf)) {
+        qc.ngroup = plan.unit_grid[ci];
+        qc.target = plan.unit_target[ci];
+        qc.dims = plan.unit_dims[ci];
+        if (plan.unit_class[ci] >= 0) {
+            const gx::UnitClass& uc = plan.unit_first[plan.unit_class[ci]];
+            qc.unit_start = plan.units.start + uc.base;
+            qc.unit_count = plan.units.count + uc.vfirst;
+        }
         if (used_b1) *used_b1 = 32;
         if (used_wpb) *used_wpb = 4;
+        if (small) {
+            GX_CUDA(gx::launch_small(k[0], k[1], k[2], k[3], dev, qc, s));
+            return;
+        }
+        qc.bra = ctx->pair_class(k[0], k[1]).dev();
+        qc.ket = ctx->pair_class(k[2], k[3]).dev();
+        qc.NL = gx::herm_count(qc.L);
+        // few entries: the blocks of a unit share its components (about one in
+        // four primitive quartets of a small plan survives)
+        const int units = (int)(pc.primitive_quartets / 128) + 1, fill = std::max(ctx->sm_count, 1);
+        qc.nchunk = gx::dense_chunks(k[0], k[1], k[2], k[3], (fill + units - 1) / units, pc.primitive_quartets <= 32);
+        GX_CUDA(gx::launch_dense(k[0], k[1], k[2], k[3], dev, qc, false, s));
+        // mixed precision: the FP32 entries are added after the FP64 ones
+        if (dev.fp32_cut > 0.0f) {
+            if (plan.unit_class32[ci] >= 0) {
+                const gx::UnitClass& u32 = plan.unit_first[plan.unit_class32[ci]];
+                qc.unit_start32 = plan.units.start + u32.base;
+                qc.unit_count32 = plan.units.count + u32.vfirst;
+            }
+            GX_CUDA(gx::launch_dense(k[0], k[1], k[2], k[3], dev, qc, true, s));
+        }
         return;
     }
-    gx::QuartetClass qc{};
     qc.bra = ctx->pair_class(k[0], k[1]).dev();
     qc.ket = ctx->pair_class(k[2], k[3]).dev();
-    qc.L = k[0] + k[1] + k[2] + k[3];
     qc.Nab = gx::herm_count(k[0] + k[1]);
     qc.NL = gx::herm_count(qc.L);
     const int ncd = qc.ket.nab;
@@ -1091,8 +1199,6 @@ void launch_class(gx_context* ctx, gx::EriDev dev, const PlanData& plan, size_t 
         }
         qc.coop = std::min(B1, (int)(lane_cost / coop_cost));
     }
-    qc.ntask = (int)pc.count;
-    qc.tasks = plan.tasks.as<gx::Task>() + pc.first;
     qc.ngroup = ngroup;
     qc.groups = groups;
     qc.minb = conf.minb == 4 ? 4 : 2;
@@ -1108,21 +1214,7 @@ void launch_class(gx_context* ctx, gx::EriDev dev, const PlanData& plan, size_t 
     const int cap = conf.wpb > 0 ? std::min(4, conf.wpb) : 4;
     const int wpb = (int)std::max<size_t>(1, std::min<size_t>(cap, (200 * 1024) / per_warp));
     const int grid = (int)std::min<long long>(((long long)qc.ngroup * qc.nchunk + wpb - 1) / wpb, 1 << 30);
-    // mixed precision: the FP32 entries of a 3 <= L <= 4 class go to the FP32
-    // lane kernel, launched after this one on the same stream
-    const bool lane = dev.fp32_cut > 0.0f && lane_groups && nlane > 0 && !conf.nolane &&
-                      gx::lane32_class(k[0], k[1], k[2], k[3]);
-    qc.no32 = lane ? 1 : 0;
     GX_CUDA(gx::launch_quartets(dev, qc, wpb, grid, s));
-    if (lane) {
-        gx::QuartetClass lq{};
-        lq.L = qc.L;
-        lq.ntask = qc.ntask;
-        lq.tasks = qc.tasks;
-        lq.ngroup = nlane;
-        lq.groups = lane_groups;
-        GX_CUDA(gx::launch_lane32(k[0], k[1], k[2], k[3], dev, lq, s));
-    }
     if (used_b1) *used_b1 = B1;
     if (used_wpb) *used_wpb = wpb;
     if (used_tiles) {
@@ -1185,6 +1277,7 @@ int enqueue_plan(gx_context* ctx, const gx::EriDev& dev, const PlanData& plan, i
     };
     if (counters && !accumulate) GX_CUDA(cudaMemsetAsync(counters, 0, 2 * plan.classes.size() * sizeof(unsigned long long), s));
     ctx->reset_status();
+    GX_CUDA(gx::launch_units(plan.units, plan.tasks.as<gx::Task>(), dev, s));
     const auto& tuned = plan.tuned[precision];
     const GroupSet& gs = tuned.valid ? tuned.groups : plan.base;
     const size_t nc = plan.classes.size();
@@ -1211,8 +1304,7 @@ int enqueue_plan(gx_context* ctx, const gx::EriDev& dev, const PlanData& plan, i
             const size_t ci = plan.order.empty() ? oi : (size_t)plan.order[oi];
             launch_class(ctx, dev, plan, ci, tuned.valid ? tuned.conf[ci] : plan.defconf[ci],
                          gs.dev.as<int2>() + gs.range[ci].first, (int)gs.range[ci].second, counters,
-                         ctx->aux[oi % K], nullptr, nullptr, nullptr, gs.dev.as<int2>() + gs.lane[ci].first,
-                         (int)gs.lane[ci].second);
+                         ctx->aux[oi % K], nullptr, nullptr, nullptr);
             copy_class(ci, ctx->aux[oi % K]);
         }
         for (int k = 0; k < K; ++k) {
@@ -1224,7 +1316,7 @@ int enqueue_plan(gx_context* ctx, const gx::EriDev& dev, const PlanData& plan, i
         for (size_t ci = 0; ci < nc; ++ci) {
             launch_class(ctx, dev, plan, ci, tuned.valid ? tuned.conf[ci] : plan.defconf[ci],
                          gs.dev.as<int2>() + gs.range[ci].first, (int)gs.range[ci].second, counters, s, nullptr,
-                         nullptr, nullptr, gs.dev.as<int2>() + gs.lane[ci].first, (int)gs.lane[ci].second);
+                         nullptr, nullptr);
             copy_class(ci, s);
         }
         join_copies();
@@ -1249,6 +1341,7 @@ void enqueue_plans(gx_context* ctx, const std::vector<std::pair<const PlanData*,
         }
         GX_CUDA(cudaEventCreateWithFlags(&ctx->fork, cudaEventDisableTiming));
     }
+    for (const auto& r : runs) GX_CUDA(gx::launch_units(r.first->units, r.first->tasks.as<gx::Task>(), r.second, s));
     GX_CUDA(cudaEventRecord(ctx->fork, s));
     for (int k = 0; k < kAux; ++k) GX_CUDA(cudaStreamWaitEvent(ctx->aux[k], ctx->fork, 0));
     int next = 0;
@@ -1260,8 +1353,7 @@ void enqueue_plans(gx_context* ctx, const std::vector<std::pair<const PlanData*,
             const size_t ci = plan.order.empty() ? oi : (size_t)plan.order[oi];
             launch_class(ctx, runs[r].second, plan, ci, tuned.valid ? tuned.conf[ci] : plan.defconf[ci],
                          gs.dev.as<int2>() + gs.range[ci].first, (int)gs.range[ci].second, counters[r],
-                         ctx->aux[next % kAux], nullptr, nullptr, nullptr, gs.dev.as<int2>() + gs.lane[ci].first,
-                         (int)gs.lane[ci].second);
+                         ctx->aux[next % kAux], nullptr, nullptr, nullptr);
         }
     }
     for (int k = 0; k < kAux; ++k) {
@@ -1305,6 +1397,7 @@ void enqueue_parts_with_copies(gx_context* ctx, const gx::EriDev& dev, const Cac
         if (counters[r])
             GX_CUDA(cudaMemsetAsync(counters[r], 0, 2 * cp.parts[r]->classes.size() * sizeof(unsigned long long), s));
     ctx->reset_status();
+    for (const auto& part : cp.parts) GX_CUDA(gx::launch_units(part->units, part->tasks.as<gx::Task>(), dev, s));
     GX_CUDA(cudaEventRecord(ctx->fork, s));
     for (int k = 0; k < kAux; ++k) GX_CUDA(cudaStreamWaitEvent(ctx->aux[k], ctx->fork, 0));
     GX_CUDA(cudaStreamWaitEvent(ctx->copy_stream, ctx->fork, 0));
@@ -1318,8 +1411,7 @@ void enqueue_parts_with_copies(gx_context* ctx, const gx::EriDev& dev, const Cac
             const size_t ci = plan.order.empty() ? oi : (size_t)plan.order[oi];
             launch_class(ctx, dev, plan, ci, tuned.valid ? tuned.conf[ci] : plan.defconf[ci],
                          gs.dev.as<int2>() + gs.range[ci].first, (int)gs.range[ci].second, counters[r],
-                         ctx->aux[next % kAux], nullptr, nullptr, nullptr, gs.dev.as<int2>() + gs.lane[ci].first,
-                         (int)gs.lane[ci].second);
+                         ctx->aux[next % kAux], nullptr, nullptr, nullptr);
         }
         // a waited event stands for its latest record, so the events are reused per part
         for (int k = 0; k < kAux; ++k) {
@@ -1519,7 +1611,7 @@ CachedPlan& lookup_parts(gx_context* ctx, gx_basis* b, uint64_t h1, uint64_t h2,
         size_t bytes = 0;
         int kept_plans = 0;
         for (auto it = cache.begin(); it != cache.end();) {
-            for (const auto& p : it->parts) bytes += p->tasks.bytes;
+            for (const auto& p : it->parts) bytes += p->tasks.bytes + p->unit_mem.bytes;
             if (++kept_plans > 4 || (kept_plans > 1 && bytes > (size_t(2) << 30)))
                 it = cache.erase(it);
             else
@@ -1885,6 +1977,7 @@ extern "C" int gx_eri_batch_packed(gx_context* ctx, int nreq, gx_basis* const* b
         ctx->out.reserve(std::max<int64_t>(total, 1) * sizeof(double2));
         gx::EriDev dev = make_dev(ctx, bases[0], field_pairs(bases[0], B, O), ctx->out.as<double2>(), precision,
                                   mixed_cutoff);
+        dev.all_real = 0;  // (of the first request alone)
         dev.basis = gx::BasisDev{};
         dev.basis.ns = pk.nseg;
         dev.basis.nprim = pk.nprim.as<int>();
@@ -2575,6 +2668,7 @@ void gx_context_destroy(gx_context* ctx) {
     for (auto st : ctx->aux) cudaStreamDestroy(st);
     for (auto ev : ctx->aux_done) cudaEventDestroy(ev);
     if (ctx->fork) cudaEventDestroy(ctx->fork);
+    if (ctx->exec_done) cudaEventDestroy(ctx->exec_done);
     if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
     if (ctx->copy_done) cudaEventDestroy(ctx->copy_done);
     for (auto st : ctx->class_copy) cudaStreamDestroy(st);
@@ -3310,6 +3404,7 @@ std::vector<long long> plan_shape(const PlanData& pd, const gx::EriDev& dev) {
                                p(dev.pairs.bound), p(dev.pairs.Epool32), p(dev.pairs.order), p(dev.pairs.sbound),
                                p(dev.pairs.g32), p(dev.boys.S), p(dev.boys.E0), p(dev.gl), p(dev.herm_xyz),
                                p(dev.rec_plan), p(dev.rec_plan_off), p(dev.out), p(dev.status)};
+    sig.push_back(dev.all_real);
     uint32_t cuts[2];
     std::memcpy(&cuts[0], &dev.skip_cut, 4);
     std::memcpy(&cuts[1], &dev.fp32_cut, 4);
@@ -3317,9 +3412,10 @@ std::vector<long long> plan_shape(const PlanData& pd, const gx::EriDev& dev) {
     sig.push_back(cuts[1]);
     for (size_t ci = 0; ci < pd.classes.size(); ++ci) {
         const auto& pc = pd.classes[ci];
+        // (the primitive-quartet count sets the class's unit count)
         sig.insert(sig.end(), {pc.key[0], pc.key[1], pc.key[2], pc.key[3], (long long)pc.first, (long long)pc.count,
-                               (long long)pd.base.range[ci].first, (long long)pd.base.range[ci].second,
-                               (long long)pd.base.lane[ci].first, (long long)pd.base.lane[ci].second});
+                               (long long)pc.primitive_quartets,
+                               (long long)pd.base.range[ci].first, (long long)pd.base.range[ci].second});
     }
     return sig;
 }
@@ -3780,7 +3876,8 @@ void cholesky_core(gx_context* ctx, gx_basis* b, const double* Bf, const double*
                     cp->counters.reserve(std::max<size_t>(2 * cp->plan.classes.size(), 2) *
                                          sizeof(unsigned long long));
                     GX_CUDA(cudaMemsetAsync(cp->counters.ptr, 0, cp->counters.bytes, st));
-                    ctx->column_plan_bytes += cp->plan.tasks.bytes + cp->plan.base.dev.bytes + cp->boff.bytes;
+                    ctx->column_plan_bytes += cp->plan.tasks.bytes + cp->plan.base.dev.bytes + cp->plan.unit_mem.bytes +
+                                              cp->boff.bytes;
                 }
                 if (!plan_base.count(cp.get())) {
                     std::vector<unsigned long long> c(2 * cp->plan.classes.size());
@@ -3846,9 +3943,9 @@ void cholesky_core(gx_context* ctx, gx_basis* b, const double* Bf, const double*
                         sp.ntask = pd.ntask;
                         sp.spread_parts = pd.spread_parts;
                         sp.base.range = pd.base.range;
-                        sp.base.lane = pd.base.lane;
                         sp.tasks.reserve(pd.tasks.bytes);
                         sp.base.dev.reserve(pd.base.dev.bytes);
+                        make_units(ctx, sp);
                         sg->counters.reserve(std::max<size_t>(2 * pd.classes.size(), 2) * sizeof(unsigned long long));
                         GX_CUDA(cudaMemsetAsync(sg->counters.ptr, 0, sg->counters.bytes, st));
                         cudaGraph_t graph = nullptr;
@@ -4195,7 +4292,7 @@ extern "C" int gx_cholesky_last_stats(gx_context* ctx, gx_cholesky_stats* out) {
 // only rewrites the pair records the graph reads.
 struct PlanGraph {
     cudaGraphExec_t exec = nullptr;
-    std::array<uintptr_t, 8> key{}, pending{};
+    std::array<uintptr_t, 9> key{}, pending{};
     bool disabled = false;
     void reset() {
         if (exec) cudaGraphExecDestroy(exec);
@@ -4219,11 +4316,35 @@ struct gx_eri_plan {
 
 extern "C" {
 
+namespace {
+bool capturing(cudaStream_t s) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
+    }
+    return st != cudaStreamCaptureStatusNone;
+}
+
+// Notes the end of an asynchronous plan execution (see gx_context_set_stream).
+void mark_execution(gx_context* ctx) {
+    if (capturing(ctx->stream)) return;
+    if (!ctx->exec_done) GX_CUDA(cudaEventCreateWithFlags(&ctx->exec_done, cudaEventDisableTiming));
+    GX_CUDA(cudaEventRecord(ctx->exec_done, ctx->stream));
+    ctx->exec_pending = true;
+}
+}  // namespace
+
 int gx_context_set_stream(gx_context* ctx, void* stream) {
     return guarded([&] {
         if (!ctx) raise(GX_EINVAL, "null context");
         std::lock_guard<std::mutex> lock(ctx->mu);
-        ctx->stream = stream ? static_cast<cudaStream_t>(stream) : ctx->own_stream;
+        cudaStream_t to = stream ? static_cast<cudaStream_t>(stream) : ctx->own_stream;
+        // a plan execution still in flight on the old stream uses its plan's
+        // unit arrays and the pair records: work on the new one follows it
+        if (to != ctx->stream && ctx->exec_pending && !capturing(to))
+            GX_CUDA(cudaStreamWaitEvent(to, ctx->exec_done, 0));
+        ctx->stream = to;
     });
 }
 
@@ -4291,9 +4412,10 @@ void plan_enqueue(gx_eri_plan* plan, const double* B, const double* O, int preci
     double cut = mixed_cutoff;
     uint64_t cut_bits;
     std::memcpy(&cut_bits, &cut, sizeof cut_bits);
-    const std::array<uintptr_t, 8> key{(uintptr_t)ctx->stream, (uintptr_t)out, (uintptr_t)precision,
+    const bool real = (B[0] == 0.0 && B[1] == 0.0 && B[2] == 0.0) || plan->basis->one_site;  // (sets the launches' shared memory)
+    const std::array<uintptr_t, 9> key{(uintptr_t)ctx->stream, (uintptr_t)out, (uintptr_t)precision,
                                        (uintptr_t)cut_bits, (uintptr_t)fp.p.ptr, (uintptr_t)fp.Epool.ptr,
-                                       (uintptr_t)fp.order.ptr, (uintptr_t)plan->generation};
+                                       (uintptr_t)fp.order.ptr, (uintptr_t)plan->generation, (uintptr_t)real};
     PlanGraph& g = plan->graph;
     const bool capturable = !g.disabled && ctx->stream != nullptr;
     if (capturable && g.exec && g.key == key) {
@@ -4349,6 +4471,7 @@ int gx_eri_plan_execute(gx_eri_plan* plan, const double* B, const double* O, int
         std::lock_guard<std::mutex> lock(ctx->mu);
         GX_CUDA(cudaSetDevice(ctx->device));
         plan_enqueue(plan, B, O, precision, mixed_cutoff, static_cast<double2*>(out_device));
+        mark_execution(ctx);
     });
 }
 
@@ -4387,11 +4510,12 @@ int gx_eri_plan_profile(gx_eri_plan* plan, const double* B, const double* O, int
         std::vector<cudaEvent_t> ev(nc + 1);
         for (auto& e : ev) GX_CUDA(cudaEventCreate(&e));
         std::vector<int> b1(nc), wpb(nc), tiles(3 * nc, 0);
+        GX_CUDA(gx::launch_units(pd.units, pd.tasks.as<gx::Task>(), dev, s));
         GX_CUDA(cudaEventRecord(ev[0], s));
         for (size_t ci = 0; ci < nc; ++ci) {
             launch_class(ctx, dev, pd, ci, tuned.valid ? tuned.conf[ci] : pd.defconf[ci],
                          gs.dev.as<int2>() + gs.range[ci].first, (int)gs.range[ci].second, counters, s, &b1[ci],
-                         &wpb[ci], &tiles[3 * ci], gs.dev.as<int2>() + gs.lane[ci].first, (int)gs.lane[ci].second);
+                         &wpb[ci], &tiles[3 * ci]);
             GX_CUDA(cudaEventRecord(ev[ci + 1], s));
         }
         GX_CUDA(cudaEventSynchronize(ev[nc]));
@@ -4491,6 +4615,7 @@ int gx_eri_plan_autotune(gx_eri_plan* plan, const double* B, const double* O, in
         cudaEvent_t e0, e1;
         GX_CUDA(cudaEventCreate(&e0));
         GX_CUDA(cudaEventCreate(&e1));
+        GX_CUDA(gx::launch_units(pd.units, pd.tasks.as<gx::Task>(), dev, s));
         std::vector<ClassConf> best = pd.defconf;
         double tot_default = 0.0, tot_best = 0.0;
         DeviceBuffer tmp;
@@ -4499,31 +4624,26 @@ int gx_eri_plan_autotune(gx_eri_plan* plan, const double* B, const double* O, in
             // the untuned configuration first (kept unless another is clearly
             // faster), then the previous built-in default and the sweep
             std::vector<ClassConf> cands{pd.defconf[ci]};
-            if (gx::small_class(k[0], k[1], k[2], k[3])) {
-                for (int per : {256, 4096}) cands.push_back(ClassConf{per, 0, 0});
-            } else {
+            const bool small = gx::small_class(k[0], k[1], k[2], k[3]);
+            if (!small) {
                 cands.push_back(ClassConf{});
                 for (int per : {16, 32, 64, 128, 256, 512, 1024})
                     for (int w : {2, 4})
                         for (int b1 : {16, 32})
                             if (!(per == 32 && w == 4 && b1 == 32)) cands.push_back(ClassConf{per, w, b1});
+                // a lane-dense class has no knobs: the sweep tries the generic kernel on it
+                for (size_t c = 1; c < cands.size(); ++c)
+                    cands[c].nolane = gx::dense_class(k[0], k[1], k[2], k[3]) ? 1 : 0;
             }
             double best_ms = 0.0, def_ms = 0.0;
             auto time_conf = [&](const ClassConf& cf) {
-                auto groups = make_groups(ctx, pd, ci, cf);
+                const auto groups = make_groups(ctx, pd, ci, cf);
                 const int ngroup = (int)groups.size();
-                int nlane = 0;
-                if (lane_class(pd.classes[ci])) {
-                    const auto lg = make_groups(ctx, pd, ci, cf, true);
-                    nlane = (int)lg.size();
-                    groups.insert(groups.end(), lg.begin(), lg.end());
-                }
                 upload(tmp, groups, s);
                 double t = 1e30;
                 for (int r = 0; r <= repeats; ++r) {  // first launch warms caches
                     GX_CUDA(cudaEventRecord(e0, s));
-                    launch_class(ctx, dev, pd, ci, cf, tmp.as<int2>(), ngroup, nullptr, s, nullptr, nullptr, nullptr,
-                                 tmp.as<int2>() + ngroup, nlane);
+                    launch_class(ctx, dev, pd, ci, cf, tmp.as<int2>(), ngroup, nullptr, s);
                     GX_CUDA(cudaEventRecord(e1, s));
                     GX_CUDA(cudaEventSynchronize(e1));
                     float ms = 0.0f;
@@ -4541,7 +4661,8 @@ int gx_eri_plan_autotune(gx_eri_plan* plan, const double* B, const double* O, in
                     best[ci] = cands[c];
                 }
             }
-            if (!gx::small_class(k[0], k[1], k[2], k[3])) {
+            const bool knobs = !small && !runs_dense(pd.classes[ci], best[ci]);
+            if (knobs) {
                 // second stage: transform tiles under the chosen work split
                 const int ncd = ctx->pair_class(k[2], k[3]).nab;
                 for (int kt : {1, 2, 4})
@@ -4581,7 +4702,7 @@ int gx_eri_plan_autotune(gx_eri_plan* plan, const double* B, const double* O, in
                         }
                     }
             }
-            if (!gx::small_class(k[0], k[1], k[2], k[3])) {
+            if (knobs) {
                 // fourth stage: stream mode (per-entry recurrences, small
                 // shared footprint, more resident warps) on the chosen split
                 const ClassConf base = best[ci];
@@ -4599,16 +4720,6 @@ int gx_eri_plan_autotune(gx_eri_plan* plan, const double* B, const double* O, in
                                 best[ci] = cf;
                             }
                         }
-            }
-            if (precision == GX_PRECISION_MIXED && lane_class(pd.classes[ci])) {
-                // fifth stage: the FP32 entries in the generic kernel instead of the lane kernel
-                ClassConf cf = best[ci];
-                cf.nolane = 1;
-                const double t = time_conf(cf);
-                if (t < 0.97 * best_ms) {
-                    best_ms = t;
-                    best[ci] = cf;
-                }
             }
             tot_default += def_ms;
             tot_best += best_ms;

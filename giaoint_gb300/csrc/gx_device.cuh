@@ -36,6 +36,23 @@ __host__ __device__ __forceinline__ double2 cmacr(double2 c, double s, double2 a
     return c2(fma(s, a.x, c.x), fma(s, a.y, c.y));
 }
 
+// Small constants of loops whose trip count is not known at compile time: a
+// division 1/(2n + 1) or an int -> double conversion there would cost FP64
+// instructions, a constant-bank read costs none.  Same values, bit for bit.
+struct DevConst {
+    double ints[40];     // n
+    double half[40];     // n + 1/2
+    double inv_odd[40];  // 1 / (2n + 1)
+    constexpr DevConst() : ints{}, half{}, inv_odd{} {
+        for (int n = 0; n < 40; ++n) {
+            ints[n] = (double)n;
+            half[n] = (double)n + 0.5;
+            inv_odd[n] = 1.0 / (double)(2 * n + 1);
+        }
+    }
+};
+static __constant__ DevConst c_dev = DevConst();
+
 // ---------------------------------------------------------------------------
 // Hermite multi-index enumeration: all (k, l, m) with k + l + m <= L, ordered
 // by total degree s, then x-major within a degree (the Cartesian order of
@@ -195,7 +212,7 @@ __device__ __forceinline__ int boys_eval(double x, double y, int L, const BoysTa
         const double2 iz = c2(x * ir2, -y * ir2);
         Sh[0] = f;
         for (int n = 0; n < L; ++n) {
-            f = cscale(cmul(f, iz), (double)n + 0.5);
+            f = cscale(cmul(f, iz), c_dev.half[n]);
             Sh[n + 1] = f;
         }
         e0 = c2(1.0, 0.0);
@@ -222,7 +239,7 @@ __device__ __forceinline__ int boys_eval(double x, double y, int L, const BoysTa
                 for (int k = BOYS_TAYLOR_TERMS - 1; k >= 1; --k) em = cmac(c2(1.0, 0.0), em, w[k]);
                 const double2 z2 = c2(x + x, y + y);
                 for (int n = L - 1; n >= 0; --n) {
-                    acc = cscale(cmac(em, z2, acc), 1.0 / (double)(2 * n + 1));
+                    acc = cscale(cmac(em, z2, acc), c_dev.inv_odd[n]);
                     Sh[n] = acc;
                 }
             }
@@ -250,6 +267,46 @@ __device__ __forceinline__ int boys_eval(double x, double y, int L, const BoysTa
     return 0;
 }
 
+// The same for a real argument x >= 0 (up to rounding): the asymptotic form or
+// the table's real line, which together cover every x >= 0 for L <= 32.
+__device__ __forceinline__ int boys_eval_real(double x, int L, const BoysTable& tab, double* Sh, double& e0) {
+    if (!isfinite(x)) return -4;
+    if (x >= 2.0 * L + 44.0) {
+        const double ir = rsqrt(x);
+        const double ix = ir * ir;
+        double f = 0.88622692545275801365 * ir;
+        Sh[0] = f;
+        for (int n = 0; n < L; ++n) {
+            f = f * ix * c_dev.half[n];
+            Sh[n + 1] = f;
+        }
+        e0 = 1.0;
+        return 0;
+    }
+    const int ix = __float2int_rn((float)(x - BOYS_X0) * (float)BOYS_INV_H);
+    const int p = ix * BOYS_NY + (BOYS_NY - 1) / 2;
+    const double d = x - (BOYS_X0 + BOYS_H * ix);
+    const double2* S = tab.S + (size_t)p * BOYS_TABLE_ORDERS;
+    e0 = __ldg(&tab.E0[p].x);
+    double w[BOYS_TAYLOR_TERMS];
+#pragma unroll
+    for (int k = 1; k < BOYS_TAYLOR_TERMS; ++k) w[k] = d * (-1.0 / (double)k);
+    double acc = __ldg(&S[L + BOYS_TAYLOR_TERMS - 1].x);
+#pragma unroll
+    for (int k = BOYS_TAYLOR_TERMS - 1; k >= 1; --k) acc = fma(acc, w[k], __ldg(&S[L + k - 1].x));
+    Sh[L] = acc;
+    if (L > 0) {
+        double em = 1.0;
+#pragma unroll
+        for (int k = BOYS_TAYLOR_TERMS - 1; k >= 1; --k) em = fma(em, w[k], 1.0);
+        const double x2 = x + x;
+        for (int n = L - 1; n >= 0; --n) {
+            acc = fma(x2, acc, em) * c_dev.inv_odd[n];
+            Sh[n] = acc;
+        }
+    }
+    return 0;
+}
 
 // ---------------------------------------------------------------------------
 // FP32 Boys values for the mixed-precision path, large |T| only: the

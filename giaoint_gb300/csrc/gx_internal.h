@@ -85,11 +85,40 @@ struct QuartetClass {
     int KT, CT;            // Hermite rows per lane in the ket transform, ket components per lane in the bra transform
     int stream;            // 1: phase 1 keeps only the seeds of the batch; each entry's R is built by the warp
                            //    into a two-column buffer right before its ket transform (small shared footprint)
-    int no32;              // 1: leave the FP32 entries of a mixed-precision pass to the FP32 lane kernel
+    int swap, axis;        // lane-dense kernel: 1 when the ket pair is its template side; the task strides of its
+                           //    component indices, two bits each (template a, b, other c, d)
     int ntask;
     const Task* tasks;
     int ngroup;
     const int2* groups;  // (first task, task count) per warp work unit
+    const int* unit_start;    // small and lane-dense kernels: first task of every unit of the class, and surviving
+    const int* unit_count;    //    FP64 primitive quartets of every task of the class
+                              //    (null: the class has few tasks, every block cuts its units itself)
+    long long target;         // weight of a unit, and the components of the four shells, one byte each, for that
+    int dims;
+    const int* unit_start32;  // lane-dense kernel: the same for the FP32 entries
+    const int* unit_count32;
+};
+
+// Work units of a plan's small and lane-dense classes with many tasks
+// (gx_dense.cu).  The tasks of the unit classes are numbered consecutively (virtual index).
+struct UnitClass {
+    long long vfirst, first;  // first virtual index; first task of the class in the plan
+    long long base;           // first entry of the class in `start`
+    long long target;         // weight of a unit
+    int mode;                 // entries counted: 0 FP64, 1 FP32, 2 FP64 with the FP32 ones adding to the weight
+    int dims;                 // components of the four shells, one byte each
+};
+struct UnitPlan {
+    const UnitClass* cls;
+    int ncls;
+    long long ntask, nunit;     // virtual tasks; entries of `start`
+    long long ntask64, nunit64; // without the FP32 unit classes, which come last
+    int* count;                 // [ntask] surviving primitive quartets (FP32 ones in mode 1)
+    long long* prefix;          // [ntask] weight prefix within the task's tile
+    long long* tile;            // [tiles] weight prefix of the tiles
+    int* start;                 // [nunit]
+    unsigned* done;             // blocks finished (0 between executions)
 };
 
 struct EriDev {
@@ -106,6 +135,7 @@ struct EriDev {
     float fp32_cut;   // ... below this (and above skip_cut) run in FP32; 0 = FP64 only.
                       // The FP32 quartets use FP32 Boys values in the asymptotic
                       // sector and FP64 ones elsewhere, then the FP32 recurrence.
+    int all_real;     // 1: every pair has q = 0 (zero field, or all shells on one centre)
     unsigned long long* counters;  // [0] FP64, [1] FP32 primitive quartets evaluated (may be null)
 };
 
@@ -216,11 +246,13 @@ cudaError_t launch_deriv_contract(const DerivContractArgs& args, int sms, cudaSt
 cudaError_t launch_gather_abs(const double2* src, const long long* idx, double* dst, long long n, int sms,
                               cudaStream_t s);
 
-// FP32 lane kernel of the mixed-precision entries of 3 <= L <= 4 classes
-// (gx_lane*.cu, dispatched in gx_small.cu); runs after the class-generic
-// kernel of the same class on the same stream
-bool lane32_class(int la, int lb, int lc, int ld);
-cudaError_t launch_lane32(int la, int lb, int lc, int ld, const EriDev& d, const QuartetClass& qc, cudaStream_t s);
+// lane-dense kernel (gx_dense.cu)
+constexpr int kUnitMinTasks = 512;  // classes with fewer tasks have no entry in the unit plan
+bool dense_class(int la, int lb, int lc, int ld);
+int dense_chunks(int la, int lb, int lc, int ld, int want, bool single);
+long long unit_tiles(long long ntask);
+cudaError_t launch_units(const UnitPlan& u, const Task* tasks, const EriDev& d, cudaStream_t s);
+cudaError_t launch_dense(int la, int lb, int lc, int ld, const EriDev& d, QuartetClass qc, bool f32, cudaStream_t s);
 
 // register-resident small classes (gx_small.cu)
 bool small_class(int la, int lb, int lc, int ld);

@@ -461,10 +461,13 @@ __device__ __forceinline__ T tmul(T a, T b);
 template <>
 __device__ __forceinline__ double2 tmul(double2 a, double2 b) { return cmul(a, b); }
 template <>
+__device__ __forceinline__ double tmul(double a, double b) { return a * b; }
+template <>
 __device__ __forceinline__ float2 tmul(float2 a, float2 b) {
     return make_float2(fmaf(a.x, b.x, -a.y * b.y), fmaf(a.x, b.y, a.y * b.x));
 }
 __device__ __forceinline__ double2 tmacr(double2 c, int k, double2 a) { return cmacr(c, c_int[k], a); }
+__device__ __forceinline__ double tmacr(double c, int k, double a) { return fma(c_int[k], a, c); }
 __device__ __forceinline__ float2 tmacr(float2 c, int k, float2 a) {
     return make_float2(fmaf((float)k, a.x, c.x), fmaf((float)k, a.y, c.y));
 }
@@ -551,11 +554,9 @@ struct WarpSmem {
 // Per-warp shared layout.  Batched mode: R columns of all B1 entries
 // (stride B1 + 1) and one seed area; stream mode: a two-column R buffer and
 // the seeds and X' of every batch entry (L + 4 slots each).
-// stage32: the E~ staging also holds the FP32 copy of a record (mixed
-// precision when this kernel takes FP32 entries; otherwise only the FP64
-// record is staged and the FP32 half is not allocated)
+// (In mixed precision the E~ staging also holds the FP32 copy of a record.)
 __host__ __device__ inline WarpSmem warp_smem(int NL, int B1, int Nab, int CH, bool mixed, int stage_e, int stream,
-                                              int L, bool stage32) {
+                                              int L) {
     WarpSmem w;
     const size_t B1p = B1 + 1;
     w.R = 0;
@@ -567,7 +568,7 @@ __host__ __device__ inline WarpSmem warp_smem(int NL, int B1, int Nab, int CH, b
     w.seed = w.eoff + (((size_t)B1 * 8 + 15) / 16) * 16;
     w.stage = w.seed + (stream ? (size_t)B1 * (L + 4) : (size_t)(BOYS_MAX_ORDER + 1 + 3)) * 16;
     // FP64 record (16 B per word) followed by its FP32 copy (8 B per word)
-    w.total = w.stage + (((size_t)stage_e * (stage32 ? 24 : 16) + 15) / 16) * 16;
+    w.total = w.stage + (((size_t)stage_e * (mixed ? 24 : 16) + 15) / 16) * 16;
     return w;
 }
 
@@ -652,6 +653,10 @@ __device__ __forceinline__ double2 group_sum(double2 v, int J) {
     }
     return v;
 }
+__device__ __forceinline__ double group_sum(double v, int J) {
+    for (int off = J >> 1; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+    return v;
+}
 __device__ __forceinline__ float2 group_sum(float2 v, int J) {
     for (int off = J >> 1; off > 0; off >>= 1) {
         v.x += __shfl_xor_sync(0xffffffffu, v.x, off);
@@ -669,7 +674,8 @@ __device__ __forceinline__ float2 group_sum(float2 v, int J) {
 // component cd, its box entries split over the item's J lanes -- contracts
 // it against the entry's R column (FP32 entries: the float2 in the first half
 // of each 16-byte slot of R, R32[(row B1p + j) 2]).  eoff[j]: E~ record of the
-// entry's ket pair; flag[j]: 0 FP32, 1 FP64.
+// entry's ket pair; flag[j]: 0 FP32, 1 FP64; with a ket pair of q = 0 (real E~)
+// 3, and with both pairs of that kind, whose R column holds doubles, 7.
 template <int KT>
 __device__ __forceinline__ void step_k_run(const QuartetClass& qc, const ClassTabs& tb, const uint32_t* herm_xyz,
                                            const PairData& pp, const double2* R, const float2* R32, int B1p,
@@ -682,7 +688,8 @@ __device__ __forceinline__ void step_k_run(const QuartetClass& qc, const ClassTa
     float2* stg32 = reinterpret_cast<float2*>(stg + qc.stage_e);
     for (int jj = j0; jj < j1; ++jj) {
         const int f = flag[jj];
-        const bool is64 = f == 1;
+        const bool is64 = f != 0;
+        const double* Rr = reinterpret_cast<const double*>(R);
         const double2* E64 = pp.Epool + eoff[jj];
         const float2* E32 = pp.Epool32 + eoff[jj];
         if (stg) {
@@ -724,7 +731,15 @@ __device__ __forceinline__ void step_k_run(const QuartetClass& qc, const ClassTa
                     const uint32_t kk = tb.kh[bo + e];
                     const int Kp = kk & 0xffff;
                     const bool neg = kk >> 16;
-                    if (is64) {
+                    if (f == 7) {
+                        const double ev = neg ? -E64[bo + e].x : E64[bo + e].x;
+#pragma unroll
+                        for (int u = 0; u < KT; ++u) a64[u].x = fma(ev, Rr[tb.hsum[hb[u] + Kp] * B1p + jj], a64[u].x);
+                    } else if (f == 3) {
+                        const double ev = neg ? -E64[bo + e].x : E64[bo + e].x;
+#pragma unroll
+                        for (int u = 0; u < KT; ++u) a64[u] = cmacr(a64[u], ev, R[tb.hsum[hb[u] + Kp] * B1p + jj]);
+                    } else if (is64) {
                         double2 ev = E64[bo + e];
                         if (neg) ev = c2(-ev.x, -ev.y);
 #pragma unroll
@@ -756,7 +771,17 @@ __device__ __forceinline__ void step_k_run(const QuartetClass& qc, const ClassTa
                     const uint32_t ke = qc.ket.ent[bo + e];
                     const int k2 = ke & 255, l2 = (ke >> 8) & 255, m2 = (ke >> 16) & 255;
                     const bool neg = (k2 + l2 + m2) & 1;
-                    if (is64) {
+                    if (f == 7 || f == 3) {
+                        const double ev = neg ? -E64[bo + e].x : E64[bo + e].x;
+#pragma unroll
+                        for (int u = 0; u < KT; ++u) {
+                            const int r = herm_index(bk[u] + k2, bl[u] + l2, bm[u] + m2) * B1p + jj;
+                            if (f == 7)
+                                a64[u].x = fma(ev, Rr[r], a64[u].x);
+                            else
+                                a64[u] = cmacr(a64[u], ev, R[r]);
+                        }
+                    } else if (is64) {
                         double2 ev = E64[bo + e];
                         if (neg) ev = c2(-ev.x, -ev.y);
 #pragma unroll
@@ -774,7 +799,9 @@ __device__ __forceinline__ void step_k_run(const QuartetClass& qc, const ClassTa
             if (J > 1) {
 #pragma unroll
                 for (int u = 0; u < KT; ++u) {
-                    if (is64)
+                    if (f == 7)
+                        a64[u].x = group_sum(a64[u].x, J);
+                    else if (is64)
                         a64[u] = group_sum(a64[u], J);
                     else
                         a32[u] = group_sum(a32[u], J);
@@ -785,7 +812,9 @@ __device__ __forceinline__ void step_k_run(const QuartetClass& qc, const ClassTa
                 for (int u = 0; u < KT; ++u) {
                     const int K = kb * KT + u;
                     if (K < qc.Nab) {
-                        if (is64) {
+                        if (f == 7) {
+                            W[K * qc.CH + cdl].x += a64[u].x;
+                        } else if (is64) {
                             W[K * qc.CH + cdl] = cadd(W[K * qc.CH + cdl], a64[u]);
                         } else {
                             float2& w = W32[K * qc.CH + cdl];
@@ -818,10 +847,11 @@ __device__ __forceinline__ void step_k_any(const QuartetClass& qc, const ClassTa
 // staging buffer (stg; null: read from global memory).  A work item is CT
 // consecutive ket components of one bra component ab (the chunk length is a
 // multiple of CT); its box entries are split over the item's J lanes.  FP32
-// partial sums are added in FP64.
+// partial sums are added in FP64.  use64: 0 no FP64 part in W, 1 complex, 3 the
+// bra pair has q = 0 (real E~), 7 and W is real too.
 template <int CT>
 __device__ __forceinline__ void step_b(const EriDev& d, const QuartetClass& qc, const ClassTabs& tb, const Task& tg,
-                                       int ip, double2* W, float2* W32, bool use64, bool use32, double2* stg, int c0,
+                                       int ip, double2* W, float2* W32, int use64, bool use32, double2* stg, int c0,
                                        int chn, int lane) {
     const int nab = qc.bra.nab;
     const int ncb = ncart(qc.bra.lb), ncdd = ncart(qc.ket.lb);
@@ -872,7 +902,21 @@ __device__ __forceinline__ void step_b(const EriDev& d, const QuartetClass& qc, 
                     for (int u = 0; u < CT; ++u) acc32[u] = tmac(acc32[u], ea32, W32[K * qc.CH + cdl0 + u]);
                 }
             }
-            if (use64) {
+            if (use64 == 7) {
+                for (int e = sub; e < nbox; e += J) {
+                    const int K = row(e);
+                    const double ea = Ea[bo + e].x;
+#pragma unroll
+                    for (int u = 0; u < CT; ++u) acc[u].x = fma(ea, W[K * qc.CH + cdl0 + u].x, acc[u].x);
+                }
+            } else if (use64 & 2) {
+                for (int e = sub; e < nbox; e += J) {
+                    const int K = row(e);
+                    const double ea = Ea[bo + e].x;
+#pragma unroll
+                    for (int u = 0; u < CT; ++u) acc[u] = cmacr(acc[u], ea, W[K * qc.CH + cdl0 + u]);
+                }
+            } else if (use64) {
                 for (int e = sub; e < nbox; e += J) {
                     const int K = row(e);
                     const double2 ea = Ea[bo + e];
@@ -905,7 +949,7 @@ __device__ __forceinline__ void step_b(const EriDev& d, const QuartetClass& qc, 
 }
 
 __device__ __forceinline__ void step_b_any(const EriDev& d, const QuartetClass& qc, const ClassTabs& tb,
-                                           const Task& tg, int ip, double2* W, float2* W32, bool use64, bool use32,
+                                           const Task& tg, int ip, double2* W, float2* W32, int use64, bool use32,
                                            double2* stg, int c0, int chn, int lane) {
     switch (qc.CT) {
         case 4: step_b<4>(d, qc, tb, tg, ip, W, W32, use64, use32, stg, c0, chn, lane); break;
@@ -913,6 +957,12 @@ __device__ __forceinline__ void step_b_any(const EriDev& d, const QuartetClass& 
         case 2: step_b<2>(d, qc, tb, tg, ip, W, W32, use64, use32, stg, c0, chn, lane); break;
         default: step_b<1>(d, qc, tb, tg, ip, W, W32, use64, use32, stg, c0, chn, lane); break;
     }
+}
+
+// True when primitive pair i has q = 0 (zero field, or both shells on one
+// centre): its E~ record and the imaginary part of its centre are real.
+__device__ __forceinline__ bool zero_q(const PairData& pp, int i) {
+    return pp.Pi[3 * i] == 0.0 && pp.Pi[3 * i + 1] == 0.0 && pp.Pi[3 * i + 2] == 0.0;
 }
 
 // Seeds of one primitive quartet: returns 1 (FP64 seeds in Sh), 0 (FP32
@@ -984,11 +1034,8 @@ __global__ void __launch_bounds__(128, MINB) quartet_kernel(EriDev d, QuartetCla
     const int wpb = blockDim.x >> 5;
     const int B1p = qc.B1 + 1;
     const float skip = d.skip_cut, cut32 = d.fp32_cut;
-    // with the FP32 lane kernel in charge of the FP32 entries, this kernel
-    // takes only the entries at or above the FP32 cutoff
-    const float skip64 = qc.no32 ? fmaxf(skip, cut32) : skip;
     const WarpSmem lay =
-        warp_smem(qc.NL, qc.B1, qc.Nab, qc.CH, cut32 > 0.0f, qc.stage_e, qc.stream, qc.L, cut32 > 0.0f && !qc.no32);
+        warp_smem(qc.NL, qc.B1, qc.Nab, qc.CH, cut32 > 0.0f, qc.stage_e, qc.stream, qc.L);
     const size_t tab_bytes = (((size_t)qc.tab_words * 4 + 15) / 16) * 16;
     char* base = reinterpret_cast<char*>(sm) + tab_bytes + (size_t)wib * lay.total;
     double2* R = reinterpret_cast<double2*>(base + lay.R);
@@ -1046,6 +1093,7 @@ __global__ void __launch_bounds__(128, MINB) quartet_kernel(EriDev d, QuartetCla
             }
             int cur = -1;  // g * Kab + P of the accumulating bra pair
             bool any64 = false, any32 = false;  // precisions accumulated into W / W32 for `cur`
+            bool cplx = false;                  // ... with complex values in W
             int cursor = 0;
             while (cursor < S) {
                 // assemble up to B1 entries of this pass
@@ -1061,7 +1109,7 @@ __global__ void __launch_bounds__(128, MINB) quartet_kernel(EriDev d, QuartetCla
                         const int op = tg.pab + P;
                         const int oq = tg.pcd + Q;
                         const float b = pp.sbound[op] * pp.sbound[oq];
-                        valid = b >= skip64;
+                        valid = b >= skip;
                     }
                     const unsigned mask = __ballot_sync(0xffffffffu, valid);
                     const int cnt = __popc(mask);
@@ -1097,7 +1145,16 @@ __global__ void __launch_bounds__(128, MINB) quartet_kernel(EriDev d, QuartetCla
                         int f = entry_seeds(d, qc.L, want32 ? 1 : 0, qa, Sh, S32, gi.x + g);
                         if (f == 2) f = 1;  // FP32 seeds out of range: this entry runs in FP64
                         double2* es = sseed + (size_t)lane * sstride;
-                        if (f == 1) {
+                        const bool bra_real = zero_q(pp, ip), ket_real = zero_q(pp, iq);
+                        if (f == 1 && bra_real && ket_real) {
+                            // real separation and seeds: a real table
+                            double* er = reinterpret_cast<double*>(es);
+                            for (int n = 0; n <= qc.L; ++n) er[n] = Sh[n].x;
+                            for (int x = 0; x < 3; ++x) er[qc.L + 1 + x] = qa.X[x].x;
+                            f = 7;
+                            cnt64 += first_chunk;
+                        } else if (f == 1) {
+                            if (ket_real) f = 3;
                             for (int n = 0; n <= qc.L; ++n) es[n] = Sh[n];
                             for (int x = 0; x < 3; ++x) es[qc.L + 1 + x] = qa.X[x];
                             cnt64 += first_chunk;
@@ -1192,7 +1249,8 @@ __global__ void __launch_bounds__(128, MINB) quartet_kernel(EriDev d, QuartetCla
                             __syncwarp();
                             const int cg = cur / Kab, cP = cur - cg * Kab;
                             const Task tc = qc.tasks[gi.x + cg];
-                            step_b_any(d, qc, tabs, tc, pp.order[tc.pab + cP], W, W32, any64,
+                            const int ipb = pp.order[tc.pab + cP];
+                            step_b_any(d, qc, tabs, tc, ipb, W, W32, !any64 ? 0 : !zero_q(pp, ipb) ? 1 : cplx ? 3 : 7,
                                        any32, stg, c0, chn, lane);
                             __syncwarp();
                             for (int it = lane; it < qc.Nab * qc.CH; it += 32) {
@@ -1202,11 +1260,12 @@ __global__ void __launch_bounds__(128, MINB) quartet_kernel(EriDev d, QuartetCla
                             __syncwarp();
                         }
                         cur = key;
-                        any64 = any32 = false;
+                        any64 = any32 = cplx = false;
                     }
                     bool has64 = false, has32 = false;
                     for (int jj = j0; jj < j1; ++jj) {
-                        has64 = has64 || flag[jj] == 1;
+                        has64 = has64 || flag[jj] != 0;
+                        cplx = cplx || flag[jj] == 1 || flag[jj] == 3;
                         has32 = has32 || flag[jj] == 0;
                     }
                     if (qc.stream) {
@@ -1216,7 +1275,11 @@ __global__ void __launch_bounds__(128, MINB) quartet_kernel(EriDev d, QuartetCla
                         for (int jj = j0; jj < j1; ++jj) {
                             __syncwarp();  // the previous entry's transform has read R
                             const double2* es = sseed + (size_t)jj * sstride;
-                            if (flag[jj] == 1) {
+                            if (flag[jj] == 7) {
+                                const double* er = reinterpret_cast<const double*>(es);
+                                coop_rec<double>(qc.L, er, er + qc.L + 1, reinterpret_cast<double*>(R), 2, 0, 1,
+                                                 d.herm_xyz, lane);
+                            } else if (flag[jj] != 0) {
                                 coop_rec<double2>(qc.L, es, es + qc.L + 1, R, 2, 0, 1, d.herm_xyz, lane);
                             } else {
                                 const float2* s32 = reinterpret_cast<const float2*>(es);
@@ -1238,7 +1301,8 @@ __global__ void __launch_bounds__(128, MINB) quartet_kernel(EriDev d, QuartetCla
                 __syncwarp();
                 const int cg = cur / Kab, cP = cur - cg * Kab;
                 const Task tc = qc.tasks[gi.x + cg];
-                step_b_any(d, qc, tabs, tc, pp.order[tc.pab + cP], W, W32, any64, any32, stg,
+                const int ipb = pp.order[tc.pab + cP];
+                step_b_any(d, qc, tabs, tc, ipb, W, W32, !any64 ? 0 : !zero_q(pp, ipb) ? 1 : cplx ? 3 : 7, any32, stg,
                            c0, chn, lane);
             }
             __syncwarp();
@@ -1258,7 +1322,7 @@ __global__ void __launch_bounds__(128, MINB) quartet_kernel(EriDev d, QuartetCla
 size_t quartet_smem_bytes(const QuartetClass& qc, int warps_per_block, bool mixed) {
     return (((size_t)qc.tab_words * 4 + 15) / 16) * 16 +
            (size_t)warps_per_block *
-               warp_smem(qc.NL, qc.B1, qc.Nab, qc.CH, mixed, qc.stage_e, qc.stream, qc.L, mixed && !qc.no32).total;
+               warp_smem(qc.NL, qc.B1, qc.Nab, qc.CH, mixed, qc.stage_e, qc.stream, qc.L).total;
 }
 
 static bool g_const_ready = false;

@@ -2,20 +2,24 @@
 //
 // One lane evaluates one primitive quartet completely: Boys values, Hermite
 // table Rh, ket transform W[K][cd] and bra transform into its contribution
-// v[ab][cd], all in registers.  A warp walks the primitive quartets of a
-// group of shell quartets with equal primitive counts as one stream and
-// compacts the ones that survive screening (and belong to the current
-// precision pass) into full batches of 32 with a ballot, so screening removes
-// issue slots instead of idling lanes.  Lanes of a batch that belong to the
-// same shell quartet are summed by a segmented warp reduction and the first
-// lane of each segment adds the sum to the output block.  Every loop is
-// expanded at compile time from constexpr plans (index-sequence folds), so
-// all register indices are constants.
+// v[ab][cd], all in registers; every loop is expanded at compile time from
+// constexpr plans (index-sequence folds), so all register indices are
+// constants.  The kernel is bound by the number of FP64 warp instructions (one
+// per 64 cycles and SM sub-partition, whatever the number of active lanes).  A
+// warp takes a work unit of consecutive shell quartets with about as many
+// surviving primitive quartets as any other (units cut on the device,
+// gx_dense.cu) and walks them in full batches of 32 (gx_stream.cuh); the lanes'
+// values go through shared memory, where every output element's entries are
+// added one after the other.  Against a segmented shuffle sum (ten FP64
+// instructions per element and batch) that costs two per 32 additions, and the
+// result does not depend on the batches.  Batches both of whose pairs have
+// q = 0 (zero field, shells on one centre) run in real arithmetic.
 #pragma once
 
 #include <utility>
 
 #include "gx_internal.h"
+#include "gx_stream.cuh"
 
 namespace gx {
 namespace small {
@@ -255,220 +259,336 @@ __device__ __forceinline__ void quartet_seeds(const EriDev& d, long long item, d
     }
 }
 
-// Segmented sum over lanes with equal key (keys non-decreasing along the
-// warp): afterwards the first lane of each run holds the run's total.
-template <int N>
-__device__ __forceinline__ void seg_sum(double2* v, int key, int lane) {
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const int ko = __shfl_down_sync(0xffffffffu, key, off);
-        const bool take = lane + off < 32 && ko == key;
-#pragma unroll
-        for (int i = 0; i < N; ++i) {
-            const double ox = __shfl_down_sync(0xffffffffu, v[i].x, off);
-            const double oy = __shfl_down_sync(0xffffffffu, v[i].y, off);
-            if (take) v[i] = c2(v[i].x + ox, v[i].y + oy);
-        }
-    }
+// Real forms of the recurrence and the transforms, for batches both of whose
+// pairs have q = 0 (E: the real parts of the complex records).
+template <int L, int... S>
+__device__ __forceinline__ void run_rec_real(double* R, const double* seed, const double* X,
+                                             std::integer_sequence<int, S...>) {
+    (
+        [&] {
+            constexpr RStep st = rstep(L, S);
+            if constexpr (st.kind == 1) {
+                R[0] = seed[st.n];
+            } else {
+                double v = X[st.axis] * R[st.s1];
+                if constexpr (st.coef > 0) v = fma((double)st.coef, R[st.s2], v);
+                R[st.dst] = v;
+            }
+        }(),
+        ...);
 }
-template <int N>
-__device__ __forceinline__ void seg_sum(float2* v, int key, int lane) {
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const int ko = __shfl_down_sync(0xffffffffu, key, off);
-        const bool take = lane + off < 32 && ko == key;
-#pragma unroll
-        for (int i = 0; i < N; ++i) {
-            const float ox = __shfl_down_sync(0xffffffffu, v[i].x, off);
-            const float oy = __shfl_down_sync(0xffffffffu, v[i].y, off);
-            if (take) v[i] = make_float2(v[i].x + ox, v[i].y + oy);
+template <int LA, int LB, int LC, int LD, int... S>
+__device__ __forceinline__ void run_k_real(double* W, const double* R, const double2* __restrict__ Ecd,
+                                           std::integer_sequence<int, S...>) {
+    (
+        [&] {
+            constexpr KMac m = kmac<LA, LB, LC, LD>(S);
+            const double e = __ldg(&Ecd[m.eoff].x);
+            W[m.w] = fma(m.neg ? -e : e, R[m.r], W[m.w]);
+        }(),
+        ...);
+}
+template <int LA, int LB, int LC, int LD, int... S>
+__device__ __forceinline__ void run_b_real(double* out, const double* W, const double2* __restrict__ Eab,
+                                           std::integer_sequence<int, S...>) {
+    (
+        [&] {
+            constexpr BMac m = bmac<LA, LB, LC, LD>(S);
+            out[m.o] = fma(__ldg(&Eab[m.eoff].x), W[m.w], out[m.o]);
+        }(),
+        ...);
+}
+
+constexpr int kWarps = 4;  // warps of a block, each with its own work unit
+
+// Shared memory of a warp: the values of a batch (33 columns: free of bank
+// conflicts both ways), the runs of lanes with one shell quartet, and the
+// queue of FP32 entries that wait for a full batch.
+template <int NOUT>
+struct WarpBuffers {
+    double2 v[NOUT * 33];
+    long long seg_off[32];
+    int4 seg_st[32];
+    int seg_lane[36];  // first lane of each run (bit 8: its first FP64 entry, store instead of adding), and the end
+    int2 queue[64];    // task, bra pair << 16 | ket pair
+};
+
+// Notes the runs of lanes with one shell quartet; returns their number.
+template <int NOUT>
+__device__ __forceinline__ int segments(WarpBuffers<NOUT>& w, const QuartetClass& qc, int task, bool first, int nb,
+                                        int lane) {
+    const int tp = __shfl_up_sync(0xffffffffu, task, 1);
+    const bool head = lane < nb && (lane == 0 || tp != task);
+    const unsigned heads = __ballot_sync(0xffffffffu, head);
+    const int nseg = __popc(heads);
+    if (head) {
+        const int s = __popc(heads & ((1u << lane) - 1u));
+        const Task* t = qc.tasks + task;
+        w.seg_off[s] = t->out_off;
+        w.seg_st[s] = make_int4(t->st[0], t->st[1], t->st[2], t->st[3]);
+        w.seg_lane[s] = lane | (first ? 256 : 0);
+    }
+    if (lane == 0) w.seg_lane[nseg] = nb;
+    return nseg;
+}
+
+// Adds the buffered values of every run to its block, one entry after the
+// other in stream order: the result does not depend on how the stream was cut
+// into batches.  REAL: the imaginary parts are zero.
+template <int LA, int LB, int LC, int LD, bool REAL>
+__device__ __forceinline__ void add_runs(double2* out, const WarpBuffers<nc(LA) * nc(LB) * nc(LC) * nc(LD)>& w, int nseg,
+                                         int lane) {
+    constexpr int NCD = nc(LC) * nc(LD), NOUT = nc(LA) * nc(LB) * NCD, NCB = nc(LB), NCDD = nc(LD);
+    for (int it = lane; it < nseg * NOUT; it += 32) {
+        const int s = it / NOUT, o = it - s * NOUT;
+        const int ab = o / NCD, cd = o - ab * NCD;
+        const int4 st = w.seg_st[s];
+        double2* p = out + w.seg_off[s] + (long long)(ab / NCB) * st.x + (long long)(ab % NCB) * st.y +
+                     (long long)(cd / NCDD) * st.z + (long long)(cd % NCDD) * st.w;
+        const double2* v = w.v + o * 33;
+        const bool store = w.seg_lane[s] & 256;
+        int l = w.seg_lane[s] & 255;
+        const int l1 = w.seg_lane[s + 1] & 255;
+        if constexpr (REAL) {
+            double sum;
+            if (store)
+                sum = v[l++].x;
+            else
+                sum = p->x;
+            for (; l < l1; ++l) sum += v[l].x;
+            if (store)
+                *p = c2(sum, 0.0);
+            else
+                p->x = sum;
+        } else {
+            double2 sum;
+            if (store)
+                sum = v[l++];
+            else
+                sum = *p;
+            for (; l < l1; ++l) sum = cadd(sum, v[l]);
+            *p = sum;
         }
     }
 }
 
 template <int LA, int LB, int LC, int LD>
-__global__ void __launch_bounds__(128) small_kernel(EriDev d, QuartetClass qc) {
+__global__ void __launch_bounds__(32 * kWarps) small_kernel(EriDev d, QuartetClass qc) {
     constexpr int L = LA + LB + LC + LD;
     constexpr int NL = hc(L), NH = hc(LA + LB);
-    constexpr int NAB = nc(LA) * nc(LB), NCD = nc(LC) * nc(LD), NOUT = NAB * NCD;
-    constexpr int NCB = nc(LB), NCDD = nc(LD);
-    __shared__ int s_queue[4][32];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    int* queue = s_queue[wib];
-    const int nwarp = gridDim.x * (blockDim.x >> 5);
+    constexpr int NCD = nc(LC) * nc(LD), NOUT = nc(LA) * nc(LB) * NCD;
+    __shared__ WarpBuffers<NOUT> s_buf[kWarps];
+    const int lane = threadIdx.x & 31;
+    WarpBuffers<NOUT>& w = s_buf[threadIdx.x >> 5];
+    const int unit = blockIdx.x * kWarps + (threadIdx.x >> 5);
+    int t0, t1;
+    if (qc.unit_start) {
+        if (unit >= qc.ngroup) return;
+        // (entries past the last unit lie beyond the class)
+        t0 = qc.unit_start[unit];
+        t1 = min(qc.unit_start[unit + 1], qc.ntask);
+    } else {
+        __shared__ int bounds[kWarps + 1];
+        __shared__ long long sums[kWarps];
+        cut_units<32 * kWarps>(d, qc, 2, blockIdx.x * kWarps, kWarps, true, bounds, sums);
+        t0 = bounds[threadIdx.x >> 5];
+        t1 = bounds[(threadIdx.x >> 5) + 1];
+    }
+    if (t0 >= t1) return;
     const PairData& pp = d.pairs;
-    const float skip = d.skip_cut, cut32 = d.fp32_cut;
-    const float cut64 = fmaxf(cut32, skip);
-    // Mixed precision: pass 0 evaluates the FP64 quartets, pass 1 the FP32
-    // quartets whose Boys argument lies in the asymptotic sector (FP32 Boys),
-    // pass 2 the other FP32 quartets (FP64 Boys, FP32 recurrence), so that
-    // every batch follows one Boys path.
-    const int npass = cut32 > 0.0f ? 3 : 1;
     unsigned n64 = 0, n32 = 0;
-    auto out_ptr = [&](const Task& t, int o) {
-        const int ab = o / NCD, cd = o - ab * NCD;
-        const int ca = ab / NCB, cb = ab - ca * NCB, cc = cd / NCDD, cdd = cd - cc * NCDD;
-        return d.out + t.out_off + (long long)ca * t.st[0] + (long long)cb * t.st[1] + (long long)cc * t.st[2] +
-               (long long)cdd * t.st[3];
-    };
-    for (int grp = blockIdx.x * (blockDim.x >> 5) + wib; grp < qc.ngroup; grp += nwarp) {
-        const int2 gi = qc.groups[grp];
-        const Task t0 = qc.tasks[gi.x];
-        const int Kab = d.basis.nprim[t0.sa] * d.basis.nprim[t0.sb];
-        const int Kcd = d.basis.nprim[t0.sc] * d.basis.nprim[t0.sd];
-        const int KK = Kab * Kcd;
-        const int S = gi.y * KK;
-        for (int it = lane; it < gi.y * NOUT; it += 32) {
-            const int g = it / NOUT;
-            *out_ptr(qc.tasks[gi.x + g], it - g * NOUT) = c2(0.0, 0.0);
+    // FP64 form of one entry into the value buffer
+    auto complex_entry = [&](const double2* X, const double2* Sh, int ip, int iq) {
+        double2 R[NL];
+        if constexpr (L == 0) {
+            R[0] = Sh[0];
+        } else {
+            R[0] = Sh[L];
+            run_rec<L>(R, Sh, X, std::make_integer_sequence<int, rsteps(L)>{});
         }
-        __syncwarp();
-        for (int pass = 0; pass < npass; ++pass) {
-            int cursor = 0;
-            while (cursor < S) {
-                // compact up to 32 surviving entries of this pass
-                int nb = 0;
-                while (nb < 32 && cursor < S) {
-                    const int idx = cursor + lane;
-                    bool valid = false;
-                    if (idx < S) {
-                        const int g = idx / KK, r = idx - g * KK;
-                        const int P = r / Kcd, Q = r - P * Kcd;
-                        const Task tg = qc.tasks[gi.x + g];
-                        const int op = tg.pab + P;
-                        const int oq = tg.pcd + Q;
-                        const float b = pp.sbound[op] * pp.sbound[oq];
-                        valid = pass == 0 ? b >= cut64 : (b >= skip && b < cut32);
-                        if (valid && pass > 0)
-                            valid = (pass == 1) == boys_asymptotic32(pp, pp.order[op], pp.order[oq], L);
-                    }
-                    const unsigned mask = __ballot_sync(0xffffffffu, valid);
-                    const int cnt = __popc(mask);
-                    const int take = min(cnt, 32 - nb);
-                    const int rank = __popc(mask & ((1u << lane) - 1u));
-                    if (valid && rank < take) queue[nb + rank] = idx;
-                    if (take < cnt) {
-                        const unsigned m2 = __ballot_sync(0xffffffffu, valid && rank == take);
-                        cursor += __ffs(m2) - 1;
-                    } else {
-                        cursor += 32;
-                    }
-                    nb += take;
-                }
-                __syncwarp();
-                if (nb == 0) break;
-                const bool active = lane < nb;
-                int key = -1 - lane;  // idle lanes never match another lane
-                double2 v[NOUT];
-                float2 v32[NOUT];
+        double2 W[NH * NCD], v[NOUT];
 #pragma unroll
-                for (int i = 0; i < NOUT; ++i) {
-                    v[i] = c2(0.0, 0.0);
-                    v32[i] = make_float2(0.0f, 0.0f);
-                }
-                bool used64 = false;
-                if (active) {
-                    const int idx = queue[lane];
-                    const int g = idx / KK, r = idx - g * KK;
-                    const int P = r / Kcd, Q = r - P * Kcd;
-                    key = g;
-                    const Task tg = qc.tasks[gi.x + g];
-                    const int ip = pp.order[tg.pab + P];
-                    const int iq = pp.order[tg.pcd + Q];
-                    const double p = pp.p[ip], q = pp.p[iq];
-                    const double2 X[3] = {c2(pp.Pr[3 * ip] - pp.Pr[3 * iq], pp.Pi[3 * ip] - pp.Pi[3 * iq]),
-                                          c2(pp.Pr[3 * ip + 1] - pp.Pr[3 * iq + 1], pp.Pi[3 * ip + 1] - pp.Pi[3 * iq + 1]),
-                                          c2(pp.Pr[3 * ip + 2] - pp.Pr[3 * iq + 2], pp.Pi[3 * ip + 2] - pp.Pi[3 * iq + 2])};
-                    const double rs = rsqrt(p + q);
-                    const double rho = p * q * rs * rs;
+        for (int i = 0; i < NH * NCD; ++i) W[i] = c2(0.0, 0.0);
+#pragma unroll
+        for (int i = 0; i < NOUT; ++i) v[i] = c2(0.0, 0.0);
+        run_k<LA, LB, LC, LD>(W, R, pp.Epool + pp.Eoff[iq],
+                              std::make_integer_sequence<int, kmacs<LA, LB, LC, LD>()>{});
+        run_b<LA, LB, LC, LD>(v, W, pp.Epool + pp.Eoff[ip], std::make_integer_sequence<int, bmacs<LA, LB, LC, LD>()>{});
+#pragma unroll
+        for (int i = 0; i < NOUT; ++i) w.v[i * 33 + lane] = v[i];
+    };
+    {
+        Stream<false> stream(d, qc, t0, t1);
+        for (;;) {
+            int task, rank = 0;
+            int2 pq;
+            const int nb = stream.next(lane, task, rank, pq);
+            if (nb == 0) break;
+            const int nseg = segments<NOUT>(w, qc, task, rank == 0, nb, lane);
+            const bool real = stream.batch_kind == 3;
+            if (lane < nb) {
+                const Task* tg = qc.tasks + task;
+                const int ip = pp.order[tg->pab + pq.x], iq = pp.order[tg->pcd + pq.y];
+                const double p = pp.p[ip], q = pp.p[iq];
+                const double rs = rsqrt(p + q);
+                const double rho = p * q * rs * rs;
+                const double x0 = pp.Pr[3 * ip] - pp.Pr[3 * iq], x1 = pp.Pr[3 * ip + 1] - pp.Pr[3 * iq + 1],
+                             x2 = pp.Pr[3 * ip + 2] - pp.Pr[3 * iq + 2];
+                if (real) {
+                    const double t = rho * fma(x0, x0, fma(x1, x1, x2 * x2));
+                    double Sh[L + 1], e0;
+                    double C = pp.F[ip].x * pp.F[iq].x * rs;
+                    if (const int rc = boys_eval_real(t, L, d.boys, Sh, e0)) {
+                        report(d.status, rc, task, L, t, 0.0);
+                        C = e0 = 0.0;
+#pragma unroll
+                        for (int n = 0; n <= L; ++n) Sh[n] = 0.0;
+                    }
+                    C *= e0;
+                    const double m2r = -2.0 * rho;
+#pragma unroll
+                    for (int n = 0; n <= L; ++n) {
+                        Sh[n] *= C;
+                        C *= m2r;
+                    }
+                    const double X[3] = {x0, x1, x2};
+                    double R[NL];
+                    if constexpr (L == 0) {
+                        R[0] = Sh[0];
+                    } else {
+                        R[0] = Sh[L];
+                        run_rec_real<L>(R, Sh, X, std::make_integer_sequence<int, rsteps(L)>{});
+                    }
+                    double W[NH * NCD], v[NOUT];
+#pragma unroll
+                    for (int i = 0; i < NH * NCD; ++i) W[i] = 0.0;
+#pragma unroll
+                    for (int i = 0; i < NOUT; ++i) v[i] = 0.0;
+                    run_k_real<LA, LB, LC, LD>(W, R, pp.Epool + pp.Eoff[iq],
+                                               std::make_integer_sequence<int, kmacs<LA, LB, LC, LD>()>{});
+                    run_b_real<LA, LB, LC, LD>(v, W, pp.Epool + pp.Eoff[ip],
+                                               std::make_integer_sequence<int, bmacs<LA, LB, LC, LD>()>{});
+#pragma unroll
+                    for (int i = 0; i < NOUT; ++i) w.v[i * 33 + lane].x = v[i];
+                } else {
+                    const double2 X[3] = {c2(x0, pp.Pi[3 * ip] - pp.Pi[3 * iq]),
+                                          c2(x1, pp.Pi[3 * ip + 1] - pp.Pi[3 * iq + 1]),
+                                          c2(x2, pp.Pi[3 * ip + 2] - pp.Pi[3 * iq + 2])};
                     const double tre = rho * (fma(X[0].x, X[0].x, fma(X[1].x, X[1].x, X[2].x * X[2].x)) -
                                               fma(X[0].y, X[0].y, fma(X[1].y, X[1].y, X[2].y * X[2].y)));
                     const double tim = 2.0 * rho * fma(X[0].x, X[0].y, fma(X[1].x, X[1].y, X[2].x * X[2].y));
                     const double2 C = cscale(cmul(pp.F[ip], pp.F[iq]), rs);
                     double2 Sh[L + 1];
-                    bool ok32 = false;
-                    if (pass > 0) {
-                        float2 S32[L + 1];
-                        ok32 = pass == 1 && seeds32(C, rho, tre, tim, L, S32);
-                        if (!ok32) {
-                            // FP64 Boys; FP32 recurrence when the seeds fit
-                            quartet_seeds<L>(d, gi.x + g, C, rho, tre, tim, Sh);
-                            ok32 = true;
-#pragma unroll
-                            for (int n = 0; n <= L; ++n) {
-                                ok32 = ok32 && fabs(Sh[n].x) + fabs(Sh[n].y) < 1.0e25;
-                                S32[n] = make_float2((float)Sh[n].x, (float)Sh[n].y);
-                            }
-                        }
-                        if (ok32) {
-                            const float2 X32[3] = {make_float2((float)X[0].x, (float)X[0].y),
-                                                   make_float2((float)X[1].x, (float)X[1].y),
-                                                   make_float2((float)X[2].x, (float)X[2].y)};
-                            float2 R32[NL];
-                            if constexpr (L == 0) {
-                                R32[0] = S32[0];
-                            } else {
-                                R32[0] = S32[L];
-                                run_rec32<L>(R32, S32, X32, std::make_integer_sequence<int, rsteps(L)>{});
-                            }
-                            float2 W32[NH * NCD];
-#pragma unroll
-                            for (int i = 0; i < NH * NCD; ++i) W32[i] = make_float2(0.0f, 0.0f);
-                            run_k32<LA, LB, LC, LD>(W32, R32, pp.Epool32 + pp.Eoff[iq],
-                                                    std::make_integer_sequence<int, kmacs<LA, LB, LC, LD>()>{});
-                            run_b32<LA, LB, LC, LD>(v32, W32, pp.Epool32 + pp.Eoff[ip],
-                                                    std::make_integer_sequence<int, bmacs<LA, LB, LC, LD>()>{});
-                            ++n32;
-                        }
-                    } else {
-                        quartet_seeds<L>(d, gi.x + g, C, rho, tre, tim, Sh);
-                    }
-                    if (!ok32) {
-                        double2 R[NL];
-                        if constexpr (L == 0) {
-                            R[0] = Sh[0];
-                        } else {
-                            R[0] = Sh[L];
-                            run_rec<L>(R, Sh, X, std::make_integer_sequence<int, rsteps(L)>{});
-                        }
-                        double2 W[NH * NCD];
-#pragma unroll
-                        for (int i = 0; i < NH * NCD; ++i) W[i] = c2(0.0, 0.0);
-                        run_k<LA, LB, LC, LD>(W, R, pp.Epool + pp.Eoff[iq],
-                                              std::make_integer_sequence<int, kmacs<LA, LB, LC, LD>()>{});
-                        run_b<LA, LB, LC, LD>(v, W, pp.Epool + pp.Eoff[ip],
-                                              std::make_integer_sequence<int, bmacs<LA, LB, LC, LD>()>{});
-                        used64 = true;
-                        ++n64;
-                    }
+                    quartet_seeds<L>(d, task, C, rho, tre, tim, Sh);
+                    complex_entry(X, Sh, ip, iq);
                 }
-                // FP32 contributions are reduced in FP32, FP64 ones in FP64, and
-                // the first lane of each segment adds both in FP64.
-                if (pass == 0 || __any_sync(0xffffffffu, used64)) seg_sum<NOUT>(v, key, lane);
-                if (pass > 0) {
-                    seg_sum<NOUT>(v32, key, lane);
-#pragma unroll
-                    for (int i = 0; i < NOUT; ++i) v[i] = cadd(v[i], c2((double)v32[i].x, (double)v32[i].y));
-                }
-                const int kprev = __shfl_up_sync(0xffffffffu, key, 1);
-                if (active && (lane == 0 || kprev != key)) {
-                    const Task tg = qc.tasks[gi.x + key];
-#pragma unroll
-                    for (int i = 0; i < NOUT; ++i) {
-                        double2* o = out_ptr(tg, i);
-                        *o = cadd(*o, v[i]);
-                    }
-                }
-                __syncwarp();
+                ++n64;
             }
+            __syncwarp();
+            if (real)
+                add_runs<LA, LB, LC, LD, true>(d.out, w, nseg, lane);
+            else
+                add_runs<LA, LB, LC, LD, false>(d.out, w, nseg, lane);
+            __syncwarp();
+        }
+    }
+    // Mixed precision: pass 0 evaluates the FP32 entries whose Boys argument
+    // lies in the asymptotic sector (FP32 Boys), pass 1 the others (FP64 Boys,
+    // FP32 recurrence), so that every batch follows one Boys path.
+    for (int pass = 0; pass < (d.fp32_cut > 0.0f ? 2 : 0); ++pass) {
+        Stream<true> stream(d, qc, t0, t1);
+        int waiting = 0;
+        bool more = true;
+        while (more || waiting > 0) {
+            while (more && waiting < 32) {
+                int task, rank;
+                int2 pq = make_int2(0, 0);
+                const int n = stream.next(lane, task, rank, pq);
+                more = n > 0;
+                bool mine = lane < n;
+                if (mine) {
+                    const Task* tg = qc.tasks + task;
+                    mine = (pass == 0) ==
+                           boys_asymptotic32(pp, pp.order[tg->pab + pq.x], pp.order[tg->pcd + pq.y], L);
+                }
+                const unsigned m = __ballot_sync(0xffffffffu, mine);
+                if (mine) w.queue[waiting + __popc(m & ((1u << lane) - 1u))] = make_int2(task, pq.x << 16 | pq.y);
+                waiting += __popc(m);
+            }
+            __syncwarp();
+            const int nb = min(waiting, 32);
+            if (nb == 0) break;
+            const int2 en = w.queue[min(lane, nb - 1)];
+            const int2 rest = w.queue[32 + lane];
+            __syncwarp();
+            if (lane < waiting - nb) w.queue[lane] = rest;
+            waiting -= nb;
+            const int nseg = segments<NOUT>(w, qc, en.x, false, nb, lane);
+            if (lane < nb) {
+                const Task* tg = qc.tasks + en.x;
+                const int ip = pp.order[tg->pab + (int)((unsigned)en.y >> 16)], iq = pp.order[tg->pcd + (en.y & 0xffff)];
+                const double p = pp.p[ip], q = pp.p[iq];
+                const double2 X[3] = {c2(pp.Pr[3 * ip] - pp.Pr[3 * iq], pp.Pi[3 * ip] - pp.Pi[3 * iq]),
+                                      c2(pp.Pr[3 * ip + 1] - pp.Pr[3 * iq + 1], pp.Pi[3 * ip + 1] - pp.Pi[3 * iq + 1]),
+                                      c2(pp.Pr[3 * ip + 2] - pp.Pr[3 * iq + 2], pp.Pi[3 * ip + 2] - pp.Pi[3 * iq + 2])};
+                const double rs = rsqrt(p + q);
+                const double rho = p * q * rs * rs;
+                const double tre = rho * (fma(X[0].x, X[0].x, fma(X[1].x, X[1].x, X[2].x * X[2].x)) -
+                                          fma(X[0].y, X[0].y, fma(X[1].y, X[1].y, X[2].y * X[2].y)));
+                const double tim = 2.0 * rho * fma(X[0].x, X[0].y, fma(X[1].x, X[1].y, X[2].x * X[2].y));
+                const double2 C = cscale(cmul(pp.F[ip], pp.F[iq]), rs);
+                double2 Sh[L + 1];
+                float2 S32[L + 1];
+                bool ok32 = pass == 0 && seeds32(C, rho, tre, tim, L, S32);
+                if (!ok32) {
+                    // FP64 Boys; FP32 recurrence when the seeds fit
+                    quartet_seeds<L>(d, en.x, C, rho, tre, tim, Sh);
+                    ok32 = true;
+#pragma unroll
+                    for (int n = 0; n <= L; ++n) {
+                        ok32 = ok32 && fabs(Sh[n].x) + fabs(Sh[n].y) < 1.0e25;
+                        S32[n] = make_float2((float)Sh[n].x, (float)Sh[n].y);
+                    }
+                }
+                if (ok32) {
+                    const float2 X32[3] = {make_float2((float)X[0].x, (float)X[0].y),
+                                           make_float2((float)X[1].x, (float)X[1].y),
+                                           make_float2((float)X[2].x, (float)X[2].y)};
+                    float2 R32[NL];
+                    if constexpr (L == 0) {
+                        R32[0] = S32[0];
+                    } else {
+                        R32[0] = S32[L];
+                        run_rec32<L>(R32, S32, X32, std::make_integer_sequence<int, rsteps(L)>{});
+                    }
+                    float2 W32[NH * NCD], v32[NOUT];
+#pragma unroll
+                    for (int i = 0; i < NH * NCD; ++i) W32[i] = make_float2(0.0f, 0.0f);
+#pragma unroll
+                    for (int i = 0; i < NOUT; ++i) v32[i] = make_float2(0.0f, 0.0f);
+                    run_k32<LA, LB, LC, LD>(W32, R32, pp.Epool32 + pp.Eoff[iq],
+                                            std::make_integer_sequence<int, kmacs<LA, LB, LC, LD>()>{});
+                    run_b32<LA, LB, LC, LD>(v32, W32, pp.Epool32 + pp.Eoff[ip],
+                                            std::make_integer_sequence<int, bmacs<LA, LB, LC, LD>()>{});
+#pragma unroll
+                    for (int i = 0; i < NOUT; ++i) w.v[i * 33 + lane] = c2(widen(v32[i].x, 0), widen(v32[i].y, 0));
+                    ++n32;
+                } else {
+                    complex_entry(X, Sh, ip, iq);
+                    ++n64;
+                }
+            }
+            __syncwarp();
+            add_runs<LA, LB, LC, LD, false>(d.out, w, nseg, lane);
+            __syncwarp();
         }
     }
     if (d.counters) {
         const unsigned a64 = __reduce_add_sync(0xffffffffu, n64);
         const unsigned a32 = __reduce_add_sync(0xffffffffu, n32);
         if (lane == 0) {
-            atomicAdd(&d.counters[0], (unsigned long long)a64);
-            atomicAdd(&d.counters[1], (unsigned long long)a32);
+            if (a64) atomicAdd(&d.counters[0], (unsigned long long)a64);
+            if (a32) atomicAdd(&d.counters[1], (unsigned long long)a32);
         }
     }
 }

@@ -450,10 +450,9 @@ int gx_eri_plan_autotune(gx_eri_plan* plan, const double* B, const double* O, in
  * cap (<= 4), phase-1 batch cap (<= 32), ket-transform rows per lane (1, 2,
  * 4), bra-transform components per lane (1-4), register-budget variant (2
  * or 4 resident blocks), 1 = no shared staging, 1 = stream mode (per-entry
- * recurrences into a two-column buffer), 1 = no FP32 lane kernel (mixed
- * precision, classes with 3 <= L <= 4: the generic kernel then also takes
- * the FP32 primitive quartets).  Fields other than per_group apply to the
- * generic kernel only. */
+ * recurrences into a two-column buffer), 1 = the generic kernel takes a
+ * class of the lane-dense kernel.  The other fields apply to the classes that
+ * the generic kernel takes. */
 typedef struct gx_class_config {
     int per_group, warps_per_block, batch, kt, ct, min_blocks, nostage, stream, nolane;
 } gx_class_config;

@@ -1,0 +1,97 @@
+"""Lane-per-quartet kernels (L <= 2 and lane-dense classes, and the real
+arithmetic of q = 0 pairs in all of them) at the places where their unit cutting
+and batching can go wrong: classes of one task, of 31 to 33 and of more than 512
+tasks, contracted tasks that span batches, units without a survivor, general
+contractions (strided blocks), and batches of every kind of pair.  FP64 within
+1e-12 of the oracle (the bar of the FP64 path) and the same bits however the
+quartet list is cut; mixed precision within 1e-10."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+import giaoint_gb300 as gi
+from giaoint_gb300 import synthetic as syn
+from giaoint_gb300.eri import _eri_batch
+
+from helpers import basis_from_records
+
+pytestmark = pytest.mark.gpu
+
+
+def _records(seed, ls, nprims, centers, contractions=1, far=0.0):
+    """One shell per (l, primitive count, centre index)."""
+    rng = np.random.default_rng(seed)
+    sites = rng.uniform(0.0, 2.5, (max(centers) + 1, 3))
+    sites[-1] += far
+    out = []
+    for l, k, c in zip(ls, nprims, centers):
+        e = np.exp(rng.uniform(np.log(0.2), np.log(20.0), k))
+        co = rng.uniform(0.1, 1.0, (contractions, k))
+        out.append(syn.ShellRecord(tuple(map(float, sites[c])), l, tuple(map(float, e)),
+                                   tuple(tuple(map(float, r)) for r in co)))
+    return out
+
+
+CASES = {
+    # every template pair and its mirror, L up to 8 and beyond (class-generic), mixed sites
+    "shells_spdf": (dict(ls=(0, 1, 2, 3, 1), nprims=(3, 2, 1, 1, 1), centers=(0, 0, 1, 1, 2)), (0.1, -0.07, 0.12), 160),
+    # one centre in a field: every pair real although B != 0
+    "one_site": (dict(ls=(0, 1, 2, 3), nprims=(4, 2, 2, 1), centers=(0, 0, 0, 0)), (0.2, 0.1, -0.3), 120),
+    # zero field, several sites: every pair real
+    "zero_field": (dict(ls=(0, 1, 2, 3, 2), nprims=(5, 3, 1, 1, 2), centers=(0, 1, 2, 2, 1)), (0.0, 0.0, 0.0), 120),
+    # general contractions: blocks written with strides
+    "contractions": (dict(ls=(0, 1, 2), nprims=(4, 3, 2), centers=(0, 1, 0), contractions=2), (0.05, 0.1, 0.0), 60),
+    # deep contractions: one task fills many batches
+    "deep": (dict(ls=(0, 0, 1), nprims=(9, 7, 6), centers=(0, 1, 1)), (-0.1, 0.02, 0.3), 81),
+    # a distant site: tasks and whole units without a surviving primitive quartet
+    "distant": (dict(ls=(0, 1, 2, 0, 1), nprims=(3, 2, 1, 3, 1), centers=(0, 0, 0, 1, 1), far=60.0), (0.01, 0.02, 0.0),
+                200),
+}
+
+
+@pytest.mark.parametrize("name", CASES)
+def test_blocks_against_oracle(name, oracle):
+    spec, B, count = CASES[name]
+    recs = _records(11, **spec)
+    basis = basis_from_records(recs)
+    ns = len(recs)
+    q = np.array([(a, b, c, d) for a in range(ns) for b in range(ns) for c in range(ns) for d in range(ns)], np.uint32)
+    rng = np.random.default_rng(5)
+    q = q[np.sort(rng.choice(len(q), min(count, len(q)), replace=False))]
+    field = gi.MagneticField(B)
+    _, _, offsets, values, _, _ = _eri_batch(basis, q, field=field)
+    ref, roff = oracle.eri_batch(recs, q, B, None, 8)
+    np.testing.assert_array_equal(offsets, roff)
+    assert np.abs(values - ref).max() <= 1e-12
+    _, _, _, exact, _, _ = _eri_batch(basis, q, field=field, precision="fp64_exact")
+    assert np.abs(exact - ref).max() <= 1e-12
+    _, _, _, mixed, _, _ = _eri_batch(basis, q, field=field, precision="mixed")
+    assert np.abs(mixed - ref).max() <= 1e-10
+    # the bits of a quartet do not depend on what it is evaluated with
+    lmax = np.array([r.angular_momentum for r in recs])[q.astype(int)].sum(1)
+    for part in (slice(0, 1), slice(3, 36), slice(1, None, 2)):
+        _, _, off2, val2, _, _ = _eri_batch(basis, q[part], field=field)
+        for i, k in enumerate(np.arange(len(q))[part]):
+            if lmax[k] <= 8:  # (beyond, the class-generic kernel splits by class size)
+                assert np.array_equal(val2[off2[i]:off2[i + 1]], values[offsets[k]:offsets[k + 1]])
+
+
+@pytest.mark.parametrize("tasks", [1, 31, 32, 33, 511, 512, 513, 1500])
+@pytest.mark.parametrize("key", [(0, 1, 0, 0), (1, 1, 0, 2), (2, 1, 2, 2)])
+def test_class_sizes(key, tasks, oracle):
+    """Classes around a batch and around the size from which the units are cut
+    by kernels of their own; the tasks repeat over few shells."""
+    rng = np.random.default_rng(tasks)
+    recs = _records(3, ls=key * 2, nprims=(2, 1, 1, 2, 1, 2, 3, 1), centers=(0, 1, 2, 0, 1, 1, 0, 2))
+    basis = basis_from_records(recs)
+    slots = [[i for i in (k, 4 + k)] for k in range(4)]
+    q = np.array([[rng.choice(s) for s in slots] for _ in range(tasks)], dtype=np.uint32)
+    B = (0.12, -0.2, 0.07)
+    _, _, offsets, values, _, _ = _eri_batch(basis, q, field=gi.MagneticField(B))
+    uniq, inv = np.unique(q, axis=0, return_inverse=True)
+    ref, roff = oracle.eri_batch(recs, uniq.astype(np.uint32), B, None, 8)
+    size = int(offsets[1])
+    want = ref.reshape(-1, size)[inv.reshape(-1)]
+    assert np.abs(values.reshape(-1, size) - want).max() <= 1e-12
