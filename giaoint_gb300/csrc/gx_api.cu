@@ -70,15 +70,20 @@ int guarded(F&& f) {
     }
 }
 
-// Grow-only device buffer.
+// Grow-only device buffer, or a view of a part of another one.
 struct DeviceBuffer {
     void* ptr = nullptr;
     size_t bytes = 0;
+    bool owned = true;
+    void view(const DeviceBuffer& of, size_t first, size_t n) {
+        release();
+        ptr = static_cast<char*>(of.ptr) + first;
+        bytes = n;
+        owned = false;
+    }
     void reserve(size_t n) {
         if (n <= bytes) return;
-        if (ptr) cudaFree(ptr);
-        ptr = nullptr;
-        bytes = 0;
+        release();
         const size_t want = std::max<size_t>(n, 256);
         cudaError_t e = cudaMalloc(&ptr, want);
         if (e != cudaSuccess) {
@@ -92,10 +97,14 @@ struct DeviceBuffer {
         return static_cast<T*>(ptr);
     }
     void release() {
-        if (ptr) cudaFree(ptr);
+        if (ptr && owned) cudaFree(ptr);
         ptr = nullptr;
         bytes = 0;
+        owned = true;
     }
+    DeviceBuffer() = default;
+    DeviceBuffer(const DeviceBuffer&) = delete;
+    DeviceBuffer& operator=(const DeviceBuffer&) = delete;
     ~DeviceBuffer() { release(); }
 };
 
@@ -327,6 +336,7 @@ void check_status(gx_context* ctx) {
 
 struct FieldPairs {
     double B[3], O[3];
+    DeviceBuffer mem;  // one allocation, and the views of its parts
     DeviceBuffer p, Pr, Pi, F, Epool, bound, Epool32, order, sbound, g32;
 };
 
@@ -344,11 +354,11 @@ struct gx_basis {
     bool one_site = true;  // all shells on one centre
     std::vector<int> seg_first, seg_l, seg_nprim, seg_primoff, seg_raw, seg_orig;
     std::vector<double> seg_center, seg_exps, seg_coefs;
-    DeviceBuffer d_center, d_l, d_nprim, d_primoff, d_exps, d_coefs, d_raw, d_sp_off;
+    DeviceBuffer mem;  // one allocation, and the views of its parts
+    DeviceBuffer d_center, d_l, d_nprim, d_primoff, d_exps, d_coefs, d_norms, d_raw, d_sp_off;
     // pair structure (field independent)
     int npp = 0;
-    std::vector<int> sp_off, pp_class;
-    std::vector<long long> Eoff;
+    std::vector<int> sp_off;
     long long Etotal = 0;
     DeviceBuffer d_pp_a, d_pp_b, d_pp_pa, d_pp_pb, d_pp_class, d_Eoff, d_classes;
     std::vector<std::pair<int, int>> class_keys;
@@ -367,7 +377,8 @@ struct gx_basis {
 
     gx::BasisDev dev() const {
         return gx::BasisDev{nseg, d_center.as<double>(), d_l.as<int>(), d_nprim.as<int>(), d_primoff.as<int>(),
-                            d_exps.as<double>(), d_coefs.as<double>(), d_raw.as<int>(), d_sp_off.as<int>()};
+                            d_exps.as<double>(), d_coefs.as<double>(), d_norms.as<double>(), d_raw.as<int>(),
+                            d_sp_off.as<int>()};
     }
     int ncart_of(int s) const { return gx::ncart(l[s]); }
     int64_t nao_of(int s) const { return (int64_t)ncontr[s] * ncart_of(s); }
@@ -397,64 +408,88 @@ void build_segments(gx_basis* b) {
         e += b->nprim[sh];
         c += (size_t)b->nprim[sh] * b->ncontr[sh];
     }
-    upload(b->d_center, b->seg_center, s);
-    upload(b->d_l, b->seg_l, s);
-    upload(b->d_nprim, b->seg_nprim, s);
-    upload(b->d_primoff, b->seg_primoff, s);
-    upload(b->d_exps, b->seg_exps, s);
-    upload(b->d_coefs, b->seg_coefs, s);
-    upload(b->d_raw, b->seg_raw, s);
+    std::vector<double> norms;
+    for (int sh = 0; sh < b->nseg; ++sh)
+        for (int p = 0; p < b->seg_nprim[sh]; ++p) {
+            const double x = b->seg_exps[b->seg_primoff[sh] + p];
+            // radial part of the primitive normalisation (src/types.cpp:60-72): (2x/pi)^{3/4} (4x)^{l/2}
+            norms.push_back(b->seg_raw[sh] ? 1.0
+                                           : std::exp(0.75 * std::log(2.0 * x / M_PI) +
+                                                      0.5 * b->seg_l[sh] * std::log(4.0 * x)));
+        }
     for (int sh = 1; sh < b->ns; ++sh)
         for (int k = 0; k < 3; ++k) b->one_site = b->one_site && b->center[3 * sh + k] == b->center[k];
-    // every ordered segmented shell pair, primitive pairs pa-major
+    // every ordered segmented shell pair: its primitive pairs (pa-major) and E~ words
     const int ns = b->nseg;
-    std::map<std::pair<int, int>, int> cls;
-    std::vector<int> pp_a, pp_b, pp_pa, pp_pb;
+    std::vector<int> cls(17 * 17, -1), sp_class((size_t)ns * ns);
+    std::vector<long long> sp_E((size_t)ns * ns);
+    std::vector<int> words;
     b->sp_off.assign((size_t)ns * ns, 0);
+    int64_t npp = 0;
     for (int a = 0; a < ns; ++a)
         for (int bb = 0; bb < ns; ++bb) {
-            b->sp_off[(size_t)a * ns + bb] = (int)pp_a.size();
-            auto key = std::make_pair(b->seg_l[a], b->seg_l[bb]);
-            auto it = cls.find(key);
-            int ci;
-            if (it == cls.end()) {
+            const size_t k = (size_t)a * ns + bb;
+            int& ci = cls[b->seg_l[a] * 17 + b->seg_l[bb]];
+            if (ci < 0) {
                 ci = (int)b->class_keys.size();
-                cls.emplace(key, ci);
-                b->class_keys.push_back(key);
-            } else {
-                ci = it->second;
+                b->class_keys.push_back({b->seg_l[a], b->seg_l[bb]});
+                words.push_back(b->ctx->pair_class(b->seg_l[a], b->seg_l[bb]).Etot);
             }
-            const PairClassHost& pc = b->ctx->pair_class(key.first, key.second);
-            for (int pa = 0; pa < b->seg_nprim[a]; ++pa)
-                for (int pb = 0; pb < b->seg_nprim[bb]; ++pb) {
-                    pp_a.push_back(a);
-                    pp_b.push_back(bb);
-                    pp_pa.push_back(pa);
-                    pp_pb.push_back(pb);
-                    b->pp_class.push_back(ci);
-                    b->Eoff.push_back(b->Etotal);
-                    b->Etotal += pc.Etot;
-                }
+            const int64_t count = (int64_t)b->seg_nprim[a] * b->seg_nprim[bb];
+            b->sp_off[k] = (int)npp;
+            sp_class[k] = ci;
+            sp_E[k] = b->Etotal;
+            npp += count;
+            b->Etotal += count * words[ci];
         }
-    b->npp = (int)pp_a.size();
-    upload(b->d_sp_off, b->sp_off, s);
-    upload(b->d_pp_a, pp_a, s);
-    upload(b->d_pp_b, pp_b, s);
-    upload(b->d_pp_pa, pp_pa, s);
-    upload(b->d_pp_pb, pp_pb, s);
-    upload(b->d_pp_class, b->pp_class, s);
-    upload(b->d_Eoff, b->Eoff, s);
+    if (npp > (int64_t)INT32_MAX) raise(GX_ELENGTH, "basis has too many primitive pairs");
+    b->npp = (int)npp;
     std::vector<gx::PairClassDev> devs;
     for (const auto& k : b->class_keys) devs.push_back(b->ctx->pair_class(k.first, k.second).dev());
-    upload(b->d_classes, devs, s);
+    // one allocation and one upload: the arrays below, then the pair structure that the device fills in
+    std::vector<char> host;
+    std::vector<std::pair<DeviceBuffer*, std::pair<size_t, size_t>>> parts;
+    size_t end = 0;
+    auto place = [&](DeviceBuffer& d, size_t bytes) {
+        parts.push_back({&d, {end, bytes}});
+        end = (end + std::max<size_t>(bytes, 1) + 15) / 16 * 16;
+    };
+    auto put = [&](DeviceBuffer& d, const auto& v) {
+        const size_t first = end, bytes = v.size() * sizeof(v[0]);
+        place(d, bytes);
+        host.resize(end);
+        if (bytes) std::memcpy(host.data() + first, v.data(), bytes);
+    };
+    DeviceBuffer d_sp_class, d_sp_E;
+    put(b->d_center, b->seg_center);
+    put(b->d_l, b->seg_l);
+    put(b->d_nprim, b->seg_nprim);
+    put(b->d_primoff, b->seg_primoff);
+    put(b->d_exps, b->seg_exps);
+    put(b->d_coefs, b->seg_coefs);
+    put(b->d_norms, norms);
+    put(b->d_raw, b->seg_raw);
+    put(b->d_sp_off, b->sp_off);
+    put(b->d_classes, devs);
+    put(d_sp_class, sp_class);
+    put(d_sp_E, sp_E);
+    for (DeviceBuffer* d : {&b->d_pp_a, &b->d_pp_b, &b->d_pp_pa, &b->d_pp_pb, &b->d_pp_class})
+        place(*d, npp * sizeof(int));
+    place(b->d_Eoff, npp * sizeof(long long));
+    b->mem.reserve(end);
+    for (auto& [d, at] : parts) d->view(b->mem, at.first, at.second);
+    GX_CUDA(cudaMemcpyAsync(b->mem.ptr, host.data(), host.size(), cudaMemcpyHostToDevice, s));
+    GX_CUDA(gx::launch_basis_pairs(b->dev(), d_sp_class.as<int>(), d_sp_E.as<long long>(),
+                                   b->d_classes.as<gx::PairClassDev>(), b->d_pp_a.as<int>(), b->d_pp_b.as<int>(),
+                                   b->d_pp_pa.as<int>(), b->d_pp_pb.as<int>(), b->d_pp_class.as<int>(),
+                                   b->d_Eoff.as<long long>(), s));
 }
 
-// Primitive-pair records for (B, O); cached on the basis for the last field.
-// Primitive-pair records for (B, O); cached on the basis for the last field.
-// After the records, every primitive pair's exact Schwarz factor is computed
-// on the device and each shell pair's primitive pairs are ordered by
-// decreasing factor, so that screened primitive quartets form a suffix of
-// every bra row and ket column.
+// Primitive-pair records for (B, O), enqueued on the context's stream; cached
+// on the basis for the last field.  After the records, every primitive pair's
+// exact Schwarz factor is computed and each shell pair's primitive pairs are
+// ordered by decreasing factor, so that screened primitive quartets form a
+// suffix of every bra row and ket column.
 gx::PairData pair_view(gx_basis* b, FieldPairs& fp) {
     return gx::PairData{b->npp,
                         fp.p.as<double>(),
@@ -478,17 +513,22 @@ FieldPairs& field_pairs(gx_basis* b, const double* B, const double* O) {
     FieldPairs& fp = *b->pairs;
     std::memcpy(fp.B, B, sizeof fp.B);
     std::memcpy(fp.O, O, sizeof fp.O);
-    const size_t n = std::max(b->npp, 1);
-    fp.p.reserve(n * sizeof(double));
-    fp.Pr.reserve(3 * n * sizeof(double));
-    fp.Pi.reserve(3 * n * sizeof(double));
-    fp.F.reserve(n * sizeof(double2));
-    fp.bound.reserve(n * sizeof(double));
-    fp.order.reserve(n * sizeof(int));
-    fp.sbound.reserve(n * sizeof(float));
-    fp.g32.reserve(2 * n * sizeof(float4));
-    fp.Epool.reserve(std::max<long long>(b->Etotal, 1) * sizeof(double2));
-    fp.Epool32.reserve(std::max<long long>(b->Etotal, 1) * sizeof(float2));
+    if (!fp.mem.ptr) {
+        const size_t n = std::max(b->npp, 1), e = std::max<long long>(b->Etotal, 1);
+        const std::pair<DeviceBuffer*, size_t> parts[] = {
+            {&fp.p, n * sizeof(double)},       {&fp.Pr, 3 * n * sizeof(double)}, {&fp.Pi, 3 * n * sizeof(double)},
+            {&fp.F, n * sizeof(double2)},      {&fp.bound, n * sizeof(double)},  {&fp.order, n * sizeof(int)},
+            {&fp.sbound, n * sizeof(float)},   {&fp.g32, 2 * n * sizeof(float4)}, {&fp.Epool, e * sizeof(double2)},
+            {&fp.Epool32, e * sizeof(float2)}};
+        size_t end = 0;
+        for (const auto& [d, bytes] : parts) end += (bytes + 255) / 256 * 256;
+        fp.mem.reserve(end);
+        end = 0;
+        for (const auto& [d, bytes] : parts) {
+            d->view(fp.mem, end, bytes);
+            end += (bytes + 255) / 256 * 256;
+        }
+    }
     gx::EriDev dev{};
     dev.basis = b->dev();
     dev.pairs = pair_view(b, fp);
@@ -502,27 +542,8 @@ FieldPairs& field_pairs(gx_basis* b, const double* B, const double* O) {
                                        b->d_classes.as<gx::PairClassDev>(), fp.p.as<double>(), fp.Pr.as<double>(),
                                        fp.Pi.as<double>(), fp.F.as<double2>(), b->d_Eoff.as<long long>(),
                                        fp.Epool.as<double2>(), fp.Epool32.as<float2>(), fp.bound.as<double>(),
-                                       fp.g32.as<float4>(), &dev, b->ctx->stream));
-    std::vector<double> bound(b->npp);
-    if (b->npp)
-        GX_CUDA(cudaMemcpyAsync(bound.data(), fp.bound.ptr, b->npp * sizeof(double), cudaMemcpyDeviceToHost,
-                                b->ctx->stream));
-    GX_CUDA(cudaStreamSynchronize(b->ctx->stream));
-    std::vector<int> order(b->npp);
-    std::vector<float> sbound(b->npp);
-    const int ns = b->nseg;
-    for (int a = 0; a < ns; ++a)
-        for (int c = 0; c < ns; ++c) {
-            const int first = b->sp_off[(size_t)a * ns + c];
-            const int count = b->seg_nprim[a] * b->seg_nprim[c];
-            std::iota(order.begin() + first, order.begin() + first + count, first);
-            std::stable_sort(order.begin() + first, order.begin() + first + count,
-                             [&](int x, int y) { return bound[x] > bound[y]; });
-            for (int k = first; k < first + count; ++k)
-                sbound[k] = (float)std::min(bound[order[k]], 3.0e38);
-        }
-    upload(fp.order, order, b->ctx->stream);
-    upload(fp.sbound, sbound, b->ctx->stream);
+                                       fp.g32.as<float4>(), fp.order.as<int>(), fp.sbound.as<float>(), dev,
+                                       b->ctx->stream));
     return fp;
 }
 

@@ -69,6 +69,7 @@ struct BasisDev {
     const int* primoff;
     const double* exps;
     const double* coefs;   // per primitive, contraction-normalised (segmented shells)
+    const double* norms;   // per primitive, radial normalisation (1 for raw shells)
     const int* raw;        // 1: no Cartesian primitive normalisation
     const int* sp_off;     // [ns*ns] first primitive pair of ordered shell pair (a, b)
 };
@@ -153,11 +154,14 @@ constexpr int REC_PLAN_MAX = 16;
 cudaError_t launch_boys_table(double2* S, double2* E0, const GLRules* gl, int* fail_count, cudaStream_t s);
 cudaError_t launch_boys_values(const double2* z, long long count, int nmax, int scaled, const BoysTable& tab,
                                const GLRules* gl, double2* out, int* region, DevStatus* st, cudaStream_t s);
+cudaError_t launch_basis_pairs(const BasisDev& basis, const int* sp_class, const long long* sp_E,
+                               const PairClassDev* classes, int* pp_a, int* pp_b, int* pp_pa, int* pp_pb,
+                               int* pp_class, long long* Eoff, cudaStream_t s);
 cudaError_t launch_pair_precompute(const BasisDev& basis, const double* B, const double* O, int npp, const int* pp_a,
                                    const int* pp_b, const int* pp_pa, const int* pp_pb, const int* pp_class,
                                    const PairClassDev* classes, double* p, double* Pr, double* Pi, double2* F,
                                    const long long* Eoff, double2* Epool, float2* Epool32, double* bound, float4* g32,
-                                   const EriDev* dev_for_bounds, cudaStream_t s);
+                                   int* order, float* sbound, const EriDev& dev, cudaStream_t s);
 size_t quartet_smem_bytes(const QuartetClass& qc, int warps_per_block, bool mixed);
 cudaError_t launch_quartets(const EriDev& dev, const QuartetClass& qc, int warps_per_block, int grid,
                             cudaStream_t s);

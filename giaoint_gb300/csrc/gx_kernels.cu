@@ -2,8 +2,8 @@
 //
 //   boys_table_kernel     scaled Boys values on the Taylor grid (setup)
 //   boys_values_kernel    F_0..F_n(z) for the boys() entry point (K2)
-//   pair_kernel           primitive-pair records: complex centre, prefactor
-//                         and complex Hermite coefficients (K1)
+//   pair_*_kernel         primitive-pair records: complex centre, prefactor,
+//                         complex Hermite coefficients, Schwarz factors (K1)
 //   quartet_kernel        class-generic shell-quartet ERIs (K3/K4)
 //   scatter_full_kernel   the four symmetry images of the full tensor (K5)
 //
@@ -18,10 +18,11 @@
 // Rh the ordinary three-index MD table of the complex centre separation
 // X' = P' - Q', seeded by common (-2 rho)^n F_n(rho X'^2).  E~ depends only
 // on the primitive pair, so it is computed once per (basis, field) by
-// pair_kernel; per primitive quartet only Rh (C(L+3,3) entries) and the two
+// the pair kernels; per primitive quartet only Rh (C(L+3,3) entries) and the two
 // contractions remain.
-#include <cstdint>
 #include <algorithm>
+#include <cmath>
+#include <cstdint>
 #include <cstdio>
 
 #include "gx_internal.h"
@@ -148,254 +149,6 @@ cudaError_t launch_boys_values(const double2* z, long long count, int nmax, int 
 }
 
 // ---------------------------------------------------------------------------
-// K1: primitive-pair records.  One thread per primitive pair.
-// ---------------------------------------------------------------------------
-
-__device__ double log_odd_double_factorial(int l) {
-    // ln((2l-1)!!) = l ln 2 + lgamma(l + 1/2) - ln(pi)/2
-    if (l == 0) return 0.0;
-    return l * 0.69314718055994530942 + lgamma(l + 0.5) - 0.57236494292470008707;
-}
-
-// Radial part of the primitive normalisation (src/types.cpp:60-72) without
-// the component factor: (2a/pi)^{3/4} (4a)^{l/2}.
-__device__ double radial_norm(double a, int l) {
-    return exp(0.75 * log(2.0 * a / 3.14159265358979323846) + 0.5 * l * log(4.0 * a));
-}
-
-// 1-D real MD coefficients E^{ij}_t, t <= i + j, by repeated raising
-// (src/hermite.cpp:8-40): first i raisings about A, then j about B.
-__device__ void hermite_1d(int i, int j, double PA, double PB, double inv2p, double* e) {
-    const int n = i + j;
-    for (int t = 0; t <= n + 1; ++t) e[t] = 0.0;
-    e[0] = 1.0;
-    for (int step = 0; step < n; ++step) {
-        const double d = step < i ? PA : PB;
-        // in place, descending t: new e[t] = inv2p e[t-1] + d e[t] + (t+1) e[t+1]
-        double upper = 0.0;  // old e[t+1]
-        for (int t = step + 1; t >= 0; --t) {
-            const double old = e[t];
-            e[t] = (t > 0 ? inv2p * e[t - 1] : 0.0) + d * old + (double)(t + 1) * upper;
-            upper = old;
-        }
-    }
-}
-
-__global__ void pair_kernel(BasisDev bs, double3 B, double3 O, int npp, const int* pp_a, const int* pp_b,
-                            const int* pp_pa, const int* pp_pb, const int* pp_class, const PairClassDev* classes,
-                            double* out_p, double* out_Pr, double* out_Pi, double2* out_F, const long long* Eoff,
-                            double2* Epool, float2* Epool32, double* out_bound, float4* out_g32) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= npp) return;
-    const int a = pp_a[i], b = pp_b[i];
-    const int pa = bs.primoff[a] + pp_pa[i], pb = bs.primoff[b] + pp_pb[i];
-    const double al = bs.exps[pa], be = bs.exps[pb];
-    const double A[3] = {bs.center[3 * a], bs.center[3 * a + 1], bs.center[3 * a + 2]};
-    const double Bc[3] = {bs.center[3 * b], bs.center[3 * b + 1], bs.center[3 * b + 2]};
-    const double p = al + be, mu = al * be / p;
-    double P[3], q[3], r2 = 0.0;
-    const double Bv[3] = {B.x, B.y, B.z}, Ov[3] = {O.x, O.y, O.z};
-    double ka[3], kb[3];
-    {
-        // London wave vectors k = B x (R - O) / 2 (src/types.cpp:179-186)
-        const double da[3] = {A[0] - Ov[0], A[1] - Ov[1], A[2] - Ov[2]};
-        const double db[3] = {Bc[0] - Ov[0], Bc[1] - Ov[1], Bc[2] - Ov[2]};
-        ka[0] = 0.5 * (Bv[1] * da[2] - Bv[2] * da[1]);
-        ka[1] = 0.5 * (Bv[2] * da[0] - Bv[0] * da[2]);
-        ka[2] = 0.5 * (Bv[0] * da[1] - Bv[1] * da[0]);
-        kb[0] = 0.5 * (Bv[1] * db[2] - Bv[2] * db[1]);
-        kb[1] = 0.5 * (Bv[2] * db[0] - Bv[0] * db[2]);
-        kb[2] = 0.5 * (Bv[0] * db[1] - Bv[1] * db[0]);
-    }
-    double qP = 0.0, qq = 0.0;
-    for (int x = 0; x < 3; ++x) {
-        P[x] = (al * A[x] + be * Bc[x]) / p;
-        q[x] = kb[x] - ka[x];
-        r2 += (A[x] - Bc[x]) * (A[x] - Bc[x]);
-        qP += q[x] * P[x];
-        qq += q[x] * q[x];
-    }
-    const int la = bs.l[a], lb = bs.l[b];
-    const bool raw_a = bs.raw[a] != 0, raw_b = bs.raw[b] != 0;
-    const double na = raw_a ? 1.0 : radial_norm(al, la);
-    const double nb = raw_b ? 1.0 : radial_norm(be, lb);
-    // 2 pi^{5/2} / (p q sqrt(p+q)) = sqrt(2 pi^{5/2})/p * sqrt(2 pi^{5/2})/q / sqrt(p+q)
-    const double mag = 5.914967172795613 * bs.coefs[pa] * bs.coefs[pb] * na * nb * exp(-mu * r2) / p;
-    double sn, cs;
-    sincos(-qP, &sn, &cs);
-    const double damp = exp(-qq / (4.0 * p));
-    out_p[i] = p;
-    for (int x = 0; x < 3; ++x) {
-        out_Pr[3 * i + x] = P[x];
-        out_Pi[3 * i + x] = -0.5 * q[x] / p;
-    }
-    out_F[i] = c2(mag * damp * cs, mag * damp * sn);
-    out_g32[2 * i] = make_float4((float)P[0], (float)P[1], (float)P[2], (float)p);
-    out_g32[2 * i + 1] = make_float4((float)(-0.5 * q[0] / p), (float)(-0.5 * q[1] / p), (float)(-0.5 * q[2] / p), 0.0f);
-
-    // complex Hermite coefficients per axis and per component pair
-    const PairClassDev pc = classes[pp_class[i]];
-    double2* rec = Epool + Eoff[i];
-    float2* rec32 = Epool32 + Eoff[i];
-    const double inv2p = 0.5 / p;
-    int ab = 0;
-    double bmax = 0.0;
-    for (int xa = la; xa >= 0; --xa)
-        for (int ya = la - xa; ya >= 0; --ya) {
-            const int ca[3] = {xa, ya, la - xa - ya};
-            for (int xb = lb; xb >= 0; --xb)
-                for (int yb = lb - xb; yb >= 0; --yb, ++ab) {
-                    const int cb[3] = {xb, yb, lb - xb - yb};
-                    double2 Et[3][34];
-                    int dim[3];
-                    double g = 1.0;
-                    for (int x = 0; x < 3; ++x) {
-                        if (!raw_a) g *= exp(-0.5 * log_odd_double_factorial(ca[x]));
-                        if (!raw_b) g *= exp(-0.5 * log_odd_double_factorial(cb[x]));
-                        double e[35];
-                        hermite_1d(ca[x], cb[x], P[x] - A[x], P[x] - Bc[x], inv2p, e);
-                        const int n = ca[x] + cb[x];
-                        dim[x] = n + 1;
-                        // E~_k = sum_{t>=k} C(t,k) (-i q)^{t-k} E_t
-                        for (int k = 0; k <= n; ++k) {
-                            double2 acc = c2(0.0, 0.0);
-                            double binom = 1.0;        // C(t, k) for t = k
-                            double2 pw = c2(1.0, 0.0); // (-i q)^{t-k}
-                            for (int t = k; t <= n; ++t) {
-                                acc = cadd(acc, cscale(pw, binom * e[t]));
-                                pw = cmul(pw, c2(0.0, -q[x]));
-                                binom = binom * (double)(t + 1) / (double)(t + 1 - k);
-                            }
-                            Et[x][k] = acc;
-                        }
-                    }
-                    const int off = pc.boxoff[ab];
-                    int e = 0;
-                    for (int k = 0; k < dim[0]; ++k)
-                        for (int l = 0; l < dim[1]; ++l) {
-                            const double2 xy = cmul(Et[0][k], Et[1][l]);
-                            for (int m = 0; m < dim[2]; ++m, ++e) {
-                                const double2 v = cscale(cmul(xy, Et[2][m]), g);
-                                rec[off + e] = v;
-                                rec32[off + e] = make_float2((float)v.x, (float)v.y);
-                                bmax = fmax(bmax, fabs(v.x) + fabs(v.y));
-                            }
-                        }
-                }
-        }
-    out_bound[i] = mag * damp * bmax;
-}
-
-// Exact primitive Schwarz factor of every primitive pair P = (a pa, b pb):
-// bound[P] = sqrt(max over component pairs |(ab|ba)_PP|), from the records of
-// P and of its reversed pair (b pb, a pa).  |(ab|cd)_PQ| <= bound[P] bound[Q]
-// holds for every component of a primitive quartet (Cauchy-Schwarz in the
-// Coulomb metric, the argument of src/eri.cpp:587-619 applied per primitive
-// pair).  Pairs with la+lb > 4 get an infinite bound (never screened).
-constexpr int BOUND_MAX_LAB = 4;
-
-__global__ void pair_bound_kernel(BasisDev bs, EriDev d, int npp, const int* pp_a, const int* pp_b, const int* pp_pa,
-                                  const int* pp_pb, const int* pp_class, const PairClassDev* classes, double* bound) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= npp) return;
-    const int a = pp_a[i], b = pp_b[i];
-    const int la = bs.l[a], lb = bs.l[b];
-    if (la + lb > BOUND_MAX_LAB) {
-        bound[i] = 1.0e300;
-        return;
-    }
-    const int j = bs.sp_off[b * bs.ns + a] + pp_pb[i] * bs.nprim[a] + pp_pa[i];
-    const PairData& pp = d.pairs;
-    const int L = 2 * (la + lb);
-    const double p = pp.p[i];
-    double2 X[3];
-    for (int x = 0; x < 3; ++x) X[x] = c2(pp.Pr[3 * i + x] - pp.Pr[3 * j + x], pp.Pi[3 * i + x] - pp.Pi[3 * j + x]);
-    const double rho = 0.5 * p;
-    const double tre = rho * (X[0].x * X[0].x + X[1].x * X[1].x + X[2].x * X[2].x - X[0].y * X[0].y -
-                              X[1].y * X[1].y - X[2].y * X[2].y);
-    const double tim = 2.0 * rho * (X[0].x * X[0].y + X[1].x * X[1].y + X[2].x * X[2].y);
-    double2 Sh[2 * BOUND_MAX_LAB + 1];
-    double2 e0;
-    if (boys_eval(tre, tim, L, d.boys, d.gl, Sh, e0)) {
-        bound[i] = 1.0e300;
-        return;
-    }
-    double2 C = cmul(cscale(cmul(pp.F[i], pp.F[j]), rsqrt(2.0 * p)), e0);
-    constexpr int NR = (2 * BOUND_MAX_LAB + 1) * (2 * BOUND_MAX_LAB + 2) * (2 * BOUND_MAX_LAB + 3) / 6;
-    double2 R[NR];
-    for (int n = 0; n <= L; ++n) {
-        Sh[n] = cmul(C, Sh[n]);
-        C = cscale(C, -2.0 * rho);
-    }
-    R[0] = Sh[L];
-    for (int n = L - 1; n >= 0; --n) {
-        for (int dg = L - n; dg >= 1; --dg)
-            for (int k = dg; k >= 0; --k)
-                for (int l = dg - k; l >= 0; --l) {
-                    const int m = dg - k - l;
-                    double2 v;
-                    if (k > 0) {
-                        v = cmul(X[0], R[herm_index(k - 1, l, m)]);
-                        if (k > 1) v = cmacr(v, (double)(k - 1), R[herm_index(k - 2, l, m)]);
-                    } else if (l > 0) {
-                        v = cmul(X[1], R[herm_index(0, l - 1, m)]);
-                        if (l > 1) v = cmacr(v, (double)(l - 1), R[herm_index(0, l - 2, m)]);
-                    } else {
-                        v = cmul(X[2], R[herm_index(0, 0, m - 1)]);
-                        if (m > 1) v = cmacr(v, (double)(m - 1), R[herm_index(0, 0, m - 2)]);
-                    }
-                    R[herm_index(k, l, m)] = v;
-                }
-        R[0] = Sh[n];
-    }
-    const PairClassDev ci = classes[pp_class[i]], cj = classes[pp_class[j]];
-    const double2* Ei = pp.Epool + pp.Eoff[i];
-    const double2* Ej = pp.Epool + pp.Eoff[j];
-    const int nb = ncart(lb), na = ncart(la);
-    double best = 0.0;
-    for (int ab = 0; ab < ci.nab; ++ab) {
-        const int ca = ab / nb, cb = ab - ca * nb;
-        const int ba = cb * na + ca;
-        const int oi = ci.boxoff[ab], di = ci.boxdim[ab];
-        const int oj = cj.boxoff[ba], dj = cj.boxdim[ba];
-        const int ni = (di & 255) * ((di >> 8) & 255) * ((di >> 16) & 255);
-        const int nj = (dj & 255) * ((dj >> 8) & 255) * ((dj >> 16) & 255);
-        double2 acc = c2(0.0, 0.0);
-        for (int e = 0; e < ni; ++e) {
-            const uint32_t ke = ci.ent[oi + e];
-            const int k1 = ke & 255, l1 = (ke >> 8) & 255, m1 = (ke >> 16) & 255;
-            double2 inner = c2(0.0, 0.0);
-            for (int f = 0; f < nj; ++f) {
-                const uint32_t kf = cj.ent[oj + f];
-                const int k2 = kf & 255, l2 = (kf >> 8) & 255, m2 = (kf >> 16) & 255;
-                double2 ev = Ej[oj + f];
-                if ((k2 + l2 + m2) & 1) ev = c2(-ev.x, -ev.y);
-                inner = cmac(inner, ev, R[herm_index(k1 + k2, l1 + l2, m1 + m2)]);
-            }
-            acc = cmac(acc, Ei[oi + e], inner);
-        }
-        best = fmax(best, sqrt(acc.x * acc.x + acc.y * acc.y));
-    }
-    bound[i] = sqrt(best) * (1.0 + 1.0e-10) + 1.0e-300;
-}
-
-cudaError_t launch_pair_precompute(const BasisDev& basis, const double* B, const double* O, int npp, const int* pp_a,
-                                   const int* pp_b, const int* pp_pa, const int* pp_pb, const int* pp_class,
-                                   const PairClassDev* classes, double* p, double* Pr, double* Pi, double2* F,
-                                   const long long* Eoff, double2* Epool, float2* Epool32, double* bound, float4* g32,
-                                   const EriDev* dev_for_bounds, cudaStream_t s) {
-    if (npp <= 0) return cudaSuccess;
-    pair_kernel<<<(npp + 63) / 64, 64, 0, s>>>(basis, make_double3(B[0], B[1], B[2]), make_double3(O[0], O[1], O[2]),
-                                               npp, pp_a, pp_b, pp_pa, pp_pb, pp_class, classes, p, Pr, Pi, F, Eoff,
-                                               Epool, Epool32, bound, g32);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess || !dev_for_bounds) return e;
-    pair_bound_kernel<<<(npp + 63) / 64, 64, 0, s>>>(basis, *dev_for_bounds, npp, pp_a, pp_b, pp_pa, pp_pb, pp_class,
-                                                     classes, bound);
-    return cudaGetLastError();
-}
-
-// ---------------------------------------------------------------------------
 // K3/K4: class-generic quartet kernel, one warp per shell quartet.
 //
 // Phase 1 (lane-parallel): up to B1 primitive quartets (P, Q..Q+B1) at a
@@ -409,8 +162,6 @@ cudaError_t launch_pair_precompute(const BasisDev& basis, const double* B, const
 // The sign (-1)^{|K'|} of the ket side is applied to the ket records when
 // they are read as kets (ket_sign below).
 // ---------------------------------------------------------------------------
-
-__constant__ double c_int[40];  // c_int[k] = k, avoids int->double conversions in inner loops
 
 // FP64 quantities of primitive quartet (ip, iq): the complex centre
 // separation X' = P' - Q', rho = pq / (p + q), the Boys argument
@@ -466,8 +217,8 @@ template <>
 __device__ __forceinline__ float2 tmul(float2 a, float2 b) {
     return make_float2(fmaf(a.x, b.x, -a.y * b.y), fmaf(a.x, b.y, a.y * b.x));
 }
-__device__ __forceinline__ double2 tmacr(double2 c, int k, double2 a) { return cmacr(c, c_int[k], a); }
-__device__ __forceinline__ double tmacr(double c, int k, double a) { return fma(c_int[k], a, c); }
+__device__ __forceinline__ double2 tmacr(double2 c, int k, double2 a) { return cmacr(c, c_dev.ints[k], a); }
+__device__ __forceinline__ double tmacr(double c, int k, double a) { return fma(c_dev.ints[k], a, c); }
 __device__ __forceinline__ float2 tmacr(float2 c, int k, float2 a) {
     return make_float2(fmaf((float)k, a.x, c.x), fmaf((float)k, a.y, c.y));
 }
@@ -636,6 +387,336 @@ __device__ __forceinline__ void coop_rec(int L, const T* seed, const T* X, T* R,
         __syncwarp();
         cur = nxt;
     }
+}
+
+// ---------------------------------------------------------------------------
+// K1: primitive-pair records, four launches per (basis, field), all bound by
+// FP64 warp instructions and latency (a field of the 12-atom molecule, 24,336
+// pairs: one thread per pair for everything and the ordering on the host took
+// 2.1 ms and a synchronisation):
+//   pair_scalar_kernel  a thread per pair: centre, prefactor (dense lanes for
+//                       the exponentials)
+//   pair_hermite_kernel a warp per pair, a lane per component pair: E~ boxes
+//   pair_bound_kernel   a warp per pair of one orientation: its exact Schwarz
+//                       factor, for both orientations
+//   pair_order_kernel   a warp per shell pair: its primitive pairs ordered by
+//                       decreasing factor
+// ---------------------------------------------------------------------------
+
+// 1-D real MD coefficients E^{ij}_t, t <= i + j, by repeated raising
+// (src/hermite.cpp:8-40): first i raisings about A, then j about B.
+__device__ void hermite_1d(int i, int j, double PA, double PB, double inv2p, double* e) {
+    const int n = i + j;
+    for (int t = 0; t <= n + 1; ++t) e[t] = 0.0;
+    e[0] = 1.0;
+    for (int step = 0; step < n; ++step) {
+        const double d = step < i ? PA : PB;
+        // in place, descending t: new e[t] = inv2p e[t-1] + d e[t] + (t+1) e[t+1]
+        double upper = 0.0;  // old e[t+1]
+        for (int t = step + 1; t >= 0; --t) {
+            const double old = e[t];
+            e[t] = (t > 0 ? inv2p * e[t - 1] : 0.0) + d * old + c_dev.ints[t + 1] * upper;
+            upper = old;
+        }
+    }
+}
+
+__global__ void pair_scalar_kernel(BasisDev bs, double3 B, double3 O, int npp, const int* pp_a, const int* pp_b,
+                                   const int* pp_pa, const int* pp_pb, double* out_p, double* out_Pr, double* out_Pi,
+                                   double2* out_F, float4* out_g32) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= npp) return;
+    const int a = pp_a[i], b = pp_b[i];
+    const int pa = bs.primoff[a] + pp_pa[i], pb = bs.primoff[b] + pp_pb[i];
+    const double al = bs.exps[pa], be = bs.exps[pb];
+    const double A[3] = {bs.center[3 * a], bs.center[3 * a + 1], bs.center[3 * a + 2]};
+    const double Bc[3] = {bs.center[3 * b], bs.center[3 * b + 1], bs.center[3 * b + 2]};
+    const double p = al + be, mu = al * be / p;
+    double P[3], q[3], r2 = 0.0;
+    const double Bv[3] = {B.x, B.y, B.z}, Ov[3] = {O.x, O.y, O.z};
+    double ka[3], kb[3];
+    {
+        // London wave vectors k = B x (R - O) / 2 (src/types.cpp:179-186)
+        const double da[3] = {A[0] - Ov[0], A[1] - Ov[1], A[2] - Ov[2]};
+        const double db[3] = {Bc[0] - Ov[0], Bc[1] - Ov[1], Bc[2] - Ov[2]};
+        ka[0] = 0.5 * (Bv[1] * da[2] - Bv[2] * da[1]);
+        ka[1] = 0.5 * (Bv[2] * da[0] - Bv[0] * da[2]);
+        ka[2] = 0.5 * (Bv[0] * da[1] - Bv[1] * da[0]);
+        kb[0] = 0.5 * (Bv[1] * db[2] - Bv[2] * db[1]);
+        kb[1] = 0.5 * (Bv[2] * db[0] - Bv[0] * db[2]);
+        kb[2] = 0.5 * (Bv[0] * db[1] - Bv[1] * db[0]);
+    }
+    double qP = 0.0, qq = 0.0;
+    for (int x = 0; x < 3; ++x) {
+        P[x] = (al * A[x] + be * Bc[x]) / p;
+        q[x] = kb[x] - ka[x];
+        r2 += (A[x] - Bc[x]) * (A[x] - Bc[x]);
+        qP += q[x] * P[x];
+        qq += q[x] * q[x];
+    }
+    // 2 pi^{5/2} / (p q sqrt(p+q)) = sqrt(2 pi^{5/2})/p * sqrt(2 pi^{5/2})/q / sqrt(p+q)
+    const double mag = 5.914967172795613 * bs.coefs[pa] * bs.coefs[pb] * bs.norms[pa] * bs.norms[pb] * exp(-mu * r2) / p;
+    double sn, cs;
+    sincos(-qP, &sn, &cs);
+    const double damp = exp(-qq / (4.0 * p));
+    out_p[i] = p;
+    for (int x = 0; x < 3; ++x) {
+        out_Pr[3 * i + x] = P[x];
+        out_Pi[3 * i + x] = -0.5 * q[x] / p;
+    }
+    out_F[i] = c2(mag * damp * cs, mag * damp * sn);
+    out_g32[2 * i] = make_float4((float)P[0], (float)P[1], (float)P[2], (float)p);
+    out_g32[2 * i + 1] = make_float4((float)(-0.5 * q[0] / p), (float)(-0.5 * q[1] / p), (float)(-0.5 * q[2] / p), 0.0f);
+}
+
+// Complex Hermite coefficients E~_k = sum_{t>=k} C(t,k) (-i q)^{t-k} E_t per
+// axis and their boxes per component pair, the component normalisation
+// ((2l-1)!!)^{-1/2} per axis folded in (inv_df).
+struct AxisNorms {
+    double v[17];
+};
+constexpr int kPairWarps = 4;
+
+__global__ void __launch_bounds__(32 * kPairWarps) pair_hermite_kernel(
+    BasisDev bs, double3 B, double3 O, int npp, const int* pp_a, const int* pp_b, const int* pp_pa, const int* pp_pb,
+    const int* pp_class, const PairClassDev* classes, AxisNorms inv_df, const double* in_p, const double* in_Pr,
+    const double* in_Pi, const long long* Eoff, double2* Epool, float2* Epool32) {
+    const int i = blockIdx.x * kPairWarps + (threadIdx.x >> 5);
+    if (i >= npp) return;
+    const int lane = threadIdx.x & 31;
+    const int a = pp_a[i], b = pp_b[i];
+    const int la = bs.l[a], lb = bs.l[b];
+    const PairClassDev pc = classes[pp_class[i]];
+    const int nb = ncart(lb);
+    if (lane >= pc.nab) return;
+    const double A[3] = {bs.center[3 * a], bs.center[3 * a + 1], bs.center[3 * a + 2]};
+    const double Bc[3] = {bs.center[3 * b], bs.center[3 * b + 1], bs.center[3 * b + 2]};
+    const double Bv[3] = {B.x, B.y, B.z}, Ov[3] = {O.x, O.y, O.z};
+    double q[3];
+    for (int x = 0; x < 3; ++x) {
+        // (zero where the pair's record says so: the kernels go by that)
+        q[x] = 0.0;
+        if (in_Pi[3 * i + x] == 0.0) continue;
+        const int y = (x + 1) % 3, z = (x + 2) % 3;
+        q[x] = 0.5 * (Bv[y] * (Bc[z] - Ov[z]) - Bv[z] * (Bc[y] - Ov[y])) -
+               0.5 * (Bv[y] * (A[z] - Ov[z]) - Bv[z] * (A[y] - Ov[y]));
+    }
+    const double inv2p = 0.5 / in_p[i];
+    const double P[3] = {in_Pr[3 * i], in_Pr[3 * i + 1], in_Pr[3 * i + 2]};
+    const bool raw_a = bs.raw[a] != 0, raw_b = bs.raw[b] != 0;
+    double2* rec = Epool + Eoff[i];
+    float2* rec32 = Epool32 + Eoff[i];
+    // Cartesian component c of degree l (x descending, then y)
+    auto component = [](int l, int c, int* v) {
+        int m = 0;  // l - x
+        while ((m + 1) * (m + 2) / 2 <= c) ++m;
+        v[0] = l - m;
+        v[2] = c - m * (m + 1) / 2;
+        v[1] = m - v[2];
+    };
+    for (int ab = lane; ab < pc.nab; ab += 32) {
+        int ca[3], cb[3];
+        component(la, ab / nb, ca);
+        component(lb, ab % nb, cb);
+        double2 Et[3][34];
+        int dim[3];
+        double g = 1.0;
+        for (int x = 0; x < 3; ++x) {
+            if (!raw_a) g *= inv_df.v[ca[x]];
+            if (!raw_b) g *= inv_df.v[cb[x]];
+            double e[35];
+            hermite_1d(ca[x], cb[x], P[x] - A[x], P[x] - Bc[x], inv2p, e);
+            const int n = ca[x] + cb[x];
+            dim[x] = n + 1;
+            for (int k = 0; k <= n; ++k) {
+                double2 acc = c2(e[k], 0.0);
+                if (q[x] != 0.0) {
+                    double binom = 1.0;         // C(t, k) for t = k
+                    double2 pw = c2(1.0, 0.0);  // (-i q)^{t-k}
+                    for (int t = k + 1; t <= n; ++t) {
+                        pw = c2(pw.y * q[x], -pw.x * q[x]);
+                        binom = binom * c_dev.ints[t] / c_dev.ints[t - k];
+                        acc = cadd(acc, cscale(pw, binom * e[t]));
+                    }
+                }
+                Et[x][k] = acc;
+            }
+        }
+        int e = pc.boxoff[ab];
+        for (int k = 0; k < dim[0]; ++k)
+            for (int l = 0; l < dim[1]; ++l) {
+                const double2 xy = cmul(Et[0][k], Et[1][l]);
+                for (int m = 0; m < dim[2]; ++m, ++e) {
+                    const double2 v = cscale(cmul(xy, Et[2][m]), g);
+                    rec[e] = v;
+                    rec32[e] = make_float2((float)v.x, (float)v.y);
+                }
+            }
+    }
+}
+
+// Exact primitive Schwarz factor of every primitive pair P = (a pa, b pb):
+// bound[P] = sqrt(max over component pairs |(ab|ba)_PP|), from the records of
+// P and of its reversed pair (b pb, a pa).  |(ab|cd)_PQ| <= bound[P] bound[Q]
+// holds for every component of a primitive quartet (Cauchy-Schwarz in the
+// Coulomb metric, the argument of src/eri.cpp:587-619 applied per primitive
+// pair).  The reversed pair has the same factor ((ab|ba) = (ba|ab) by the
+// exchange of the electrons), so one orientation is evaluated.  Pairs with
+// la+lb > 4 get an infinite bound (never screened).
+constexpr int BOUND_MAX_LAB = 4;
+
+__global__ void __launch_bounds__(32 * kPairWarps) pair_bound_kernel(BasisDev bs, EriDev d, int npp, const int* pp_a,
+                                                                     const int* pp_b, const int* pp_pa,
+                                                                     const int* pp_pb, const int* pp_class,
+                                                                     const PairClassDev* classes, double* bound) {
+    constexpr int MAXL = 2 * BOUND_MAX_LAB;
+    constexpr int NR = (MAXL + 1) * (MAXL + 2) * (MAXL + 3) / 6;
+    __shared__ double2 s_R[kPairWarps][2 * NR];
+    __shared__ double2 s_seed[kPairWarps][MAXL + 4];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int i = blockIdx.x * kPairWarps + warp;
+    if (i >= npp) return;
+    const int a = pp_a[i], b = pp_b[i];
+    if (a > b || (a == b && pp_pa[i] > pp_pb[i])) return;
+    const int la = bs.l[a], lb = bs.l[b];
+    const int j = bs.sp_off[b * bs.ns + a] + pp_pb[i] * bs.nprim[a] + pp_pa[i];
+    if (la + lb > BOUND_MAX_LAB) {
+        if (lane == 0) bound[i] = bound[j] = 1.0e300;
+        return;
+    }
+    const PairData& pp = d.pairs;
+    const int L = 2 * (la + lb);
+    const double p = pp.p[i];
+    double2 X[3];
+    for (int x = 0; x < 3; ++x) X[x] = c2(pp.Pr[3 * i + x] - pp.Pr[3 * j + x], pp.Pi[3 * i + x] - pp.Pi[3 * j + x]);
+    const double rho = 0.5 * p;
+    const double tre = rho * (X[0].x * X[0].x + X[1].x * X[1].x + X[2].x * X[2].x - X[0].y * X[0].y -
+                              X[1].y * X[1].y - X[2].y * X[2].y);
+    const double tim = 2.0 * rho * (X[0].x * X[0].y + X[1].x * X[1].y + X[2].x * X[2].y);
+    double2 Sh[MAXL + 1];
+    double2 e0;
+    if (boys_eval(tre, tim, L, d.boys, d.gl, Sh, e0)) {  // (the same on every lane)
+        if (lane == 0) bound[i] = bound[j] = 1.0e300;
+        return;
+    }
+    double2 C = cmul(cscale(cmul(pp.F[i], pp.F[j]), rsqrt(2.0 * p)), e0);
+    double2* R = s_R[warp];
+    double2* seed = s_seed[warp];
+    for (int n = 0; n <= L; ++n) {
+        if (lane == 0) seed[n] = cmul(C, Sh[n]);
+        C = cscale(C, -2.0 * rho);
+    }
+    if (lane < 3) seed[L + 1 + lane] = lane == 0 ? X[0] : (lane == 1 ? X[1] : X[2]);
+    __syncwarp();
+    coop_rec<double2>(L, seed, seed + L + 1, R, 2, 0, 1, d.herm_xyz, lane);
+    const PairClassDev ci = classes[pp_class[i]], cj = classes[pp_class[j]];
+    const double2* Ei = pp.Epool + pp.Eoff[i];
+    const double2* Ej = pp.Epool + pp.Eoff[j];
+    const int nb = ncart(lb), na = ncart(la);
+    double best = 0.0;
+    for (int ab = lane; ab < ci.nab; ab += 32) {
+        const int ca = ab / nb, cb = ab - ca * nb;
+        const int ba = cb * na + ca;
+        const int oi = ci.boxoff[ab], di = ci.boxdim[ab];
+        const int oj = cj.boxoff[ba], dj = cj.boxdim[ba];
+        const int ni = (di & 255) * ((di >> 8) & 255) * ((di >> 16) & 255);
+        const int nj = (dj & 255) * ((dj >> 8) & 255) * ((dj >> 16) & 255);
+        double2 acc = c2(0.0, 0.0);
+        for (int e = 0; e < ni; ++e) {
+            const uint32_t ke = ci.ent[oi + e];
+            const int k1 = ke & 255, l1 = (ke >> 8) & 255, m1 = (ke >> 16) & 255;
+            double2 inner = c2(0.0, 0.0);
+            for (int f = 0; f < nj; ++f) {
+                const uint32_t kf = cj.ent[oj + f];
+                const int k2 = kf & 255, l2 = (kf >> 8) & 255, m2 = (kf >> 16) & 255;
+                double2 ev = Ej[oj + f];
+                if ((k2 + l2 + m2) & 1) ev = c2(-ev.x, -ev.y);
+                inner = cmac(inner, ev, R[2 * herm_index(k1 + k2, l1 + l2, m1 + m2)]);
+            }
+            acc = cmac(acc, Ei[oi + e], inner);
+        }
+        best = fmax(best, acc.x * acc.x + acc.y * acc.y);
+    }
+    for (int off = 16; off > 0; off >>= 1) best = fmax(best, __shfl_xor_sync(0xffffffffu, best, off));
+    if (lane == 0) bound[i] = bound[j] = sqrt(sqrt(best)) * (1.0 + 1.0e-10) + 1.0e-300;
+}
+
+// The primitive pairs of every shell pair by decreasing factor (equal ones in
+// record order): the rank of a pair is the number of pairs before it.
+__global__ void pair_order_kernel(BasisDev bs, const double* bound, int* order, float* sbound) {
+    const int sp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (sp >= bs.ns * bs.ns) return;
+    const int a = sp / bs.ns, b = sp - a * bs.ns;
+    const int first = bs.sp_off[sp], count = bs.nprim[a] * bs.nprim[b];
+    for (int x = threadIdx.x & 31; x < count; x += 32) {
+        const double v = bound[first + x];
+        int rank = 0;
+        for (int y = 0; y < count; ++y) {
+            const double w = bound[first + y];
+            rank += w > v || (w == v && y < x);
+        }
+        order[first + rank] = first + x;
+        sbound[first + rank] = (float)fmin(v, 3.0e38);
+    }
+}
+
+// Primitive pairs of every ordered shell pair (sp_class, sp_E: pair class and
+// first E~ word of the shell pair), pa-major.
+__global__ void basis_pairs_kernel(BasisDev bs, const int* sp_class, const long long* sp_E, const PairClassDev* classes,
+                                   int* pp_a, int* pp_b, int* pp_pa, int* pp_pb, int* pp_class, long long* Eoff) {
+    const int sp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (sp >= bs.ns * bs.ns) return;
+    const int a = sp / bs.ns, b = sp - a * bs.ns;
+    const int first = bs.sp_off[sp], nb = bs.nprim[b], count = bs.nprim[a] * nb, cls = sp_class[sp];
+    const long long E = sp_E[sp];
+    const int words = classes[cls].Etot;
+    for (int x = threadIdx.x & 31; x < count; x += 32) {
+        pp_a[first + x] = a;
+        pp_b[first + x] = b;
+        pp_pa[first + x] = x / nb;
+        pp_pb[first + x] = x % nb;
+        pp_class[first + x] = cls;
+        Eoff[first + x] = E + (long long)x * words;
+    }
+}
+
+cudaError_t launch_basis_pairs(const BasisDev& basis, const int* sp_class, const long long* sp_E,
+                               const PairClassDev* classes, int* pp_a, int* pp_b, int* pp_pa, int* pp_pb,
+                               int* pp_class, long long* Eoff, cudaStream_t s) {
+    if (basis.ns <= 0) return cudaSuccess;
+    const unsigned pairs = (unsigned)basis.ns * (unsigned)basis.ns;
+    basis_pairs_kernel<<<(pairs + 7) / 8, 256, 0, s>>>(basis, sp_class, sp_E, classes, pp_a, pp_b, pp_pa, pp_pb,
+                                                       pp_class, Eoff);
+    return cudaGetLastError();
+}
+
+static AxisNorms axis_norms() {
+    AxisNorms n;
+    double df = 1.0;  // (2l - 1)!!
+    for (int l = 0; l < 17; ++l) {
+        if (l > 0) df *= 2.0 * l - 1.0;
+        n.v[l] = 1.0 / std::sqrt(df);
+    }
+    return n;
+}
+
+cudaError_t launch_pair_precompute(const BasisDev& basis, const double* B, const double* O, int npp, const int* pp_a,
+                                   const int* pp_b, const int* pp_pa, const int* pp_pb, const int* pp_class,
+                                   const PairClassDev* classes, double* p, double* Pr, double* Pi, double2* F,
+                                   const long long* Eoff, double2* Epool, float2* Epool32, double* bound, float4* g32,
+                                   int* order, float* sbound, const EriDev& dev, cudaStream_t s) {
+    if (npp <= 0) return cudaSuccess;
+    const double3 Bv = make_double3(B[0], B[1], B[2]), Ov = make_double3(O[0], O[1], O[2]);
+    const unsigned warps = (unsigned)((npp + kPairWarps - 1) / kPairWarps);
+    pair_scalar_kernel<<<(npp + 63) / 64, 64, 0, s>>>(basis, Bv, Ov, npp, pp_a, pp_b, pp_pa, pp_pb, p, Pr, Pi, F, g32);
+    pair_hermite_kernel<<<warps, 32 * kPairWarps, 0, s>>>(basis, Bv, Ov, npp, pp_a, pp_b, pp_pa, pp_pb, pp_class,
+                                                          classes, axis_norms(), p, Pr, Pi, Eoff, Epool,
+                                                          Epool32);
+    pair_bound_kernel<<<warps, 32 * kPairWarps, 0, s>>>(basis, dev, npp, pp_a, pp_b, pp_pa, pp_pb, pp_class, classes,
+                                                        bound);
+    const unsigned pairs = (unsigned)basis.ns * (unsigned)basis.ns;
+    pair_order_kernel<<<(pairs + 3) / 4, 128, 0, s>>>(basis, bound, order, sbound);
+    return cudaGetLastError();
 }
 
 // Work split of a transform with `items` work items: J lanes share an item
@@ -1325,18 +1406,9 @@ size_t quartet_smem_bytes(const QuartetClass& qc, int warps_per_block, bool mixe
                warp_smem(qc.NL, qc.B1, qc.Nab, qc.CH, mixed, qc.stage_e, qc.stream, qc.L).total;
 }
 
-static bool g_const_ready = false;
-
 cudaError_t launch_quartets(const EriDev& dev, const QuartetClass& qc, int warps_per_block, int grid,
                             cudaStream_t s) {
     if (qc.ntask <= 0) return cudaSuccess;
-    if (!g_const_ready) {
-        double v[40];
-        for (int i = 0; i < 40; ++i) v[i] = (double)i;
-        cudaError_t e = cudaMemcpyToSymbol(c_int, v, sizeof v);
-        if (e != cudaSuccess) return e;
-        g_const_ready = true;
-    }
     const size_t smem = quartet_smem_bytes(qc, warps_per_block, dev.fp32_cut > 0.0f);
     static size_t configured[2] = {0, 0};
     const int v = qc.minb == 4 ? 1 : 0;

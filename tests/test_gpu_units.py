@@ -45,6 +45,8 @@ CASES = {
     "contractions": (dict(ls=(0, 1, 2), nprims=(4, 3, 2), centers=(0, 1, 0), contractions=2), (0.05, 0.1, 0.0), 60),
     # deep contractions: one task fills many batches
     "deep": (dict(ls=(0, 0, 1), nprims=(9, 7, 6), centers=(0, 1, 1)), (-0.1, 0.02, 0.3), 81),
+    # order above the Schwarz factors' limit, beyond a warp's lanes of component pairs
+    "high_l": (dict(ls=(5, 4, 0), nprims=(1, 2, 2), centers=(0, 1, 1)), (0.1, 0.2, -0.1), 12),
     # a distant site: tasks and whole units without a surviving primitive quartet
     "distant": (dict(ls=(0, 1, 2, 0, 1), nprims=(3, 2, 1, 3, 1), centers=(0, 0, 0, 1, 1), far=60.0), (0.01, 0.02, 0.0),
                 200),
@@ -95,3 +97,17 @@ def test_class_sizes(key, tasks, oracle):
     size = int(offsets[1])
     want = ref.reshape(-1, size)[inv.reshape(-1)]
     assert np.abs(values.reshape(-1, size) - want).max() <= 1e-12
+
+
+def test_equal_schwarz_factors(oracle):
+    """Shells with repeated primitives: the order of equal factors is that of
+    the records, and 24 primitives fill several rounds of the ranking."""
+    e = tuple([0.8] * 12 + [1.7] * 12)
+    c = ((0.1,) * 24,)
+    recs = [syn.ShellRecord((0.0, 0.0, 0.1 * k), l, e, c) for k, l in enumerate((0, 1))]
+    basis = basis_from_records(recs)
+    q = np.array([(0, 1, 0, 1), (1, 1, 0, 0)], np.uint32)
+    B = (0.3, -0.1, 0.2)
+    _, _, _, values, _, _ = _eri_batch(basis, q, field=gi.MagneticField(B))
+    ref, _ = oracle.eri_batch(recs, q, B, None, 8)
+    assert np.abs(values - ref).max() <= 1e-12
