@@ -215,15 +215,15 @@ struct Out {
     const long long* seg_off;   // block of each segment (run of lanes with one shell quartet)
     const int4* seg_st;         // its strides: template a, b, other c, d
     const int* shift;           // FP32: per lane, the power of two that undoes its seed scale
-    const int* seg_lane;        // first lane of each segment (bit 8: store, not add), and the end
+    const int* seg_lane;        // first lane and flags of each segment, and the end
     int nseg, ndd, lane;
     bool inner_c;               // the other side's components are the inner ones of the block
 };
 
 // The lanes of each segment over the value buffer (components ab0 .. of the
-// other side's components c .. c + cg - 1), added to its block one after the
-// other in stream order and in FP64: the result depends neither on where the batches
-// of a unit begin or end, nor on what else they hold.
+// other side's components c .. c + cg - 1), added to its block in stream order
+// and in FP64: the result depends neither on where the batches of a unit begin
+// or end, nor on what else they hold.
 template <int LB, typename RT>
 __device__ __forceinline__ void reduce_out(const Out& o, const RT* vb, int ab0, int nab, int c, int cg) {
     constexpr int NCB = nc(LB);
@@ -238,31 +238,22 @@ __device__ __forceinline__ void reduce_out(const Out& o, const RT* vb, int ab0, 
         double2* p = o.out + o.seg_off[s] + (long long)(ab / NCB) * st.x + (long long)(ab % NCB) * st.y +
                      (long long)cc * st.z + (long long)cdd * st.w;
         const RT* v = vb + (u * nab + i) * 33;
-        const bool store = o.seg_lane[s] & 256;
-        int l = o.seg_lane[s] & 255;
-        const int l1 = o.seg_lane[s + 1] & 255;
+        const int flags = o.seg_lane[s], l0 = flags & 255, l1 = o.seg_lane[s + 1] & 255;
+        const bool store = flags & kStore;
+        auto at = [&](int k) { return v[k]; };
         if constexpr (std::is_same_v<RT, double2>) {
-            double2 sum;
-            if (store)
-                sum = v[l++];
-            else
-                sum = *p;
-            for (; l < l1; ++l) sum = add(sum, v[l]);
-            *p = sum;
+            const double2 old = store ? c2(0.0, 0.0) : *p;
+            *p = add_by_runs(old, flags, l0, l1, at);
         } else if constexpr (std::is_same_v<RT, double>) {
-            double sum;
-            if (store)
-                sum = v[l++];
-            else
-                sum = p->x;
-            for (; l < l1; ++l) sum += v[l];
+            const double old = store ? 0.0 : p->x;
+            const double sum = add_by_runs(old, flags, l0, l1, at);
             if (store)
                 *p = c2(sum, 0.0);
             else
                 p->x = sum;
         } else {
             double2 sum = *p;
-            for (; l < l1; ++l) sum = cadd(sum, c2(widen(v[l].x, o.shift[l]), widen(v[l].y, o.shift[l])));
+            for (int l = l0; l < l1; ++l) sum = cadd(sum, c2(widen(v[l].x, o.shift[l]), widen(v[l].y, o.shift[l])));
             *p = sum;
         }
     }
@@ -466,8 +457,7 @@ __global__ void __launch_bounds__(32 * kWarps) dense_kernel(EriDev d, QuartetCla
                     const int s = __popc(heads & ((1u << lane) - 1u));
                     seg_off[s] = tg->out_off;
                     seg_st[s] = strides(tg);
-                    // bit 8: the shell quartet's first FP64 entry, whose batch stores instead of adding
-                    seg_lane[s] = lane | (!F32 && rank == 0 ? 256 : 0);
+                    seg_lane[s] = lane | (!F32 && rank == 0 ? kStore : 0) | (stream.run == 32 ? kLongRuns : 0);
                 }
                 const double pi0 = pp.Pi[3 * ip], pi1 = pp.Pi[3 * ip + 1], pi2 = pp.Pi[3 * ip + 2];
                 const double qi0 = pp.Pi[3 * iq], qi1 = pp.Pi[3 * iq + 1], qi2 = pp.Pi[3 * iq + 2];

@@ -9,10 +9,10 @@
 // warp takes a work unit of consecutive shell quartets with about as many
 // surviving primitive quartets as any other (units cut on the device,
 // gx_dense.cu) and walks them in full batches of 32 (gx_stream.cuh); the lanes'
-// values go through shared memory, where every output element's entries are
-// added one after the other.  Against a segmented shuffle sum (ten FP64
-// instructions per element and batch) that costs two per 32 additions, and the
-// result does not depend on the batches.  Batches both of whose pairs have
+// values go through shared memory, where a lane adds the entries of an output
+// element in stream order.  Against a segmented shuffle sum (ten FP64
+// instructions per element and batch) that costs about two per 32 additions,
+// and the result does not depend on the batches.  Batches both of whose pairs have
 // q = 0 (zero field, shells on one centre) run in real arithmetic.
 #pragma once
 
@@ -302,20 +302,20 @@ __device__ __forceinline__ void run_b_real(double* out, const double* W, const d
 constexpr int kWarps = 4;  // warps of a block, each with its own work unit
 
 // Shared memory of a warp: the values of a batch (33 columns: free of bank
-// conflicts both ways), the runs of lanes with one shell quartet, and the
+// conflicts both ways), the segments (lanes with one shell quartet), and the
 // queue of FP32 entries that wait for a full batch.
 template <int NOUT>
 struct WarpBuffers {
     double2 v[NOUT * 33];
     long long seg_off[32];
     int4 seg_st[32];
-    int seg_lane[36];  // first lane of each run (bit 8: its first FP64 entry, store instead of adding), and the end
+    int seg_lane[36];  // first lane and flags of each segment, and the end
     int2 queue[64];    // task, bra pair << 16 | ket pair
 };
 
-// Notes the runs of lanes with one shell quartet; returns their number.
+// Notes the segments; flags: those of the lane's task.  Returns their number.
 template <int NOUT>
-__device__ __forceinline__ int segments(WarpBuffers<NOUT>& w, const QuartetClass& qc, int task, bool first, int nb,
+__device__ __forceinline__ int segments(WarpBuffers<NOUT>& w, const QuartetClass& qc, int task, int flags, int nb,
                                         int lane) {
     const int tp = __shfl_up_sync(0xffffffffu, task, 1);
     const bool head = lane < nb && (lane == 0 || tp != task);
@@ -326,16 +326,17 @@ __device__ __forceinline__ int segments(WarpBuffers<NOUT>& w, const QuartetClass
         const Task* t = qc.tasks + task;
         w.seg_off[s] = t->out_off;
         w.seg_st[s] = make_int4(t->st[0], t->st[1], t->st[2], t->st[3]);
-        w.seg_lane[s] = lane | (first ? 256 : 0);
+        w.seg_lane[s] = lane | flags;
     }
     if (lane == 0) w.seg_lane[nseg] = nb;
     return nseg;
 }
 
-// Adds the buffered values of every run to its block, one entry after the
-// other in stream order: the result does not depend on how the stream was cut
-// into batches.  REAL: the imaginary parts are zero.
-template <int LA, int LB, int LC, int LD, bool REAL>
+// Adds the buffered values of every shell quartet's lanes to its block in
+// stream order: the result does not depend on how the stream was cut into
+// batches.  kReal: the imaginary parts are zero.
+enum AddMode { kReal, kComplex, kFP32 };
+template <int LA, int LB, int LC, int LD, AddMode MODE>
 __device__ __forceinline__ void add_runs(double2* out, const WarpBuffers<nc(LA) * nc(LB) * nc(LC) * nc(LD)>& w, int nseg,
                                          int lane) {
     constexpr int NCD = nc(LC) * nc(LD), NOUT = nc(LA) * nc(LB) * NCD, NCB = nc(LB), NCDD = nc(LD);
@@ -346,27 +347,22 @@ __device__ __forceinline__ void add_runs(double2* out, const WarpBuffers<nc(LA) 
         double2* p = out + w.seg_off[s] + (long long)(ab / NCB) * st.x + (long long)(ab % NCB) * st.y +
                      (long long)(cd / NCDD) * st.z + (long long)(cd % NCDD) * st.w;
         const double2* v = w.v + o * 33;
-        const bool store = w.seg_lane[s] & 256;
-        int l = w.seg_lane[s] & 255;
-        const int l1 = w.seg_lane[s + 1] & 255;
-        if constexpr (REAL) {
-            double sum;
-            if (store)
-                sum = v[l++].x;
-            else
-                sum = p->x;
-            for (; l < l1; ++l) sum += v[l].x;
+        const int flags = w.seg_lane[s], l0 = flags & 255, l1 = w.seg_lane[s + 1] & 255;
+        const bool store = flags & kStore;
+        if constexpr (MODE == kReal) {
+            const double old = store ? 0.0 : p->x;
+            const double sum = add_by_runs(old, flags, l0, l1, [&](int k) { return v[k].x; });
             if (store)
                 *p = c2(sum, 0.0);
             else
                 p->x = sum;
+        } else if constexpr (MODE == kComplex) {
+            const double2 old = store ? c2(0.0, 0.0) : *p;
+            *p = add_by_runs(old, flags, l0, l1, [&](int k) { return v[k]; });
         } else {
-            double2 sum;
-            if (store)
-                sum = v[l++];
-            else
-                sum = *p;
-            for (; l < l1; ++l) sum = cadd(sum, v[l]);
+            // (FP32 values: their passes cut the stream where the Boys paths part)
+            double2 sum = *p;
+            for (int l = l0; l < l1; ++l) sum = cadd(sum, v[l]);
             *p = sum;
         }
     }
@@ -424,7 +420,8 @@ __global__ void __launch_bounds__(32 * kWarps) small_kernel(EriDev d, QuartetCla
             int2 pq;
             const int nb = stream.next(lane, task, rank, pq);
             if (nb == 0) break;
-            const int nseg = segments<NOUT>(w, qc, task, rank == 0, nb, lane);
+            const int nseg = segments<NOUT>(
+                w, qc, task, (rank == 0 ? kStore : 0) | (stream.run == 32 ? kLongRuns : 0), nb, lane);
             const bool real = stream.batch_kind == 3;
             if (lane < nb) {
                 const Task* tg = qc.tasks + task;
@@ -486,9 +483,9 @@ __global__ void __launch_bounds__(32 * kWarps) small_kernel(EriDev d, QuartetCla
             }
             __syncwarp();
             if (real)
-                add_runs<LA, LB, LC, LD, true>(d.out, w, nseg, lane);
+                add_runs<LA, LB, LC, LD, kReal>(d.out, w, nseg, lane);
             else
-                add_runs<LA, LB, LC, LD, false>(d.out, w, nseg, lane);
+                add_runs<LA, LB, LC, LD, kComplex>(d.out, w, nseg, lane);
             __syncwarp();
         }
     }
@@ -523,7 +520,7 @@ __global__ void __launch_bounds__(32 * kWarps) small_kernel(EriDev d, QuartetCla
             __syncwarp();
             if (lane < waiting - nb) w.queue[lane] = rest;
             waiting -= nb;
-            const int nseg = segments<NOUT>(w, qc, en.x, false, nb, lane);
+            const int nseg = segments<NOUT>(w, qc, en.x, 0, nb, lane);
             if (lane < nb) {
                 const Task* tg = qc.tasks + en.x;
                 const int ip = pp.order[tg->pab + (int)((unsigned)en.y >> 16)], iq = pp.order[tg->pcd + (en.y & 0xffff)];
@@ -579,7 +576,7 @@ __global__ void __launch_bounds__(32 * kWarps) small_kernel(EriDev d, QuartetCla
                 }
             }
             __syncwarp();
-            add_runs<LA, LB, LC, LD, false>(d.out, w, nseg, lane);
+            add_runs<LA, LB, LC, LD, kFP32>(d.out, w, nseg, lane);
             __syncwarp();
         }
     }

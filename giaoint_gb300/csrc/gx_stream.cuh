@@ -7,6 +7,9 @@
 
 namespace gx {
 
+__device__ __forceinline__ double plus(double a, double b) { return a + b; }
+__device__ __forceinline__ double2 plus(double2 a, double2 b) { return cadd(a, b); }
+
 // Number of primitive quartets of a task with lo <= B_P B_Q < hi (FP32
 // products of the sorted factors, so that for every bra pair they are a run of
 // ket pairs whose ends move down as the bra pair's factor decreases).
@@ -115,6 +118,13 @@ __device__ __forceinline__ void cut_units(const EriDev& d, const QuartetClass& q
     }
 }
 
+// A task's FP64 values are summed in runs of entries, and the run sums one
+// after the other, so that the rounding of a deep contraction grows with the
+// number of runs; batches never split a run, so the sums do not depend on how
+// the stream is cut into batches.  Runs of 8 cost a batch two lanes on average;
+// a task of 256 entries or more has room for runs of 32.
+__device__ __forceinline__ int run_length(int survivors) { return survivors >= 256 ? 32 : 8; }
+
 // The surviving primitive quartets of the tasks t0 .. t1 - 1 in stream order
 // (task, bra pair, ket pair), up to 32 at a time, one per lane.  32 tasks are
 // looked at together: their survivor counts as an inclusive prefix over the
@@ -127,6 +137,7 @@ struct Stream {
     const QuartetClass& qc;
     float lo, hi;
     int t1, next_task, chunk = 0, incl = 0, cnt = 0, kind = 0, total = 0, used = 0, batch_kind = 0;
+    int run = 8;  // run length of the lane's task
 
     __device__ __forceinline__ Stream(const EriDev& dev, const QuartetClass& cls, int first, int last)
         : d(dev), qc(cls), t1(last), next_task(first) {
@@ -183,7 +194,22 @@ struct Stream {
                 const int stop = __shfl_sync(0xffffffffu, incl - cnt, other ? __ffs(other) - 1 : 31);
                 if (other) end = stop;
             }
-            const int take = min(32 - got, end - used);
+            int take = min(32 - got, end - used);
+            bool full = false;
+            if constexpr (!F32) {
+                // a batch that ends within a task ends after a whole run
+                if (used + take < end) {
+                    int at = 0;
+#pragma unroll
+                    for (int h = 16; h > 0; h >>= 1) {
+                        const int v = __shfl_sync(0xffffffffu, incl, at + h - 1);
+                        if (v <= used + take) at += h;
+                    }
+                    const int out = used + take - __shfl_sync(0xffffffffu, incl - cnt, at);
+                    take -= out % run_length(__shfl_sync(0xffffffffu, cnt, at));
+                    full = true;
+                }
+            }
             const int e = used + lane - got;
             int src = 0;
 #pragma unroll
@@ -192,12 +218,15 @@ struct Stream {
                 if (v <= e) src += h;
             }
             const int before = __shfl_sync(0xffffffffu, incl - cnt, src & 31);
+            const int whole = __shfl_sync(0xffffffffu, cnt, src & 31);
             if (lane >= got && lane < got + take) {
                 task = chunk + src;
                 rank = e - before;
+                run = run_length(whole);
             }
             used += take;
             got += take;
+            if (full) break;
         }
         if (lane < got) {
             const Task* tg = qc.tasks + task;
@@ -207,6 +236,26 @@ struct Stream {
         return got;
     }
 };
+
+// Flags of a batch's segment beside its first lane: the batch holds the shell
+// quartet's first FP64 entry, which stores instead of adding; long runs.
+constexpr int kStore = 256, kLongRuns = 512;
+
+// A segment's values v(l0) .. v(l1 - 1) by runs, added to sum (or, with
+// kStore, in its place).
+template <typename T, typename Get>
+__device__ __forceinline__ T add_by_runs(T sum, int flags, int l0, int l1, Get&& v) {
+    const int run = flags & kLongRuns ? 32 : 8;
+    bool fresh = flags & kStore;
+    for (int l = l0; l < l1; l += run) {
+        T part = v(l);
+        const int end = l + run < l1 ? l + run : l1;
+        for (int k = l + 1; k < end; ++k) part = plus(part, v(k));
+        sum = fresh ? part : plus(sum, part);
+        fresh = false;
+    }
+    return sum;
+}
 
 // v 2^shift as a double by integer work (a conversion is an FP64 instruction);
 // results below the normal range become zero.
