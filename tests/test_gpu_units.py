@@ -114,3 +114,18 @@ def test_equal_schwarz_factors(oracle):
     merged = [syn.ShellRecord(r.center, r.angular_momentum, (0.8, 1.7), ((1.2, 1.2),)) for r in recs]
     ref, _ = oracle.eri_batch(merged, q, B, None, 8)
     assert np.abs(values - ref).max() <= 1e-12
+
+
+@pytest.mark.parametrize("nuclei", [1, 31, 33, 70])
+@pytest.mark.parametrize("B", [(0.0, 0.0, 0.0), (0.1, -0.2, 0.15)])
+def test_nuclear_batches(nuclei, B, oracle):
+    """Nuclear attraction with lanes that hold (primitive pair, nucleus): fewer
+    nuclei than lanes, more, and shells on both sides of the table limit
+    (la + lb <= 8).  Tolerance: that of the reference comparison."""
+    recs = _records(17, ls=(0, 1, 2, 3, 5, 4), nprims=(5, 3, 2, 1, 1, 1), centers=(0, 0, 1, 2, 1, 2))
+    basis = basis_from_records(recs)
+    rng = np.random.default_rng(nuclei)
+    nucs = [(float(rng.integers(1, 9)), tuple(map(float, rng.uniform(-2.0, 4.0, 3)))) for _ in range(nuclei)]
+    got = gi.nuclear_attraction(basis, [gi.Nucleus(z, c) for z, c in nucs], field=gi.MagneticField(B))
+    ref = oracle.nuclear(recs, nucs, B, None)
+    np.testing.assert_allclose(got, ref, rtol=1e-12, atol=1e-12 * np.abs(ref).max())
