@@ -138,16 +138,19 @@ __host__ __device__ inline Layout layout(int NH, int NAB, int ncdh, int etot_ket
 // order L, in place: level by level, and within a level degree by degree from
 // the top, whose entries only read lower degrees of the previous level and are
 // shared by the block's warps.  seeds: [L + 1] seeds and X'[3] of every lane.
+// (seeds, col: of the lane's entry; part, parts: its share of every degree, over
+// the block's warps and the lanes that share the entry.)
 template <typename T>
-__device__ __forceinline__ void recurrence(const int2* __restrict__ plan, int L, const T* seeds, T* col, int warp) {
+__device__ __forceinline__ void recurrence(const int2* __restrict__ plan, int L, const T* seeds, T* col, int part,
+                                           int parts) {
     const T X0 = seeds[(L + 1) * 32], X1 = seeds[(L + 2) * 32], X2 = seeds[(L + 3) * 32];
-    if (warp == 0) col[0] = seeds[L * 32];
+    if (part == 0) col[0] = seeds[L * 32];
     int pos = 0;
     for (int n = L - 1; n >= 0; --n) {
         __syncthreads();
         for (int dg = L - n; dg >= 1; --dg) {
             const int cnt = (dg + 1) * (dg + 2) / 2;
-            for (int i = warp; i < cnt; i += kWarps) {
+            for (int i = part; i < cnt; i += parts) {
                 const int2 st = __ldg(&plan[pos + i]);
                 const int dst = st.x & 0xffff, s1 = (st.x >> 16) & 0xffff;
                 const int s2 = st.y & 0x3fff, axis = (st.y >> 14) & 3, coef = (st.y >> 16) & 63;
@@ -159,7 +162,7 @@ __device__ __forceinline__ void recurrence(const int2* __restrict__ plan, int L,
             pos += cnt;
             __syncthreads();
         }
-        if (warp == 0) col[0] = seeds[n * 32];
+        if (part == 0) col[0] = seeds[n * 32];
         ++pos;  // (the list's seed step)
     }
     __syncthreads();
@@ -216,28 +219,32 @@ struct Out {
     const int4* seg_st;         // its strides: template a, b, other c, d
     const int* shift;           // FP32: per lane, the power of two that undoes its seed scale
     const int* seg_lane;        // first lane and flags of each segment, and the end
-    int nseg, ndd, lane;
+    int nseg, cbegin, cend, ndd, lane;  // (components of this block)
+    int width, parts;           // lanes of an entry set, and how many sets (with their own components) fill the warp
     bool inner_c;               // the other side's components are the inner ones of the block
 };
 
 // The lanes of each segment over the value buffer (components ab0 .. of the
-// other side's components c .. c + cg - 1), added to its block in stream order
+// other side's components c .. c + cg - 1 of lane set 0, the following groups of
+// `stride` components of the other sets), added to its block in stream order
 // and in FP64: the result depends neither on where the batches of a unit begin
 // or end, nor on what else they hold.
 template <int LB, typename RT>
-__device__ __forceinline__ void reduce_out(const Out& o, const RT* vb, int ab0, int nab, int c, int cg) {
+__device__ __forceinline__ void reduce_out(const Out& o, const RT* vb, int ab0, int nab, int c, int cg, int stride) {
     constexpr int NCB = nc(LB);
-    const int per = nab * cg;
+    const int one = nab * cg, per = one * o.parts;
     for (int it = o.lane; it < o.nseg * per; it += 32) {
-        const int s = it / per, m = it - s * per;
+        const int s = it / per, rest = it - s * per;
+        const int set = rest / one, m = rest - set * one;
         // neighbouring lanes take neighbouring elements of the block
         const int i = o.inner_c ? m / cg : m % nab, u = o.inner_c ? m - i * cg : m / nab;
-        const int ab = ab0 + i;
-        const int cc = (c + u) / o.ndd, cdd = (c + u) - cc * o.ndd;
+        const int ab = ab0 + i, cx = c + set * stride + u;
+        if (cx >= o.cend) continue;
+        const int cc = cx / o.ndd, cdd = cx - cc * o.ndd;
         const int4 st = o.seg_st[s];
         double2* p = o.out + o.seg_off[s] + (long long)(ab / NCB) * st.x + (long long)(ab % NCB) * st.y +
                      (long long)cc * st.z + (long long)cdd * st.w;
-        const RT* v = vb + (u * nab + i) * 33;
+        const RT* v = vb + (u * nab + i) * 33 + set * o.width;
         const int flags = o.seg_lane[s], l0 = flags & 255, l1 = o.seg_lane[s + 1] & 255;
         const bool store = flags & kStore;
         auto at = [&](int k) { return v[k]; };
@@ -278,41 +285,44 @@ __device__ __forceinline__ void slices(const Out& o, const RT* W, RT* vb, const 
             }
             if constexpr (group_of(nc(LA) * nc(LB)) == 1) {
                 __syncwarp();
-                reduce_out<LB, RT>(o, vb, S * SL, SL, c, 1);
+                reduce_out<LB, RT>(o, vb, S * SL, SL, c, 1, 1);
                 __syncwarp();
             }
         }(),
         ...);
 }
 
-// The component groups first, first + step, ... of one batch.
+// The component groups of one batch: sets of o.parts consecutive groups, dealt
+// out to the block's warps; each lane set takes one group of a set.
 template <int LA, int LB, typename RT, typename EP>
 __device__ __forceinline__ void transforms(const Out& o, const RT* R, RT* vb, const int* hsum, const int* kh,
                                            const int2* kb, const EP* Ek, const EP* Eb, bool ket_real, bool bra_real,
-                                           int first, int step, int ncd) {
+                                           int warp) {
     constexpr int NH = hc(LA + LB), NAB = nc(LA) * nc(LB), CG = group_of(NAB);
-    const RT* col = R + o.lane;
-    for (int c1 = first * CG; c1 < ncd; c1 += step * CG) {
-        const int cg = min(CG, ncd - c1);
+    const RT* col = R + (o.lane & (o.width - 1));
+    const int set = o.lane / o.width;
+    for (int c1 = o.cbegin + warp * o.parts * CG; c1 < o.cend; c1 += kWarps * o.parts * CG) {
+        const int cg = min(CG, o.cend - c1);
         for (int u = 0; u < cg; ++u) {
-            const int bo = kb[c1 + u].x, nbox = kb[c1 + u].y;
+            // (a set beyond the last component repeats it; it is not added)
+            const int2 box = kb[min(c1 + set * CG + u, o.cend - 1)];
             RT W[NH];
             if constexpr (std::is_same_v<RT, double>) {
-                ket<NH, double, RT>(W, col, Ek + bo, kh + bo, nbox, hsum);
+                ket<NH, double, RT>(W, col, Ek + box.x, kh + box.x, box.y, hsum);
             } else if constexpr (std::is_same_v<RT, double2>) {
                 if (ket_real)
-                    ket<NH, double, RT>(W, col, Ek + bo, kh + bo, nbox, hsum);
+                    ket<NH, double, RT>(W, col, Ek + box.x, kh + box.x, box.y, hsum);
                 else
-                    ket<NH, double2, RT>(W, col, Ek + bo, kh + bo, nbox, hsum);
+                    ket<NH, double2, RT>(W, col, Ek + box.x, kh + box.x, box.y, hsum);
             } else {
-                ket<NH, float2, RT>(W, col, Ek + bo, kh + bo, nbox, hsum);
+                ket<NH, float2, RT>(W, col, Ek + box.x, kh + box.x, box.y, hsum);
             }
-            slices<LA, LB, RT>(o, W, vb + u * NAB * 33, Eb, bra_real, c1 + u,
+            slices<LA, LB, RT>(o, W, vb + u * NAB * 33, Eb, bra_real, c1,
                                std::make_integer_sequence<int, NAB / slice_of(NAB)>{});
         }
         if constexpr (CG > 1) {
             __syncwarp();
-            reduce_out<LB, RT>(o, vb, 0, NAB, c1, cg);
+            reduce_out<LB, RT>(o, vb, 0, NAB, c1, cg, CG);
             __syncwarp();
         }
     }
@@ -427,8 +437,9 @@ __global__ void __launch_bounds__(32 * kWarps) dense_kernel(EriDev d, QuartetCla
         return make_int4(t->st[qc.axis & 3], t->st[(qc.axis >> 2) & 3], t->st[(qc.axis >> 4) & 3],
                          t->st[(qc.axis >> 6) & 3]);
     };
-    // component groups of this warp (of gridDim.y blocks that share a unit)
-    const int first = blockIdx.y * kWarps + warp, step = gridDim.y * kWarps;
+    // component groups of this block (of gridDim.y that share the unit)
+    const int groups = (ncd + CG - 1) / CG, share = (groups + gridDim.y - 1) / gridDim.y * CG;
+    const int cbegin = blockIdx.y * share, cend = min(ncd, cbegin + share);
     const int2* plan = d.rec_plan + d.rec_plan_off[L];
     const bool leader = warp == (int)(blockIdx.x % kWarps);
     unsigned count = 0;
@@ -564,25 +575,30 @@ __global__ void __launch_bounds__(32 * kWarps) dense_kernel(EriDev d, QuartetCla
         __syncthreads();
         if (info[0] == 0) break;
         const bool bra_real = info[2] & 1, ket_real = info[2] & 2;
-        const Out o{d.out, seg_off, seg_st, s_shift, seg_lane, info[1], ndd, lane, !qc.swap};
+        // a batch of at most 16 entries is repeated over the lanes, and the
+        // sets of lanes share the recurrence and the components
+        int width = 32;
+        while (width > 1 && info[0] <= width / 2) width /= 2;
+        const Out o{d.out, seg_off, seg_st,  s_shift, seg_lane,   info[1],
+                    cbegin, cend,  ndd,     lane,    width,      32 / width, !qc.swap};
+        const int ent = lane & (width - 1), part = warp * o.parts + lane / width, parts = kWarps * o.parts;
         if constexpr (F32) {
-            recurrence<float2>(plan, L, reinterpret_cast<const float2*>(seeds) + lane,
-                               reinterpret_cast<float2*>(R) + lane, warp);
+            recurrence<float2>(plan, L, reinterpret_cast<const float2*>(seeds) + ent,
+                               reinterpret_cast<float2*>(R) + ent, part, parts);
             transforms<LA, LB, float2>(o, reinterpret_cast<const float2*>(R), reinterpret_cast<float2*>(vb), hsum, kh,
-                                       kb, pp.Epool32 + s_ek[lane], pp.Epool32 + s_eb[lane], false, false, first, step,
-                                       ncd);
+                                       kb, pp.Epool32 + s_ek[ent], pp.Epool32 + s_eb[ent], false, false, warp);
         } else {
-            const double2 *Ek = pp.Epool + s_ek[lane], *Eb = pp.Epool + s_eb[lane];
+            const double2 *Ek = pp.Epool + s_ek[ent], *Eb = pp.Epool + s_eb[ent];
             if (bra_real && ket_real) {
-                recurrence<double>(plan, L, reinterpret_cast<const double*>(seeds) + lane,
-                                   reinterpret_cast<double*>(R) + lane, warp);
+                recurrence<double>(plan, L, reinterpret_cast<const double*>(seeds) + ent,
+                                   reinterpret_cast<double*>(R) + ent, part, parts);
                 transforms<LA, LB, double>(o, reinterpret_cast<const double*>(R), reinterpret_cast<double*>(vb), hsum,
-                                           kh, kb, Ek, Eb, true, true, first, step, ncd);
+                                           kh, kb, Ek, Eb, true, true, warp);
             } else {
-                recurrence<double2>(plan, L, reinterpret_cast<const double2*>(seeds) + lane,
-                                    reinterpret_cast<double2*>(R) + lane, warp);
+                recurrence<double2>(plan, L, reinterpret_cast<const double2*>(seeds) + ent,
+                                    reinterpret_cast<double2*>(R) + ent, part, parts);
                 transforms<LA, LB, double2>(o, reinterpret_cast<const double2*>(R), reinterpret_cast<double2*>(vb),
-                                            hsum, kh, kb, Ek, Eb, ket_real, bra_real, first, step, ncd);
+                                            hsum, kh, kb, Ek, Eb, ket_real, bra_real, warp);
             }
         }
         __syncthreads();  // the next batch overwrites the table
