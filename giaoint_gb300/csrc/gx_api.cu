@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <array>
 #include <chrono>
+#include <functional>
 #include <limits>
 #include <cmath>
 #include <complex>
@@ -1103,6 +1104,48 @@ gx::EriDev make_dev(gx_context* ctx, gx_basis* b, FieldPairs& fp, double2* out, 
     return dev;
 }
 
+// Small or lane-dense class ci as its kernels take it (a lane-dense one not
+// yet oriented).
+gx::QuartetClass unit_class(gx_context* ctx, const PlanData& plan, size_t ci, unsigned long long* counters) {
+    const auto& pc = plan.classes[ci];
+    const auto& k = pc.key;
+    gx::QuartetClass qc{};
+    qc.L = k[0] + k[1] + k[2] + k[3];
+    qc.ntask = (int)pc.count;
+    qc.tasks = plan.tasks.as<gx::Task>() + pc.first;
+    qc.counters = counters ? counters + 2 * ci : nullptr;
+    qc.ngroup = plan.unit_grid[ci];
+    qc.target = plan.unit_target[ci];
+    qc.dims = plan.unit_dims[ci];
+    if (plan.unit_class[ci] >= 0) {
+        const gx::UnitClass& uc = plan.unit_first[plan.unit_class[ci]];
+        qc.unit_start = plan.units.start + uc.base;
+        qc.unit_count = plan.units.count + uc.vfirst;
+    }
+    if (plan.unit_class32[ci] >= 0) {
+        const gx::UnitClass& u32 = plan.unit_first[plan.unit_class32[ci]];
+        qc.unit_start32 = plan.units.start + u32.base;
+        qc.unit_count32 = plan.units.count + u32.vfirst;
+    }
+    qc.nchunk = 1;
+    if (gx::small_class(k[0], k[1], k[2], k[3])) return qc;
+    qc.bra = ctx->pair_class(k[0], k[1]).dev();
+    qc.ket = ctx->pair_class(k[2], k[3]).dev();
+    // few entries: the blocks of a unit share its components (about one in
+    // four primitive quartets of a small plan survives)
+    const int units = (int)(pc.primitive_quartets / 128) + 1, fill = std::max(ctx->sm_count, 1);
+    qc.nchunk = gx::dense_chunks(k[0], k[1], k[2], k[3], (fill + units - 1) / units, pc.primitive_quartets <= 32);
+    return qc;
+}
+
+// Lane-dense classes of one template pair; in mixed precision their FP32
+// entries are added after the FP64 ones.
+void launch_dense_classes(int pair, const gx::EriDev& dev, const std::vector<gx::QuartetClass>& classes,
+                          cudaStream_t s) {
+    GX_CUDA(gx::launch_dense(pair, dev, classes, false, s));
+    if (dev.fp32_cut > 0.0f) GX_CUDA(gx::launch_dense(pair, dev, classes, true, s));
+}
+
 // Enqueue the kernel of class ci with configuration conf and work units
 // groups[0..ngroup).  Returns the (batch, warps per block) used through the
 // optional pointers.
@@ -1112,45 +1155,23 @@ void launch_class(gx_context* ctx, gx::EriDev dev, const PlanData& plan, size_t 
     const auto& pc = plan.classes[ci];
     const auto& k = pc.key;
     dev.counters = counters ? counters + 2 * ci : nullptr;
+    const bool small = gx::small_class(k[0], k[1], k[2], k[3]);
+    if (small || runs_dense(pc, conf)) {
+        gx::QuartetClass uc = unit_class(ctx, plan, ci, counters);
+        if (small) {
+            GX_CUDA(gx::launch_small(k[0], k[1], k[2], k[3], dev, uc, s));
+        } else {
+            const int pair = gx::dense_orient(k[0], k[1], k[2], k[3], uc);
+            launch_dense_classes(pair, dev, {uc}, s);
+        }
+        if (used_b1) *used_b1 = 32;
+        if (used_wpb) *used_wpb = 4;
+        return;
+    }
     gx::QuartetClass qc{};
     qc.L = k[0] + k[1] + k[2] + k[3];
     qc.ntask = (int)pc.count;
     qc.tasks = plan.tasks.as<gx::Task>() + pc.first;
-    const bool small = gx::small_class(k[0], k[1], k[2], k[3]);
-    if (small || runs_dense(pc, conf)) {
-        qc.ngroup = plan.unit_grid[ci];
-        qc.target = plan.unit_target[ci];
-        qc.dims = plan.unit_dims[ci];
-        if (plan.unit_class[ci] >= 0) {
-            const gx::UnitClass& uc = plan.unit_first[plan.unit_class[ci]];
-            qc.unit_start = plan.units.start + uc.base;
-            qc.unit_count = plan.units.count + uc.vfirst;
-        }
-        if (used_b1) *used_b1 = 32;
-        if (used_wpb) *used_wpb = 4;
-        if (small) {
-            GX_CUDA(gx::launch_small(k[0], k[1], k[2], k[3], dev, qc, s));
-            return;
-        }
-        qc.bra = ctx->pair_class(k[0], k[1]).dev();
-        qc.ket = ctx->pair_class(k[2], k[3]).dev();
-        qc.NL = gx::herm_count(qc.L);
-        // few entries: the blocks of a unit share its components (about one in
-        // four primitive quartets of a small plan survives)
-        const int units = (int)(pc.primitive_quartets / 128) + 1, fill = std::max(ctx->sm_count, 1);
-        qc.nchunk = gx::dense_chunks(k[0], k[1], k[2], k[3], (fill + units - 1) / units, pc.primitive_quartets <= 32);
-        GX_CUDA(gx::launch_dense(k[0], k[1], k[2], k[3], dev, qc, false, s));
-        // mixed precision: the FP32 entries are added after the FP64 ones
-        if (dev.fp32_cut > 0.0f) {
-            if (plan.unit_class32[ci] >= 0) {
-                const gx::UnitClass& u32 = plan.unit_first[plan.unit_class32[ci]];
-                qc.unit_start32 = plan.units.start + u32.base;
-                qc.unit_count32 = plan.units.count + u32.vfirst;
-            }
-            GX_CUDA(gx::launch_dense(k[0], k[1], k[2], k[3], dev, qc, true, s));
-        }
-        return;
-    }
     qc.bra = ctx->pair_class(k[0], k[1]).dev();
     qc.ket = ctx->pair_class(k[2], k[3]).dev();
     qc.Nab = gx::herm_count(k[0] + k[1]);
@@ -1245,6 +1266,73 @@ void launch_class(gx_context* ctx, gx::EriDev dev, const PlanData& plan, size_t 
     }
 }
 
+// One launch of a plan: its classes, and the function that enqueues it.
+struct PlanLaunch {
+    std::vector<size_t> classes;
+    std::function<void(cudaStream_t)> enqueue;
+};
+
+// The launches of one plan (`dev` and `plan` outlive them).  Small and lane-dense classes with few primitive
+// quartets share launches -- the small ones one, the lane-dense ones one per
+// template pair -- because a plan of them is bound by the launches (the 36
+// classes of a 19-function atom: 0.41 ms with a launch each, of which the device
+// was busy 0.26).  Classes above the limit keep their own, and a plan above a
+// limit shares launches among classes of one total order only: a launch carries
+// the shared memory of its largest class (by template pair alone the gradient
+// of three atoms took 29.1 ms instead of 27.7).
+constexpr int64_t kSharedLaunch = 4096, kSharedPlan = 65536;
+
+std::vector<PlanLaunch> plan_launches(gx_context* ctx, const gx::EriDev& dev, const PlanData& plan, int precision,
+                                      unsigned long long* counters) {
+    std::vector<PlanLaunch> out;
+    const auto& tuned = plan.tuned[precision];
+    const GroupSet& gs = tuned.valid ? tuned.groups : plan.base;
+    const size_t nc = plan.classes.size();
+    std::map<int, std::vector<size_t>> shared;  // by (order and) template pair; small classes at -1
+    std::vector<size_t> own;
+    for (size_t oi = 0; oi < nc; ++oi) {
+        const size_t ci = plan.order.empty() ? oi : (size_t)plan.order[oi];
+        const PlanClass& pc = plan.classes[ci];
+        const auto& k = pc.key;
+        const ClassConf& conf = tuned.valid ? tuned.conf[ci] : plan.defconf[ci];
+        const bool small = gx::small_class(k[0], k[1], k[2], k[3]);
+        if ((small || runs_dense(pc, conf)) && pc.primitive_quartets <= kSharedLaunch) {
+            gx::QuartetClass qc{};
+            const int L = k[0] + k[1] + k[2] + k[3];
+            const int by_order = plan.primitive_quartets > kSharedPlan ? L : 0;
+            shared[small ? -1 : by_order * 16 + gx::dense_orient(k[0], k[1], k[2], k[3], qc)].push_back(ci);
+        } else {
+            own.push_back(ci);
+        }
+    }
+    // (the higher template pairs first: theirs are the longest blocks)
+    for (auto it = shared.rbegin(); it != shared.rend(); ++it) {
+        const int pair = it->first < 0 ? -1 : it->first % 16;
+        const std::vector<size_t> cs = it->second;
+        out.push_back({cs, [=, &dev, &plan](cudaStream_t s) {
+            std::vector<gx::QuartetClass> classes;
+            std::vector<int> keys;
+            for (size_t ci : cs) {
+                const auto& k = plan.classes[ci].key;
+                gx::QuartetClass qc = unit_class(ctx, plan, ci, counters);
+                if (pair >= 0) gx::dense_orient(k[0], k[1], k[2], k[3], qc);
+                classes.push_back(qc);
+                keys.push_back(((k[0] * 3 + k[1]) * 3 + k[2]) * 3 + k[3]);
+            }
+            if (pair < 0)
+                GX_CUDA(gx::launch_small_list(dev, keys, classes, s));
+            else
+                launch_dense_classes(pair, dev, classes, s);
+        }});
+    }
+    for (size_t ci : own)
+        out.push_back({{ci}, [=, &dev, &plan, &tuned, &gs](cudaStream_t s) {
+            launch_class(ctx, dev, plan, ci, tuned.valid ? tuned.conf[ci] : plan.defconf[ci],
+                         gs.dev.as<int2>() + gs.range[ci].first, (int)gs.range[ci].second, counters, s);
+        }});
+    return out;
+}
+
 // Enqueue the pair records for (B, O) and every class launch; no host sync
 // unless the field changed (the pair bounds are sorted on the host).  Uses
 // the autotuned configuration of the precision mode when there is one.
@@ -1299,16 +1387,14 @@ int enqueue_plan(gx_context* ctx, const gx::EriDev& dev, const PlanData& plan, i
     if (counters && !accumulate) GX_CUDA(cudaMemsetAsync(counters, 0, 2 * plan.classes.size() * sizeof(unsigned long long), s));
     ctx->reset_status();
     GX_CUDA(gx::launch_units(plan.units, plan.tasks.as<gx::Task>(), dev, s));
-    const auto& tuned = plan.tuned[precision];
-    const GroupSet& gs = tuned.valid ? tuned.groups : plan.base;
-    const size_t nc = plan.classes.size();
+    const std::vector<PlanLaunch> launches = plan_launches(ctx, dev, plan, precision, counters);
     // The classes write disjoint output blocks, so they run concurrently on
     // the auxiliary streams: a plan of many small classes (a Cholesky column
     // batch) costs about its longest class instead of the sum, and the tails
     // of large classes overlap.  Under stream capture this becomes parallel
     // graph branches.
     constexpr int kAux = 32;
-    const int K = (int)std::min<size_t>(nc, kAux);
+    const int K = (int)std::min<size_t>(launches.size(), kAux);
     if (K > 1) {
         if (ctx->aux.empty()) {
             ctx->aux.resize(kAux);
@@ -1321,28 +1407,19 @@ int enqueue_plan(gx_context* ctx, const gx::EriDev& dev, const PlanData& plan, i
         }
         GX_CUDA(cudaEventRecord(ctx->fork, s));
         for (int k = 0; k < K; ++k) GX_CUDA(cudaStreamWaitEvent(ctx->aux[k], ctx->fork, 0));
-        for (size_t oi = 0; oi < nc; ++oi) {
-            const size_t ci = plan.order.empty() ? oi : (size_t)plan.order[oi];
-            launch_class(ctx, dev, plan, ci, tuned.valid ? tuned.conf[ci] : plan.defconf[ci],
-                         gs.dev.as<int2>() + gs.range[ci].first, (int)gs.range[ci].second, counters,
-                         ctx->aux[oi % K], nullptr, nullptr, nullptr);
-            copy_class(ci, ctx->aux[oi % K]);
-        }
+    }
+    for (size_t i = 0; i < launches.size(); ++i) {
+        cudaStream_t to = K > 1 ? ctx->aux[i % K] : s;
+        launches[i].enqueue(to);
+        for (size_t ci : launches[i].classes) copy_class(ci, to);
+    }
+    if (K > 1)
         for (int k = 0; k < K; ++k) {
             GX_CUDA(cudaEventRecord(ctx->aux_done[k], ctx->aux[k]));
             GX_CUDA(cudaStreamWaitEvent(s, ctx->aux_done[k], 0));
         }
-        join_copies();
-    } else {
-        for (size_t ci = 0; ci < nc; ++ci) {
-            launch_class(ctx, dev, plan, ci, tuned.valid ? tuned.conf[ci] : plan.defconf[ci],
-                         gs.dev.as<int2>() + gs.range[ci].first, (int)gs.range[ci].second, counters, s, nullptr,
-                         nullptr, nullptr);
-            copy_class(ci, s);
-        }
-        join_copies();
-    }
-    return 1 + (int)nc;
+    join_copies();
+    return 1 + (int)launches.size();
 }
 
 // Enqueue several plans (each with its own evaluation view and counters,
@@ -1363,21 +1440,15 @@ void enqueue_plans(gx_context* ctx, const std::vector<std::pair<const PlanData*,
         GX_CUDA(cudaEventCreateWithFlags(&ctx->fork, cudaEventDisableTiming));
     }
     for (const auto& r : runs) GX_CUDA(gx::launch_units(r.first->units, r.first->tasks.as<gx::Task>(), r.second, s));
+    std::vector<PlanLaunch> launches;
+    for (size_t r = 0; r < runs.size(); ++r)
+        for (PlanLaunch& l : plan_launches(ctx, runs[r].second, *runs[r].first, precision, counters[r]))
+            launches.push_back(std::move(l));
+    const int K = (int)std::min<size_t>(launches.size(), kAux);
     GX_CUDA(cudaEventRecord(ctx->fork, s));
-    for (int k = 0; k < kAux; ++k) GX_CUDA(cudaStreamWaitEvent(ctx->aux[k], ctx->fork, 0));
-    int next = 0;
-    for (size_t r = 0; r < runs.size(); ++r) {
-        const PlanData& plan = *runs[r].first;
-        const auto& tuned = plan.tuned[precision];
-        const GroupSet& gs = tuned.valid ? tuned.groups : plan.base;
-        for (size_t oi = 0; oi < plan.classes.size(); ++oi, ++next) {
-            const size_t ci = plan.order.empty() ? oi : (size_t)plan.order[oi];
-            launch_class(ctx, runs[r].second, plan, ci, tuned.valid ? tuned.conf[ci] : plan.defconf[ci],
-                         gs.dev.as<int2>() + gs.range[ci].first, (int)gs.range[ci].second, counters[r],
-                         ctx->aux[next % kAux], nullptr, nullptr, nullptr);
-        }
-    }
-    for (int k = 0; k < kAux; ++k) {
+    for (int k = 0; k < K; ++k) GX_CUDA(cudaStreamWaitEvent(ctx->aux[k], ctx->fork, 0));
+    for (size_t i = 0; i < launches.size(); ++i) launches[i].enqueue(ctx->aux[i % K]);
+    for (int k = 0; k < K; ++k) {
         GX_CUDA(cudaEventRecord(ctx->aux_done[k], ctx->aux[k]));
         GX_CUDA(cudaStreamWaitEvent(s, ctx->aux_done[k], 0));
     }
@@ -1425,15 +1496,8 @@ void enqueue_parts_with_copies(gx_context* ctx, const gx::EriDev& dev, const Cac
     int next = 0;
     int64_t start = 0;
     for (size_t r = 0; r < cp.parts.size(); ++r) {
-        const PlanData& plan = *cp.parts[r];
-        const auto& tuned = plan.tuned[precision];
-        const GroupSet& gs = tuned.valid ? tuned.groups : plan.base;
-        for (size_t oi = 0; oi < plan.classes.size(); ++oi, ++next) {
-            const size_t ci = plan.order.empty() ? oi : (size_t)plan.order[oi];
-            launch_class(ctx, dev, plan, ci, tuned.valid ? tuned.conf[ci] : plan.defconf[ci],
-                         gs.dev.as<int2>() + gs.range[ci].first, (int)gs.range[ci].second, counters[r],
-                         ctx->aux[next % kAux], nullptr, nullptr, nullptr);
-        }
+        for (const PlanLaunch& l : plan_launches(ctx, dev, *cp.parts[r], precision, counters[r]))
+            l.enqueue(ctx->aux[next++ % kAux]);
         // a waited event stands for its latest record, so the events are reused per part
         for (int k = 0; k < kAux; ++k) {
             GX_CUDA(cudaEventRecord(ctx->aux_done[k], ctx->aux[k]));

@@ -3,14 +3,14 @@
 #include "gx_dense.cuh"
 
 #include <algorithm>
-#include <atomic>
+#include <cstdint>
 
 namespace gx {
 
 namespace {
 
 using dense::kMaxOrder;
-constexpr int kMaxSmem = 200 * 1024;
+using dense::kMaxSmem;
 
 // template pairs: (l, 0) runs as (0, l), whose components, boxes and Hermite
 // records are the same in the same order
@@ -49,20 +49,6 @@ int side_of(int la, int lb, int lc, int ld) {
     return work(la, lb, lc, ld) <= work(lc, ld, la, lb) ? 1 : 2;
 }
 
-template <int LA, int LB, bool F32>
-cudaError_t go(const EriDev& d, const QuartetClass& qc, int smem, cudaStream_t s) {
-    static std::atomic<bool> ready{false};
-    if (!ready.load(std::memory_order_acquire)) {
-        const cudaError_t e = cudaFuncSetAttribute(dense::dense_kernel<LA, LB, F32>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
-        if (e != cudaSuccess) return e;
-        ready.store(true, std::memory_order_release);
-    }
-    dense::dense_kernel<LA, LB, F32>
-        <<<dim3((unsigned)qc.ngroup, (unsigned)qc.nchunk), 32 * dense::kWarps, smem, s>>>(d, qc);
-    return cudaGetLastError();
-}
-
 }  // namespace
 
 bool dense_class(int la, int lb, int lc, int ld) { return side_of(la, lb, lc, ld) != 0; }
@@ -85,10 +71,8 @@ int dense_chunks(int la, int lb, int lc, int ld, int want, bool single) {
     return std::max(1, std::min(want, most));
 }
 
-cudaError_t launch_dense(int la, int lb, int lc, int ld, const EriDev& d, QuartetClass qc, bool f32, cudaStream_t s) {
-    if (qc.ntask <= 0 || qc.ngroup <= 0) return cudaSuccess;
+int dense_orient(int la, int lb, int lc, int ld, QuartetClass& qc) {
     const int side = side_of(la, lb, lc, ld);
-    if (side == 0) return cudaErrorInvalidValue;
     int a = 0, b = 1, c = 2, e = 3;  // task strides of the template and the other side
     if (side == 2) {
         std::swap(la, lc);
@@ -103,24 +87,35 @@ cudaError_t launch_dense(int la, int lb, int lc, int ld, const EriDev& d, Quarte
     }
     qc.swap = side == 2;
     qc.axis = a | b << 2 | c << 4 | e << 6;
-    const int smem = smem_bytes(la, lb, lc, ld, f32 || d.all_real ? 8 : 16);
-    switch (la * 4 + lb) {
-#define GX_CASE(A, B) \
-    case A * 4 + B: return f32 ? go<A, B, true>(d, qc, smem, s) : go<A, B, false>(d, qc, smem, s);
-        GX_CASE(0, 0)
-        GX_CASE(0, 1)
-        GX_CASE(0, 2)
-        GX_CASE(0, 3)
-        GX_CASE(1, 1)
-        GX_CASE(1, 2)
-        GX_CASE(2, 1)
-        GX_CASE(1, 3)
-        GX_CASE(3, 1)
-        GX_CASE(2, 2)
-#undef GX_CASE
-        default:
-            return cudaErrorInvalidValue;
+    return la * 4 + lb;
+}
+
+cudaError_t launch_dense(int pair, const EriDev& d, const std::vector<QuartetClass>& classes, bool f32, cudaStream_t s) {
+    const int la = pair / 4, lb = pair % 4;
+    dense::ClassList list;
+    for (size_t k = 0; k < classes.size();) {
+        list.n = 0;
+        list.first[0] = 0;
+        int smem = 0;
+        for (; k < classes.size() && list.n < dense::kMaxClasses; ++k) {
+            const QuartetClass& qc = classes[k];
+            const long long blocks = (long long)qc.ngroup * qc.nchunk;
+            if (qc.ntask <= 0 || blocks <= 0) continue;
+            if (list.n > 0 && list.first[list.n] + blocks > INT32_MAX) break;
+            list.cls[list.n] = qc;
+            list.first[list.n + 1] = (int)(list.first[list.n] + blocks);
+            ++list.n;
+            smem = std::max(smem, smem_bytes(la, lb, qc.ket.la, qc.ket.lb, f32 || d.all_real ? 8 : 16));
+        }
+        if (list.n == 0) continue;
+        cudaError_t e;
+        if (list.n == 1)
+            e = f32 ? dense::run_one_f32(pair, d, list.cls[0], smem, s) : dense::run_one_f64(pair, d, list.cls[0], smem, s);
+        else
+            e = f32 ? dense::run_list_f32(pair, d, list, smem, s) : dense::run_list_f64(pair, d, list, smem, s);
+        if (e != cudaSuccess) return e;
     }
+    return cudaSuccess;
 }
 
 // ---------------------------------------------------------------------------

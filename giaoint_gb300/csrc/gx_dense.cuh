@@ -40,6 +40,7 @@
 // asymptotic sector, seeds and every sum into the blocks in FP64), after the FP64 one on the same stream.
 #pragma once
 
+#include <atomic>
 #include <type_traits>
 #include <utility>
 
@@ -372,8 +373,19 @@ __device__ __forceinline__ Seeds32 seeds32_begin(const float2* x, double p, doub
     return s;
 }
 
+// The classes of one launch: all have the same template pair; block b works on
+// class c with first[c] <= b < first[c + 1], on unit (b - first[c]) / nchunk and
+// that unit's share (b - first[c]) % nchunk of the components.
+constexpr int kMaxClasses = 24;
+struct ClassList {
+    int n;
+    int first[kMaxClasses + 1];
+    QuartetClass cls[kMaxClasses];
+};
+
+// Unit `unit` of a class; share_of: which of the nchunk blocks that share it.
 template <int LA, int LB, bool F32>
-__global__ void __launch_bounds__(32 * kWarps) dense_kernel(EriDev d, QuartetClass qc) {
+__device__ __forceinline__ void dense_block(const EriDev& d, const QuartetClass& qc, int unit, int share_of) {
     constexpr int NH = hc(LA + LB), NHP = (NH + 3) / 4 * 4;
     constexpr int NAB = nc(LA) * nc(LB), NCB = nc(LB), CG = group_of(NAB);
     extern __shared__ double2 dsm[];
@@ -400,12 +412,12 @@ __global__ void __launch_bounds__(32 * kWarps) dense_kernel(EriDev d, QuartetCla
     const int* start = F32 ? qc.unit_start32 : qc.unit_start;
     int t0, t1;
     if (start) {
-        t0 = start[blockIdx.x];
-        t1 = min(start[blockIdx.x + 1], qc.ntask);
+        t0 = start[unit];
+        t1 = min(start[unit + 1], qc.ntask);
     } else {
         __shared__ int bounds[2];
         __shared__ long long sums[kWarps];
-        cut_units<32 * kWarps>(d, qc, F32 ? 1 : 0, blockIdx.x, 1, !F32 && blockIdx.y == 0, bounds, sums);
+        cut_units<32 * kWarps>(d, qc, F32 ? 1 : 0, unit, 1, !F32 && share_of == 0, bounds, sums);
         t0 = bounds[0];
         t1 = bounds[1];
     }
@@ -437,9 +449,9 @@ __global__ void __launch_bounds__(32 * kWarps) dense_kernel(EriDev d, QuartetCla
         return make_int4(t->st[qc.axis & 3], t->st[(qc.axis >> 2) & 3], t->st[(qc.axis >> 4) & 3],
                          t->st[(qc.axis >> 6) & 3]);
     };
-    // component groups of this block (of gridDim.y that share the unit)
-    const int groups = (ncd + CG - 1) / CG, share = (groups + gridDim.y - 1) / gridDim.y * CG;
-    const int cbegin = blockIdx.y * share, cend = min(ncd, cbegin + share);
+    // component groups of this block (of nchunk that share the unit)
+    const int groups = (ncd + CG - 1) / CG, share = (groups + qc.nchunk - 1) / qc.nchunk * CG;
+    const int cbegin = share_of * share, cend = min(ncd, cbegin + share);
     const int2* plan = d.rec_plan + d.rec_plan_off[L];
     const bool leader = warp == (int)(blockIdx.x % kWarps);
     unsigned count = 0;
@@ -485,7 +497,7 @@ __global__ void __launch_bounds__(32 * kWarps) dense_kernel(EriDev d, QuartetCla
                     info[1] = nseg;
                     info[2] = stream.batch_kind;
                 }
-                count += active && blockIdx.y == 0;
+                count += active && share_of == 0;
                 if (!F32 && bra_real && ket_real) {
                     const double rho = p * q * rs * rs;
                     const double t = rho * fma(x0, x0, fma(x1, x1, x2 * x2));
@@ -603,11 +615,61 @@ __global__ void __launch_bounds__(32 * kWarps) dense_kernel(EriDev d, QuartetCla
         }
         __syncthreads();  // the next batch overwrites the table
     }
-    if (d.counters && leader && blockIdx.y == 0) {
+    if (qc.counters && leader && share_of == 0) {
         const unsigned a = __reduce_add_sync(0xffffffffu, count);
-        if (lane == 0 && a) atomicAdd(&d.counters[F32 ? 1 : 0], (unsigned long long)a);
+        if (lane == 0 && a) atomicAdd(&qc.counters[F32 ? 1 : 0], (unsigned long long)a);
     }
 }
+
+template <int LA, int LB, bool F32>
+__global__ void __launch_bounds__(32 * kWarps) dense_kernel(const __grid_constant__ EriDev d,
+                                                            const __grid_constant__ QuartetClass qc) {
+    dense_block<LA, LB, F32>(d, qc, blockIdx.x, blockIdx.y);
+}
+
+// (reading the class through the list costs the FP64-bound plans 1.5%, so a
+// class with a launch of its own has the kernel above)
+template <int LA, int LB, bool F32>
+__global__ void __launch_bounds__(32 * kWarps) dense_list_kernel(const __grid_constant__ EriDev d,
+                                                                 const __grid_constant__ ClassList list) {
+    int ci = 0;
+    while (ci + 1 < list.n && (int)blockIdx.x >= list.first[ci + 1]) ++ci;
+    const int b = (int)blockIdx.x - list.first[ci], nchunk = list.cls[ci].nchunk;
+    dense_block<LA, LB, F32>(d, list.cls[ci], b / nchunk, b % nchunk);
+}
+
+constexpr int kMaxSmem = 200 * 1024;
+
+// Launches of the template pair LA * 4 + LB, one translation unit for each
+// pair of (one class or a list, FP64 or FP32).
+cudaError_t run_one_f64(int pair, const EriDev& d, const QuartetClass& qc, int smem, cudaStream_t s);
+cudaError_t run_one_f32(int pair, const EriDev& d, const QuartetClass& qc, int smem, cudaStream_t s);
+cudaError_t run_list_f64(int pair, const EriDev& d, const ClassList& list, int smem, cudaStream_t s);
+cudaError_t run_list_f32(int pair, const EriDev& d, const ClassList& list, int smem, cudaStream_t s);
+
+template <class Arg>
+cudaError_t launch_with_smem(void (*kernel)(EriDev, Arg), std::atomic<bool>& ready, dim3 grid, int smem, cudaStream_t s,
+                             const EriDev& d, const Arg& arg) {
+    if (!ready.load(std::memory_order_acquire)) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
+        if (e != cudaSuccess) return e;
+        ready.store(true, std::memory_order_release);
+    }
+    kernel<<<grid, 32 * kWarps, smem, s>>>(d, arg);
+    return cudaGetLastError();
+}
+
+#define GX_DENSE_PAIRS \
+    GX_CASE(0, 0)      \
+    GX_CASE(0, 1)      \
+    GX_CASE(0, 2)      \
+    GX_CASE(0, 3)      \
+    GX_CASE(1, 1)      \
+    GX_CASE(1, 2)      \
+    GX_CASE(2, 1)      \
+    GX_CASE(1, 3)      \
+    GX_CASE(3, 1)      \
+    GX_CASE(2, 2)
 
 }  // namespace dense
 }  // namespace gx

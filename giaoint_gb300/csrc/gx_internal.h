@@ -6,6 +6,7 @@
 #include <stdint.h>
 
 #include <string>
+#include <vector>
 
 #include "gx_device.cuh"
 
@@ -97,6 +98,7 @@ struct QuartetClass {
                               //    (null: the class has few tasks, every block cuts its units itself)
     long long target;         // weight of a unit, and the components of the four shells, one byte each, for that
     int dims;
+    unsigned long long* counters;  // [0] FP64, [1] FP32 primitive quartets evaluated (may be null)
     const int* unit_start32;  // lane-dense kernel: the same for the FP32 entries
     const int* unit_count32;
 };
@@ -137,7 +139,7 @@ struct EriDev {
                       // The FP32 quartets use FP32 Boys values in the asymptotic
                       // sector and FP64 ones elsewhere, then the FP32 recurrence.
     int all_real;     // 1: every pair has q = 0 (zero field, or all shells on one centre)
-    unsigned long long* counters;  // [0] FP64, [1] FP32 primitive quartets evaluated (may be null)
+    unsigned long long* counters;  // class-generic kernel: [0] FP64, [1] FP32 primitive quartets evaluated (may be null)
 };
 
 // In-place descending-level Hermite recurrence as a step list per total order
@@ -256,11 +258,17 @@ bool dense_class(int la, int lb, int lc, int ld);
 int dense_chunks(int la, int lb, int lc, int ld, int want, bool single);
 long long unit_tiles(long long ntask);
 cudaError_t launch_units(const UnitPlan& u, const Task* tasks, const EriDev& d, cudaStream_t s);
-cudaError_t launch_dense(int la, int lb, int lc, int ld, const EriDev& d, QuartetClass qc, bool f32, cudaStream_t s);
+// A dense class oriented for its template pair (LA, LB): returns LA * 4 + LB.
+int dense_orient(int la, int lb, int lc, int ld, QuartetClass& qc);
+// Classes of one template pair in as few launches as hold them.
+cudaError_t launch_dense(int pair, const EriDev& d, const std::vector<QuartetClass>& classes, bool f32, cudaStream_t s);
 
 // register-resident small classes (gx_small.cu)
 bool small_class(int la, int lb, int lc, int ld);
 cudaError_t launch_small(int la, int lb, int lc, int ld, const EriDev& d, const QuartetClass& qc, cudaStream_t s);
+// small classes (up to 15, keys[i] = ((la 3 + lb) 3 + lc) 3 + ld) in one launch
+cudaError_t launch_small_list(const EriDev& d, const std::vector<int>& keys, const std::vector<QuartetClass>& classes,
+                              cudaStream_t s);
 
 // Cholesky (gx_chol.cu)
 cudaError_t launch_chol_diag(const double2* packed, const long long* boff, const int* info, int nblocks, int n,

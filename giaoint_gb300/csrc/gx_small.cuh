@@ -369,14 +369,13 @@ __device__ __forceinline__ void add_runs(double2* out, const WarpBuffers<nc(LA) 
 }
 
 template <int LA, int LB, int LC, int LD>
-__global__ void __launch_bounds__(32 * kWarps) small_kernel(EriDev d, QuartetClass qc) {
+__device__ __forceinline__ void small_block(const EriDev& d, const QuartetClass& qc, int block, char* smem) {
     constexpr int L = LA + LB + LC + LD;
     constexpr int NL = hc(L), NH = hc(LA + LB);
     constexpr int NCD = nc(LC) * nc(LD), NOUT = nc(LA) * nc(LB) * NCD;
-    __shared__ WarpBuffers<NOUT> s_buf[kWarps];
     const int lane = threadIdx.x & 31;
-    WarpBuffers<NOUT>& w = s_buf[threadIdx.x >> 5];
-    const int unit = blockIdx.x * kWarps + (threadIdx.x >> 5);
+    WarpBuffers<NOUT>& w = reinterpret_cast<WarpBuffers<NOUT>*>(smem)[threadIdx.x >> 5];
+    const int unit = block * kWarps + (threadIdx.x >> 5);
     int t0, t1;
     if (qc.unit_start) {
         if (unit >= qc.ngroup) return;
@@ -386,7 +385,7 @@ __global__ void __launch_bounds__(32 * kWarps) small_kernel(EriDev d, QuartetCla
     } else {
         __shared__ int bounds[kWarps + 1];
         __shared__ long long sums[kWarps];
-        cut_units<32 * kWarps>(d, qc, 2, blockIdx.x * kWarps, kWarps, true, bounds, sums);
+        cut_units<32 * kWarps>(d, qc, 2, block * kWarps, kWarps, true, bounds, sums);
         t0 = bounds[threadIdx.x >> 5];
         t1 = bounds[(threadIdx.x >> 5) + 1];
     }
@@ -580,15 +579,31 @@ __global__ void __launch_bounds__(32 * kWarps) small_kernel(EriDev d, QuartetCla
             __syncwarp();
         }
     }
-    if (d.counters) {
+    if (qc.counters) {
         const unsigned a64 = __reduce_add_sync(0xffffffffu, n64);
         const unsigned a32 = __reduce_add_sync(0xffffffffu, n32);
         if (lane == 0) {
-            if (a64) atomicAdd(&d.counters[0], (unsigned long long)a64);
-            if (a32) atomicAdd(&d.counters[1], (unsigned long long)a32);
+            if (a64) atomicAdd(&qc.counters[0], (unsigned long long)a64);
+            if (a32) atomicAdd(&qc.counters[1], (unsigned long long)a32);
         }
     }
 }
+
+template <int LA, int LB, int LC, int LD>
+__global__ void __launch_bounds__(32 * kWarps) small_kernel(const __grid_constant__ EriDev d,
+                                                            const __grid_constant__ QuartetClass qc) {
+    __shared__ WarpBuffers<nc(LA) * nc(LB) * nc(LC) * nc(LD)> s_buf[kWarps];
+    small_block<LA, LB, LC, LD>(d, qc, blockIdx.x, reinterpret_cast<char*>(s_buf));
+}
+
+// The small classes of a small plan in one launch: block b works on class c with
+// first[c] <= b < first[c + 1].
+struct ClassList {
+    int n;
+    int key[15];
+    int first[16];
+    QuartetClass cls[15];
+};
 
 }  // namespace small
 }  // namespace gx
