@@ -43,7 +43,13 @@ struct DevConst {
     double ints[40];     // n
     double half[40];     // n + 1/2
     double inv_odd[40];  // 1 / (2n + 1)
-    constexpr DevConst() : ints{}, half{}, inv_odd{} {
+    double binom[561];   // C(t, k) at t (t + 1) / 2 + k, t <= 32
+    constexpr DevConst() : ints{}, half{}, inv_odd{}, binom{} {
+        for (int t = 0; t <= 32; ++t) {
+            binom[t * (t + 1) / 2] = binom[t * (t + 1) / 2 + t] = 1.0;
+            for (int k = 1; k < t; ++k)
+                binom[t * (t + 1) / 2 + k] = binom[(t - 1) * t / 2 + k - 1] + binom[(t - 1) * t / 2 + k];
+        }
         for (int n = 0; n < 40; ++n) {
             ints[n] = (double)n;
             half[n] = (double)n + 0.5;

@@ -531,12 +531,10 @@ __global__ void __launch_bounds__(32 * kPairWarps) pair_hermite_kernel(
             for (int k = 0; k <= n; ++k) {
                 double2 acc = c2(e[k], 0.0);
                 if (q[x] != 0.0) {
-                    double binom = 1.0;         // C(t, k) for t = k
                     double2 pw = c2(1.0, 0.0);  // (-i q)^{t-k}
                     for (int t = k + 1; t <= n; ++t) {
                         pw = c2(pw.y * q[x], -pw.x * q[x]);
-                        binom = binom * c_dev.ints[t] / c_dev.ints[t - k];
-                        acc = cadd(acc, cscale(pw, binom * e[t]));
+                        acc = cadd(acc, cscale(pw, c_dev.binom[t * (t + 1) / 2 + k] * e[t]));
                     }
                 }
                 Et[x][k] = acc;
@@ -565,16 +563,21 @@ __global__ void __launch_bounds__(32 * kPairWarps) pair_hermite_kernel(
 // la+lb > 4 get an infinite bound (never screened).
 constexpr int BOUND_MAX_LAB = 4;
 
-__global__ void __launch_bounds__(32 * kPairWarps) pair_bound_kernel(BasisDev bs, EriDev d, int npp, const int* pp_a,
+constexpr int kBoundWords = 336;  // E~ words of (dd), the largest pair class with la + lb <= 4
+constexpr int kBoundWarps = 2;
+
+__global__ void __launch_bounds__(32 * kBoundWarps) pair_bound_kernel(BasisDev bs, EriDev d, int npp, const int* pp_a,
                                                                      const int* pp_b, const int* pp_pa,
                                                                      const int* pp_pb, const int* pp_class,
                                                                      const PairClassDev* classes, double* bound) {
     constexpr int MAXL = 2 * BOUND_MAX_LAB;
     constexpr int NR = (MAXL + 1) * (MAXL + 2) * (MAXL + 3) / 6;
-    __shared__ double2 s_R[kPairWarps][2 * NR];
-    __shared__ double2 s_seed[kPairWarps][MAXL + 4];
+    __shared__ double2 s_R[kBoundWarps][2 * NR];
+    __shared__ double2 s_E[kBoundWarps][kBoundWords], s_t[kBoundWarps][kBoundWords];
+    __shared__ uint32_t s_k[kBoundWarps][kBoundWords];
+    __shared__ double2 s_seed[kBoundWarps][MAXL + 4];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int i = blockIdx.x * kPairWarps + warp;
+    const int i = blockIdx.x * kBoundWarps + warp;
     if (i >= npp) return;
     const int a = pp_a[i], b = pp_b[i];
     if (a > b || (a == b && pp_pa[i] > pp_pb[i])) return;
@@ -609,32 +612,54 @@ __global__ void __launch_bounds__(32 * kPairWarps) pair_bound_kernel(BasisDev bs
     if (lane < 3) seed[L + 1 + lane] = lane == 0 ? X[0] : (lane == 1 ? X[1] : X[2]);
     __syncwarp();
     coop_rec<double2>(L, seed, seed + L + 1, R, 2, 0, 1, d.herm_xyz, lane);
+    // (ab|ba) = sum_e E~ab[e] sum_f (-1)^{|f|} E~ba[f] R[e + f]: a lane per word
+    // e of the record (its table row and component pair are found once), the
+    // words of a component pair then summed by a lane each.  The records and the
+    // rows of the other side's words are staged in shared memory: read from
+    // global memory, one load per multiply-add, they took most of the time.
     const PairClassDev ci = classes[pp_class[i]], cj = classes[pp_class[j]];
     const double2* Ei = pp.Epool + pp.Eoff[i];
     const double2* Ej = pp.Epool + pp.Eoff[j];
+    double2* s_Ej = s_E[warp];
+    uint32_t* s_kj = s_k[warp];
+    double2* s_term = s_t[warp];
+    for (int f = lane; f < cj.Etot; f += 32) {
+        const uint32_t kf = cj.ent[f];
+        double2 ev = Ej[f];
+        if (((kf & 255) + ((kf >> 8) & 255) + ((kf >> 16) & 255)) & 1) ev = c2(-ev.x, -ev.y);
+        s_Ej[f] = ev;
+        s_kj[f] = kf;
+    }
+    __syncwarp();
     const int nb = ncart(lb), na = ncart(la);
     double best = 0.0;
-    for (int ab = lane; ab < ci.nab; ab += 32) {
-        const int ca = ab / nb, cb = ab - ca * nb;
-        const int ba = cb * na + ca;
-        const int oi = ci.boxoff[ab], di = ci.boxdim[ab];
-        const int oj = cj.boxoff[ba], dj = cj.boxdim[ba];
-        const int ni = (di & 255) * ((di >> 8) & 255) * ((di >> 16) & 255);
-        const int nj = (dj & 255) * ((dj >> 8) & 255) * ((dj >> 16) & 255);
-        double2 acc = c2(0.0, 0.0);
-        for (int e = 0; e < ni; ++e) {
-            const uint32_t ke = ci.ent[oi + e];
-            const int k1 = ke & 255, l1 = (ke >> 8) & 255, m1 = (ke >> 16) & 255;
+    int ab = 0, e_end = 0;  // component pair of the lane's word (words of a pair are consecutive)
+    for (int e0 = 0; e0 < ci.Etot; e0 += 32) {
+        const int e = e0 + lane;
+        if (e < ci.Etot) {
+            while (e >= e_end) {
+                const int di = ci.boxdim[ab];
+                e_end = ci.boxoff[ab] + (di & 255) * ((di >> 8) & 255) * ((di >> 16) & 255);
+                if (e >= e_end) ++ab;
+            }
+            const int ca = ab / nb, ba = (ab - ca * nb) * na + ca;
+            const int oj = cj.boxoff[ba], dj = cj.boxdim[ba];
+            const int nj = (dj & 255) * ((dj >> 8) & 255) * ((dj >> 16) & 255);
+            const uint32_t ke = ci.ent[e];
             double2 inner = c2(0.0, 0.0);
             for (int f = 0; f < nj; ++f) {
-                const uint32_t kf = cj.ent[oj + f];
-                const int k2 = kf & 255, l2 = (kf >> 8) & 255, m2 = (kf >> 16) & 255;
-                double2 ev = Ej[oj + f];
-                if ((k2 + l2 + m2) & 1) ev = c2(-ev.x, -ev.y);
-                inner = cmac(inner, ev, R[2 * herm_index(k1 + k2, l1 + l2, m1 + m2)]);
+                const uint32_t k = ke + s_kj[oj + f];  // (bytes do not overflow: orders <= 8)
+                inner = cmac(inner, s_Ej[oj + f], R[2 * herm_index(k & 255, (k >> 8) & 255, (k >> 16) & 255)]);
             }
-            acc = cmac(acc, Ei[oi + e], inner);
+            s_term[e] = cmul(Ei[e], inner);
         }
+    }
+    __syncwarp();
+    for (int c = lane; c < ci.nab; c += 32) {
+        const int o = ci.boxoff[c], dc = ci.boxdim[c];
+        const int n = (dc & 255) * ((dc >> 8) & 255) * ((dc >> 16) & 255);
+        double2 acc = s_term[o];
+        for (int e = 1; e < n; ++e) acc = cadd(acc, s_term[o + e]);
         best = fmax(best, acc.x * acc.x + acc.y * acc.y);
     }
     for (int off = 16; off > 0; off >>= 1) best = fmax(best, __shfl_xor_sync(0xffffffffu, best, off));
@@ -712,7 +737,7 @@ cudaError_t launch_pair_precompute(const BasisDev& basis, const double* B, const
     pair_hermite_kernel<<<warps, 32 * kPairWarps, 0, s>>>(basis, Bv, Ov, npp, pp_a, pp_b, pp_pa, pp_pb, pp_class,
                                                           classes, axis_norms(), p, Pr, Pi, Eoff, Epool,
                                                           Epool32);
-    pair_bound_kernel<<<warps, 32 * kPairWarps, 0, s>>>(basis, dev, npp, pp_a, pp_b, pp_pa, pp_pb, pp_class, classes,
+    pair_bound_kernel<<<(unsigned)((npp + kBoundWarps - 1) / kBoundWarps), 32 * kBoundWarps, 0, s>>>(basis, dev, npp, pp_a, pp_b, pp_pa, pp_pb, pp_class, classes,
                                                         bound);
     const unsigned pairs = (unsigned)basis.ns * (unsigned)basis.ns;
     pair_order_kernel<<<(pairs + 3) / 4, 128, 0, s>>>(basis, bound, order, sbound);
