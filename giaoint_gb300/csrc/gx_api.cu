@@ -783,7 +783,7 @@ void make_units(gx_context* ctx, PlanData& plan) {
             const PlanClass& pc = plan.classes[ci];
             const bool small = gx::small_class(pc.key[0], pc.key[1], pc.key[2], pc.key[3]);
             if (!gx::dense_class(pc.key[0], pc.key[1], pc.key[2], pc.key[3]) && !(small && !fp32)) continue;
-            const int64_t full = 8 * (int64_t)std::max(ctx->sm_count, 1);
+            const int64_t full = (small ? 64 : 8) * (int64_t)std::max(ctx->sm_count, 1);
             const int64_t all = pc.primitive_quartets * std::max(plan.spread_parts, 1);
             int entries = 256;
             while (entries > 32 && all / entries < full) entries /= 2;
@@ -1062,8 +1062,15 @@ void build_plan_parts(gx_context* ctx, const std::vector<PlanPart>& parts, PlanD
     for (size_t ci = 0; ci < plan.classes.size(); ++ci) plan.defconf[ci] = default_conf(plan.classes[ci].key);
     plan.order.resize(plan.classes.size());
     std::iota(plan.order.begin(), plan.order.end(), 0);
+    // by decreasing work, but the small classes first: their work is little and
+    // their warps are slow, and launched last they were the end of the plan
+    // (one field of five atoms in mixed precision, with their shorter units:
+    // 3.74 -> 3.56 ms; molecules of 12 atoms unchanged)
     std::stable_sort(plan.order.begin(), plan.order.end(), [&](int x, int y) {
         const PlanClass &a = plan.classes[x], &c = plan.classes[y];
+        const bool sa = gx::small_class(a.key[0], a.key[1], a.key[2], a.key[3]);
+        const bool sc = gx::small_class(c.key[0], c.key[1], c.key[2], c.key[3]);
+        if (sa != sc) return sa;
         return (double)a.primitive_quartets * a.flops_per_primitive_quartet >
                (double)c.primitive_quartets * c.flops_per_primitive_quartet;
     });

@@ -122,17 +122,23 @@ cudaError_t launch_dense(int pair, const EriDev& d, const std::vector<QuartetCla
 // Work units.  How many primitive quartets of a task survive depends on the
 // field, so the units are cut on the device at every execution: unit u of a
 // class starts at the first task whose weight prefix (task_weight) within the
-// class reaches u * target.  Two launches for the classes with many tasks: counts with prefixes over tiles of 1024 tasks (the last block to
-// finish turns the tile sums into a prefix), then the starts; the others' blocks
-// cut their units themselves (cut_units).  Bound by memory:
-// 48 bytes read and 16 written per task, and the blocks of the tasks without an
-// FP64 survivor, which are cleared here (the kernels store the first batch of
-// every other block).
+// class reaches u * target.  Two launches for the classes with many tasks:
+// counts with prefixes over tiles of tasks (the last block to finish turns the
+// tile sums into a prefix), then the starts; the others' blocks cut their units
+// themselves (cut_units).  A large plan is bound by memory: 48 bytes read and 16
+// written per task, and the blocks of the tasks without an FP64 survivor, which
+// are cleared here (the kernels store the first batch of every other block).  A
+// small one waits for a warp's chain of dependent loads (a task's shells, their
+// primitives, the walk over its pair factors) once per row of 32 tasks: up to
+// kFewTasks tasks a warp takes one row and a tile is 256 tasks (300,000 tasks:
+// 122 us with four rows, 63 with one); beyond, four rows and tiles of 1024, which
+// leave the last block a quarter of the tile sums.
 // ---------------------------------------------------------------------------
 
 namespace {
 
-constexpr int kTile = 1024, kUnitThreads = 256, kPer = kTile / kUnitThreads, kNoTask = 0x7f7f7f7f;
+constexpr int kUnitThreads = 256, kNoTask = 0x7f7f7f7f;
+constexpr long long kFewTasks = 1 << 20;
 
 __device__ __forceinline__ int class_of(const UnitClass* cls, int n, long long v) {
     int lo = 0, hi = n - 1;
@@ -167,6 +173,8 @@ __device__ long long block_prefix(long long x, long long* smem, long long* total
     return before + inc - x;
 }
 
+// ROWS: rows of 32 tasks per warp; a block's tile is ROWS * kUnitThreads tasks
+template <int ROWS>
 __global__ void __launch_bounds__(kUnitThreads) unit_count_kernel(UnitPlan u, const Task* tasks, PairData pp,
                                                                   const int* nprim, float skip, float cut32,
                                                                   double2* out) {
@@ -176,11 +184,12 @@ __global__ void __launch_bounds__(kUnitThreads) unit_count_kernel(UnitPlan u, co
          i += (long long)gridDim.x * kUnitThreads)
         u.start[i] = kNoTask;
     const int lane = threadIdx.x & 31;
-    // a warp takes 128 consecutive tasks, 32 at a time: lane-coalesced, and the
+    // a warp takes consecutive tasks, 32 at a time: lane-coalesced, and the
     // lanes' weights are put in order by the prefix below
-    const long long v0 = (long long)blockIdx.x * kTile + (threadIdx.x >> 5) * (32 * kPer);
-    long long w[kPer], before[kPer], sum = 0;
-    for (int k = 0; k < kPer; ++k) {
+    const long long v0 = ((long long)blockIdx.x * kUnitThreads + (threadIdx.x & ~31)) * ROWS;
+    long long w[ROWS], before[ROWS], sum = 0;
+#pragma unroll
+    for (int k = 0; k < ROWS; ++k) {
         const long long v = v0 + 32 * k + lane;
         w[k] = 0;
         const Task* t = nullptr;
@@ -217,7 +226,8 @@ __global__ void __launch_bounds__(kUnitThreads) unit_count_kernel(UnitPlan u, co
     long long total;
     const long long at = block_prefix(lane == 0 ? sum : 0, smem, &total);
     const long long base = __shfl_sync(0xffffffffu, at, 0);
-    for (int k = 0; k < kPer; ++k)
+#pragma unroll
+    for (int k = 0; k < ROWS; ++k)
         if (v0 + 32 * k + lane < u.ntask) u.prefix[v0 + 32 * k + lane] = base + before[k];
     if (threadIdx.x == 0) {
         u.tile[blockIdx.x] = total;
@@ -239,11 +249,11 @@ __global__ void __launch_bounds__(kUnitThreads) unit_count_kernel(UnitPlan u, co
     if (threadIdx.x == 0) *u.done = 0;
 }
 
-__global__ void unit_start_kernel(UnitPlan u) {
+__global__ void unit_start_kernel(UnitPlan u, int tile) {
     const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= u.ntask) return;
     const UnitClass c = u.cls[class_of(u.cls, u.ncls, v)];
-    auto at = [&](long long x) { return u.tile[x / kTile] + u.prefix[x]; };
+    auto at = [&](long long x) { return u.tile[x / tile] + u.prefix[x]; };
     const long long base = at(c.vfirst);
     const int here = (int)((at(v) - base) / c.target);
     const int prev = v == c.vfirst ? -1 : (int)((at(v - 1) - base) / c.target);
@@ -252,7 +262,7 @@ __global__ void unit_start_kernel(UnitPlan u) {
 
 }  // namespace
 
-long long unit_tiles(long long ntask) { return (ntask + kTile - 1) / kTile; }
+long long unit_tiles(long long ntask) { return (ntask + kUnitThreads - 1) / kUnitThreads; }
 
 cudaError_t launch_units(const UnitPlan& plan, const Task* tasks, const EriDev& d, cudaStream_t s) {
     UnitPlan u = plan;
@@ -261,11 +271,13 @@ cudaError_t launch_units(const UnitPlan& plan, const Task* tasks, const EriDev& 
         u.nunit = plan.nunit64;
     }
     if (u.ntask <= 0) return cudaSuccess;
-    unit_count_kernel<<<(unsigned)unit_tiles(u.ntask), kUnitThreads, 0, s>>>(u, tasks, d.pairs, d.basis.nprim,
-                                                                             d.skip_cut, d.fp32_cut, d.out);
+    const int tile = (u.ntask <= kFewTasks ? 1 : 4) * kUnitThreads;
+    auto* count = u.ntask <= kFewTasks ? unit_count_kernel<1> : unit_count_kernel<4>;
+    count<<<(unsigned)((u.ntask + tile - 1) / tile), kUnitThreads, 0, s>>>(u, tasks, d.pairs, d.basis.nprim, d.skip_cut,
+                                                                           d.fp32_cut, d.out);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    unit_start_kernel<<<(unsigned)((u.ntask + 255) / 256), 256, 0, s>>>(u);
+    unit_start_kernel<<<(unsigned)((u.ntask + 255) / 256), 256, 0, s>>>(u, tile);
     return cudaGetLastError();
 }
 
