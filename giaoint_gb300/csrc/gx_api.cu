@@ -723,9 +723,12 @@ void record_tuning(const gx_context* ctx, const gx_basis* b, int precision, cons
 }
 
 // The class runs in the lane-dense kernel (unless it is pinned to the
-// class-generic one).
-bool runs_dense(const PlanClass& pc, const ClassConf& conf) {
-    return !conf.nolane && gx::dense_class(pc.key[0], pc.key[1], pc.key[2], pc.key[3]);
+// class-generic one).  all_real: of the execution.  A stable plan takes the
+// real table's classes to the class-generic kernel, as an execution packed
+// with others does, which is not known to be real.
+bool runs_dense(const PlanData& plan, const PlanClass& pc, const ClassConf& conf, int all_real) {
+    return !conf.nolane &&
+           gx::dense_class(pc.key[0], pc.key[1], pc.key[2], pc.key[3], all_real && !plan.stable);
 }
 
 // Warp work units of class ci in the class-generic kernel: runs of tasks with
@@ -734,7 +737,7 @@ bool runs_dense(const PlanClass& pc, const ClassConf& conf) {
 // fewer tasks when the class is too small to give every SM eight warps.
 std::vector<int2> make_groups(const gx_context* ctx, const PlanData& plan, size_t ci, const ClassConf& conf) {
     const PlanClass& pc = plan.classes[ci];
-    if (gx::small_class(pc.key[0], pc.key[1], pc.key[2], pc.key[3]) || runs_dense(pc, conf)) return {};
+    if (gx::small_class(pc.key[0], pc.key[1], pc.key[2], pc.key[3]) || runs_dense(plan, pc, conf, 0)) return {};
     const int per = conf.per_group > 0 ? conf.per_group : 32;
     const size_t count = pc.count * (size_t)std::max(plan.spread_parts, 1);
     const int spread = std::max<int>(1, (int)(count / (size_t)(8 * std::max(ctx->sm_count, 1))));
@@ -782,7 +785,9 @@ void make_units(gx_context* ctx, PlanData& plan) {
         for (size_t ci = 0; ci < nc; ++ci) {
             const PlanClass& pc = plan.classes[ci];
             const bool small = gx::small_class(pc.key[0], pc.key[1], pc.key[2], pc.key[3]);
-            if (!gx::dense_class(pc.key[0], pc.key[1], pc.key[2], pc.key[3]) && !(small && !fp32)) continue;
+            const bool complex = gx::dense_class(pc.key[0], pc.key[1], pc.key[2], pc.key[3], false);
+            const bool dense = gx::dense_class(pc.key[0], pc.key[1], pc.key[2], pc.key[3], !plan.stable);
+            if (!dense && !(small && !fp32)) continue;
             const int64_t full = (small ? 64 : 8) * (int64_t)std::max(ctx->sm_count, 1);
             const int64_t all = pc.primitive_quartets * std::max(plan.spread_parts, 1);
             int entries = 256;
@@ -798,7 +803,8 @@ void make_units(gx_context* ctx, PlanData& plan) {
             plan.unit_dims[ci] = dims;
             if (pc.count < (size_t)gx::kUnitMinTasks) continue;
             (fp32 ? plan.unit_class32 : plan.unit_class)[ci] = (int)cls.size();
-            cls.push_back(gx::UnitClass{vtask, (long long)pc.first, nunit, target, fp32 ? 1 : (small ? 2 : 0), dims});
+            cls.push_back(gx::UnitClass{vtask, (long long)pc.first, nunit, target, fp32 ? 1 : (small ? 2 : 0), dims,
+                                        dense && !complex ? 1 : 0});
             vtask += (int64_t)pc.count;
             nunit += grid + 1;
         }
@@ -1163,7 +1169,7 @@ void launch_class(gx_context* ctx, gx::EriDev dev, const PlanData& plan, size_t 
     const auto& k = pc.key;
     dev.counters = counters ? counters + 2 * ci : nullptr;
     const bool small = gx::small_class(k[0], k[1], k[2], k[3]);
-    if (small || runs_dense(pc, conf)) {
+    if (small || runs_dense(plan, pc, conf, dev.all_real)) {
         gx::QuartetClass uc = unit_class(ctx, plan, ci, counters);
         if (small) {
             GX_CUDA(gx::launch_small(k[0], k[1], k[2], k[3], dev, uc, s));
@@ -1303,7 +1309,7 @@ std::vector<PlanLaunch> plan_launches(gx_context* ctx, const gx::EriDev& dev, co
         const auto& k = pc.key;
         const ClassConf& conf = tuned.valid ? tuned.conf[ci] : plan.defconf[ci];
         const bool small = gx::small_class(k[0], k[1], k[2], k[3]);
-        if ((small || runs_dense(pc, conf)) && pc.primitive_quartets <= kSharedLaunch) {
+        if ((small || runs_dense(plan, pc, conf, dev.all_real)) && pc.primitive_quartets <= kSharedLaunch) {
             gx::QuartetClass qc{};
             const int L = k[0] + k[1] + k[2] + k[3];
             const int by_order = plan.primitive_quartets > kSharedPlan ? L : 0;
@@ -4725,7 +4731,7 @@ int gx_eri_plan_autotune(gx_eri_plan* plan, const double* B, const double* O, in
                             if (!(per == 32 && w == 4 && b1 == 32)) cands.push_back(ClassConf{per, w, b1});
                 // a lane-dense class has no knobs: the sweep tries the generic kernel on it
                 for (size_t c = 1; c < cands.size(); ++c)
-                    cands[c].nolane = gx::dense_class(k[0], k[1], k[2], k[3]) ? 1 : 0;
+                    cands[c].nolane = runs_dense(pd, pd.classes[ci], pd.defconf[ci], dev.all_real) ? 1 : 0;
             }
             double best_ms = 0.0, def_ms = 0.0;
             auto time_conf = [&](const ClassConf& cf) {
@@ -4753,7 +4759,7 @@ int gx_eri_plan_autotune(gx_eri_plan* plan, const double* B, const double* O, in
                     best[ci] = cands[c];
                 }
             }
-            const bool knobs = !small && !runs_dense(pd.classes[ci], best[ci]);
+            const bool knobs = !small && !runs_dense(pd, pd.classes[ci], best[ci], dev.all_real);
             if (knobs) {
                 // second stage: transform tiles under the chosen work split
                 const int ncd = ctx->pair_class(k[2], k[3]).nab;

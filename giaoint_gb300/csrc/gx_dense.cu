@@ -10,6 +10,7 @@ namespace gx {
 namespace {
 
 using dense::kMaxOrder;
+using dense::kMaxOrderReal;
 using dense::kMaxSmem;
 
 // template pairs: (l, 0) runs as (0, l), whose components, boxes and Hermite
@@ -36,9 +37,10 @@ int smem_bytes(int la, int lb, int lc, int ld, int word) {
 // as the template side, 438 with (12)).
 int side_of(int la, int lb, int lc, int ld) {
     const int L = la + lb + lc + ld;
-    if (L < 3 || L > kMaxOrder) return 0;
-    const bool ab = template_pair(la, lb) && smem_bytes(la, lb, lc, ld, 16) <= kMaxSmem;
-    const bool cd = template_pair(lc, ld) && smem_bytes(lc, ld, la, lb, 16) <= kMaxSmem;
+    if (L < 3 || L > kMaxOrderReal) return 0;
+    const int word = L <= kMaxOrder ? 16 : 8;
+    const bool ab = template_pair(la, lb) && smem_bytes(la, lb, lc, ld, word) <= kMaxSmem;
+    const bool cd = template_pair(lc, ld) && smem_bytes(lc, ld, la, lb, word) <= kMaxSmem;
     if (!ab || !cd) return ab ? 1 : (cd ? 2 : 0);
     auto groups = [](int a, int b, int c, int d) {
         const int cg = dense::group_of(small::nc(a) * small::nc(b));
@@ -51,7 +53,9 @@ int side_of(int la, int lb, int lc, int ld) {
 
 }  // namespace
 
-bool dense_class(int la, int lb, int lc, int ld) { return side_of(la, lb, lc, ld) != 0; }
+bool dense_class(int la, int lb, int lc, int ld, bool real) {
+    return la + lb + lc + ld <= (real ? kMaxOrderReal : kMaxOrder) && side_of(la, lb, lc, ld) != 0;
+}
 
 // Blocks that share a work unit's components when `want` would fill the GPU:
 // at most as many as have components for their warps, and (unless the class
@@ -177,7 +181,7 @@ __device__ long long block_prefix(long long x, long long* smem, long long* total
 template <int ROWS>
 __global__ void __launch_bounds__(kUnitThreads) unit_count_kernel(UnitPlan u, const Task* tasks, PairData pp,
                                                                   const int* nprim, float skip, float cut32,
-                                                                  double2* out) {
+                                                                  int all_real, double2* out) {
     __shared__ long long smem[kUnitThreads / 32];
     __shared__ bool last;
     for (long long i = (long long)blockIdx.x * kUnitThreads + threadIdx.x; i < u.nunit;
@@ -197,12 +201,14 @@ __global__ void __launch_bounds__(kUnitThreads) unit_count_kernel(UnitPlan u, co
         bool clear = false;
         if (v < u.ntask) {
             const UnitClass c = u.cls[class_of(u.cls, u.ncls, v)];
-            t = tasks + c.first + (v - c.vfirst);
-            dims = c.dims;
-            int n64, n32;
-            w[k] = task_weight(c.mode, t, pp, nprim, skip, cut32, n64, n32);
-            u.count[v] = c.mode == 1 ? n32 : n64;
-            clear = c.mode != 1 && n64 == 0;
+            if (!c.real_only || all_real) {
+                t = tasks + c.first + (v - c.vfirst);
+                dims = c.dims;
+                int n64, n32;
+                w[k] = task_weight(c.mode, t, pp, nprim, skip, cut32, n64, n32);
+                u.count[v] = c.mode == 1 ? n32 : n64;
+                clear = c.mode != 1 && n64 == 0;
+            }
         }
         // clear this row's empty blocks, the warp together on each
         unsigned m = __ballot_sync(0xffffffffu, clear);
@@ -274,7 +280,7 @@ cudaError_t launch_units(const UnitPlan& plan, const Task* tasks, const EriDev& 
     const int tile = (u.ntask <= kFewTasks ? 1 : 4) * kUnitThreads;
     auto* count = u.ntask <= kFewTasks ? unit_count_kernel<1> : unit_count_kernel<4>;
     count<<<(unsigned)((u.ntask + tile - 1) / tile), kUnitThreads, 0, s>>>(u, tasks, d.pairs, d.basis.nprim, d.skip_cut,
-                                                                           d.fp32_cut, d.out);
+                                                                           d.fp32_cut, d.all_real, d.out);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     unit_start_kernel<<<(unsigned)((u.ntask + 255) / 256), 256, 0, s>>>(u, tile);

@@ -99,8 +99,13 @@ __device__ __forceinline__ double coef_of(double*, int k) { return c_dev.ints[k]
 __device__ __forceinline__ float coef_of(float2*, int k) { return (float)k; }
 
 constexpr int kWarps = 4;
-constexpr int kMaxOrder = 8;         // FP64 table of 165 rows: 84 KB a block, two blocks an SM
-constexpr int kMaxSeeds = kMaxOrder + 1;
+// Highest order of an execution, and of one whose pairs are all real.  The table
+// of order 8 takes 84 KB a block (165 rows), two blocks an SM; at 9 and 10 there
+// is room for one, and five atoms with f shells in a field took 35.2 ms instead
+// of the class-generic kernel's 29.6.  A real table has half the bytes: 73 KB at
+// order 10, and the same atoms at zero field take 11.7 ms instead of 13.4.
+constexpr int kMaxOrder = 8, kMaxOrderReal = 10;
+constexpr int kMaxSeeds = kMaxOrderReal + 1;
 
 // Value buffer of a warp: the components ab of `group` components of the other
 // side, or of a slice of one, 9 to 12 rows of 33 columns (the odd width keeps

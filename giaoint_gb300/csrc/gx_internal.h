@@ -111,6 +111,7 @@ struct UnitClass {
     long long target;         // weight of a unit
     int mode;                 // entries counted: 0 FP64, 1 FP32, 2 FP64 with the FP32 ones adding to the weight
     int dims;                 // components of the four shells, one byte each
+    int real_only;            // counted in real executions alone (the lane-dense kernel takes the class in no other)
 };
 struct UnitPlan {
     const UnitClass* cls;
@@ -254,7 +255,7 @@ cudaError_t launch_gather_abs(const double2* src, const long long* idx, double* 
 
 // lane-dense kernel (gx_dense.cu)
 constexpr int kUnitMinTasks = 512;  // classes with fewer tasks have no entry in the unit plan
-bool dense_class(int la, int lb, int lc, int ld);
+bool dense_class(int la, int lb, int lc, int ld, bool real);  // real: the execution's pairs all have q = 0
 int dense_chunks(int la, int lb, int lc, int ld, int want, bool single);
 long long unit_tiles(long long ntask);
 cudaError_t launch_units(const UnitPlan& u, const Task* tasks, const EriDev& d, cudaStream_t s);

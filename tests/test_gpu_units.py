@@ -129,3 +129,28 @@ def test_nuclear_batches(nuclei, B, oracle):
     got = gi.nuclear_attraction(basis, [gi.Nucleus(z, c) for z, c in nucs], field=gi.MagneticField(B))
     ref = oracle.nuclear(recs, nucs, B, None)
     np.testing.assert_allclose(got, ref, rtol=1e-12, atol=1e-12 * np.abs(ref).max())
+
+
+@pytest.mark.parametrize("key", [(2, 1, 3, 3), (3, 0, 3, 3), (2, 2, 2, 3), (3, 3, 1, 3), (3, 3, 2, 2), (3, 2, 3, 2)])
+@pytest.mark.parametrize("tasks", [1, 40, 600])
+def test_real_orders_9_and_10(key, tasks, oracle):
+    """Classes that the lane-dense kernel takes at zero field alone, their
+    mirrors and one without a template pair, with units cut by the blocks and by
+    kernels of their own; then the same plan in a field (class-generic kernel)
+    and at zero field again.  Tolerances: the bars of the two precision modes."""
+    rng = np.random.default_rng(tasks + sum(key))
+    recs = _records(23, ls=key * 2, nprims=(2, 1, 1, 2, 1, 1, 2, 1), centers=(0, 1, 1, 2, 2, 1, 0, 2))
+    basis = basis_from_records(recs)
+    q = np.array([[rng.choice([k, 4 + k]) for k in range(4)] for _ in range(tasks)], dtype=np.uint32)
+    uniq, inv = np.unique(q, axis=0, return_inverse=True)
+    bits = {}
+    for turn, B in enumerate([(0.0, 0.0, 0.0), (0.12, -0.2, 0.07), (0.0, 0.0, 0.0)]):
+        ref, _ = oracle.eri_batch(recs, uniq.astype(np.uint32), B, None, 8)
+        for precision, bar in (("fp64", 1e-12), ("mixed", 1e-10)):
+            _, _, offsets, values, _, _ = _eri_batch(basis, q, field=gi.MagneticField(B), precision=precision)
+            want = ref.reshape(len(uniq), -1)[inv.reshape(-1)].reshape(-1)
+            assert np.abs(values - want).max() <= bar * max(1.0, np.abs(ref).max())
+            if turn == 0:
+                bits[precision] = values.copy()
+            elif turn == 2:
+                assert np.array_equal(values, bits[precision])
