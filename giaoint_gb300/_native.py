@@ -177,6 +177,7 @@ SIGNATURES = {
     "gx_measure_fp64_peak": (ctypes.c_int, [_vp, _d]),
     "gx_measure_fp32_peak": (ctypes.c_int, [_vp, _d]),
     "gx_canonical_quartets": (ctypes.c_int64, [ctypes.c_int, _u32]),
+    "gx_canonical_rows": (ctypes.c_int64, [ctypes.c_int, ctypes.c_int64, ctypes.c_int64, _u32]),
     "gx_cholesky_step_noalloc": (ctypes.c_int, [_vp, ctypes.c_int64, ctypes.c_int64, _vp, ctypes.c_int, ctypes.c_int,
                                                 _vp, _vp, _vp, _vp]),
 }

@@ -4895,25 +4895,30 @@ int gx_measure_fp32_peak(gx_context* ctx, double* tflops) {
 // Canonical representatives of the finite-field orbit {(ab|cd), (cd|ab),
 // (ba|dc)*, (dc|ba)*} in lexicographic order (src/eri.cpp:414-429, 825-843).
 // out may be NULL to count; returns the count.
-extern "C" int64_t gx_canonical_quartets(int ns, uint32_t* out) {
+// (a, b, c, d) is the least of its orbit: (a, b) <= (c, d) and (a, b) <= (d, c)
+// by their shells in order, a <= b, and c <= d when a == b.
+extern "C" int64_t gx_canonical_rows(int ns, int64_t first, int64_t last, uint32_t* out) {
     int64_t n = 0;
-    for (int a = 0; a < ns; ++a)
-        for (int b = 0; b < ns; ++b)
-            for (int c = 0; c < ns; ++c)
-                for (int d = 0; d < ns; ++d) {
-                    const std::array<int, 4> me{a, b, c, d};
-                    if (std::array<int, 4>{c, d, a, b} < me || std::array<int, 4>{b, a, d, c} < me ||
-                        std::array<int, 4>{d, c, b, a} < me)
-                        continue;
-                    if (out) {
-                        out[4 * n] = (uint32_t)a;
-                        out[4 * n + 1] = (uint32_t)b;
-                        out[4 * n + 2] = (uint32_t)c;
-                        out[4 * n + 3] = (uint32_t)d;
-                    }
-                    ++n;
+    for (int64_t row = std::max<int64_t>(first, 0); row < std::min(last, (int64_t)ns * ns); ++row) {
+        const int a = (int)(row / ns), b = (int)(row % ns);
+        if (b < a) continue;
+        for (int c = a; c < ns; ++c)
+            for (int d = a; d < ns; ++d) {
+                if ((c == a && d < b) || (d == a && c < b) || (a == b && d < c)) continue;
+                if (out) {
+                    out[4 * n] = (uint32_t)a;
+                    out[4 * n + 1] = (uint32_t)b;
+                    out[4 * n + 2] = (uint32_t)c;
+                    out[4 * n + 3] = (uint32_t)d;
                 }
+                ++n;
+            }
+    }
     return n;
+}
+
+extern "C" int64_t gx_canonical_quartets(int ns, uint32_t* out) {
+    return gx_canonical_rows(ns, 0, (int64_t)ns * ns, out);
 }
 
 namespace gx {

@@ -468,6 +468,8 @@ int gx_eri_plan_set_config(gx_eri_plan* plan, int precision, const gx_class_conf
  * order of compute_eri_tensor (src/eri.cpp:825-843).  out[4*count] may be
  * NULL to count only; returns the count. */
 int64_t gx_canonical_quartets(int ns, uint32_t* out);
+/* Those of the bra pairs a * ns + b in [first, last), in the same order. */
+int64_t gx_canonical_rows(int ns, int64_t first, int64_t last, uint32_t* out);
 
 /* Measured FP64 FMA throughput of the device (TFLOP/s) from a dependent-
  * chain probe kernel: the roofline denominator of the FP64-bound kernels. */
