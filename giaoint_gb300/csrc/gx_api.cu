@@ -258,7 +258,7 @@ struct gx_context {
     std::map<std::vector<long long>, std::shared_ptr<ShapeGraph>> shape_graphs;
     // page-locked staging of the Cholesky host loop (chain state, reduction,
     // status, chain log; the column-slot map), so its small copies never stall
-    PinnedHost chol_mail, chol_slots;
+    PinnedHost chol_mail, chol_slots, chol_cands, chol_residual, chol_counts;
     // Cholesky column plans by (basis, pivot shell pair, real path), kept
     // across factorisations of the same basis (fields change only the pair
     // records); dropped with the basis, cleared beyond kMaxColumnPlanBytes
@@ -3457,6 +3457,13 @@ struct gx_cholesky_factors {
 
 namespace {
 
+// Host's knowledge of a device counter array that accumulates over
+// factorisations: its value, when no evaluation has run since it was read.
+struct EvaluationCounts {
+    std::vector<unsigned long long> value;
+    bool known = false;
+};
+
 // Column evaluations replayed as CUDA graphs.  Pivot shell pairs of the
 // same kind (angular momenta and primitive counts) give column plans of the
 // same shape: the same classes, task counts and work units, only the task
@@ -3470,6 +3477,7 @@ namespace {
 struct ShapeGraph {
     PlanData plan;  // the shape's classes and units over buffers of its own
     DeviceBuffer counters;
+    EvaluationCounts counts;
     cudaGraphExec_t exec = nullptr;
     ~ShapeGraph() {
         if (exec) cudaGraphExecDestroy(exec);
@@ -3482,6 +3490,7 @@ struct ShapeGraph {
 struct ColumnPlan {
     PlanData plan;
     DeviceBuffer boff, flip, counters;
+    EvaluationCounts counts;
     int nblocks = 0;
     int64_t entries = 0;
 };
@@ -3584,11 +3593,19 @@ void cholesky_core(gx_context* ctx, gx_basis* b, const double* Bf, const double*
     };
 
     // ---- diagonal (with optional Schwarz skip of initial blocks) ----
-    DeviceBuffer d_D, d_res, d_partial, d_red, d_scale, d_work, d_boff, d_info, d_cand, d_dst;
+    DeviceBuffer d_D, d_res, d_partial, d_red, d_scale, d_work, d_boff, d_info, d_cand;
     d_D.reserve(N * sizeof(double));
     d_res.reserve(N * sizeof(double));
     d_partial.reserve(gx::chol_partial_bytes());
-    d_red.reserve(gx::chol_red_bytes());
+    // the loop's reduction result, chain state and cache slots side by side:
+    // one copy each way (red and state to the host, state and slots back)
+    constexpr size_t kRedBytes = 64, kStateBytes = 64;
+    static_assert(sizeof(CholRed) <= kRedBytes && sizeof(gx::ChainState) <= kStateBytes, "loop mailbox");
+    DeviceBuffer d_loop, d_state, d_slot_of;
+    d_loop.reserve(kRedBytes + kStateBytes + N * sizeof(int));
+    d_red.view(d_loop, 0, kRedBytes);
+    d_state.view(d_loop, kRedBytes, kStateBytes);
+    d_slot_of.view(d_loop, kRedBytes + kStateBytes, N * sizeof(int));
     d_scale.reserve(sizeof(double));
     GX_CUDA(cudaMemsetAsync(d_D.ptr, 0, N * sizeof(double), st));
     std::vector<double> q;
@@ -3651,20 +3668,33 @@ void cholesky_core(gx_context* ctx, gx_basis* b, const double* Bf, const double*
     // page-locked mailbox of the loop's small transfers (asynchronous both ways)
     constexpr int kMailLog = 256;
     struct Mail {
-        gx::ChainState cs_in, cs_out;
-        CholRed red;
+        char loop[kRedBytes + kStateBytes];
         int status, pad;
         long long log[kMailLog];
     };
     ctx->chol_mail.reserve(sizeof(Mail));
     Mail* mail = static_cast<Mail*>(ctx->chol_mail.p);
+    // Residual on the host after every wait, up to 512 KB (about 10 us; the
+    // copy and wait for one block of it 17 us, once per evaluation): the
+    // candidates are chosen from it without a wait of their own.
+    constexpr int64_t kMirror = 1 << 16;
+    double* mirror = nullptr;
+    if (N <= kMirror) {
+        ctx->chol_residual.reserve(N * sizeof(double));
+        mirror = static_cast<double*>(ctx->chol_residual.p);
+    }
+    gx::ChainState chain_state{};
     auto fetch_red = [&] {
-        // the reduction result and the kernels' status word in one wait (a
-        // failure in a column batch is reported before the next pivot)
-        GX_CUDA(cudaMemcpyAsync(&mail->red, d_red.ptr, sizeof(CholRed), cudaMemcpyDeviceToHost, st));
+        // the reduction result, the chain's state and the kernels' status word
+        // in one wait (a failure in a column batch is reported before the next
+        // pivot)
+        GX_CUDA(cudaMemcpyAsync(mail->loop, d_loop.ptr, sizeof mail->loop, cudaMemcpyDeviceToHost, st));
         GX_CUDA(cudaMemcpyAsync(&mail->status, ctx->status.ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
+        if (mirror)
+            GX_CUDA(cudaMemcpyAsync(mirror, d_res.ptr, N * sizeof(double), cudaMemcpyDeviceToHost, st));
         GX_CUDA(cudaStreamSynchronize(st));
-        red = mail->red;
+        std::memcpy(&red, mail->loop, sizeof red);
+        std::memcpy(&chain_state, mail->loop + kRedBytes, sizeof chain_state);
         status_code = mail->status;
         collect_times();
         if (status_code) check_status(ctx);
@@ -3710,16 +3740,14 @@ void cholesky_core(gx_context* ctx, gx_basis* b, const double* Bf, const double*
     // Chained steps (no local block rule): the device takes the next pivots
     // itself while their raw columns are cached; slot_of mirrors the cache.
     const bool chain_ok = !local_rule;
-    DeviceBuffer d_slot_of, d_state, d_log;
+    DeviceBuffer d_log;
     std::vector<int> slot_of_h;
     bool slot_dirty = true;
     int chain_k = 8;
     slot_of_h.assign(N, -1);  // cache slot of every flat index (-1: not cached)
     if (chain_ok) {
-        d_slot_of.reserve(N * sizeof(int));
-        d_state.reserve(sizeof(gx::ChainState));
         d_log.reserve(std::max<int64_t>(limit, 1) * sizeof(long long));
-        ctx->chol_slots.reserve(N * sizeof(int));
+        ctx->chol_slots.reserve(kStateBytes + N * sizeof(int));
     }
     struct GraphSet {  // instantiated chain graphs, destroyed with the factorisation
         std::map<std::tuple<int, void*, int>, cudaGraphExec_t> m;
@@ -3746,9 +3774,27 @@ void cholesky_core(gx_context* ctx, gx_basis* b, const double* Bf, const double*
     std::vector<int64_t> ref_cands, block_cands;
     KeyOrder ref_cache;
     std::vector<double> hostblk;
-    // the context's column plans this factorisation used (held) and their
-    // counters when it began
-    std::map<ColumnPlan*, std::pair<std::shared_ptr<ColumnPlan>, std::vector<unsigned long long>>> plan_base;
+    // the context's column plans this factorisation used (held), their counters
+    // when it began, and whether their launches were its own (not a graph's)
+    struct PlanBase {
+        std::shared_ptr<ColumnPlan> plan;
+        std::vector<unsigned long long> counts;
+        bool direct;
+    };
+    std::map<ColumnPlan*, PlanBase> plan_base;
+    // counters of a plan or shape at the start of its use here: read from the
+    // device only when the last factorisation that used it did not finish
+    auto counts_before = [&](EvaluationCounts& ec, const DeviceBuffer& counters, size_t classes) {
+        if (!ec.known) {
+            ec.value.assign(2 * classes, 0);
+            if (classes)
+                GX_CUDA(cudaMemcpyAsync(ec.value.data(), counters.ptr, 2 * classes * sizeof(unsigned long long),
+                                        cudaMemcpyDeviceToHost, st));
+            GX_CUDA(cudaStreamSynchronize(st));
+        }
+        ec.known = false;
+        return ec.value;
+    };
     DeviceBuffer column_info;
     // Column evaluations replayed as CUDA graphs (ShapeGraph), cached in the
     // context across factorisations.
@@ -3768,6 +3814,10 @@ void cholesky_core(gx_context* ctx, gx_basis* b, const double* Bf, const double*
     int64_t rank = 0;
     auto residual_at = [&](const std::vector<int64_t>& idx, std::vector<double>& vals) {
         vals.resize(idx.size());
+        if (mirror) {
+            for (size_t k = 0; k < idx.size(); ++k) vals[k] = mirror[idx[k]];
+            return;
+        }
         for (size_t k = 0; k < idx.size(); ++k)
             GX_CUDA(cudaMemcpyAsync(&vals[k], d_res.as<double>() + idx[k], sizeof(double), cudaMemcpyDeviceToHost,
                                     st));
@@ -3778,8 +3828,8 @@ void cholesky_core(gx_context* ctx, gx_basis* b, const double* Bf, const double*
         cands.clear();
         cand_slot.clear();
     };
-    // Residual of the pivot's shell-pair block on the host (one strided 2-D
-    // copy) and the reference's candidate list: the contraction variants of
+    // Residual of the pivot's shell-pair block on the host (from the mirror, or
+    // by one strided 2-D copy) and the reference's candidate list: the contraction variants of
     // the pivot (reuse) or the whole block, above the tolerance, largest
     // residual first (stable), at most `count`, the pivot forced in
     // (cholesky.py:225-242).
@@ -3791,10 +3841,14 @@ void cholesky_core(gx_context* ctx, gx_basis* b, const double* Bf, const double*
         if (a == blk_a && c == blk_c && blk_rank == rank) return;
         const int64_t na = b->nao_of(a), nc = b->nao_of(c);
         hostblk.resize(na * nc);
-        GX_CUDA(cudaMemcpy2DAsync(hostblk.data(), nc * sizeof(double),
-                                  d_res.as<double>() + b->ao_off[a] * n + b->ao_off[c], n * sizeof(double),
-                                  nc * sizeof(double), na, cudaMemcpyDeviceToHost, st));
-        GX_CUDA(cudaStreamSynchronize(st));
+        const int64_t first = b->ao_off[a] * n + b->ao_off[c];
+        if (mirror) {
+            for (int64_t i = 0; i < na; ++i) std::copy_n(mirror + first + i * n, nc, hostblk.data() + i * nc);
+        } else {
+            GX_CUDA(cudaMemcpy2DAsync(hostblk.data(), nc * sizeof(double), d_res.as<double>() + first,
+                                      n * sizeof(double), nc * sizeof(double), na, cudaMemcpyDeviceToHost, st));
+            GX_CUDA(cudaStreamSynchronize(st));
+        }
         blk_a = a;
         blk_c = c;
         blk_rank = rank;
@@ -3974,18 +4028,13 @@ void cholesky_core(gx_context* ctx, gx_basis* b, const double* Bf, const double*
                     cp->counters.reserve(std::max<size_t>(2 * cp->plan.classes.size(), 2) *
                                          sizeof(unsigned long long));
                     GX_CUDA(cudaMemsetAsync(cp->counters.ptr, 0, cp->counters.bytes, st));
+                    cp->counts = {std::vector<unsigned long long>(2 * cp->plan.classes.size(), 0), true};
                     ctx->column_plan_bytes += cp->plan.tasks.bytes + cp->plan.base.dev.bytes + cp->plan.unit_mem.bytes +
                                               cp->boff.bytes;
                 }
-                if (!plan_base.count(cp.get())) {
-                    std::vector<unsigned long long> c(2 * cp->plan.classes.size());
-                    if (!c.empty()) {
-                        GX_CUDA(cudaMemcpyAsync(c.data(), cp->counters.ptr, c.size() * sizeof(unsigned long long),
-                                                cudaMemcpyDeviceToHost, st));
-                        GX_CUDA(cudaStreamSynchronize(st));
-                    }
-                    plan_base.emplace(cp.get(), std::make_pair(cp, std::move(c)));
-                }
+                if (!plan_base.count(cp.get()))
+                    plan_base.emplace(cp.get(), PlanBase{cp, counts_before(cp->counts, cp->counters,
+                                                                           cp->plan.classes.size()), false});
                 cps.push_back(cp.get());
                 sbase.push_back(stot);
                 stot += cp->entries;
@@ -3999,20 +4048,28 @@ void cholesky_core(gx_context* ctx, gx_basis* b, const double* Bf, const double*
                                                  (int)b->nao_of(y), x == y ? 1 : 0});
                 upload(column_info, info, st);
             }
-            std::vector<int> cl;
-            std::vector<void*> dst;
+            // column destinations, then the columns' components, in one copy from
+            // page-locked memory (the last one from there ended with the previous
+            // iteration's wait)
+            size_t ncol = 0;
+            for (const auto& bl : blocks) ncol += bl.cols.size();
+            const size_t col_words = ncol * (sizeof(void*) + 2 * sizeof(int));
+            ctx->chol_cands.reserve(col_words);
+            void** dst = static_cast<void**>(ctx->chol_cands.p);
+            int* cl = reinterpret_cast<int*>(dst + ncol);
+            size_t col = 0;
             std::vector<std::vector<int>> bslots(blocks.size());
             for (size_t k = 0; k < blocks.size(); ++k)
                 for (int64_t fl : blocks[k].cols) {
-                    cl.push_back((int)(fl % n - b->ao_off[blocks[k].sb]));  // c: p1 within sb
-                    cl.push_back((int)(fl / n - b->ao_off[blocks[k].sa]));  // d: p0 within sa
+                    cl[2 * col] = (int)(fl % n - b->ao_off[blocks[k].sb]);      // c: p1 within sb
+                    cl[2 * col + 1] = (int)(fl / n - b->ao_off[blocks[k].sa]);  // d: p0 within sa
                     const int slot = pool.take();
                     bslots[k].push_back(slot);
-                    dst.push_back(pool.ptr(slot));
+                    dst[col++] = pool.ptr(slot);
                 }
             cand_slot = bslots[0];
-            upload(d_cand, cl, st);
-            upload(d_dst, dst, st);
+            d_cand.reserve(col_words);
+            GX_CUDA(cudaMemcpyAsync(d_cand.ptr, dst, col_words, cudaMemcpyHostToDevice, st));
             GX_CUDA(cudaEventRecord(ev_col.a, st));
             {
                 // the blocks' class launches share one fork/join over the
@@ -4046,6 +4103,7 @@ void cholesky_core(gx_context* ctx, gx_basis* b, const double* Bf, const double*
                         make_units(ctx, sp);
                         sg->counters.reserve(std::max<size_t>(2 * pd.classes.size(), 2) * sizeof(unsigned long long));
                         GX_CUDA(cudaMemsetAsync(sg->counters.ptr, 0, sg->counters.bytes, st));
+                        sg->counts = {std::vector<unsigned long long>(2 * pd.classes.size(), 0), true};
                         cudaGraph_t graph = nullptr;
                         GX_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
                         try {
@@ -4065,17 +4123,14 @@ void cholesky_core(gx_context* ctx, gx_basis* b, const double* Bf, const double*
                                             cudaMemcpyDeviceToDevice, st));
                     GX_CUDA(cudaMemcpyAsync(sg->plan.base.dev.ptr, pd.base.dev.ptr, pd.base.dev.bytes,
                                             cudaMemcpyDeviceToDevice, st));
-                    if (!shape_base.count(sg.get())) {
-                        // the counters accumulate across factorisations: note where this one starts
-                        std::vector<unsigned long long> c(2 * pd.classes.size());
-                        GX_CUDA(cudaMemcpyAsync(c.data(), sg->counters.ptr, c.size() * sizeof(unsigned long long),
-                                                cudaMemcpyDeviceToHost, st));
-                        GX_CUDA(cudaStreamSynchronize(st));
-                        shape_base.emplace(sg.get(), std::make_pair(sg, std::move(c)));
-                    }
+                    // the counters accumulate across factorisations: note where this one starts
+                    if (!shape_base.count(sg.get()))
+                        shape_base.emplace(sg.get(), std::make_pair(sg, counts_before(sg->counts, sg->counters,
+                                                                                      pd.classes.size())));
                     GX_CUDA(cudaGraphLaunch(sg->exec, st));
                 } else {
                     enqueue_plans(ctx, runs, GX_PRECISION_FP64, ctr);
+                    for (auto* cp : cps) plan_base[cp].direct = true;
                 }
             }
             int64_t coff = 0;
@@ -4084,9 +4139,9 @@ void cholesky_core(gx_context* ctx, gx_basis* b, const double* Bf, const double*
                 if (ncand)
                     GX_CUDA(gx::launch_chol_cols(real, ctx->scratch_a.as<double2>() + sbase[k], cps[k]->boff.as<long long>(),
                                                  column_info.as<int>(), cps[k]->flip.as<int>(), cps[k]->nblocks,
-                                                 d_cand.as<int>() + 2 * coff,
+                                                 reinterpret_cast<int*>(d_cand.as<void*>() + ncol) + 2 * coff,
                                                  ncand, (int)b->nao_of(blocks[k].sb), (int)b->nao_of(blocks[k].sa),
-                                                 (int)n, d_dst.as<void*>() + coff, st));
+                                                 (int)n, d_cand.as<void*>() + coff, st));
                 coff += ncand;
             }
             GX_CUDA(cudaEventRecord(ev_col.b, st));
@@ -4141,21 +4196,19 @@ void cholesky_core(gx_context* ctx, gx_basis* b, const double* Bf, const double*
         std::vector<long long> chain_log;
         int64_t nlog = 0;
         if (chained) {
-            if (slot_dirty) {
-                // (the previous upload from the staging copy ended with the
-                // previous iteration's synchronisation)
-                std::memcpy(ctx->chol_slots.p, slot_of_h.data(), N * sizeof(int));
-                GX_CUDA(cudaMemcpyAsync(d_slot_of.ptr, ctx->chol_slots.p, N * sizeof(int), cudaMemcpyHostToDevice,
-                                        st));
-                slot_dirty = false;
-            }
             gx::ChainState cs{};
             cs.slot = -1;
             cs.rank = (int)rank + 1;
             cs.active = 1;
             cs.rank_limit = (int)std::min<int64_t>(limit, f.cap_rows);
-            mail->cs_in = cs;
-            GX_CUDA(cudaMemcpyAsync(d_state.ptr, &mail->cs_in, sizeof cs, cudaMemcpyHostToDevice, st));
+            // (the previous upload from the staging copy ended with the
+            // previous iteration's synchronisation)
+            char* staged = static_cast<char*>(ctx->chol_slots.p);
+            std::memcpy(staged, &cs, sizeof cs);
+            if (slot_dirty) std::memcpy(staged + kStateBytes, slot_of_h.data(), N * sizeof(int));
+            GX_CUDA(cudaMemcpyAsync(d_state.ptr, staged, slot_dirty ? kStateBytes + N * sizeof(int) : sizeof cs,
+                                    cudaMemcpyHostToDevice, st));
+            slot_dirty = false;
             // the chain's launches replayed as one CUDA graph per (length,
             // factor buffer, rank-chunk count): one launch instead of three per step
             const int rank_hi = (int)rank + 1 + chain_k;
@@ -4190,7 +4243,6 @@ void cholesky_core(gx_context* ctx, gx_basis* b, const double* Bf, const double*
                 git = chain_graphs.emplace(gkey, exec).first;
             }
             if (capturable) GX_CUDA(cudaGraphLaunch(git->second, st));
-            GX_CUDA(cudaMemcpyAsync(&mail->cs_out, d_state.ptr, sizeof cs_out, cudaMemcpyDeviceToHost, st));
             // the log holds `limit` entries; the chain writes at most up to rank_limit <= limit
             nlog = std::min<int64_t>(std::min<int64_t>(chain_k, kMailLog), limit - (rank + 1));
             GX_CUDA(cudaMemcpyAsync(mail->log, d_log.as<long long>() + rank + 1, nlog * sizeof(long long),
@@ -4204,7 +4256,7 @@ void cholesky_core(gx_context* ctx, gx_basis* b, const double* Bf, const double*
         stats.update_flops += (real ? 2.0 : 8.0) * (double)rank * N;
         fetch_red();
         if (chained) {
-            cs_out = mail->cs_out;
+            cs_out = chain_state;
             chain_log.assign(mail->log, mail->log + nlog);
         }
         f.pivots.push_back(pivot / n);
@@ -4247,20 +4299,43 @@ void cholesky_core(gx_context* ctx, gx_basis* b, const double* Bf, const double*
     }
     // primitive quartets of the column evaluations and their FP64 FLOP model
     // (counted per plan when launched directly, per shape when replayed)
-    auto add_counts = [&](const PlanData& pd, const DeviceBuffer& counters, const std::vector<unsigned long long>* base) {
-        std::vector<unsigned long long> c(2 * pd.classes.size());
-        if (c.empty()) return;
-        GX_CUDA(cudaMemcpyAsync(c.data(), counters.ptr, c.size() * sizeof(unsigned long long),
-                                cudaMemcpyDeviceToHost, st));
-        GX_CUDA(cudaStreamSynchronize(st));
-        for (size_t i = 0; i < pd.classes.size(); ++i) {
-            const unsigned long long v = c[2 * i] - (base ? (*base)[2 * i] : 0ull);
-            stats.column_primitive_quartets += (int64_t)v;
-            stats.column_model_flops += (double)v * pd.classes[i].flops_per_primitive_quartet;
-        }
+    struct Counted {
+        const PlanData* plan;
+        EvaluationCounts* counts;
+        const DeviceBuffer* counters;
+        const std::vector<unsigned long long>* before;
     };
-    for (const auto& kv : plan_base) add_counts(kv.first->plan, kv.first->counters, &kv.second.second);
-    for (const auto& kv : shape_base) add_counts(kv.first->plan, kv.first->counters, &kv.second.second);
+    std::vector<Counted> counted;
+    for (auto& kv : plan_base) {
+        if (kv.second.direct)
+            counted.push_back({&kv.first->plan, &kv.first->counts, &kv.first->counters, &kv.second.counts});
+        else
+            kv.first->counts.known = true;  // (no launch of this factorisation added to them)
+    }
+    for (auto& kv : shape_base)
+        counted.push_back({&kv.first->plan, &kv.first->counts, &kv.first->counters, &kv.second.second});
+    size_t nread = 0;
+    for (const auto& c : counted) nread += c.before->size();
+    ctx->chol_counts.reserve(std::max<size_t>(nread, 1) * sizeof(unsigned long long));
+    auto* now = static_cast<unsigned long long*>(ctx->chol_counts.p);
+    for (const auto& c : counted) {
+        if (!c.before->empty())
+            GX_CUDA(cudaMemcpyAsync(now, c.counters->ptr, c.before->size() * sizeof(unsigned long long),
+                                    cudaMemcpyDeviceToHost, st));
+        now += c.before->size();
+    }
+    GX_CUDA(cudaStreamSynchronize(st));
+    now = static_cast<unsigned long long*>(ctx->chol_counts.p);
+    for (const auto& c : counted) {
+        for (size_t i = 0; i < c.plan->classes.size(); ++i) {
+            const unsigned long long v = now[2 * i] - (*c.before)[2 * i];
+            stats.column_primitive_quartets += (int64_t)v;
+            stats.column_model_flops += (double)v * c.plan->classes[i].flops_per_primitive_quartet;
+        }
+        c.counts->value.assign(now, now + c.before->size());
+        c.counts->known = true;
+        now += c.before->size();
+    }
     f.rank = rank;
     f.max_residual = final_max;
     stats.rank = rank;
