@@ -13,6 +13,7 @@
 //                        (cholesky.py:269-281)
 //   argmax reductions    lowest flat index on ties (NumPy argmax order)
 #include <algorithm>
+#include <type_traits>
 
 #include "gx_internal.h"
 
@@ -98,67 +99,92 @@ cudaError_t launch_chol_cols(bool real, const double2* packed, const long long* 
 
 // ---- argmax / min reductions -------------------------------------------------
 
+// Largest value (the lowest index among equals) and smallest value.  The
+// reductions compare order-preserving integer keys: an FP64 comparison occupies
+// its sub-partition for 64 cycles, and the butterflies over (value, index,
+// minimum) were most of a 9 us step end (chain_update_kernel, 1,600 entries).
 struct Red {
     double maxv;
     long long idx;
     double minv;
 };
+struct RedKey {
+    long long maxk, idx, mink;
+};
 
-__device__ __forceinline__ void red_merge(Red& a, const Red& b) {
-    if (b.maxv > a.maxv || (b.maxv == a.maxv && b.idx < a.idx)) {
-        a.maxv = b.maxv;
-        a.idx = b.idx;
-    }
-    a.minv = fmin(a.minv, b.minv);
+__device__ __forceinline__ long long red_order(long long bits) { return bits ^ ((bits >> 63) & 0x7fffffffffffffffll); }
+// (NaN takes part in neither, as in a comparison; -0 counts as 0)
+__device__ __forceinline__ RedKey red_key(double v, long long j, double low) {
+    const long long v0 = __double_as_longlong(v), l0 = __double_as_longlong(low);
+    constexpr long long kInf = 0x7ff0000000000000ll, kAbs = 0x7fffffffffffffffll;
+    RedKey k;
+    k.maxk = (v0 & kAbs) > kInf ? red_order(kInf | (1ll << 63)) : red_order((v0 & kAbs) == 0 ? 0 : v0);
+    k.idx = j;
+    k.mink = (l0 & kAbs) > kInf ? kInf : red_order((l0 & kAbs) == 0 ? 0 : l0);
+    return k;
+}
+__device__ __forceinline__ RedKey red_none() { return red_key(-1.0 / 0.0, (long long)1 << 62, 1.0 / 0.0); }
+__device__ __forceinline__ Red red_value(const RedKey& k) {
+    return Red{__longlong_as_double(red_order(k.maxk)), k.idx, __longlong_as_double(red_order(k.mink))};
 }
 
-__device__ Red block_reduce(Red r) {
-    __shared__ Red sh[32];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int o = 16; o > 0; o >>= 1) {
-        Red t;
-        t.maxv = __shfl_down_sync(0xffffffffu, r.maxv, o);
-        t.idx = __shfl_down_sync(0xffffffffu, r.idx, o);
-        t.minv = __shfl_down_sync(0xffffffffu, r.minv, o);
-        red_merge(r, t);
+__device__ __forceinline__ void red_merge(RedKey& a, const RedKey& b) {
+    if (b.maxk > a.maxk || (b.maxk == a.maxk && b.idx < a.idx)) {
+        a.maxk = b.maxk;
+        a.idx = b.idx;
     }
-    if (lane == 0) sh[w] = r;
-    __syncthreads();
-    if (w == 0) {
-        r = lane < (int)(blockDim.x >> 5) ? sh[lane] : Red{-1.0 / 0.0, (long long)1 << 62, 1.0 / 0.0};
-        for (int o = 16; o > 0; o >>= 1) {
-            Red t;
-            t.maxv = __shfl_down_sync(0xffffffffu, r.maxv, o);
-            t.idx = __shfl_down_sync(0xffffffffu, r.idx, o);
-            t.minv = __shfl_down_sync(0xffffffffu, r.minv, o);
-            red_merge(r, t);
-        }
+    a.mink = min(a.mink, b.mink);
+}
+
+__device__ __forceinline__ RedKey warp_reduce(RedKey r, int lanes) {
+    for (int o = lanes / 2; o > 0; o >>= 1) {
+        RedKey t;
+        t.maxk = __shfl_down_sync(0xffffffffu, r.maxk, o);
+        t.idx = __shfl_down_sync(0xffffffffu, r.idx, o);
+        t.mink = __shfl_down_sync(0xffffffffu, r.mink, o);
+        red_merge(r, t);
     }
     return r;
 }
 
-constexpr int RED_BLOCKS = 256;
+// (blocks of at most eight warps)
+__device__ RedKey block_reduce(RedKey r) {
+    __shared__ RedKey sh[8];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    r = warp_reduce(r, 32);
+    if (lane == 0) sh[w] = r;
+    __syncthreads();
+    if (w == 0) r = warp_reduce(lane < (int)(blockDim.x >> 5) ? sh[lane] : red_none(), 8);
+    return r;
+}
 
-__global__ void chol_scan_kernel(const double* res, long long N, Red* partial) {
-    Red r{-1.0 / 0.0, (long long)1 << 62, 1.0 / 0.0};
+// Blocks of the reductions over N entries, an entry per thread until the
+// partials fill one block.
+constexpr int RED_BLOCKS = 256, RED_THREADS = 128;
+int red_blocks(long long N) {
+    return (int)std::max<long long>(1, std::min<long long>((N + RED_THREADS - 1) / RED_THREADS, RED_BLOCKS));
+}
+
+__global__ void chol_scan_kernel(const double* res, long long N, RedKey* partial) {
+    RedKey r = red_none();
     for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j < N; j += (long long)gridDim.x * blockDim.x) {
         const double v = res[j];
-        red_merge(r, Red{v, j, v});
+        red_merge(r, red_key(v, j, v));
     }
     r = block_reduce(r);
     if (threadIdx.x == 0) partial[blockIdx.x] = r;
 }
 
-__global__ void chol_final_kernel(const Red* partial, int np, Red* out) {
-    Red r{-1.0 / 0.0, (long long)1 << 62, 1.0 / 0.0};
+__global__ void chol_final_kernel(const RedKey* partial, int np, Red* out) {
+    RedKey r = red_none();
     for (int i = threadIdx.x; i < np; i += blockDim.x) red_merge(r, partial[i]);
     r = block_reduce(r);
-    if (threadIdx.x == 0) *out = r;
+    if (threadIdx.x == 0) *out = red_value(r);
 }
 
 cudaError_t launch_chol_scan(const double* res, long long N, void* partial, void* out, cudaStream_t s) {
-    chol_scan_kernel<<<RED_BLOCKS, 256, 0, s>>>(res, N, static_cast<Red*>(partial));
-    chol_final_kernel<<<1, 256, 0, s>>>(static_cast<const Red*>(partial), RED_BLOCKS, static_cast<Red*>(out));
+    chol_scan_kernel<<<red_blocks(N), RED_THREADS, 0, s>>>(res, N, static_cast<RedKey*>(partial));
+    chol_final_kernel<<<1, 256, 0, s>>>(static_cast<const RedKey*>(partial), red_blocks(N), static_cast<Red*>(out));
     return cudaGetLastError();
 }
 
@@ -173,74 +199,95 @@ __device__ __forceinline__ double2 conj_mul_sub(double2 acc, double2 a, double2 
     return c2(fma(-a.y, b.y, fma(-a.x, b.x, acc.x)), fma(a.y, b.x, fma(-a.x, b.y, acc.y)));
 }
 
-template <typename T>
-__global__ void chol_gemv_kernel(const T* L, long long ld, int rank, long long piv, const T* col_in, T* col_out,
-                                 long long N) {
-    __shared__ T coef[256];
-    const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    T acc;
-    if constexpr (sizeof(T) == 8) {
-        acc = j < N ? col_in[j] : T(0);
-    } else {
-        acc = j < N ? col_in[j] : c2(0.0, 0.0);
+// What a thread of the factor update sums: a column entry, or with HALVES the
+// real or imaginary part of one.  The rows of a few thousand entries come from
+// the L2 cache, and an entry's four dependent-pair FMAs per complex row, 31 ns
+// each for a warp alone on its sub-partition, are the time of the update: two
+// threads halve it (1,000 entries at rank 400, eight chunks: @@ us for one,
+// @@ for two) with the same operations in the same order.  Long columns, bound
+// by memory, keep whole entries.
+template <typename T, bool HALVES>
+struct Entry {
+    using Acc = std::conditional_t<HALVES, double, T>;
+    long long j;
+    int part = 0;
+    __device__ __forceinline__ explicit Entry(long long t) : j(HALVES ? t >> 1 : t) {
+        if (HALVES) part = (int)(t & 1);
     }
-    for (int r0 = 0; r0 < rank; r0 += 256) {
-        const int nr = min(256, rank - r0);
+    __device__ __forceinline__ static Acc zero() {
+        if constexpr (std::is_same_v<Acc, double>)
+            return 0.0;
+        else
+            return c2(0.0, 0.0);
+    }
+    __device__ __forceinline__ long long at(long long row) const { return HALVES ? 2 * row + part : row; }
+};
+
+// acc +/- the sum of conj(L[r, piv]) L[r, j] over rows rbeg .. rend - 1, in
+// order (all threads of a block call this; coef: 256 entries of shared memory)
+template <typename T, bool HALVES, bool SUB>
+__device__ __forceinline__ typename Entry<T, HALVES>::Acc gemv_rows(typename Entry<T, HALVES>::Acc acc,
+                                                                   const Entry<T, HALVES>& e, const T* L,
+                                                                   long long ld, int rbeg, int rend, long long piv,
+                                                                   long long N, T* coef) {
+    for (int r0 = rbeg; r0 < rend; r0 += 256) {
+        const int nr = min(256, rend - r0);
         __syncthreads();
         for (int i = threadIdx.x; i < nr; i += blockDim.x) coef[i] = L[(long long)(r0 + i) * ld + piv];
         __syncthreads();
-        if (j < N) {
-            // eight independent row loads in flight per thread: the GEMV is
-            // bound by HBM bandwidth, not by load latency
+        if (e.j < N) {
+            // eight independent row loads in flight per thread: the GEMV of a
+            // long column is bound by HBM bandwidth, not by load latency
 #pragma unroll 8
             for (int r = 0; r < nr; ++r) {
-                const T lv = __ldg(&L[(long long)(r0 + r) * ld + j]);
+                const T lv = __ldg(&L[(long long)(r0 + r) * ld + e.j]);
                 if constexpr (sizeof(T) == 8) {
-                    acc -= coef[r] * lv;
+                    acc = fma(SUB ? -coef[r] : coef[r], lv, acc);
+                } else if constexpr (HALVES) {
+                    // re: fma(a.y, b.y, fma(a.x, b.x, acc)); im: fma(-a.y, b.x, fma(a.x, b.y, acc))
+                    const double2 a = SUB ? c2(-coef[r].x, -coef[r].y) : coef[r];
+                    const double u = e.part ? lv.y : lv.x;
+                    const double w = e.part ? __hiloint2double(__double2hiint(lv.x) ^ 0x80000000, __double2loint(lv.x))
+                                            : lv.y;
+                    acc = fma(a.y, w, fma(a.x, u, acc));
                 } else {
-                    acc = conj_mul_sub(acc, coef[r], lv);
+                    acc = SUB ? conj_mul_sub(acc, coef[r], lv) : conj_mul_add(acc, coef[r], lv);
                 }
             }
         }
     }
-    if (j < N) col_out[j] = acc;
+    return acc;
+}
+
+template <typename T, bool HALVES>
+__global__ void chol_gemv_kernel(const T* L, long long ld, int rank, long long piv, const T* col_in, T* col_out,
+                                 long long N) {
+    __shared__ T coef[256];
+    using Acc = typename Entry<T, HALVES>::Acc;
+    const Entry<T, HALVES> e((long long)blockIdx.x * blockDim.x + threadIdx.x);
+    Acc acc = e.j < N ? reinterpret_cast<const Acc*>(col_in)[e.at(e.j)] : Entry<T, HALVES>::zero();
+    acc = gemv_rows<T, HALVES, true>(acc, e, L, ld, 0, rank, piv, N, coef);
+    if (e.j < N) reinterpret_cast<Acc*>(col_out)[e.at(e.j)] = acc;
 }
 
 // The same update with the rank split over blockIdx.y: block (x, y) sums
 // conj(L[r, piv]) L[r, j] over its rows into partials[y][j], and
 // chol_gemv_sum_kernel subtracts the chunks in order.  Small n (few column
 // entries) otherwise leaves too few loads in flight to stream L at HBM speed.
-template <typename T>
+template <typename T, bool HALVES>
 __global__ void chol_gemv_split_kernel(const T* L, long long ld, int rank, long long piv, int chunk, T* partials,
                                        long long N) {
     __shared__ T coef[256];
-    const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    using Acc = typename Entry<T, HALVES>::Acc;
+    const Entry<T, HALVES> e((long long)blockIdx.x * blockDim.x + threadIdx.x);
     const int rbeg = blockIdx.y * chunk, rend = min(rank, rbeg + chunk);
-    T acc;
-    if constexpr (sizeof(T) == 8) {
-        acc = T(0);
-    } else {
-        acc = c2(0.0, 0.0);
-    }
-    for (int r0 = rbeg; r0 < rend; r0 += 256) {
-        const int nr = min(256, rend - r0);
-        __syncthreads();
-        for (int i = threadIdx.x; i < nr; i += blockDim.x) coef[i] = L[(long long)(r0 + i) * ld + piv];
-        __syncthreads();
-        if (j < N) {
-#pragma unroll 8
-            for (int r = 0; r < nr; ++r) {
-                const T lv = __ldg(&L[(long long)(r0 + r) * ld + j]);
-                if constexpr (sizeof(T) == 8) {
-                    acc += coef[r] * lv;
-                } else {
-                    acc = conj_mul_add(acc, coef[r], lv);
-                }
-            }
-        }
-    }
-    if (j < N) partials[(long long)blockIdx.y * N + j] = acc;
+    const Acc acc = gemv_rows<T, HALVES, false>(Entry<T, HALVES>::zero(), e, L, ld, rbeg, rend, piv, N, coef);
+    if (e.j < N) reinterpret_cast<Acc*>(partials)[e.at((long long)blockIdx.y * N + e.j)] = acc;
 }
+
+// Two threads per complex entry while the doubled grid leaves at most two
+// warps on a sub-partition.
+bool gemv_halves(bool real, int blocks, int nchunks, int sms) { return !real && 2 * blocks * nchunks <= 2 * sms; }
 
 template <typename T>
 __global__ void chol_gemv_sum_kernel(const T* col_in, const T* partials, int nchunks, long long N, T* col_out) {
@@ -257,20 +304,25 @@ __global__ void chol_gemv_sum_kernel(const T* col_in, const T* partials, int nch
     }
 }
 
+// entry (nu mu) of entry j = (mu nu)
+__device__ __forceinline__ long long transposed(long long j, int n) {
+    const unsigned mu = (unsigned long long)j >> 32 ? (unsigned)(j / n) : (unsigned)j / (unsigned)n;
+    return (j - (long long)mu * n) * n + mu;
+}
+
 // scale = 1/sqrt(residual[piv]) (read before the update)
 __global__ void chol_scale_kernel(const double* res, long long piv, double* scale) { *scale = rsqrt(res[piv]); }
 
 template <typename T>
 __global__ void chol_update_kernel(const T* col, int n, long long piv, const double* scale, T* Lrow, double* res,
-                                   Red* partial) {
+                                   RedKey* partial) {
     const long long N = (long long)n * n;
     const double sc = *scale;
-    Red r{-1.0 / 0.0, (long long)1 << 62, 1.0 / 0.0};
+    RedKey r = red_none();
     for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j < N; j += (long long)gridDim.x * blockDim.x) {
         double mag2;
         if constexpr (sizeof(T) == 8) {
-            const long long mu = j / n, nu = j - mu * n;
-            const double c = (col[j] + col[nu * n + mu]) * 0.5 * sc;
+            const double c = (col[j] + col[transposed(j, n)]) * 0.5 * sc;
             Lrow[j] = c;
             mag2 = c * c;
         } else {
@@ -281,7 +333,7 @@ __global__ void chol_update_kernel(const T* col, int n, long long piv, const dou
         const double nr = res[j] - mag2;
         const double kept = j == piv ? 0.0 : fmax(nr, 0.0);
         res[j] = kept;
-        red_merge(r, Red{kept, j, nr});
+        red_merge(r, red_key(kept, j, nr));
     }
     r = block_reduce(r);
     if (threadIdx.x == 0) partial[blockIdx.x] = r;
@@ -302,37 +354,41 @@ cudaError_t launch_chol_step(bool real, const void* L, long long ld, int rank, l
         const dim3 grid(blocks, nchunks);
         const int sblocks = (int)std::min<long long>((N + 255) / 256, 8LL * sms);
         if (real) {
-            chol_gemv_split_kernel<double><<<grid, 128, 0, s>>>(static_cast<const double*>(L), ld, rank, piv, chunk,
-                                                                static_cast<double*>(gemv_partials), N);
+            chol_gemv_split_kernel<double, false><<<grid, 128, 0, s>>>(
+                static_cast<const double*>(L), ld, rank, piv, chunk, static_cast<double*>(gemv_partials), N);
             chol_gemv_sum_kernel<double><<<sblocks, 256, 0, s>>>(static_cast<const double*>(column),
                                                                   static_cast<const double*>(gemv_partials), nchunks,
                                                                   N, static_cast<double*>(work));
         } else {
-            chol_gemv_split_kernel<double2><<<grid, 128, 0, s>>>(static_cast<const double2*>(L), ld, rank, piv, chunk,
-                                                                 static_cast<double2*>(gemv_partials), N);
+            const bool halves = gemv_halves(real, blocks, nchunks, sms);
+            auto* gemv = halves ? chol_gemv_split_kernel<double2, true> : chol_gemv_split_kernel<double2, false>;
+            gemv<<<halves ? dim3(2 * blocks, nchunks) : grid, 128, 0, s>>>(
+                static_cast<const double2*>(L), ld, rank, piv, chunk, static_cast<double2*>(gemv_partials), N);
             chol_gemv_sum_kernel<double2><<<sblocks, 256, 0, s>>>(static_cast<const double2*>(column),
                                                                    static_cast<const double2*>(gemv_partials), nchunks,
                                                                    N, static_cast<double2*>(work));
         }
     } else if (real) {
-        chol_gemv_kernel<double><<<blocks, 128, 0, s>>>(static_cast<const double*>(L), ld, rank, piv,
-                                                        static_cast<const double*>(column),
-                                                        static_cast<double*>(work), N);
+        chol_gemv_kernel<double, false><<<blocks, 128, 0, s>>>(static_cast<const double*>(L), ld, rank, piv,
+                                                               static_cast<const double*>(column),
+                                                               static_cast<double*>(work), N);
     } else {
-        chol_gemv_kernel<double2><<<blocks, 128, 0, s>>>(static_cast<const double2*>(L), ld, rank, piv,
-                                                         static_cast<const double2*>(column),
-                                                         static_cast<double2*>(work), N);
+        const bool halves = gemv_halves(real, blocks, 1, sms);
+        auto* gemv = halves ? chol_gemv_kernel<double2, true> : chol_gemv_kernel<double2, false>;
+        gemv<<<halves ? 2 * blocks : blocks, 128, 0, s>>>(static_cast<const double2*>(L), ld, rank, piv,
+                                                          static_cast<const double2*>(column),
+                                                          static_cast<double2*>(work), N);
     }
     chol_scale_kernel<<<1, 1, 0, s>>>(res, piv, scale);
     if (real)
-        chol_update_kernel<double><<<RED_BLOCKS, 256, 0, s>>>(static_cast<const double*>(work), n, piv, scale,
-                                                              static_cast<double*>(Lrow), res,
-                                                              static_cast<Red*>(partial));
+        chol_update_kernel<double><<<red_blocks(N), RED_THREADS, 0, s>>>(static_cast<const double*>(work), n, piv,
+                                                                         scale, static_cast<double*>(Lrow), res,
+                                                                         static_cast<RedKey*>(partial));
     else
-        chol_update_kernel<double2><<<RED_BLOCKS, 256, 0, s>>>(static_cast<const double2*>(work), n, piv, scale,
-                                                               static_cast<double2*>(Lrow), res,
-                                                               static_cast<Red*>(partial));
-    chol_final_kernel<<<1, 256, 0, s>>>(static_cast<const Red*>(partial), RED_BLOCKS, static_cast<Red*>(out));
+        chol_update_kernel<double2><<<red_blocks(N), RED_THREADS, 0, s>>>(static_cast<const double2*>(work), n, piv,
+                                                                          scale, static_cast<double2*>(Lrow), res,
+                                                                          static_cast<RedKey*>(partial));
+    chol_final_kernel<<<1, 256, 0, s>>>(static_cast<const RedKey*>(partial), red_blocks(N), static_cast<Red*>(out));
     return cudaGetLastError();
 }
 
@@ -380,40 +436,18 @@ __global__ void chain_select_kernel(ChainState* st, const Red* red, int* slot_of
     chain_select(st, *red, slot_of, log, tol, psd);
 }
 
-template <typename T>
+template <typename T, bool HALVES>
 __global__ void chain_gemv_split_kernel(const T* L, long long ld, const ChainState* st, int nchunks, T* partials,
                                         long long N) {
     if (!st->active) return;
     __shared__ T coef[256];
+    using Acc = typename Entry<T, HALVES>::Acc;
     const int rank = st->rank;
-    const long long piv = st->pivot;
     const int chunk = (rank + nchunks - 1) / nchunks;
-    const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const Entry<T, HALVES> e((long long)blockIdx.x * blockDim.x + threadIdx.x);
     const int rbeg = blockIdx.y * chunk, rend = min(rank, rbeg + chunk);
-    T acc;
-    if constexpr (sizeof(T) == 8) {
-        acc = T(0);
-    } else {
-        acc = c2(0.0, 0.0);
-    }
-    for (int r0 = rbeg; r0 < rend; r0 += 256) {
-        const int nr = min(256, rend - r0);
-        __syncthreads();
-        for (int i = threadIdx.x; i < nr; i += blockDim.x) coef[i] = L[(long long)(r0 + i) * ld + piv];
-        __syncthreads();
-        if (j < N) {
-#pragma unroll 8
-            for (int r = 0; r < nr; ++r) {
-                const T lv = __ldg(&L[(long long)(r0 + r) * ld + j]);
-                if constexpr (sizeof(T) == 8) {
-                    acc += coef[r] * lv;
-                } else {
-                    acc = conj_mul_add(acc, coef[r], lv);
-                }
-            }
-        }
-    }
-    if (j < N) partials[(long long)blockIdx.y * N + j] = acc;
+    const Acc acc = gemv_rows<T, HALVES, false>(Entry<T, HALVES>::zero(), e, L, ld, rbeg, rend, st->pivot, N, coef);
+    if (e.j < N) reinterpret_cast<Acc*>(partials)[e.at((long long)blockIdx.y * N + e.j)] = acc;
 }
 
 // Updated column entry j: the cached raw column minus the rank-chunk partial
@@ -439,7 +473,7 @@ __device__ __forceinline__ T chain_column(const T* col_in, const T* partials, in
 // count) and, unless this is the chain's last step, selects the next pivot.
 template <typename T>
 __global__ void chain_update_kernel(ChainState* st, const T* pool, const T* partials, int nchunks, int n, T* L,
-                                    double* res, Red* partial, Red* out, int* slot_of, long long* log, double tol,
+                                    double* res, RedKey* partial, Red* out, int* slot_of, long long* log, double tol,
                                     double psd, int select_next) {
     if (!st->active) return;
     const long long N = (long long)n * n;
@@ -447,13 +481,12 @@ __global__ void chain_update_kernel(ChainState* st, const T* pool, const T* part
     const T* col_in = pool + (long long)st->slot * N;
     T* Lrow = L + (long long)st->rank * N;
     const double sc = st->scale;
-    Red r{-1.0 / 0.0, (long long)1 << 62, 1.0 / 0.0};
+    RedKey r = red_none();
     for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j < N; j += (long long)gridDim.x * blockDim.x) {
         double mag2;
         if constexpr (sizeof(T) == 8) {
-            const long long mu = j / n, nu = j - mu * n;
             const double wj = chain_column(col_in, partials, nchunks, N, j);
-            const double wt = chain_column(col_in, partials, nchunks, N, nu * n + mu);
+            const double wt = chain_column(col_in, partials, nchunks, N, transposed(j, n));
             const double c = (wj + wt) * 0.5 * sc;
             Lrow[j] = c;
             mag2 = c * c;
@@ -465,7 +498,7 @@ __global__ void chain_update_kernel(ChainState* st, const T* pool, const T* part
         const double nr = res[j] - mag2;
         const double kept = j == piv ? 0.0 : fmax(nr, 0.0);
         res[j] = kept;
-        red_merge(r, Red{kept, j, nr});
+        red_merge(r, red_key(kept, j, nr));
     }
     r = block_reduce(r);
     __shared__ int last;
@@ -477,11 +510,13 @@ __global__ void chain_update_kernel(ChainState* st, const T* pool, const T* part
     __syncthreads();
     if (!last) return;
     __threadfence();
-    Red q{-1.0 / 0.0, (long long)1 << 62, 1.0 / 0.0};
-    const volatile Red* vp = partial;
-    for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) red_merge(q, Red{vp[i].maxv, vp[i].idx, vp[i].minv});
-    q = block_reduce(q);
+    RedKey k = red_none();
+    const volatile RedKey* vp = partial;
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x)
+        red_merge(k, RedKey{vp[i].maxk, vp[i].idx, vp[i].mink});
+    k = block_reduce(k);
     if (threadIdx.x == 0) {
+        const Red q = red_value(k);
         *out = q;
         st->done = 0;
         st->rank += 1;
@@ -503,17 +538,19 @@ cudaError_t launch_chol_chain(bool real, void* L, long long N, int n, int rank_h
     for (int k = 0; k < steps; ++k) {
         const int select_next = k + 1 < steps ? 1 : 0;
         if (real) {
-            chain_gemv_split_kernel<double><<<grid, 128, 0, s>>>(static_cast<const double*>(L), N, st, nchunks,
-                                                                 static_cast<double*>(gemv_partials), N);
-            chain_update_kernel<double><<<RED_BLOCKS, 256, 0, s>>>(
+            chain_gemv_split_kernel<double, false><<<grid, 128, 0, s>>>(static_cast<const double*>(L), N, st, nchunks,
+                                                                        static_cast<double*>(gemv_partials), N);
+            chain_update_kernel<double><<<red_blocks(N), RED_THREADS, 0, s>>>(
                 st, static_cast<const double*>(pool), static_cast<const double*>(gemv_partials), nchunks, n,
-                static_cast<double*>(L), res, static_cast<Red*>(partial), red, slot_of, log, tol, psd, select_next);
+                static_cast<double*>(L), res, static_cast<RedKey*>(partial), red, slot_of, log, tol, psd, select_next);
         } else {
-            chain_gemv_split_kernel<double2><<<grid, 128, 0, s>>>(static_cast<const double2*>(L), N, st, nchunks,
-                                                                  static_cast<double2*>(gemv_partials), N);
-            chain_update_kernel<double2><<<RED_BLOCKS, 256, 0, s>>>(
+            const bool halves = gemv_halves(real, blocks, nchunks, sms);
+            auto* gemv = halves ? chain_gemv_split_kernel<double2, true> : chain_gemv_split_kernel<double2, false>;
+            gemv<<<halves ? dim3(2 * blocks, nchunks) : grid, 128, 0, s>>>(
+                static_cast<const double2*>(L), N, st, nchunks, static_cast<double2*>(gemv_partials), N);
+            chain_update_kernel<double2><<<red_blocks(N), RED_THREADS, 0, s>>>(
                 st, static_cast<const double2*>(pool), static_cast<const double2*>(gemv_partials), nchunks, n,
-                static_cast<double2*>(L), res, static_cast<Red*>(partial), red, slot_of, log, tol, psd, select_next);
+                static_cast<double2*>(L), res, static_cast<RedKey*>(partial), red, slot_of, log, tol, psd, select_next);
         }
     }
     return cudaGetLastError();
@@ -560,6 +597,6 @@ cudaError_t launch_chol_final_residual(bool real, const double* D, const void* L
 }
 
 size_t chol_red_bytes() { return sizeof(Red); }
-size_t chol_partial_bytes() { return sizeof(Red) * RED_BLOCKS; }
+size_t chol_partial_bytes() { return sizeof(RedKey) * RED_BLOCKS; }
 
 }  // namespace gx
