@@ -770,8 +770,17 @@ std::vector<int2> make_groups(const gx_context* ctx, const PlanData& plan, size_
 // least eight such units per SM before screening, else 128, 64 or 32 (16 and 8
 // were measured too: the half-empty batches cost small plans with f shells
 // more than their shorter units gave); a few less, because a unit ends with a
-// whole task and should not spill into a batch of its own.  Classes with few tasks have no
-// entry in the unit arrays: their blocks cut the units themselves.
+// whole task and should not spill into a batch of its own.  A plan that has
+// fewer than three units per SM at that size (the column evaluations of a
+// Cholesky factorisation, one or two atoms) is bound by the time of one unit,
+// and a short batch repeats its entries over the lanes: down to 8 entries.  Two
+// atoms' factorisation 19.8 -> 18.8 ms (16 entries: 19.7, 4: 18.7), their s/p
+// shells in a field 73 -> 48 us; at four units per SM the 98 classes of an s-f
+// atom took 309 us instead of 290.  In the small classes (L <= 2) a unit is one
+// warp's work, not a block's, so they go on halving until there are 64 units
+// per SM: at eight a warp walked up to 256 entries alone while the rest of a
+// five-atom molecule had finished.  Classes with few tasks have no entry in the
+// unit arrays: their blocks cut the units themselves.
 void make_units(gx_context* ctx, PlanData& plan) {
     std::vector<gx::UnitClass> cls;
     const size_t nc = plan.classes.size();
@@ -781,6 +790,7 @@ void make_units(gx_context* ctx, PlanData& plan) {
     plan.unit_target.assign(nc, 0);
     plan.unit_dims.assign(nc, 0);
     int64_t vtask = 0, nunit = 0, vtask64 = 0, nunit64 = 0;
+    const int64_t plan_all = plan.primitive_quartets * std::max(plan.spread_parts, 1);
     for (int fp32 = 0; fp32 < 2; ++fp32) {
         for (size_t ci = 0; ci < nc; ++ci) {
             const PlanClass& pc = plan.classes[ci];
@@ -792,6 +802,8 @@ void make_units(gx_context* ctx, PlanData& plan) {
             const int64_t all = pc.primitive_quartets * std::max(plan.spread_parts, 1);
             int entries = 256;
             while (entries > 32 && all / entries < full) entries /= 2;
+            while (entries > 8 && entries <= 32 && plan_all / entries < 3 * (int64_t)std::max(ctx->sm_count, 1))
+                entries /= 2;
             const int64_t mean = pc.primitive_quartets / std::max<int64_t>((int64_t)pc.count, 1);
             const int64_t target = 64 * (entries - std::min<int64_t>(entries / 16, mean / 4));
             // as many units as an execution without screening has
