@@ -201,6 +201,7 @@ struct ColumnPlan;  // the column-evaluation plan of one pivot shell pair (see c
 // Page-locked host memory that grows on demand.
 struct PinnedHost {
     void* p = nullptr;
+    void* dev = nullptr;  // the same memory as kernels address it
     size_t n = 0;
     PinnedHost() = default;
     PinnedHost(const PinnedHost&) = delete;
@@ -214,6 +215,7 @@ struct PinnedHost {
         p = nullptr;
         n = 0;
         GX_CUDA(cudaHostAlloc(&p, bytes, cudaHostAllocDefault));
+        GX_CUDA(cudaHostGetDevicePointer(&dev, p, 0));
         n = bytes;
     }
 };
@@ -3681,14 +3683,13 @@ void cholesky_core(gx_context* ctx, gx_basis* b, const double* Bf, const double*
     constexpr int kMailLog = 256;
     struct Mail {
         char loop[kRedBytes + kStateBytes];
-        int status, pad;
+        long long status;
         long long log[kMailLog];
     };
     ctx->chol_mail.reserve(sizeof(Mail));
     Mail* mail = static_cast<Mail*>(ctx->chol_mail.p);
-    // Residual on the host after every wait, up to 512 KB (about 10 us; the
-    // copy and wait for one block of it 17 us, once per evaluation): the
-    // candidates are chosen from it without a wait of their own.
+    // Residual on the host after every wait, up to 512 KB: the candidates are
+    // chosen from it without a wait of their own.
     constexpr int64_t kMirror = 1 << 16;
     double* mirror = nullptr;
     if (N <= kMirror) {
@@ -3696,18 +3697,20 @@ void cholesky_core(gx_context* ctx, gx_basis* b, const double* Bf, const double*
         mirror = static_cast<double*>(ctx->chol_residual.p);
     }
     gx::ChainState chain_state{};
-    auto fetch_red = [&] {
-        // the reduction result, the chain's state and the kernels' status word
-        // in one wait (a failure in a column batch is reported before the next
-        // pivot)
-        GX_CUDA(cudaMemcpyAsync(mail->loop, d_loop.ptr, sizeof mail->loop, cudaMemcpyDeviceToHost, st));
-        GX_CUDA(cudaMemcpyAsync(&mail->status, ctx->status.ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
-        if (mirror)
-            GX_CUDA(cudaMemcpyAsync(mirror, d_res.ptr, N * sizeof(double), cudaMemcpyDeviceToHost, st));
+    // the reduction result, the chain's state and log, the kernels' status word
+    // and the residual by one kernel into the mailbox, and one wait (a failure
+    // in a column batch is reported before the next pivot)
+    auto fetch_red = [&](const long long* log = nullptr, int64_t nlog = 0) {
+        char* to = static_cast<char*>(ctx->chol_mail.dev);
+        GX_CUDA(gx::launch_copy_words({gx::WordCopy{to, d_loop.ptr, (int64_t)sizeof(Mail::loop) / 8},
+                                       gx::WordCopy{to + offsetof(Mail, status), ctx->status.ptr, 1},
+                                       gx::WordCopy{to + offsetof(Mail, log), log, nlog},
+                                       gx::WordCopy{ctx->chol_residual.dev, d_res.ptr, mirror ? N : 0}},
+                                      ctx->sm_count, st));
         GX_CUDA(cudaStreamSynchronize(st));
         std::memcpy(&red, mail->loop, sizeof red);
         std::memcpy(&chain_state, mail->loop + kRedBytes, sizeof chain_state);
-        status_code = mail->status;
+        status_code = (int)(mail->status & 0xffffffff);
         collect_times();
         if (status_code) check_status(ctx);
     };
@@ -4060,9 +4063,9 @@ void cholesky_core(gx_context* ctx, gx_basis* b, const double* Bf, const double*
                                                  (int)b->nao_of(y), x == y ? 1 : 0});
                 upload(column_info, info, st);
             }
-            // column destinations, then the columns' components, in one copy from
-            // page-locked memory (the last one from there ended with the previous
-            // iteration's wait)
+            // column destinations, then the columns' components, copied from
+            // page-locked memory by a kernel (the last copy from there ended with
+            // the previous iteration's wait)
             size_t ncol = 0;
             for (const auto& bl : blocks) ncol += bl.cols.size();
             const size_t col_words = ncol * (sizeof(void*) + 2 * sizeof(int));
@@ -4081,7 +4084,7 @@ void cholesky_core(gx_context* ctx, gx_basis* b, const double* Bf, const double*
                 }
             cand_slot = bslots[0];
             d_cand.reserve(col_words);
-            GX_CUDA(cudaMemcpyAsync(d_cand.ptr, dst, col_words, cudaMemcpyHostToDevice, st));
+            const gx::WordCopy columns{d_cand.ptr, ctx->chol_cands.dev, (int64_t)col_words / 8};
             GX_CUDA(cudaEventRecord(ev_col.a, st));
             {
                 // the blocks' class launches share one fork/join over the
@@ -4131,16 +4134,19 @@ void cholesky_core(gx_context* ctx, gx_basis* b, const double* Bf, const double*
                         cudaGraphDestroy(graph);
                         GX_CUDA(ie);
                     }
-                    GX_CUDA(cudaMemcpyAsync(sg->plan.tasks.ptr, pd.tasks.ptr, sizeof(gx::Task) * pd.ntask,
-                                            cudaMemcpyDeviceToDevice, st));
-                    GX_CUDA(cudaMemcpyAsync(sg->plan.base.dev.ptr, pd.base.dev.ptr, pd.base.dev.bytes,
-                                            cudaMemcpyDeviceToDevice, st));
+                    static_assert(sizeof(gx::Task) % 8 == 0 && sizeof(int2) == 8, "copied by words");
+                    GX_CUDA(gx::launch_copy_words(
+                        {columns,
+                         gx::WordCopy{sg->plan.tasks.ptr, pd.tasks.ptr, (int64_t)(sizeof(gx::Task) / 8) * pd.ntask},
+                         gx::WordCopy{sg->plan.base.dev.ptr, pd.base.dev.ptr, (int64_t)pd.base.dev.bytes / 8}},
+                        ctx->sm_count, st));
                     // the counters accumulate across factorisations: note where this one starts
                     if (!shape_base.count(sg.get()))
                         shape_base.emplace(sg.get(), std::make_pair(sg, counts_before(sg->counts, sg->counters,
                                                                                       pd.classes.size())));
                     GX_CUDA(cudaGraphLaunch(sg->exec, st));
                 } else {
+                    GX_CUDA(gx::launch_copy_words({columns}, ctx->sm_count, st));
                     enqueue_plans(ctx, runs, GX_PRECISION_FP64, ctr);
                     for (auto* cp : cps) plan_base[cp].direct = true;
                 }
@@ -4257,8 +4263,6 @@ void cholesky_core(gx_context* ctx, gx_basis* b, const double* Bf, const double*
             if (capturable) GX_CUDA(cudaGraphLaunch(git->second, st));
             // the log holds `limit` entries; the chain writes at most up to rank_limit <= limit
             nlog = std::min<int64_t>(std::min<int64_t>(chain_k, kMailLog), limit - (rank + 1));
-            GX_CUDA(cudaMemcpyAsync(mail->log, d_log.as<long long>() + rank + 1, nlog * sizeof(long long),
-                                    cudaMemcpyDeviceToHost, st));
         }
         GX_CUDA(cudaEventRecord(ev_upd.b, st));
         upd_pending = true;
@@ -4266,7 +4270,7 @@ void cholesky_core(gx_context* ctx, gx_basis* b, const double* Bf, const double*
         // column read, the new row written, the residual read and written
         stats.update_bytes += (double)col_bytes * (rank + 2) + 16.0 * N;
         stats.update_flops += (real ? 2.0 : 8.0) * (double)rank * N;
-        fetch_red();
+        fetch_red(chained ? d_log.as<long long>() + rank + 1 : nullptr, nlog);
         if (chained) {
             cs_out = chain_state;
             chain_log.assign(mail->log, mail->log + nlog);

@@ -278,6 +278,14 @@ cudaError_t launch_chol_diag(const double2* packed, const long long* boff, const
 cudaError_t launch_chol_cols(bool real, const double2* packed, const long long* boff, const int* info,
                              const int* flip, int nblocks, const int* cand, int ncand, int nc, int nd, int n,
                              void* const* dst, cudaStream_t s);
+// Several small copies of 8-byte words (device memory, or page-locked host
+// memory at its device address) by one kernel.
+struct WordCopy {
+    void* dst;
+    const void* src;
+    int64_t words;
+};
+cudaError_t launch_copy_words(std::initializer_list<WordCopy> copies, int sms, cudaStream_t s);
 cudaError_t launch_chol_scan(const double* res, long long N, void* partial, void* out, cudaStream_t s);
 // gemv_partials (max_chunks x n^2 values, may be null): splits the factor
 // update over rank chunks when that gives more blocks; sms: SM count.
