@@ -21,6 +21,7 @@
 // through the electron-repulsion class kernels; this kernel gathers them into
 // the (4, 3, na, nb, nc, nd) blocks of the reference layout.
 #include <algorithm>
+#include <type_traits>
 
 #include "gx_internal.h"
 
@@ -43,6 +44,11 @@ __device__ __forceinline__ void comp_of(int l, int c, int& lx, int& ly, int& lz)
     ly = m - lz;
 }
 
+// Bound by the instructions of an element (a third of three atoms' quartets:
+// 344 -> 285 us): its FP64 ones (about 20) occupy a
+// sub-partition for 64 cycles each, and index arithmetic comes next (64-bit
+// divisions cost some 70 instructions; a block has fewer than 2^32 elements:
+// with its derived blocks it would not fit the device memory otherwise).
 __global__ void __launch_bounds__(256) deriv_combine_kernel(DerivCombineArgs a) {
     const long long total = a.offsets[a.nq];
     const bool centre = a.mode == 0;
@@ -67,20 +73,23 @@ __global__ void __launch_bounds__(256) deriv_combine_kernel(DerivCombineArgs a) 
             size *= dim[k];
         }
         const long long rel = e - __ldg(&a.offsets[qi]);
-        const int d = (int)(rel / size);
-        const long long r0 = rel - (long long)d * size;
-        long long r = r0;
+        const int d = (unsigned long long)rel >> 32 ? (int)(rel / size) : (int)((unsigned)rel / (unsigned)size);
+        const unsigned r0 = (unsigned)(rel - (long long)d * size);
+        unsigned r = r0;
         int idx[4];
         for (int j = 3; j >= 0; --j) {
-            idx[j] = (int)(r % dim[j]);
-            r /= dim[j];
+            const unsigned q = r / (unsigned)dim[j];
+            idx[j] = (int)(r - q * (unsigned)dim[j]);
+            r = q;
         }
+        const long long d01 = (long long)dim[0] * dim[1], d23 = (long long)dim[2] * dim[3];
+        const long long others[4] = {dim[1] * d23, dim[0] * d23, d01 * dim[3], d01 * dim[2]};
         // this quartet's derived blocks: per slot [Z, D if l > 0] (centre), [U]; then [plain]
         long long off = __ldg(&a.derived_offsets[qi]);
         long long zoff[4], doff[4], uoff[4], boff = -1;
         double uscale[4];  // U = Z / (2 alpha) for a single-primitive shell in centre mode
         for (int j = 0; j < 4; ++j) {
-            const long long up = size / dim[j] * (nc[j] * ncart(l[j] + 1));
+            const long long up = others[j] * (nc[j] * ncart(l[j] + 1));
             zoff[j] = doff[j] = uoff[j] = -1;
             uscale[j] = 1.0;
             if (centre) {
@@ -88,7 +97,7 @@ __global__ void __launch_bounds__(256) deriv_combine_kernel(DerivCombineArgs a) 
                 off += up;
                 if (l[j] > 0) {
                     doff[j] = off;
-                    off += size / dim[j] * (nc[j] * ncart(l[j] - 1));
+                    off += others[j] * (nc[j] * ncart(l[j] - 1));
                 }
             }
             const double inv2a = centre ? __ldg(&a.shell_inv2a[sh[j]]) : 0.0;
@@ -135,8 +144,9 @@ __global__ void __launch_bounds__(256) deriv_combine_kernel(DerivCombineArgs a) 
                     int dn[3] = {ang[0], ang[1], ang[2]};
                     --dn[x];
                     const double2 t = __ldg(&a.derived[doff[k] + derived(k, xk, lk - 1, dn[0], dn[2])]);
-                    v.x -= ang[x] * t.x;
-                    v.y -= ang[x] * t.y;
+                    const double ax = c_dev.ints[ang[x]];
+                    v.x -= ax * t.x;
+                    v.y -= ax * t.y;
                 }
                 res = c2(hk * v.x, hk * v.y);
                 if (!a.field) break;
@@ -151,19 +161,22 @@ __global__ void __launch_bounds__(256) deriv_combine_kernel(DerivCombineArgs a) 
                 w[1] = b == 2 ? D[0] : (b == 0 ? -D[2] : 0.0);
                 w[2] = b == 0 ? D[1] : (b == 1 ? -D[0] : 0.0);
             }
+            // sum_c coef_c (h U_c + R_c base), the parts of U and of base apart
             double2 t = c2(0.0, 0.0);
+            double rb = 0.0;
             for (int c = 0; c < 3; ++c) {
-                const double coef = phi * w[c];
-                if (coef == 0.0) continue;
+                if ((__double_as_longlong(w[c]) & 0x7fffffffffffffffll) == 0) continue;
                 int uc[3] = {ang[0], ang[1], ang[2]};
                 ++uc[c];
                 const double2 u = __ldg(&a.derived[uoff[k] + derived(k, xk, lk + 1, uc[0], uc[2])]);
-                const double R = __ldg(&a.shell_center[3 * sh[k] + c]);
-                const double hu = hk * uscale[k];
-                // coef * (h U + R base)
-                t.x += coef * (hu * u.x + R * base.x);
-                t.y += coef * (hu * u.y + R * base.y);
+                t.x = fma(w[c], u.x, t.x);
+                t.y = fma(w[c], u.y, t.y);
+                rb = fma(w[c], __ldg(&a.shell_center[3 * sh[k] + c]), rb);
             }
+            const double hu = phi * (hk * uscale[k]);
+            rb *= phi;
+            t.x = fma(rb, base.x, hu * t.x);
+            t.y = fma(rb, base.y, hu * t.y);
             // + i t
             res.x -= t.y;
             res.y += t.x;
@@ -304,6 +317,9 @@ __global__ void __launch_bounds__(256) deriv_mixed_kernel(DerivMixedArgs a) {
 // at the image's AO indices multiplies the derivative (conjugated for the
 // last two images); lanes stride over the elements and a fixed shuffle tree
 // sums the twelve partial sums, so the result does not depend on scheduling.
+// Bound by FP64 issue (64 cycles an instruction on each sub-partition): the four
+// combined weights leave four FMAs per derivative, and the tree halves the
+// values with every exchange (the same quartets: 405 -> 295 us).
 __global__ void __launch_bounds__(128) deriv_contract_kernel(DerivContractArgs a) {
     const int lane = threadIdx.x & 31;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -330,12 +346,13 @@ __global__ void __launch_bounds__(128) deriv_contract_kernel(DerivContractArgs a
         double2 acc[12];
 #pragma unroll
         for (int t = 0; t < 12; ++t) acc[t] = c2(0.0, 0.0);
-        for (long long loc = lane; loc < size; loc += 32) {
+        for (unsigned loc = lane; loc < (unsigned)size; loc += 32) {
             long long ao[4];
-            long long rest = loc;
+            unsigned rest = loc;
             for (int k = 3; k >= 0; --k) {
-                ao[k] = st[k] + rest % dim[k];
-                rest /= dim[k];
+                const unsigned q = rest / (unsigned)dim[k];
+                ao[k] = st[k] + (int)(rest - q * (unsigned)dim[k]);
+                rest = q;
             }
             double2 wd = c2(0.0, 0.0), wc = c2(0.0, 0.0);  // direct / conjugated images
             for (int o = 0; o < 4; ++o) {
@@ -360,22 +377,47 @@ __global__ void __launch_bounds__(128) deriv_contract_kernel(DerivContractArgs a
                 else
                     wc = cadd(wc, w);
             }
+            // d wd + conj(d) wc
+            const double xx = wd.x + wc.x, xy = wc.y - wd.y, yx = wd.y + wc.y, yy = wd.x - wc.x;
 #pragma unroll
             for (int t = 0; t < 12; ++t) {
                 const double2 dv = __ldg(&blk[(long long)t * size + loc]);
-                // d wd + conj(d) wc
-                acc[t].x += dv.x * wd.x - dv.y * wd.y + dv.x * wc.x + dv.y * wc.y;
-                acc[t].y += dv.x * wd.y + dv.y * wd.x + dv.x * wc.y - dv.y * wc.x;
+                acc[t].x = fma(dv.y, xy, fma(dv.x, xx, acc[t].x));
+                acc[t].y = fma(dv.y, yy, fma(dv.x, yx, acc[t].y));
             }
         }
+        // halving exchanges: a lane keeps half of its values and adds the other
+        // lane's share of them (24 additions instead of 120)
+        double v[24];
 #pragma unroll
-        for (int t = 0; t < 12; ++t)
-            for (int off = 16; off > 0; off >>= 1) {
-                acc[t].x += __shfl_xor_sync(0xffffffffu, acc[t].x, off);
-                acc[t].y += __shfl_xor_sync(0xffffffffu, acc[t].y, off);
+        for (int t = 0; t < 12; ++t) {
+            v[2 * t] = acc[t].x;
+            v[2 * t + 1] = acc[t].y;
+        }
+        auto halve = [&](auto count, int off) {
+            constexpr int H = decltype(count)::value;  // values kept
+            const bool up = lane & off;
+#pragma unroll
+            for (int k = 0; k < H; ++k) {
+                const double keep = up ? v[H + k] : v[k], give = up ? v[k] : v[H + k];
+                v[k] = keep + __shfl_xor_sync(0xffffffffu, give, off);
             }
-        if (lane == 0)
-            for (int t = 0; t < 12; ++t) a.partials[(long long)qi * 12 + t] = acc[t];
+        };
+        halve(std::integral_constant<int, 12>{}, 16);
+        halve(std::integral_constant<int, 6>{}, 8);
+        halve(std::integral_constant<int, 3>{}, 4);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            v[k] += __shfl_xor_sync(0xffffffffu, v[k], 2);
+            v[k] += __shfl_xor_sync(0xffffffffu, v[k], 1);
+        }
+        // lanes 0, 4, .. 28 hold three consecutive values each
+        if ((lane & 3) == 0) {
+            const int first = (lane & 16 ? 12 : 0) + (lane & 8 ? 6 : 0) + (lane & 4 ? 3 : 0);
+            double* out = reinterpret_cast<double*>(a.partials + (long long)qi * 12);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) out[first + k] = v[k];
+        }
     }
 }
 
