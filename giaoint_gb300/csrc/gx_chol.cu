@@ -158,11 +158,14 @@ __device__ RedKey block_reduce(RedKey r) {
     return r;
 }
 
-// Blocks of the reductions over N entries, an entry per thread until the
-// partials fill one block.
-constexpr int RED_BLOCKS = 256, RED_THREADS = 128;
+// Blocks of the reductions over N entries, at most as many as one block merges,
+// and their threads: an entry each, in blocks of 128 (of 1,000 entries every
+// warp then has a sub-partition to itself) until those run out.
+constexpr int RED_BLOCKS = 256;
+int red_threads(long long N) { return N <= 128 * RED_BLOCKS ? 128 : 256; }
 int red_blocks(long long N) {
-    return (int)std::max<long long>(1, std::min<long long>((N + RED_THREADS - 1) / RED_THREADS, RED_BLOCKS));
+    const int threads = red_threads(N);
+    return (int)std::max<long long>(1, std::min<long long>((N + threads - 1) / threads, RED_BLOCKS));
 }
 
 __global__ void chol_scan_kernel(const double* res, long long N, RedKey* partial) {
@@ -183,7 +186,7 @@ __global__ void chol_final_kernel(const RedKey* partial, int np, Red* out) {
 }
 
 cudaError_t launch_chol_scan(const double* res, long long N, void* partial, void* out, cudaStream_t s) {
-    chol_scan_kernel<<<red_blocks(N), RED_THREADS, 0, s>>>(res, N, static_cast<RedKey*>(partial));
+    chol_scan_kernel<<<red_blocks(N), red_threads(N), 0, s>>>(res, N, static_cast<RedKey*>(partial));
     chol_final_kernel<<<1, 256, 0, s>>>(static_cast<const RedKey*>(partial), red_blocks(N), static_cast<Red*>(out));
     return cudaGetLastError();
 }
@@ -418,11 +421,11 @@ cudaError_t launch_chol_step(bool real, const void* L, long long ld, int rank, l
     }
     chol_scale_kernel<<<1, 1, 0, s>>>(res, piv, scale);
     if (real)
-        chol_update_kernel<double><<<red_blocks(N), RED_THREADS, 0, s>>>(static_cast<const double*>(work), n, piv,
+        chol_update_kernel<double><<<red_blocks(N), red_threads(N), 0, s>>>(static_cast<const double*>(work), n, piv,
                                                                          scale, static_cast<double*>(Lrow), res,
                                                                          static_cast<RedKey*>(partial));
     else
-        chol_update_kernel<double2><<<red_blocks(N), RED_THREADS, 0, s>>>(static_cast<const double2*>(work), n, piv,
+        chol_update_kernel<double2><<<red_blocks(N), red_threads(N), 0, s>>>(static_cast<const double2*>(work), n, piv,
                                                                           scale, static_cast<double2*>(Lrow), res,
                                                                           static_cast<RedKey*>(partial));
     chol_final_kernel<<<1, 256, 0, s>>>(static_cast<const RedKey*>(partial), red_blocks(N), static_cast<Red*>(out));
@@ -577,7 +580,7 @@ cudaError_t launch_chol_chain(bool real, void* L, long long N, int n, int rank_h
         if (real) {
             chain_gemv_split_kernel<double, false><<<grid, 128, 0, s>>>(static_cast<const double*>(L), N, st, nchunks,
                                                                         static_cast<double*>(gemv_partials), N);
-            chain_update_kernel<double><<<red_blocks(N), RED_THREADS, 0, s>>>(
+            chain_update_kernel<double><<<red_blocks(N), red_threads(N), 0, s>>>(
                 st, static_cast<const double*>(pool), static_cast<const double*>(gemv_partials), nchunks, n,
                 static_cast<double*>(L), res, static_cast<RedKey*>(partial), red, slot_of, log, tol, psd, select_next);
         } else {
@@ -585,7 +588,7 @@ cudaError_t launch_chol_chain(bool real, void* L, long long N, int n, int rank_h
             auto* gemv = halves ? chain_gemv_split_kernel<double2, true> : chain_gemv_split_kernel<double2, false>;
             gemv<<<halves ? dim3(2 * blocks, nchunks) : grid, 128, 0, s>>>(
                 static_cast<const double2*>(L), N, st, nchunks, static_cast<double2*>(gemv_partials), N);
-            chain_update_kernel<double2><<<red_blocks(N), RED_THREADS, 0, s>>>(
+            chain_update_kernel<double2><<<red_blocks(N), red_threads(N), 0, s>>>(
                 st, static_cast<const double2*>(pool), static_cast<const double2*>(gemv_partials), nchunks, n,
                 static_cast<double2*>(L), res, static_cast<RedKey*>(partial), red, slot_of, log, tol, psd, select_next);
         }
