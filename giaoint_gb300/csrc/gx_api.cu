@@ -1360,9 +1360,8 @@ std::vector<PlanLaunch> plan_launches(gx_context* ctx, const gx::EriDev& dev, co
     return out;
 }
 
-// Enqueue the pair records for (B, O) and every class launch; no host sync
-// unless the field changed (the pair bounds are sorted on the host).  Uses
-// the autotuned configuration of the precision mode when there is one.
+// Enqueue the pair records for (B, O) and every class launch without a wait.
+// Uses the autotuned configuration of the precision mode when there is one.
 // counters: 2 per class (FP64, FP32 primitive quartets evaluated) or null;
 // zeroed first unless `accumulate`.
 // host_mapped (may be null): page-locked host output, its mapped address;
