@@ -71,6 +71,15 @@ int guarded(F&& f) {
     }
 }
 
+bool capturing(cudaStream_t s) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
+    }
+    return st != cudaStreamCaptureStatusNone;
+}
+
 // Grow-only device buffer, or a view of a part of another one.
 struct DeviceBuffer {
     void* ptr = nullptr;
@@ -339,6 +348,7 @@ void check_status(gx_context* ctx) {
 
 struct FieldPairs {
     double B[3], O[3];
+    bool valid = false;  // the records of (B, O) are complete, or enqueued to be
     DeviceBuffer mem;  // one allocation, and the views of its parts
     DeviceBuffer p, Pr, Pi, F, Epool, bound, Epool32, order, sbound, g32;
 };
@@ -492,7 +502,9 @@ void build_segments(gx_basis* b) {
 // on the basis for the last field.  After the records, every primitive pair's
 // exact Schwarz factor is computed and each shell pair's primitive pairs are
 // ordered by decreasing factor, so that screened primitive quartets form a
-// suffix of every bra row and ket column.
+// suffix of every bra row and ket column.  While the stream is captured by the caller
+// nothing runs until the graph is replayed (and each replay runs it again, over
+// whatever field the records hold by then), so new records are refused there.
 gx::PairData pair_view(gx_basis* b, FieldPairs& fp) {
     return gx::PairData{b->npp,
                         fp.p.as<double>(),
@@ -509,11 +521,15 @@ gx::PairData pair_view(gx_basis* b, FieldPairs& fp) {
 }
 
 FieldPairs& field_pairs(gx_basis* b, const double* B, const double* O) {
-    if (b->pairs && std::memcmp(b->pairs->B, B, sizeof(double) * 3) == 0 &&
+    if (b->pairs && b->pairs->valid && std::memcmp(b->pairs->B, B, sizeof(double) * 3) == 0 &&
         std::memcmp(b->pairs->O, O, sizeof(double) * 3) == 0)
         return *b->pairs;
+    if (capturing(b->ctx->stream))
+        raise(GX_ECUDA, "the stream is being captured and the pair records of this field are not on the device: "
+                        "evaluate the basis once in this field before the capture");
     if (!b->pairs) b->pairs = std::make_unique<FieldPairs>();
     FieldPairs& fp = *b->pairs;
+    fp.valid = false;  // until everything below is enqueued
     std::memcpy(fp.B, B, sizeof fp.B);
     std::memcpy(fp.O, O, sizeof fp.O);
     if (!fp.mem.ptr) {
@@ -547,6 +563,7 @@ FieldPairs& field_pairs(gx_basis* b, const double* B, const double* O) {
                                        fp.Epool.as<double2>(), fp.Epool32.as<float2>(), fp.bound.as<double>(),
                                        fp.g32.as<float4>(), fp.order.as<int>(), fp.sbound.as<float>(), dev,
                                        b->ctx->stream));
+    fp.valid = true;
     return fp;
 }
 
@@ -4505,15 +4522,6 @@ struct gx_eri_plan {
 extern "C" {
 
 namespace {
-bool capturing(cudaStream_t s) {
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
-        cudaGetLastError();
-        return true;
-    }
-    return st != cudaStreamCaptureStatusNone;
-}
-
 // Notes the end of an asynchronous plan execution (see gx_context_set_stream).
 void mark_execution(gx_context* ctx) {
     if (capturing(ctx->stream)) return;
