@@ -80,6 +80,41 @@ bool capturing(cudaStream_t s) {
     return st != cudaStreamCaptureStatusNone;
 }
 
+// End of work that was enqueued on one stream and that later work, possibly on
+// another one, has to follow.
+struct StreamMark {
+    cudaEvent_t ev = nullptr;
+    cudaStream_t stream = nullptr;
+    bool set = false;
+    StreamMark() = default;
+    StreamMark(const StreamMark&) = delete;
+    StreamMark& operator=(const StreamMark&) = delete;
+    ~StreamMark() {
+        if (ev) cudaEventDestroy(ev);
+    }
+    void record(cudaStream_t s) {
+        if (!ev) GX_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+        GX_CUDA(cudaEventRecord(ev, s));
+        stream = s;
+        set = true;
+    }
+    // Work enqueued on s from here on follows the mark.  (The per-thread default
+    // stream is another stream in every thread.)  A stream that is being captured
+    // cannot wait for an event outside its graph: the host waits.
+    void follow(cudaStream_t s) const {
+        if (!set || (s == stream && s != cudaStreamPerThread)) return;
+        if (!capturing(s)) {
+            GX_CUDA(cudaStreamWaitEvent(s, ev, 0));
+            return;
+        }
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        GX_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+        const cudaError_t e = cudaEventSynchronize(ev);
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        GX_CUDA(e);
+    }
+};
+
 // Grow-only device buffer, or a view of a part of another one.
 struct DeviceBuffer {
     void* ptr = nullptr;
@@ -239,8 +274,6 @@ struct gx_context {
     std::vector<cudaStream_t> aux;
     std::vector<cudaEvent_t> aux_done;
     cudaEvent_t fork = nullptr;
-    cudaEvent_t exec_done = nullptr;  // end of the last asynchronous plan execution
-    bool exec_pending = false;
     std::shared_ptr<SharedTables> t;  // shared immutable tables of the device
     DeviceBuffer status;
     std::mutex mu;
@@ -349,6 +382,7 @@ void check_status(gx_context* ctx) {
 struct FieldPairs {
     double B[3], O[3];
     bool valid = false;  // the records of (B, O) are complete, or enqueued to be
+    StreamMark written;
     DeviceBuffer mem;  // one allocation, and the views of its parts
     DeviceBuffer p, Pr, Pi, F, Epool, bound, Epool32, order, sbound, g32;
 };
@@ -376,6 +410,8 @@ struct gx_basis {
     DeviceBuffer d_pp_a, d_pp_b, d_pp_pa, d_pp_pb, d_pp_class, d_Eoff, d_classes;
     std::vector<std::pair<int, int>> class_keys;
     std::unique_ptr<FieldPairs> pairs;
+    // the last executions of the basis's plans, which may still read `pairs`
+    std::vector<std::shared_ptr<StreamMark>> readers;
     // centre-derivative basis (built on first use): the shells of this basis
     // followed by their Z, U and D shells, and per-shell arrays for the
     // combine kernel
@@ -522,14 +558,19 @@ gx::PairData pair_view(gx_basis* b, FieldPairs& fp) {
 
 FieldPairs& field_pairs(gx_basis* b, const double* B, const double* O) {
     if (b->pairs && b->pairs->valid && std::memcmp(b->pairs->B, B, sizeof(double) * 3) == 0 &&
-        std::memcmp(b->pairs->O, O, sizeof(double) * 3) == 0)
+        std::memcmp(b->pairs->O, O, sizeof(double) * 3) == 0) {
+        b->pairs->written.follow(b->ctx->stream);
         return *b->pairs;
+    }
     if (capturing(b->ctx->stream))
         raise(GX_ECUDA, "the stream is being captured and the pair records of this field are not on the device: "
                         "evaluate the basis once in this field before the capture");
     if (!b->pairs) b->pairs = std::make_unique<FieldPairs>();
     FieldPairs& fp = *b->pairs;
     fp.valid = false;  // until everything below is enqueued
+    fp.written.follow(b->ctx->stream);
+    for (const auto& r : b->readers) r->follow(b->ctx->stream);
+    std::erase_if(b->readers, [](const auto& r) { return r.use_count() == 1; });  // (of plans that are gone)
     std::memcpy(fp.B, B, sizeof fp.B);
     std::memcpy(fp.O, O, sizeof fp.O);
     if (!fp.mem.ptr) {
@@ -563,6 +604,7 @@ FieldPairs& field_pairs(gx_basis* b, const double* B, const double* O) {
                                        fp.Epool.as<double2>(), fp.Epool32.as<float2>(), fp.bound.as<double>(),
                                        fp.g32.as<float4>(), fp.order.as<int>(), fp.sbound.as<float>(), dev,
                                        b->ctx->stream));
+    fp.written.record(b->ctx->stream);
     fp.valid = true;
     return fp;
 }
@@ -784,6 +826,22 @@ std::vector<int2> make_groups(const gx_context* ctx, const PlanData& plan, size_
     return groups;
 }
 
+// Arrays that an execution writes its units to, in `mem` (grown), their block
+// counter cleared on s.  Returns `tail` bytes that follow them.
+void* unit_arrays(gx::UnitPlan& u, DeviceBuffer& mem, size_t tail, cudaStream_t s) {
+    const int64_t o_prefix = 16, o_tile = o_prefix + 8 * u.ntask, o_count = o_tile + 8 * gx::unit_tiles(u.ntask),
+                  o_start = o_count + 4 * u.ntask, o_tail = (o_start + 4 * u.nunit + 15) / 16 * 16;
+    mem.reserve((size_t)o_tail + tail);
+    char* base = mem.as<char>();
+    GX_CUDA(cudaMemsetAsync(base, 0, 16, s));
+    u.done = reinterpret_cast<unsigned*>(base);
+    u.prefix = reinterpret_cast<long long*>(base + o_prefix);
+    u.tile = reinterpret_cast<long long*>(base + o_tile);
+    u.count = reinterpret_cast<int*>(base + o_count);
+    u.start = reinterpret_cast<int*>(base + o_start);
+    return base + o_tail;
+}
+
 // Work units of the small and lane-dense classes.  A unit holds about 256
 // surviving primitive quartets (eight batches of 32) in classes that have at
 // least eight such units per SM before screening, else 128, 64 or 32 (16 and 8
@@ -847,26 +905,15 @@ void make_units(gx_context* ctx, PlanData& plan) {
     plan.units = gx::UnitPlan{};
     plan.unit_first = cls;
     if (cls.empty()) return;
-    const int64_t tiles = gx::unit_tiles(vtask);
-    auto align = [](int64_t x) { return (x + 15) / 16 * 16; };
-    const int64_t o_cls = 16, o_prefix = align(o_cls + (int64_t)(cls.size() * sizeof(gx::UnitClass))),
-                  o_tile = o_prefix + 8 * vtask, o_count = o_tile + 8 * tiles, o_start = o_count + 4 * vtask;
-    plan.unit_mem.reserve((size_t)(o_start + 4 * nunit));
-    char* base = plan.unit_mem.as<char>();
-    GX_CUDA(cudaMemsetAsync(base, 0, 16, ctx->stream));
-    GX_CUDA(cudaMemcpyAsync(base + o_cls, cls.data(), cls.size() * sizeof(gx::UnitClass), cudaMemcpyHostToDevice,
-                            ctx->stream));
-    plan.units = gx::UnitPlan{reinterpret_cast<gx::UnitClass*>(base + o_cls),
-                              (int)cls.size(),
-                              vtask,
-                              nunit,
-                              vtask64,
-                              nunit64,
-                              reinterpret_cast<int*>(base + o_count),
-                              reinterpret_cast<long long*>(base + o_prefix),
-                              reinterpret_cast<long long*>(base + o_tile),
-                              reinterpret_cast<int*>(base + o_start),
-                              reinterpret_cast<unsigned*>(base)};
+    plan.units.ncls = (int)cls.size();
+    plan.units.ntask = vtask;
+    plan.units.nunit = nunit;
+    plan.units.ntask64 = vtask64;
+    plan.units.nunit64 = nunit64;
+    const size_t bytes = cls.size() * sizeof(gx::UnitClass);
+    void* d_cls = unit_arrays(plan.units, plan.unit_mem, bytes, ctx->stream);
+    GX_CUDA(cudaMemcpyAsync(d_cls, cls.data(), bytes, cudaMemcpyHostToDevice, ctx->stream));
+    plan.units.cls = static_cast<gx::UnitClass*>(d_cls);
 }
 
 // Generic-kernel work units of every class in one device array.
@@ -2796,7 +2843,6 @@ void gx_context_destroy(gx_context* ctx) {
     for (auto st : ctx->aux) cudaStreamDestroy(st);
     for (auto ev : ctx->aux_done) cudaEventDestroy(ev);
     if (ctx->fork) cudaEventDestroy(ctx->fork);
-    if (ctx->exec_done) cudaEventDestroy(ctx->exec_done);
     if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
     if (ctx->copy_done) cudaEventDestroy(ctx->copy_done);
     for (auto st : ctx->class_copy) cudaStreamDestroy(st);
@@ -4515,32 +4561,23 @@ struct gx_eri_plan {
     int64_t total = 0;
     int last_launches = 0;
     PlanGraph graph;
+    // The last execution that was not captured by the caller: the next one, on
+    // whichever stream, follows it (both write the unit arrays).  One that the
+    // caller captures into a graph of its own has unit arrays of its own, kept
+    // for the graph's sake as long as the plan.
+    std::shared_ptr<StreamMark> done = std::make_shared<StreamMark>();
+    std::vector<std::unique_ptr<DeviceBuffer>> captured_units;
     int generation = 0;  // bumped when the launch configuration changes
     int graph_replays = 0;
 };
 
 extern "C" {
 
-namespace {
-// Notes the end of an asynchronous plan execution (see gx_context_set_stream).
-void mark_execution(gx_context* ctx) {
-    if (capturing(ctx->stream)) return;
-    if (!ctx->exec_done) GX_CUDA(cudaEventCreateWithFlags(&ctx->exec_done, cudaEventDisableTiming));
-    GX_CUDA(cudaEventRecord(ctx->exec_done, ctx->stream));
-    ctx->exec_pending = true;
-}
-}  // namespace
-
 int gx_context_set_stream(gx_context* ctx, void* stream) {
     return guarded([&] {
         if (!ctx) raise(GX_EINVAL, "null context");
         std::lock_guard<std::mutex> lock(ctx->mu);
-        cudaStream_t to = stream ? static_cast<cudaStream_t>(stream) : ctx->own_stream;
-        // a plan execution still in flight on the old stream uses its plan's
-        // unit arrays and the pair records: work on the new one follows it
-        if (to != ctx->stream && ctx->exec_pending && !capturing(to))
-            GX_CUDA(cudaStreamWaitEvent(to, ctx->exec_done, 0));
-        ctx->stream = to;
+        ctx->stream = stream ? static_cast<cudaStream_t>(stream) : ctx->own_stream;
     });
 }
 
@@ -4575,6 +4612,7 @@ int gx_eri_plan_create(gx_context* ctx, gx_basis* b, const uint32_t* quartets, i
         plan->total = off;
         build_plan(ctx, b, req, plan->data);
         GX_CUDA(cudaStreamSynchronize(ctx->stream));
+        b->readers.push_back(plan->done);
         *out = plan.release();
     });
 }
@@ -4613,6 +4651,33 @@ void plan_enqueue(gx_eri_plan* plan, const double* B, const double* O, int preci
                                        (uintptr_t)cut_bits, (uintptr_t)fp.p.ptr, (uintptr_t)fp.Epool.ptr,
                                        (uintptr_t)fp.order.ptr, (uintptr_t)plan->generation, (uintptr_t)real};
     PlanGraph& g = plan->graph;
+    if (capturing(ctx->stream)) {
+        // the caller's graph: the launches themselves, on unit arrays of their own
+        auto mem = std::make_unique<DeviceBuffer>();
+        const gx::UnitPlan own = pd.units;
+        if (own.ntask > 0) {
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // (for the allocation)
+            GX_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+            try {
+                unit_arrays(pd.units, *mem, 0, ctx->stream);
+            } catch (...) {
+                cudaThreadExchangeStreamCaptureMode(&mode);
+                pd.units = own;
+                throw;
+            }
+            cudaThreadExchangeStreamCaptureMode(&mode);
+        }
+        plan->captured_units.push_back(std::move(mem));
+        try {
+            plan->last_launches = execute_plan(ctx, plan->basis, B, O, pd, out, precision, mixed_cutoff,
+                                               pd.counters.as<unsigned long long>());
+        } catch (...) {
+            pd.units = own;
+            throw;
+        }
+        pd.units = own;
+        return;
+    }
     const bool capturable = !g.disabled && ctx->stream != nullptr;
     if (capturable && g.exec && g.key == key) {
         GX_CUDA(cudaGraphLaunch(g.exec, ctx->stream));
@@ -4666,8 +4731,18 @@ int gx_eri_plan_execute(gx_eri_plan* plan, const double* B, const double* O, int
         gx_context* ctx = plan->ctx;
         std::lock_guard<std::mutex> lock(ctx->mu);
         GX_CUDA(cudaSetDevice(ctx->device));
-        plan_enqueue(plan, B, O, precision, mixed_cutoff, static_cast<double2*>(out_device));
-        mark_execution(ctx);
+        if (capturing(ctx->stream)) {
+            plan_enqueue(plan, B, O, precision, mixed_cutoff, static_cast<double2*>(out_device));
+            return;
+        }
+        plan->done->follow(ctx->stream);
+        try {
+            plan_enqueue(plan, B, O, precision, mixed_cutoff, static_cast<double2*>(out_device));
+        } catch (...) {
+            plan->done->record(ctx->stream);
+            throw;
+        }
+        plan->done->record(ctx->stream);
     });
 }
 
@@ -4692,6 +4767,7 @@ int gx_eri_plan_profile(gx_eri_plan* plan, const double* B, const double* O, int
         std::lock_guard<std::mutex> lock(ctx->mu);
         GX_CUDA(cudaSetDevice(ctx->device));
         PlanData& pd = plan->data;
+        plan->done->follow(ctx->stream);
         const size_t nc = pd.classes.size();
         pd.counters.reserve(std::max<size_t>(2 * nc, 2) * sizeof(unsigned long long));
         auto* counters = pd.counters.as<unsigned long long>();
@@ -4781,6 +4857,7 @@ int gx_eri_plan_set_config(gx_eri_plan* plan, int precision, const gx_class_conf
                                  c.stream, c.nolane};
         }
         auto& tuned = pd.tuned[precision];
+        plan->done->follow(ctx->stream);
         make_group_set(ctx, pd, conf, tuned.groups);
         tuned.conf = conf;
         tuned.valid = true;
@@ -4802,6 +4879,7 @@ int gx_eri_plan_autotune(gx_eri_plan* plan, const double* B, const double* O, in
         std::lock_guard<std::mutex> lock(ctx->mu);
         GX_CUDA(cudaSetDevice(ctx->device));
         PlanData& pd = plan->data;
+        plan->done->follow(ctx->stream);
         const size_t nc = pd.classes.size();
         FieldPairs& fp = field_pairs(plan->basis, B, O);
         const gx::EriDev dev = make_dev(ctx, plan->basis, fp, static_cast<double2*>(out_device), precision,
@@ -4943,6 +5021,7 @@ int gx_eri_plan_counts(gx_eri_plan* plan, int64_t* fp64_quartets, int64_t* fp32_
         std::lock_guard<std::mutex> lock(plan->ctx->mu);
         const size_t nc = plan->data.classes.size();
         std::vector<unsigned long long> c(2 * nc);
+        plan->done->follow(plan->ctx->stream);
         GX_CUDA(cudaStreamSynchronize(plan->ctx->stream));
         if (nc)
             GX_CUDA(cudaMemcpy(c.data(), plan->data.counters.ptr, c.size() * sizeof(unsigned long long),

@@ -350,7 +350,15 @@ int gx_nuclear_attraction(gx_context* ctx, gx_basis* basis, const double* B, con
 
 /* Enqueue all later device work of `ctx` on `stream` (a cudaStream_t);
  * NULL restores the context's own stream.  No reference counterpart: the
- * reference runs synchronously on host threads (src/eri.cpp:708-763). */
+ * reference runs synchronously on host threads (src/eri.cpp:708-763).
+ * Executions of one plan follow each other, whichever streams they are on
+ * (they share its work-unit arrays), and new pair records of a basis follow the
+ * executions that read the old ones; different plans are not ordered.
+ * Under the caller's stream capture gx_eri_plan_execute is recorded with
+ * work-unit arrays of its own (allocated then, freed with the plan) and reads
+ * the basis's pair records when the graph is replayed: the field's records must
+ * be on the device before (a new field is refused with GX_ECUDA), and ordering
+ * replays against calls that change the field is the caller's. */
 int gx_context_set_stream(gx_context* ctx, void* stream);
 /* Wait for the context's stream and report any device status word. */
 int gx_context_synchronize(gx_context* ctx);

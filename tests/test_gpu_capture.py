@@ -72,3 +72,85 @@ def test_new_field_under_capture_is_refused(setup):
         graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(out, ref)
+
+
+def test_replay_beside_eager_executions_of_the_same_plan(setup):
+    """A captured execution has work units of its own: its replays on one stream and eager executions with
+    another cutoff (other units) on a second one give what each gives alone."""
+    torch, ctx, use = setup
+    _, basis = molecule(seed=7, natoms=3)
+    field = gi.MagneticField((0.05, -0.1, 0.12))
+    plan = EriPlan(basis, context=ctx)
+    outs = [torch.empty(plan.total, dtype=torch.complex128, device="cuda:0") for _ in range(2)]
+    refs = []
+    for out, precision in zip(outs, ("fp64", "mixed")):
+        plan.execute(out, field, precision=precision)
+        plan.synchronize()
+        refs.append(out.clone())
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    use(streams[0])
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=streams[0]):
+        plan.execute(outs[0], field, precision="fp64")
+    use(streams[1])
+    for _ in range(10):
+        for out in outs:
+            out.zero_()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(streams[0]):
+            graph.replay()
+        plan.execute(outs[1], field, precision="mixed")
+        torch.cuda.synchronize()
+        for out, ref in zip(outs, refs):
+            assert torch.equal(out, ref)
+
+
+def test_one_plan_and_two_fields_on_alternating_streams(setup):
+    """Executions on alternating streams without a wait between them, with the field (and so the pair records that
+    all of them read) changing every second time."""
+    torch, ctx, use = setup
+    _, basis = molecule(seed=11, natoms=3)
+    fields = [gi.MagneticField((0.05, -0.1, 0.12)), gi.MagneticField((-0.15, 0.02, 0.08))]
+    plan = EriPlan(basis, context=ctx)
+    refs = [_values(torch, ctx, basis, f) for f in fields]
+    outs = [torch.zeros(plan.total, dtype=torch.complex128, device="cuda:0") for _ in range(8)]
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    torch.cuda.synchronize()
+    for i, out in enumerate(outs):
+        use(streams[i % 2])
+        plan.execute(out, fields[(i // 2) % 2])
+    torch.cuda.synchronize()
+    for i, out in enumerate(outs):
+        assert torch.equal(out, refs[(i // 2) % 2]), i
+
+
+def test_plans_on_two_streams_do_not_wait_for_each_other(setup):
+    """A plan's execution finishes while another plan's is still queued behind a long kernel of its own stream.
+    (One class, so that the launches are on that stream alone; streams can share a hardware queue: one of several
+    suffices.)"""
+    torch, ctx, use = setup
+    _, basis = molecule(seed=7, natoms=2)
+    field = gi.MagneticField((0.05, -0.1, 0.12))
+    plans = [EriPlan(basis, [(0, 0, 0, 0)], context=ctx) for _ in range(2)]
+    outs = [torch.empty(p.total, dtype=torch.complex128, device="cuda:0") for p in plans]
+    streams = [torch.cuda.Stream() for _ in range(5)]
+    overlapped = False
+    for other in streams[1:]:
+        for plan, out, stream in zip(plans, outs, (streams[0], other)):
+            use(stream)
+            plan.execute(out, field)
+            plan.synchronize()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(streams[0]):
+            torch.cuda._sleep(400_000_000)
+        use(streams[0])
+        plans[0].execute(outs[0], field)
+        queued = torch.cuda.Event()
+        queued.record(streams[0])
+        use(other)
+        plans[1].execute(outs[1], field)
+        other.synchronize()
+        overlapped = overlapped or not queued.query()
+        torch.cuda.synchronize()
+    assert overlapped
+    assert torch.equal(outs[0], outs[1])
