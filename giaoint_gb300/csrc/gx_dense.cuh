@@ -40,11 +40,11 @@
 // asymptotic sector, seeds and every sum into the blocks in FP64), after the FP64 one on the same stream.
 #pragma once
 
-#include <atomic>
 #include <type_traits>
 #include <utility>
 
 #include "gx_internal.h"
+#include "gx_per_device.h"
 #include "gx_small.cuh"
 #include "gx_stream.cuh"
 
@@ -653,12 +653,15 @@ cudaError_t run_list_f64(int pair, const EriDev& d, const ClassList& list, int s
 cudaError_t run_list_f32(int pair, const EriDev& d, const ClassList& list, int smem, cudaStream_t s);
 
 template <class Arg>
-cudaError_t launch_with_smem(void (*kernel)(EriDev, Arg), std::atomic<bool>& ready, dim3 grid, int smem, cudaStream_t s,
+cudaError_t launch_with_smem(void (*kernel)(EriDev, Arg), PerDevice& limit, dim3 grid, int smem, cudaStream_t s,
                              const EriDev& d, const Arg& arg) {
-    if (!ready.load(std::memory_order_acquire)) {
-        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    if (limit.needs(device, kMaxSmem)) {
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
         if (e != cudaSuccess) return e;
-        ready.store(true, std::memory_order_release);
+        limit.done(device, kMaxSmem);
     }
     kernel<<<grid, 32 * kWarps, smem, s>>>(d, arg);
     return cudaGetLastError();

@@ -8,8 +8,8 @@ cudaError_t run_one_f64(int pair, const EriDev& d, const QuartetClass& qc, int s
     switch (pair) {
 #define GX_CASE(A, B)                                                                                             \
     case A * 4 + B: {                                                                                             \
-        static std::atomic<bool> ready{false};                                                                    \
-        return launch_with_smem(dense_kernel<A, B, false>, ready, dim3(qc.ngroup, qc.nchunk), smem, s, d, qc); \
+        static PerDevice limit;                                                                                   \
+        return launch_with_smem(dense_kernel<A, B, false>, limit, dim3(qc.ngroup, qc.nchunk), smem, s, d, qc);    \
     }
         GX_DENSE_PAIRS
 #undef GX_CASE

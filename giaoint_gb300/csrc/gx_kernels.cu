@@ -26,6 +26,7 @@
 #include <cstdio>
 
 #include "gx_internal.h"
+#include "gx_per_device.h"
 
 namespace gx {
 
@@ -1435,15 +1436,21 @@ cudaError_t launch_quartets(const EriDev& dev, const QuartetClass& qc, int warps
                             cudaStream_t s) {
     if (qc.ntask <= 0) return cudaSuccess;
     const size_t smem = quartet_smem_bytes(qc, warps_per_block, dev.fp32_cut > 0.0f);
-    static size_t configured[2] = {0, 0};
+    // (all that a block may have, whatever this launch takes: a smaller value set
+    // later by another thread would lower the limit)
+    constexpr size_t kLimit = 227 * 1024;
+    static PerDevice limit[2];
     const int v = qc.minb == 4 ? 1 : 0;
-    if (smem > 48 * 1024 && smem > configured[v]) {
-        cudaError_t e = v ? cudaFuncSetAttribute(quartet_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)smem)
-                          : cudaFuncSetAttribute(quartet_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)smem);
+    if (smem > 48 * 1024) {
+        int device = 0;
+        cudaError_t e = cudaGetDevice(&device);
         if (e != cudaSuccess) return e;
-        configured[v] = smem;
+        if (limit[v].needs(device, kLimit)) {
+            e = v ? cudaFuncSetAttribute(quartet_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLimit)
+                  : cudaFuncSetAttribute(quartet_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLimit);
+            if (e != cudaSuccess) return e;
+            limit[v].done(device, kLimit);
+        }
     }
     if (v)
         quartet_kernel<4><<<grid, warps_per_block * 32, smem, s>>>(dev, qc);
