@@ -903,6 +903,7 @@ void make_units(gx_context* ctx, PlanData& plan) {
         }
     }
     plan.units = gx::UnitPlan{};
+    plan.units.wide = reinterpret_cast<int*>(plan.tasks.as<gx::Task>() + plan.ntask);
     plan.unit_first = cls;
     if (cls.empty()) return;
     plan.units.ncls = (int)cls.size();
@@ -1140,7 +1141,8 @@ void build_plan_parts(gx_context* ctx, const std::vector<PlanPart>& parts, PlanD
     }
     plan.ntask = T;
     plan.stable = ctx->stable_launch;
-    plan.tasks.reserve(sizeof(gx::Task) * std::max<int64_t>(T, 1));
+    // (and a flag per class behind them, see UnitPlan)
+    plan.tasks.reserve(sizeof(gx::Task) * std::max<int64_t>(T, 1) + sizeof(int) * bkeys.size());
     if (T) GX_CUDA(cudaMemcpyAsync(plan.tasks.ptr, all.get(), sizeof(gx::Task) * T, cudaMemcpyHostToDevice, ctx->stream));
     plan.defconf.resize(plan.classes.size());
     for (size_t ci = 0; ci < plan.classes.size(); ++ci) plan.defconf[ci] = default_conf(plan.classes[ci].key);
@@ -1220,6 +1222,7 @@ gx::QuartetClass unit_class(gx_context* ctx, const PlanData& plan, size_t ci, un
     }
     qc.nchunk = 1;
     if (gx::small_class(k[0], k[1], k[2], k[3])) return qc;
+    if (qc.L >= gx::kWideOrder) qc.wide = plan.units.wide + ci;
     qc.bra = ctx->pair_class(k[0], k[1]).dev();
     qc.ket = ctx->pair_class(k[2], k[3]).dev();
     // few entries: the blocks of a unit share its components (about one in
@@ -1230,11 +1233,17 @@ gx::QuartetClass unit_class(gx_context* ctx, const PlanData& plan, size_t ci, un
 }
 
 // Lane-dense classes of one template pair; in mixed precision their FP32
-// entries are added after the FP64 ones.
-void launch_dense_classes(int pair, const gx::EriDev& dev, const std::vector<gx::QuartetClass>& classes,
-                          cudaStream_t s) {
+// entries are added after the FP64 ones, and, when `wide` is set, those that FP32
+// left to FP64 (otherwise launch_wide_classes follows for the whole plan).
+void launch_dense_classes(gx_context* ctx, int pair, const gx::EriDev& dev,
+                          const std::vector<gx::QuartetClass>& classes, cudaStream_t s, bool wide) {
     GX_CUDA(gx::launch_dense(pair, dev, classes, false, s));
-    if (dev.fp32_cut > 0.0f) GX_CUDA(gx::launch_dense(pair, dev, classes, true, s));
+    if (!(dev.fp32_cut > 0.0f)) return;
+    GX_CUDA(gx::launch_dense(pair, dev, classes, true, s));
+    if (!wide) return;
+    std::vector<std::pair<int, gx::QuartetClass>> list;
+    for (const auto& qc : classes) list.push_back({pair, qc});
+    GX_CUDA(gx::launch_wide(dev, list, ctx->sm_count, s));
 }
 
 // Enqueue the kernel of class ci with configuration conf and work units
@@ -1242,7 +1251,7 @@ void launch_dense_classes(int pair, const gx::EriDev& dev, const std::vector<gx:
 // optional pointers.
 void launch_class(gx_context* ctx, gx::EriDev dev, const PlanData& plan, size_t ci, const ClassConf& conf,
                   const int2* groups, int ngroup, unsigned long long* counters, cudaStream_t s, int* used_b1 = nullptr,
-                  int* used_wpb = nullptr, int* used_tiles = nullptr) {
+                  int* used_wpb = nullptr, int* used_tiles = nullptr, bool wide = true) {
     const auto& pc = plan.classes[ci];
     const auto& k = pc.key;
     dev.counters = counters ? counters + 2 * ci : nullptr;
@@ -1253,7 +1262,7 @@ void launch_class(gx_context* ctx, gx::EriDev dev, const PlanData& plan, size_t 
             GX_CUDA(gx::launch_small(k[0], k[1], k[2], k[3], dev, uc, s));
         } else {
             const int pair = gx::dense_orient(k[0], k[1], k[2], k[3], uc);
-            launch_dense_classes(pair, dev, {uc}, s);
+            launch_dense_classes(ctx, pair, dev, {uc}, s, wide);
         }
         if (used_b1) *used_b1 = 32;
         if (used_wpb) *used_wpb = 4;
@@ -1373,8 +1382,9 @@ struct PlanLaunch {
 // of three atoms took 29.1 ms instead of 27.7).
 constexpr int64_t kSharedLaunch = 4096, kSharedPlan = 65536;
 
+// wide: see launch_dense_classes.
 std::vector<PlanLaunch> plan_launches(gx_context* ctx, const gx::EriDev& dev, const PlanData& plan, int precision,
-                                      unsigned long long* counters) {
+                                      unsigned long long* counters, bool wide) {
     std::vector<PlanLaunch> out;
     const auto& tuned = plan.tuned[precision];
     const GroupSet& gs = tuned.valid ? tuned.groups : plan.base;
@@ -1413,15 +1423,36 @@ std::vector<PlanLaunch> plan_launches(gx_context* ctx, const gx::EriDev& dev, co
             if (pair < 0)
                 GX_CUDA(gx::launch_small_list(dev, keys, classes, s));
             else
-                launch_dense_classes(pair, dev, classes, s);
+                launch_dense_classes(ctx, pair, dev, classes, s, wide);
         }});
     }
     for (size_t ci : own)
         out.push_back({{ci}, [=, &dev, &plan, &tuned, &gs](cudaStream_t s) {
             launch_class(ctx, dev, plan, ci, tuned.valid ? tuned.conf[ci] : plan.defconf[ci],
-                         gs.dev.as<int2>() + gs.range[ci].first, (int)gs.range[ci].second, counters, s);
+                         gs.dev.as<int2>() + gs.range[ci].first, (int)gs.range[ci].second, counters, s, nullptr,
+                         nullptr, nullptr, wide);
         }});
     return out;
+}
+
+// What the FP32 launches of a mixed-precision plan left to FP64, for all its
+// lane-dense classes at once: a launch for every class cost a field of five atoms
+// 0.3 ms of 3.8.
+void launch_wide_classes(gx_context* ctx, const gx::EriDev& dev, const PlanData& plan, int precision,
+                         unsigned long long* counters, cudaStream_t s) {
+    if (!(dev.fp32_cut > 0.0f)) return;
+    const auto& tuned = plan.tuned[precision];
+    std::vector<std::pair<int, gx::QuartetClass>> list;
+    for (size_t ci = 0; ci < plan.classes.size(); ++ci) {
+        const auto& k = plan.classes[ci].key;
+        if (k[0] + k[1] + k[2] + k[3] < gx::kWideOrder ||
+            !runs_dense(plan, plan.classes[ci], tuned.valid ? tuned.conf[ci] : plan.defconf[ci], dev.all_real))
+            continue;
+        gx::QuartetClass qc = unit_class(ctx, plan, ci, counters);
+        const int pair = gx::dense_orient(k[0], k[1], k[2], k[3], qc);
+        list.push_back({pair, qc});
+    }
+    GX_CUDA(gx::launch_wide(dev, list, ctx->sm_count, s));
 }
 
 // Enqueue the pair records for (B, O) and every class launch without a wait.
@@ -1477,7 +1508,9 @@ int enqueue_plan(gx_context* ctx, const gx::EriDev& dev, const PlanData& plan, i
     if (counters && !accumulate) GX_CUDA(cudaMemsetAsync(counters, 0, 2 * plan.classes.size() * sizeof(unsigned long long), s));
     ctx->reset_status();
     GX_CUDA(gx::launch_units(plan.units, plan.tasks.as<gx::Task>(), dev, s));
-    const std::vector<PlanLaunch> launches = plan_launches(ctx, dev, plan, precision, counters);
+    // (a class that is copied to the host as soon as it is done has to be complete)
+    const std::vector<PlanLaunch> launches =
+        plan_launches(ctx, dev, plan, precision, counters, host_mapped != nullptr);
     // The classes write disjoint output blocks, so they run concurrently on
     // the auxiliary streams: a plan of many small classes (a Cholesky column
     // batch) costs about its longest class instead of the sum, and the tails
@@ -1508,6 +1541,7 @@ int enqueue_plan(gx_context* ctx, const gx::EriDev& dev, const PlanData& plan, i
             GX_CUDA(cudaEventRecord(ctx->aux_done[k], ctx->aux[k]));
             GX_CUDA(cudaStreamWaitEvent(s, ctx->aux_done[k], 0));
         }
+    if (!host_mapped) launch_wide_classes(ctx, dev, plan, precision, counters, s);
     join_copies();
     return 1 + (int)launches.size();
 }
@@ -1532,7 +1566,7 @@ void enqueue_plans(gx_context* ctx, const std::vector<std::pair<const PlanData*,
     for (const auto& r : runs) GX_CUDA(gx::launch_units(r.first->units, r.first->tasks.as<gx::Task>(), r.second, s));
     std::vector<PlanLaunch> launches;
     for (size_t r = 0; r < runs.size(); ++r)
-        for (PlanLaunch& l : plan_launches(ctx, runs[r].second, *runs[r].first, precision, counters[r]))
+        for (PlanLaunch& l : plan_launches(ctx, runs[r].second, *runs[r].first, precision, counters[r], false))
             launches.push_back(std::move(l));
     const int K = (int)std::min<size_t>(launches.size(), kAux);
     GX_CUDA(cudaEventRecord(ctx->fork, s));
@@ -1542,6 +1576,8 @@ void enqueue_plans(gx_context* ctx, const std::vector<std::pair<const PlanData*,
         GX_CUDA(cudaEventRecord(ctx->aux_done[k], ctx->aux[k]));
         GX_CUDA(cudaStreamWaitEvent(s, ctx->aux_done[k], 0));
     }
+    for (size_t r = 0; r < runs.size(); ++r)
+        launch_wide_classes(ctx, runs[r].second, *runs[r].first, precision, counters[r], s);
 }
 
 // Blocks of the SM copy to page-locked host memory: a few dozen saturate the
@@ -1586,7 +1622,7 @@ void enqueue_parts_with_copies(gx_context* ctx, const gx::EriDev& dev, const Cac
     int next = 0;
     int64_t start = 0;
     for (size_t r = 0; r < cp.parts.size(); ++r) {
-        for (const PlanLaunch& l : plan_launches(ctx, dev, *cp.parts[r], precision, counters[r]))
+        for (const PlanLaunch& l : plan_launches(ctx, dev, *cp.parts[r], precision, counters[r], true))
             l.enqueue(ctx->aux[next++ % kAux]);
         // a waited event stands for its latest record, so the events are reused per part
         for (int k = 0; k < kAux; ++k) {
@@ -4655,18 +4691,17 @@ void plan_enqueue(gx_eri_plan* plan, const double* B, const double* O, int preci
         // the caller's graph: the launches themselves, on unit arrays of their own
         auto mem = std::make_unique<DeviceBuffer>();
         const gx::UnitPlan own = pd.units;
-        if (own.ntask > 0) {
-            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // (for the allocation)
-            GX_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
-            try {
-                unit_arrays(pd.units, *mem, 0, ctx->stream);
-            } catch (...) {
-                cudaThreadExchangeStreamCaptureMode(&mode);
-                pd.units = own;
-                throw;
-            }
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // (for the allocation)
+        GX_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+        try {
+            pd.units.wide = static_cast<int*>(
+                unit_arrays(pd.units, *mem, std::max<size_t>(pd.classes.size(), 1) * sizeof(int), ctx->stream));
+        } catch (...) {
             cudaThreadExchangeStreamCaptureMode(&mode);
+            pd.units = own;
+            throw;
         }
+        cudaThreadExchangeStreamCaptureMode(&mode);
         plan->captured_units.push_back(std::move(mem));
         try {
             plan->last_launches = execute_plan(ctx, plan->basis, B, O, pd, out, precision, mixed_cutoff,

@@ -94,8 +94,11 @@ int dense_orient(int la, int lb, int lc, int ld, QuartetClass& qc) {
     return la * 4 + lb;
 }
 
+int dense_smem(int pair, const QuartetClass& qc, int word) {
+    return smem_bytes(pair / 4, pair % 4, qc.ket.la, qc.ket.lb, word);
+}
+
 cudaError_t launch_dense(int pair, const EriDev& d, const std::vector<QuartetClass>& classes, bool f32, cudaStream_t s) {
-    const int la = pair / 4, lb = pair % 4;
     dense::ClassList list;
     for (size_t k = 0; k < classes.size();) {
         list.n = 0;
@@ -109,7 +112,7 @@ cudaError_t launch_dense(int pair, const EriDev& d, const std::vector<QuartetCla
             list.cls[list.n] = qc;
             list.first[list.n + 1] = (int)(list.first[list.n] + blocks);
             ++list.n;
-            smem = std::max(smem, smem_bytes(la, lb, qc.ket.la, qc.ket.lb, f32 || d.all_real ? 8 : 16));
+            smem = std::max(smem, dense_smem(pair, qc, f32 || d.all_real ? 8 : 16));
         }
         if (list.n == 0) continue;
         cudaError_t e;

@@ -36,8 +36,11 @@
 // are products with exact zeros.
 //
 // FP32.  The same kernel evaluates the FP32 entries of mixed precision (tables,
-// transforms in FP32; separation, prefactor, Boys function outside its
-// asymptotic sector, seeds and every sum into the blocks in FP64), after the FP64 one on the same stream.
+// transforms in FP32; separation, T, prefactor, Boys function outside its
+// asymptotic sector, seeds and every sum into the blocks in FP64), after the FP64
+// one on the same stream.  Entries whose seeds may leave the FP32 range (tight
+// primitives on one centre at high orders) are skipped there and evaluated in
+// FP64 by a launch for all classes (gx_dense_wide.cu).
 #pragma once
 
 #include <type_traits>
@@ -337,25 +340,22 @@ __device__ __forceinline__ void transforms(const Out& o, const RT* R, RT* vb, co
 // 2^e as a double (|e| <= 1000)
 __device__ __forceinline__ double pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }
 
-// FP32 seeds of a lane, scaled by a power of two.  Asymptotic sector
-// (T in FP32 from the FP64 separation): F_0 = sqrt(pi) / (2 sqrt T) and
-// S_{n+1} = -(2n + 1) S_n / X'.X'.  Elsewhere FP64 Boys values and seeds, which
-// are then rounded.  seed32[0 .. L]; `e_lane`: a binary exponent that bounds
-// the seeds.
+// FP32 seeds of a lane, scaled by a power of two.  Asymptotic sector (T and
+// X'.X' formed in FP64, then rounded): F_0 = sqrt(pi) / (2 sqrt T) and
+// S_{n+1} = -(2n + 1) S_n / X'.X'.  Elsewhere, and where |C| is not between 1e-30
+// and 1e30, FP64 Boys values and seeds, which are then rounded.  seed32[0 .. L];
+// `e_lane`: a binary exponent that bounds the seeds.  used: the lane's entry is
+// evaluated here (C is zero otherwise).
 struct Seeds32 {
     float2 F0, iXX;
     bool asymptotic;
     int e_lane;
 };
-__device__ __forceinline__ Seeds32 seeds32_begin(const float2* x, double p, double q, double2 C, int L) {
+__device__ __forceinline__ Seeds32 seeds32_begin(double2 XX64, double tre, double tim, double2 C, bool used, int L) {
     Seeds32 s{};
     s.e_lane = -1000;
-    const float pf = (float)p, qf = (float)q;
-    const float rho = __fdividef(pf * qf, pf + qf);
-    const float2 XX = make_float2(
-        fmaf(x[0].x, x[0].x, fmaf(x[1].x, x[1].x, x[2].x * x[2].x)) - fmaf(x[0].y, x[0].y, fmaf(x[1].y, x[1].y, x[2].y * x[2].y)),
-        2.0f * fmaf(x[0].x, x[0].y, fmaf(x[1].x, x[1].y, x[2].x * x[2].y)));
-    const float tr = rho * XX.x, ti = rho * XX.y;
+    const float2 XX = make_float2((float)XX64.x, (float)XX64.y);
+    const float tr = (float)tre, ti = (float)tim;
     const float r2 = fmaf(tr, tr, ti * ti);
     s.asymptotic = tr >= 2.0f * L + 24.0f && fabsf(ti) <= 0.5f * tr && (r2 <= 160.0f * 160.0f || tr >= 2.0f * L + 60.0f);
     if (!s.asymptotic) return s;
@@ -364,8 +364,8 @@ __device__ __forceinline__ Seeds32 seeds32_begin(const float2* x, double p, doub
     const float k0 = 0.886226925452758f * ir;  // sqrt(pi) / 2 / |T|
     s.F0 = make_float2(k0 * sq, -k0 * (0.5f * ti / sq));
     const float m2 = fmaf(XX.x, XX.x, XX.y * XX.y);
-    s.iXX = make_float2(__fdividef(XX.x, m2), -__fdividef(XX.y, m2));
     const float ixx = rsqrtf(m2);
+    s.iXX = make_float2(XX.x * ixx * ixx, -XX.y * ixx * ixx);
     float gm = 1.0f, gmax = 1.0f;
     for (int n = 0; n < L; ++n) {
         gm *= (2.0f * n + 1.0f) * ixx;
@@ -374,9 +374,60 @@ __device__ __forceinline__ Seeds32 seeds32_begin(const float2* x, double p, doub
     const int ec = max((__double2hiint(C.x) >> 20) & 0x7ff, (__double2hiint(C.y) >> 20) & 0x7ff);
     const int ef = (__float_as_int(fmaxf(fabsf(s.F0.x), fabsf(s.F0.y))) >> 23) & 0xff;
     const int eg = (__float_as_int(gmax) >> 23) & 0xff;
+    if (used && (ec < 1023 - 99 || ec > 1023 + 99 || eg == 0xff)) s.asymptotic = false;
     if (ec > 0 && ec < 0x7ff && ef > 0 && ef < 0xff && eg < 0xff) s.e_lane = (ec - 1023) + (ef - 127) + (eg - 127) + 2;
+    if (!s.asymptotic) s.e_lane = -1000;
     return s;
 }
+
+// The entries of a stream that FP32 leaves to FP64, in stream order and up to 32
+// at a time, of tasks of one kind (see Stream): they are few among the stream's,
+// so they wait in a queue until there are 32, the kind changes or the stream ends.
+struct WideEntries {
+    int waiting = 0, kind = 0;  // queued entries and their kind
+    unsigned held = 0;          // lanes whose entry of the last batch has yet to be queued
+    int htask = 0;
+    int2 hpq = make_int2(0, 0);
+    bool done = false;
+
+    __device__ __forceinline__ int next(Stream<false>& stream, int4* queue, int lane, int L, int& task, int2& pq,
+                                        int& batch_kind) {
+        const PairData& pp = stream.d.pairs;
+        for (;;) {
+            if (held && (waiting == 0 || kind == stream.batch_kind)) {
+                if (held >> lane & 1)
+                    queue[waiting + __popc(held & ((1u << lane) - 1u))] = make_int4(htask, hpq.x, hpq.y, 0);
+                waiting += __popc(held);
+                kind = stream.batch_kind;
+                held = 0;
+                __syncwarp();
+            }
+            if (waiting >= 32 || (waiting > 0 && (held || done))) {
+                const int nb = min(waiting, 32);
+                const int4 e = queue[min(lane, nb - 1)], rest = queue[32 + lane];
+                __syncwarp();
+                if (lane < waiting - nb) queue[lane] = rest;
+                __syncwarp();
+                waiting -= nb;
+                task = e.x;
+                pq = make_int2(e.y, e.z);
+                batch_kind = kind;
+                return nb;
+            }
+            if (done) return 0;
+            int rank;
+            const int n = stream.next(lane, htask, rank, hpq);
+            done = n == 0;
+            bool wide = false;
+            if (lane < n) {
+                const Task* tg = stream.qc.tasks + htask;
+                const int op = pp.order[tg->pab + hpq.x], oq = pp.order[tg->pcd + hpq.y];
+                wide = stream.qc.swap ? seeds_exceed_fp32(pp, oq, op, L) : seeds_exceed_fp32(pp, op, oq, L);
+            }
+            held = __ballot_sync(0xffffffffu, wide);
+        }
+    }
+};
 
 // The classes of one launch: all have the same template pair; block b works on
 // class c with first[c] <= b < first[c + 1], on unit (b - first[c]) / nchunk and
@@ -388,9 +439,12 @@ struct ClassList {
     QuartetClass cls[kMaxClasses];
 };
 
-// Unit `unit` of a class; share_of: which of the nchunk blocks that share it.
-template <int LA, int LB, bool F32>
-__device__ __forceinline__ void dense_block(const EriDev& d, const QuartetClass& qc, int unit, int share_of) {
+// Unit `unit` of a class; share_of: which of the nchunk blocks that share it;
+// queue: 64 entries of shared memory (kDenseWide).
+template <int LA, int LB, DenseMode MODE>
+__device__ __forceinline__ void dense_block(const EriDev& d, const QuartetClass& qc, int unit, int share_of,
+                                            int4* queue = nullptr) {
+    constexpr bool F32 = MODE == kDenseF32, WIDE = MODE == kDenseWide;
     constexpr int NH = hc(LA + LB), NHP = (NH + 3) / 4 * 4;
     constexpr int NAB = nc(LA) * nc(LB), NCB = nc(LB), CG = group_of(NAB);
     extern __shared__ double2 dsm[];
@@ -413,16 +467,19 @@ __device__ __forceinline__ void dense_block(const EriDev& d, const QuartetClass&
     int* s_shift = reinterpret_cast<int*>(base + lay.shift);
     int* seg_lane = reinterpret_cast<int*>(base + lay.seg_lane);
     int* info = reinterpret_cast<int*>(base + lay.info);  // entries, segments, real sides
+    // (set by the FP32 launch, which follows the FP64 one)
+    if (MODE == kDenseF64 && qc.wide && unit == 0 && share_of == 0 && threadIdx.x == 0) *qc.wide = 0;
     // the unit's tasks (entries past the last unit lie beyond the class)
-    const int* start = F32 ? qc.unit_start32 : qc.unit_start;
+    const int* start = MODE == kDenseF64 ? qc.unit_start : qc.unit_start32;
     int t0, t1;
     if (start) {
-        t0 = start[unit];
-        t1 = min(start[unit + 1], qc.ntask);
+        t0 = start[unit] & 0x7fffffff;
+        t1 = min(start[unit + 1] & 0x7fffffff, qc.ntask);
     } else {
         __shared__ int bounds[2];
         __shared__ long long sums[kWarps];
-        cut_units<32 * kWarps>(d, qc, F32 ? 1 : 0, unit, 1, !F32 && share_of == 0, bounds, sums);
+        cut_units<32 * kWarps>(d, qc, MODE == kDenseF64 ? 0 : 1, unit, 1, MODE == kDenseF64 && share_of == 0, bounds,
+                               sums);
         t0 = bounds[0];
         t1 = bounds[1];
     }
@@ -460,13 +517,22 @@ __device__ __forceinline__ void dense_block(const EriDev& d, const QuartetClass&
     const int2* plan = d.rec_plan + d.rec_plan_off[L];
     const bool leader = warp == (int)(blockIdx.x % kWarps);
     unsigned count = 0;
-    Stream<F32> stream(d, qc, t0, t1);
+    Stream<F32> stream(d, qc, t0, t1, MODE == kDenseF64 ? fmaxf(d.skip_cut, d.fp32_cut) : d.skip_cut,
+                       MODE == kDenseF64 ? 3.4e38f : d.fp32_cut, MODE == kDenseF64 ? qc.unit_count : qc.unit_count32);
+    WideEntries wide;
+    unsigned skipped = 0;  // FP32: lanes that met an entry left to FP64
     __syncthreads();
     for (;;) {
         if (leader) {
-            int task, rank;
+            int task, rank = 0, kind;
             int2 pq;
-            const int nb = stream.next(lane, task, rank, pq);
+            int nb;
+            if constexpr (WIDE) {
+                nb = wide.next(stream, queue, lane, L, task, pq, kind);
+            } else {
+                nb = stream.next(lane, task, rank, pq);
+                kind = stream.batch_kind;
+            }
             if (nb > 0) {
                 // the lanes past a short batch repeat its last entry with a zero prefactor
                 const bool active = lane < nb;
@@ -485,11 +551,17 @@ __device__ __forceinline__ void dense_block(const EriDev& d, const QuartetClass&
                     const int s = __popc(heads & ((1u << lane) - 1u));
                     seg_off[s] = tg->out_off;
                     seg_st[s] = strides(tg);
-                    seg_lane[s] = lane | (!F32 && rank == 0 ? kStore : 0) | (stream.run == 32 ? kLongRuns : 0);
+                    seg_lane[s] = lane | (MODE == kDenseF64 && rank == 0 ? kStore : 0) |
+                                  (WIDE ? kSingle : (stream.run == 32 ? kLongRuns : 0));
                 }
                 const double pi0 = pp.Pi[3 * ip], pi1 = pp.Pi[3 * ip + 1], pi2 = pp.Pi[3 * ip + 2];
                 const double qi0 = pp.Pi[3 * iq], qi1 = pp.Pi[3 * iq + 1], qi2 = pp.Pi[3 * iq + 2];
-                const bool bra_real = stream.batch_kind & 1, ket_real = stream.batch_kind & 2;
+                const bool bra_real = kind & 1, ket_real = kind & 2;
+                bool mine = active;
+                if constexpr (F32) {
+                    if (L >= kWideOrder && seeds_exceed_fp32(pp, ip, iq, L)) mine = false;
+                    skipped |= active && !mine;
+                }
                 const double p = pp.p[ip], q = pp.p[iq];
                 const double rs = rsqrt(p + q);
                 const double x0 = pp.Pr[3 * ip] - pp.Pr[3 * iq], x1 = pp.Pr[3 * ip + 1] - pp.Pr[3 * iq + 1],
@@ -500,9 +572,9 @@ __device__ __forceinline__ void dense_block(const EriDev& d, const QuartetClass&
                     seg_lane[nseg] = nb;
                     info[0] = nb;
                     info[1] = nseg;
-                    info[2] = stream.batch_kind;
+                    info[2] = kind;
                 }
-                count += active && share_of == 0;
+                count += mine && share_of == 0;
                 if (!F32 && bra_real && ket_real) {
                     const double rho = p * q * rs * rs;
                     const double t = rho * fma(x0, x0, fma(x1, x1, x2 * x2));
@@ -527,20 +599,20 @@ __device__ __forceinline__ void dense_block(const EriDev& d, const QuartetClass&
                     sd[(L + 3) * 32] = x2;
                 } else {
                     const double2 X[3] = {c2(x0, pi0 - qi0), c2(x1, pi1 - qi1), c2(x2, pi2 - qi2)};
-                    double2 C = active ? cscale(cmul(pp.F[ip], pp.F[iq]), rs) : c2(0.0, 0.0);
+                    double2 C = mine ? cscale(cmul(pp.F[ip], pp.F[iq]), rs) : c2(0.0, 0.0);
+                    const double rho = p * q * rs * rs;
+                    const double2 XX = c2(fma(X[0].x, X[0].x, fma(X[1].x, X[1].x, X[2].x * X[2].x)) -
+                                              fma(X[0].y, X[0].y, fma(X[1].y, X[1].y, X[2].y * X[2].y)),
+                                          2.0 * fma(X[0].x, X[0].y, fma(X[1].x, X[1].y, X[2].x * X[2].y)));
+                    const double tre = rho * XX.x, tim = rho * XX.y;
                     float2 X32[3];
                     Seeds32 s32{};
                     if constexpr (F32) {
                         for (int k = 0; k < 3; ++k) X32[k] = make_float2((float)X[k].x, (float)X[k].y);
-                        s32 = seeds32_begin(X32, p, q, C, L);
+                        s32 = seeds32_begin(XX, tre, tim, C, mine, L);
                     }
                     double2 Sh[kMaxSeeds];
                     if (!F32 || !s32.asymptotic) {
-                        const double rho = p * q * rs * rs;
-                        const double tre =
-                            rho * (fma(X[0].x, X[0].x, fma(X[1].x, X[1].x, X[2].x * X[2].x)) -
-                                   fma(X[0].y, X[0].y, fma(X[1].y, X[1].y, X[2].y * X[2].y)));
-                        const double tim = 2.0 * rho * fma(X[0].x, X[0].y, fma(X[1].x, X[1].y, X[2].x * X[2].y));
                         double2 e0;
                         if (const int rc = boys_eval(tre, tim, L, d.boys, d.gl, Sh, e0)) {
                             report(d.status, rc, task, L, tre, tim);
@@ -620,27 +692,33 @@ __device__ __forceinline__ void dense_block(const EriDev& d, const QuartetClass&
         }
         __syncthreads();  // the next batch overwrites the table
     }
+    if constexpr (F32) {
+        if (leader && __any_sync(0xffffffffu, skipped) && lane == 0) {
+            *qc.wide = 1;
+            if (start) const_cast<int*>(start)[unit] = t0 | (int)0x80000000;
+        }
+    }
     if (qc.counters && leader && share_of == 0) {
         const unsigned a = __reduce_add_sync(0xffffffffu, count);
         if (lane == 0 && a) atomicAdd(&qc.counters[F32 ? 1 : 0], (unsigned long long)a);
     }
 }
 
-template <int LA, int LB, bool F32>
+template <int LA, int LB, DenseMode MODE>
 __global__ void __launch_bounds__(32 * kWarps) dense_kernel(const __grid_constant__ EriDev d,
                                                             const __grid_constant__ QuartetClass qc) {
-    dense_block<LA, LB, F32>(d, qc, blockIdx.x, blockIdx.y);
+    dense_block<LA, LB, MODE>(d, qc, blockIdx.x, blockIdx.y);
 }
 
 // (reading the class through the list costs the FP64-bound plans 1.5%, so a
 // class with a launch of its own has the kernel above)
-template <int LA, int LB, bool F32>
+template <int LA, int LB, DenseMode MODE>
 __global__ void __launch_bounds__(32 * kWarps) dense_list_kernel(const __grid_constant__ EriDev d,
                                                                  const __grid_constant__ ClassList list) {
     int ci = 0;
     while (ci + 1 < list.n && (int)blockIdx.x >= list.first[ci + 1]) ++ci;
     const int b = (int)blockIdx.x - list.first[ci], nchunk = list.cls[ci].nchunk;
-    dense_block<LA, LB, F32>(d, list.cls[ci], b / nchunk, b % nchunk);
+    dense_block<LA, LB, MODE>(d, list.cls[ci], b / nchunk, b % nchunk);
 }
 
 constexpr int kMaxSmem = 200 * 1024;

@@ -9,7 +9,7 @@ cudaError_t run_list_f32(int pair, const EriDev& d, const ClassList& list, int s
 #define GX_CASE(A, B)                                                                                             \
     case A * 4 + B: {                                                                                             \
         static PerDevice limit;                                                                                   \
-        return launch_with_smem(dense_list_kernel<A, B, true>, limit, dim3(list.first[list.n]), smem, s, d, list); \
+        return launch_with_smem(dense_list_kernel<A, B, kDenseF32>, limit, dim3(list.first[list.n]), smem, s, d, list); \
     }
         GX_DENSE_PAIRS
 #undef GX_CASE

@@ -9,7 +9,7 @@ cudaError_t run_one_f64(int pair, const EriDev& d, const QuartetClass& qc, int s
 #define GX_CASE(A, B)                                                                                             \
     case A * 4 + B: {                                                                                             \
         static PerDevice limit;                                                                                   \
-        return launch_with_smem(dense_kernel<A, B, false>, limit, dim3(qc.ngroup, qc.nchunk), smem, s, d, qc);    \
+        return launch_with_smem(dense_kernel<A, B, kDenseF64>, limit, dim3(qc.ngroup, qc.nchunk), smem, s, d, qc);    \
     }
         GX_DENSE_PAIRS
 #undef GX_CASE

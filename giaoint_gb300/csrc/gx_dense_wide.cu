@@ -1,0 +1,82 @@
+// Lane-dense kernel (gx_dense.cuh): the entries that FP32 leaves to FP64, of all
+// classes of a plan in one launch.  There are few of them, so a small grid looks
+// through the units (a thread each) for those in which the FP32 launch met one.
+#include <algorithm>
+
+#include "gx_dense.cuh"
+
+namespace gx {
+
+namespace {
+
+constexpr int kMaxWide = 48;
+struct WideList {
+    int n;
+    int pair[kMaxWide];
+    QuartetClass cls[kMaxWide];
+};
+
+__global__ void __launch_bounds__(32 * dense::kWarps) wide_kernel(const __grid_constant__ EriDev d,
+                                                                  const __grid_constant__ WideList list) {
+    constexpr int THREADS = 32 * dense::kWarps;
+    __shared__ int4 queue[64];
+    __shared__ long long hits[THREADS];
+    __shared__ int nhit;
+    for (int c = 0; c < list.n; ++c) {
+        const QuartetClass& qc = list.cls[c];
+        if (*qc.wide == 0) continue;
+        const long long items = (long long)qc.ngroup * qc.nchunk;
+        for (long long i0 = blockIdx.x; i0 < items; i0 += (long long)THREADS * gridDim.x) {
+            if (threadIdx.x == 0) nhit = 0;
+            __syncthreads();
+            const long long i = i0 + (long long)threadIdx.x * gridDim.x;
+            // (any order: they write disjoint elements)
+            if (i < items && (!qc.unit_start32 || qc.unit_start32[i / qc.nchunk] < 0)) hits[atomicAdd(&nhit, 1)] = i;
+            __syncthreads();
+            const int n = nhit;
+            for (int k = 0; k < n; ++k) {
+                switch (list.pair[c]) {
+#define GX_CASE(A, B)                                                              \
+    case A * 4 + B:                                                                \
+        dense::dense_block<A, B, kDenseWide>(d, qc, (int)(hits[k] / qc.nchunk),    \
+                                             (int)(hits[k] % qc.nchunk), queue);   \
+        break;
+                    GX_DENSE_PAIRS
+#undef GX_CASE
+                }
+                __syncthreads();
+            }
+        }
+    }
+}
+
+}  // namespace
+
+cudaError_t launch_wide(const EriDev& d, const std::vector<std::pair<int, QuartetClass>>& classes, int sms,
+                        cudaStream_t s) {
+    static PerDevice limit;
+    WideList list;
+    for (size_t k = 0; k < classes.size();) {
+        long long units = 0;
+        int smem = 0;
+        for (list.n = 0; k < classes.size() && list.n < kMaxWide; ++k) {
+            const auto& [pair, qc] = classes[k];
+            if (qc.ntask <= 0 || qc.ngroup <= 0 || !qc.wide) continue;
+            list.pair[list.n] = pair;
+            list.cls[list.n] = qc;
+            // (blocks that share a unit's components: few units have anything to do,
+            // and the launch is the end of its plan)
+            const int nchunk = dense_chunks(qc.bra.la, qc.bra.lb, qc.ket.la, qc.ket.lb, 8, true);
+            list.cls[list.n++].nchunk = nchunk;
+            units += (long long)qc.ngroup * nchunk;
+            smem = std::max(smem, dense_smem(pair, qc, d.all_real ? 8 : 16));
+        }
+        if (list.n == 0) continue;
+        const dim3 grid((unsigned)std::min<long long>(units, 2ll * std::max(sms, 1)));
+        const cudaError_t e = dense::launch_with_smem(wide_kernel, limit, grid, smem, s, d, list);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
+}  // namespace gx

@@ -6,6 +6,7 @@
 #include <stdint.h>
 
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "gx_device.cuh"
@@ -44,7 +45,7 @@ struct PairData {
     const float2* Epool32; // the same coefficients in FP32 (mixed precision)
     const int* order;      // [npp] records of each shell pair sorted by decreasing bound
     const float* sbound;   // [npp] bound of order[i] (FP32, for gating)
-    const float4* g32;     // [2*npp] (P, p) and (Im P', 0) in FP32, for classifying Boys arguments
+    const float4* g32;     // [2*npp] (P, p) and (Im P', bound of log2 |F|) in FP32, for classifying entries
 };
 
 // True when the Boys argument T of primitive quartet (ip, iq) lies in the
@@ -60,6 +61,49 @@ __device__ __forceinline__ bool boys_asymptotic32(const PairData& pp, int ip, in
     const float x = rho * (fmaf(dx, dx, fmaf(dy, dy, dz * dz)) - fmaf(ex, ex, fmaf(ey, ey, ez * ez)));
     const float y = 2.0f * rho * fmaf(dx, ex, fmaf(dy, ey, dz * ez));
     return x >= 2.0f * L + 25.0f && fabsf(y) <= 0.45f * x && (x * x + y * y <= 150.0f * 150.0f || x >= 2.0f * L + 61.0f);
+}
+
+// True when a seed C (-2 rho)^n F_n(T), n <= L, of primitive quartet (ip, iq) may
+// reach 1e25 in magnitude, from the FP32 pair geometry: the mixed-precision
+// evaluation leaves such an entry in FP64.  An upper bound of the seeds decides
+// (|F_n(T)| <= F_n(Re T), whose values over n are log-convex, so that n = 0 and
+// n = L suffice), and with operations that are never fused or reordered, because
+// the kernel that skips the entry and the one that takes it both ask.
+__device__ __forceinline__ bool seeds_exceed_fp32(const PairData& pp, int ip, int iq, int L) {
+    const float4 a = pp.g32[2 * ip], b = pp.g32[2 * iq];
+    const float4 ai = pp.g32[2 * ip + 1], bi = pp.g32[2 * iq + 1];
+    // |Re X'|^2 from below and |Im X'|^2 from above
+    float re = 0.0f, im = 0.0f;
+    auto axis = [&](float x, float y, float u, float v) {
+        const float dr = fmaxf(0.0f, __fsub_rn(fabsf(__fsub_rn(x, y)),
+                                               __fmul_rn(0x1p-22f, __fadd_rn(fabsf(x), fabsf(y)))));
+        const float di = __fadd_rn(fabsf(__fsub_rn(u, v)), __fmul_rn(0x1p-22f, __fadd_rn(fabsf(u), fabsf(v))));
+        re = __fmaf_rn(dr, dr, re);
+        im = __fmaf_rn(di, di, im);
+    };
+    axis(a.x, b.x, ai.x, bi.x);
+    axis(a.y, b.y, ai.y, bi.y);
+    axis(a.z, b.z, ai.z, bi.z);
+    const float s = __fadd_rn(a.w, b.w);
+    const float rho = __fmul_rn(a.w, __fdiv_rn(b.w, s));
+    float t = __fmul_rn(rho, __fsub_rn(__fmul_rn(re, 1.0f - 0x1p-20f), __fmul_rn(im, 1.0f + 0x1p-20f)));
+    t = __fmul_rn(t, t > 0.0f ? 1.0f - 0x1p-20f : 1.0f + 0x1p-20f);  // Re T from below
+    // log2 of F_0 and F_L: e^{-t} / (2n + 1), and Gamma(n + 1/2) / (2 t^{n + 1/2}) for t > 0
+    float f0 = 0.0f, fl = -__log2f((float)(2 * L + 1));
+    if (t > 0.0f) {
+        float g = 0.88622693f;  // sqrt(pi) / 2
+        for (int n = 0; n < L; ++n) g = __fmul_rn(g, (float)n + 0.5f);
+        const float lt = __log2f(t);
+        f0 = fminf(0.0f, __fsub_rn(-0.17426f, __fmul_rn(0.5f, lt)));
+        fl = fminf(fl, __fsub_rn(__log2f(g), __fmul_rn((float)L + 0.5f, lt)));
+    } else {
+        f0 = __fmul_rn(-1.442696f, t);
+        fl = __fadd_rn(fl, f0);
+    }
+    const float c = __fsub_rn(__fadd_rn(ai.w, bi.w), __fmul_rn(0.5f, __log2f(s)));
+    const float top = fmaxf(__fadd_rn(c, f0),
+                            __fadd_rn(__fadd_rn(c, fl), __fmul_rn((float)L, __fadd_rn(1.0f, __log2f(rho)))));
+    return !(top < 82.0f);  // log2(1e25) = 83.05; half a unit for |x| + |y|, half for the rounding here
 }
 
 struct BasisDev {
@@ -99,8 +143,9 @@ struct QuartetClass {
     long long target;         // weight of a unit, and the components of the four shells, one byte each, for that
     int dims;
     unsigned long long* counters;  // [0] FP64, [1] FP32 primitive quartets evaluated (may be null)
-    const int* unit_start32;  // lane-dense kernel: the same for the FP32 entries
-    const int* unit_count32;
+    const int* unit_start32;  // lane-dense kernel: the same for the FP32 entries (bit 31 of a start: the unit
+    const int* unit_count32;  //    has entries that FP32 left to FP64)
+    int* wide;                // 1: the class has such entries (null: it can have none)
 };
 
 // Work units of a plan's small and lane-dense classes with many tasks
@@ -123,6 +168,7 @@ struct UnitPlan {
     long long* tile;            // [tiles] weight prefix of the tiles
     int* start;                 // [nunit]
     unsigned* done;             // blocks finished (0 between executions)
+    int* wide;                  // [classes of the plan] see QuartetClass
 };
 
 struct EriDev {
@@ -257,12 +303,22 @@ cudaError_t launch_gather_abs(const double2* src, const long long* idx, double* 
 constexpr int kUnitMinTasks = 512;  // classes with fewer tasks have no entry in the unit plan
 bool dense_class(int la, int lb, int lc, int ld, bool real);  // real: the execution's pairs all have q = 0
 int dense_chunks(int la, int lb, int lc, int ld, int want, bool single);
+// FP64 entries; FP32 entries; those of the FP32 range whose seeds leave it, in
+// FP64 (classes of order kWideOrder and up).
+enum DenseMode { kDenseF64, kDenseF32, kDenseWide };
+constexpr int kWideOrder = 5;
 long long unit_tiles(long long ntask);
 cudaError_t launch_units(const UnitPlan& u, const Task* tasks, const EriDev& d, cudaStream_t s);
 // A dense class oriented for its template pair (LA, LB): returns LA * 4 + LB.
 int dense_orient(int la, int lb, int lc, int ld, QuartetClass& qc);
 // Classes of one template pair in as few launches as hold them.
 cudaError_t launch_dense(int pair, const EriDev& d, const std::vector<QuartetClass>& classes, bool f32, cudaStream_t s);
+// Shared memory of a block (qc oriented for `pair`; word: bytes of a table entry).
+int dense_smem(int pair, const QuartetClass& qc, int word);
+// The entries that FP32 left to FP64, of classes of any template pair (given
+// with their pair), after their FP32 launches.
+cudaError_t launch_wide(const EriDev& d, const std::vector<std::pair<int, QuartetClass>>& classes, int sms,
+                        cudaStream_t s);
 
 // register-resident small classes (gx_small.cu)
 bool small_class(int la, int lb, int lc, int ld);

@@ -467,7 +467,10 @@ __global__ void pair_scalar_kernel(BasisDev bs, double3 B, double3 O, int npp, c
     }
     out_F[i] = c2(mag * damp * cs, mag * damp * sn);
     out_g32[2 * i] = make_float4((float)P[0], (float)P[1], (float)P[2], (float)p);
-    out_g32[2 * i + 1] = make_float4((float)(-0.5 * q[0] / p), (float)(-0.5 * q[1] / p), (float)(-0.5 * q[2] / p), 0.0f);
+    // log2 |F|, at most 1.5 too large
+    const int ef = max((__double2hiint(out_F[i].x) >> 20) & 0x7ff, (__double2hiint(out_F[i].y) >> 20) & 0x7ff);
+    out_g32[2 * i + 1] = make_float4((float)(-0.5 * q[0] / p), (float)(-0.5 * q[1] / p), (float)(-0.5 * q[2] / p),
+                                     (float)ef - 1021.5f);
 }
 
 // Complex Hermite coefficients E~_k = sum_{t>=k} C(t,k) (-i q)^{t-k} E_t per

@@ -128,7 +128,9 @@ __device__ __forceinline__ int run_length(int survivors) { return survivors >= 2
 // The surviving primitive quartets of the tasks t0 .. t1 - 1 in stream order
 // (task, bra pair, ket pair), up to 32 at a time, one per lane.  32 tasks are
 // looked at together: their survivor counts as an inclusive prefix over the
-// lanes, and how many of those have been handed out.  FP64 batches hold tasks
+// lanes, and how many of those have been handed out.  Entries with
+// lo <= B_P B_Q < hi; counts: their number in every task of the class (may be
+// null).  FP64 batches hold tasks
 // of one kind (bit 0: template pair real, bit 1: other pair real), so that a
 // task's arithmetic does not depend on its neighbours.
 template <bool F32>
@@ -136,14 +138,13 @@ struct Stream {
     const EriDev& d;
     const QuartetClass& qc;
     float lo, hi;
+    const int* counts;
     int t1, next_task, chunk = 0, incl = 0, cnt = 0, kind = 0, total = 0, used = 0, batch_kind = 0;
     int run = 8;  // run length of the lane's task
 
-    __device__ __forceinline__ Stream(const EriDev& dev, const QuartetClass& cls, int first, int last)
-        : d(dev), qc(cls), t1(last), next_task(first) {
-        lo = F32 ? d.skip_cut : fmaxf(d.skip_cut, d.fp32_cut);
-        hi = F32 ? d.fp32_cut : 3.4e38f;
-    }
+    __device__ __forceinline__ Stream(const EriDev& dev, const QuartetClass& cls, int first, int last, float from,
+                                      float below, const int* task_counts)
+        : d(dev), qc(cls), lo(from), hi(below), counts(task_counts), t1(last), next_task(first) {}
     // Returns the number of entries; every lane below it has its task, the
     // entry's rank within the task, and its bra and ket pair.
     __device__ __forceinline__ int next(int lane, int& task, int& rank, int2& pq) {
@@ -166,7 +167,6 @@ struct Stream {
                                (pk[0] == 0.0 && pk[1] == 0.0 && pk[2] == 0.0 ? (qc.swap ? 1 : 2) : 0);
                         if (d.all_real) kind = 3;  // (every pair has q = 0; the table is sized for that)
                     }
-                    const int* counts = F32 ? qc.unit_count32 : qc.unit_count;
                     if (!counts)
                         cnt = survivors(pp.sbound + tg->pab, np[tg->sa] * np[tg->sb], pp.sbound + tg->pcd,
                                         np[tg->sc] * np[tg->sd], lo, hi);
@@ -239,13 +239,14 @@ struct Stream {
 
 // Flags of a batch's segment beside its first lane: the batch holds the shell
 // quartet's first FP64 entry, which stores instead of adding; long runs.
-constexpr int kStore = 256, kLongRuns = 512;
+// kSingle: entry by entry (entries queued over several batches of the stream).
+constexpr int kStore = 256, kLongRuns = 512, kSingle = 1024;
 
 // A segment's values v(l0) .. v(l1 - 1) by runs, added to sum (or, with
 // kStore, in its place).
 template <typename T, typename Get>
 __device__ __forceinline__ T add_by_runs(T sum, int flags, int l0, int l1, Get&& v) {
-    const int run = flags & kLongRuns ? 32 : 8;
+    const int run = flags & kSingle ? 1 : (flags & kLongRuns ? 32 : 8);
     bool fresh = flags & kStore;
     for (int l = l0; l < l1; l += run) {
         T part = v(l);
