@@ -25,17 +25,27 @@ __device__ __forceinline__ int survivors(const float* __restrict__ sp, int Kab, 
     return n;
 }
 
-// The j-th of them in stream order (bra pair, then ket pair).
-__device__ __forceinline__ int2 survivor(const float* __restrict__ sp, int Kab, const float* __restrict__ sq, int Kcd,
-                                         float lo, float hi, int j) {
-    int qb = Kcd, qa = hi < 3.0e38f ? Kcd : 0;
-    for (int P = 0; P < Kab; ++P) {
+// Where a survivor lies: its bra pair, the ends of that one's run of ket pairs, and
+// the survivors of the bra pairs before it.
+struct Row {
+    int P, qb, qa, before;
+};
+
+// The j-th of them in stream order (bra pair, then ket pair), from `row` on (of the
+// task's start, or of an earlier survivor), which is left at the survivor's.
+__device__ __forceinline__ int2 survivor(const float* __restrict__ sp, int Kab, const float* __restrict__ sq, float lo,
+                                         float hi, int j, Row& row) {
+    int qb = row.qb, qa = row.qa, before = row.before;
+    for (int P = row.P; P < Kab; ++P) {
         const float b = sp[P];
         while (qb > 0 && !(b * sq[qb - 1] >= lo)) --qb;
         while (qa > 0 && b * sq[qa - 1] < hi) --qa;
         const int n = qb - qa > 0 ? qb - qa : 0;
-        if (j < n) return make_int2(P, qa + j);
-        j -= n;
+        if (j - before < n) {
+            row = Row{P, qb, qa, before};
+            return make_int2(P, qa + j - before);
+        }
+        before += n;
     }
     return make_int2(0, 0);
 }
@@ -141,6 +151,11 @@ struct Stream {
     const int* counts;
     int t1, next_task, chunk = 0, incl = 0, cnt = 0, kind = 0, total = 0, used = 0, batch_kind = 0;
     int run = 8;  // run length of the lane's task
+    // The last entry handed out: the next one of its task is sought from there
+    // (from the task's start every batch of a deep contraction walked over all its
+    // bra pairs: one (ss|ss) of 20 primitives a shell, 1.6e5 entries, 141 ms).
+    int row_task = -1;
+    Row row{};
 
     __device__ __forceinline__ Stream(const EriDev& dev, const QuartetClass& cls, int first, int last, float from,
                                       float below, const int* task_counts)
@@ -228,11 +243,19 @@ struct Stream {
             got += take;
             if (full) break;
         }
+        if (got == 0) return 0;
+        Row r = row;
         if (lane < got) {
             const Task* tg = qc.tasks + task;
-            pq = survivor(pp.sbound + tg->pab, np[tg->sa] * np[tg->sb], pp.sbound + tg->pcd, np[tg->sc] * np[tg->sd],
-                          lo, hi, rank);
+            if (task != row_task) {
+                const int Kcd = np[tg->sc] * np[tg->sd];
+                r = Row{0, Kcd, hi < 3.0e38f ? Kcd : 0, 0};
+            }
+            pq = survivor(pp.sbound + tg->pab, np[tg->sa] * np[tg->sb], pp.sbound + tg->pcd, lo, hi, rank, r);
         }
+        row_task = __shfl_sync(0xffffffffu, task, got - 1);
+        row = Row{__shfl_sync(0xffffffffu, r.P, got - 1), __shfl_sync(0xffffffffu, r.qb, got - 1),
+                  __shfl_sync(0xffffffffu, r.qa, got - 1), __shfl_sync(0xffffffffu, r.before, got - 1)};
         return got;
     }
 };

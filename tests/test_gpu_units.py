@@ -154,3 +154,23 @@ def test_real_orders_9_and_10(key, tasks, oracle):
                 bits[precision] = values.copy()
             elif turn == 2:
                 assert np.array_equal(values, bits[precision])
+
+
+def test_cost_of_an_entry_does_not_grow_with_the_contraction():
+    """One (ss|ss) of 20 primitives a shell against one of 14: 4.2 times the entries.  (Sought from the task's first
+    bra pair for every batch, they took 6.6 times as long.)"""
+    import time
+
+    field = gi.MagneticField((0.1, 0.05, 0.0))
+    seconds = []
+    for nprim in (14, 20):
+        rng = np.random.default_rng(1)
+        shells = [gi.Shell((0.3 * i, 0.0, 0.1 * i), 0, np.exp(rng.uniform(-2.0, 8.0, nprim)),
+                           rng.uniform(0.1, 1.0, nprim)) for i in range(2)]
+        best = np.inf
+        for _ in range(5):
+            start = time.perf_counter()
+            gi.eri_shell(shells[0], shells[1], shells[0], shells[1], field=field)
+            best = min(best, time.perf_counter() - start)
+        seconds.append(best)
+    assert seconds[1] <= 5.2 * seconds[0], seconds
