@@ -121,7 +121,7 @@ __host__ __device__ constexpr int rows_of(int nab) { return slice_of(nab) * grou
 // FP64, 8 complex FP32 or an execution all of whose pairs are real).  hsum rows are padded to four entries so
 // that the table rows of one Hermite index of the other side are read as int4.
 struct Layout {
-    int hsum, kh, kb, R, v, seed, eb, ek, seg_off, seg_st, shift, seg_lane, info, total;
+    int hsum, kh, kb, R, v, seed, eb, ek, seg_off, seg_st, shift, seg_lane, info, walk, total;
 };
 __host__ __device__ inline Layout layout(int NH, int NAB, int ncdh, int etot_ket, int ncd, int L, int word) {
     const int NHP = (NH + 3) / 4 * 4, NL = (L + 1) * (L + 2) * (L + 3) / 6;
@@ -139,7 +139,8 @@ __host__ __device__ inline Layout layout(int NH, int NAB, int ncdh, int etot_ket
     w.shift = w.seg_st + 32 * 16;
     w.seg_lane = w.shift + 32 * 4;
     w.info = w.seg_lane + 36 * 4;
-    w.total = w.info + 16;
+    w.walk = w.info + 16;
+    w.total = w.walk + 32;
     return w;
 }
 
@@ -518,7 +519,8 @@ __device__ __forceinline__ void dense_block(const EriDev& d, const QuartetClass&
     const bool leader = warp == (int)(blockIdx.x % kWarps);
     unsigned count = 0;
     Stream<F32> stream(d, qc, t0, t1, MODE == kDenseF64 ? fmaxf(d.skip_cut, d.fp32_cut) : d.skip_cut,
-                       MODE == kDenseF64 ? 3.4e38f : d.fp32_cut, MODE == kDenseF64 ? qc.unit_count : qc.unit_count32);
+                       MODE == kDenseF64 ? 3.4e38f : d.fp32_cut, MODE == kDenseF64 ? qc.unit_count : qc.unit_count32,
+                       reinterpret_cast<Walk*>(base + lay.walk));
     WideEntries wide;
     unsigned skipped = 0;  // FP32: lanes that met an entry left to FP64
     __syncthreads();

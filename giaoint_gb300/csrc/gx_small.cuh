@@ -311,6 +311,7 @@ struct WarpBuffers {
     int4 seg_st[32];
     int seg_lane[36];  // first lane and flags of each segment, and the end
     int2 queue[64];    // task, bra pair << 16 | ket pair
+    Walk walk;
 };
 
 // Notes the segments; flags: those of the lane's task.  Returns their number.
@@ -413,7 +414,7 @@ __device__ __forceinline__ void small_block(const EriDev& d, const QuartetClass&
         for (int i = 0; i < NOUT; ++i) w.v[i * 33 + lane] = v[i];
     };
     {
-        Stream<false> stream(d, qc, t0, t1, fmaxf(d.skip_cut, d.fp32_cut), 3.4e38f, qc.unit_count);
+        Stream<false> stream(d, qc, t0, t1, fmaxf(d.skip_cut, d.fp32_cut), 3.4e38f, qc.unit_count, &w.walk);
         for (;;) {
             int task, rank = 0;
             int2 pq;
@@ -492,7 +493,7 @@ __device__ __forceinline__ void small_block(const EriDev& d, const QuartetClass&
     // lies in the asymptotic sector (FP32 Boys), pass 1 the others (FP64 Boys,
     // FP32 recurrence), so that every batch follows one Boys path.
     for (int pass = 0; pass < (d.fp32_cut > 0.0f ? 2 : 0); ++pass) {
-        Stream<true> stream(d, qc, t0, t1, d.skip_cut, d.fp32_cut, qc.unit_count32);
+        Stream<true> stream(d, qc, t0, t1, d.skip_cut, d.fp32_cut, qc.unit_count32, &w.walk);
         int waiting = 0;
         bool more = true;
         while (more || waiting > 0) {

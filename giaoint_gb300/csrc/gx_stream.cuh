@@ -30,6 +30,11 @@ __device__ __forceinline__ int survivors(const float* __restrict__ sp, int Kab, 
 struct Row {
     int P, qb, qa, before;
 };
+// The row of a stream's last entry, of the task it is in (-1: not kept).
+struct Walk {
+    Row row;
+    int task;
+};
 
 // The j-th of them in stream order (bra pair, then ket pair), from `row` on (of the
 // task's start, or of an earlier survivor), which is left at the survivor's.
@@ -151,15 +156,20 @@ struct Stream {
     const int* counts;
     int t1, next_task, chunk = 0, incl = 0, cnt = 0, kind = 0, total = 0, used = 0, batch_kind = 0;
     int run = 8;  // run length of the lane's task
-    // The last entry handed out: the next one of its task is sought from there
-    // (from the task's start every batch of a deep contraction walked over all its
-    // bra pairs: one (ss|ss) of 20 primitives a shell, 1.6e5 entries, 141 ms).
-    int row_task = -1;
-    Row row{};
+    // The last entry handed out, when its task goes on and the walk to it was a long
+    // one: the next entry is sought from there (from the task's start every batch of
+    // a deep contraction walked over all its bra pairs: one (ss|ss) of 20 primitives
+    // a shell, 1.6e5 entries, 141 instead of 37.6 ms).  In shared memory: held in
+    // registers it cost the (pp| template an occupancy step, 1% of twelve atoms.
+    Walk* walk;
 
     __device__ __forceinline__ Stream(const EriDev& dev, const QuartetClass& cls, int first, int last, float from,
-                                      float below, const int* task_counts)
-        : d(dev), qc(cls), lo(from), hi(below), counts(task_counts), t1(last), next_task(first) {}
+                                      float below, const int* task_counts, Walk* kept)
+        : d(dev), qc(cls), lo(from), hi(below), counts(task_counts), t1(last), next_task(first), walk(kept) {
+        __syncwarp();
+        walk->task = -1;  // (every lane of the stream's warp)
+        __syncwarp();
+    }
     // Returns the number of entries; every lane below it has its task, the
     // entry's rank within the task, and its bra and ket pair.
     __device__ __forceinline__ int next(int lane, int& task, int& rank, int2& pq) {
@@ -167,6 +177,7 @@ struct Stream {
         const int* np = d.basis.nprim;
         int got = 0;
         task = -1;
+        int left = 0;  // entries of the lane's task after its own
         while (got < 32) {
             if (used == total) {
                 if (next_task >= t1) break;
@@ -238,24 +249,32 @@ struct Stream {
                 task = chunk + src;
                 rank = e - before;
                 run = run_length(whole);
+                left = whole - 1 - rank;
             }
             used += take;
             got += take;
             if (full) break;
         }
         if (got == 0) return 0;
-        Row r = row;
+        Row r{};
         if (lane < got) {
             const Task* tg = qc.tasks + task;
-            if (task != row_task) {
+            if (task == walk->task) {
+                r = walk->row;
+            } else {
                 const int Kcd = np[tg->sc] * np[tg->sd];
                 r = Row{0, Kcd, hi < 3.0e38f ? Kcd : 0, 0};
             }
             pq = survivor(pp.sbound + tg->pab, np[tg->sa] * np[tg->sb], pp.sbound + tg->pcd, lo, hi, rank, r);
         }
-        row_task = __shfl_sync(0xffffffffu, task, got - 1);
-        row = Row{__shfl_sync(0xffffffffu, r.P, got - 1), __shfl_sync(0xffffffffu, r.qb, got - 1),
-                  __shfl_sync(0xffffffffu, r.qa, got - 1), __shfl_sync(0xffffffffu, r.before, got - 1)};
+        // (a kept row stays valid until the stream has left its task: entries are only
+        // sought further on)
+        const bool keep = lane == got - 1 && left > 0 && r.P >= 16;
+        if (__any_sync(0xffffffffu, keep)) {
+            __syncwarp();
+            if (keep) *walk = Walk{r, task};
+            __syncwarp();
+        }
         return got;
     }
 };
