@@ -1423,7 +1423,7 @@ std::vector<PlanLaunch> plan_launches(gx_context* ctx, const gx::EriDev& dev, co
             if (pair < 0)
                 GX_CUDA(gx::launch_small_list(dev, keys, classes, s));
             else
-                launch_dense_classes(ctx, pair, dev, classes, s, wide);
+                launch_dense_classes(ctx, pair, dev, classes, s, true);
         }});
     }
     for (size_t ci : own)
@@ -1436,8 +1436,10 @@ std::vector<PlanLaunch> plan_launches(gx_context* ctx, const gx::EriDev& dev, co
 }
 
 // What the FP32 launches of a mixed-precision plan left to FP64, for all its
-// lane-dense classes at once: a launch for every class cost a field of five atoms
-// 0.3 ms of 3.8.
+// lane-dense classes with launches of their own at once (a launch for every class
+// cost a field of five atoms 0.3 ms of 3.8).  The shared launches are followed by
+// theirs, which then run beside the rest of the plan: a unit of (dd|dd) takes 0.2
+// ms, most of it latency.
 void launch_wide_classes(gx_context* ctx, const gx::EriDev& dev, const PlanData& plan, int precision,
                          unsigned long long* counters, cudaStream_t s) {
     if (!(dev.fp32_cut > 0.0f)) return;
@@ -1446,6 +1448,7 @@ void launch_wide_classes(gx_context* ctx, const gx::EriDev& dev, const PlanData&
     for (size_t ci = 0; ci < plan.classes.size(); ++ci) {
         const auto& k = plan.classes[ci].key;
         if (k[0] + k[1] + k[2] + k[3] < gx::kWideOrder ||
+            plan.classes[ci].primitive_quartets <= kSharedLaunch ||
             !runs_dense(plan, plan.classes[ci], tuned.valid ? tuned.conf[ci] : plan.defconf[ci], dev.all_real))
             continue;
         gx::QuartetClass qc = unit_class(ctx, plan, ci, counters);

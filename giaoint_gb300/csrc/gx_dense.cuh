@@ -696,7 +696,8 @@ __device__ __forceinline__ void dense_block(const EriDev& d, const QuartetClass&
     }
     if constexpr (F32) {
         if (leader && __any_sync(0xffffffffu, skipped) && lane == 0) {
-            *qc.wide = 1;
+            const int old = atomicCAS(qc.wide, 0, unit + 1);
+            if (old != 0 && old != unit + 1) *qc.wide = -1;
             if (start) const_cast<int*>(start)[unit] = t0 | (int)0x80000000;
         }
     }

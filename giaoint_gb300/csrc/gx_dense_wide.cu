@@ -1,6 +1,7 @@
-// Lane-dense kernel (gx_dense.cuh): the entries that FP32 leaves to FP64, of all
-// classes of a plan in one launch.  There are few of them, so a small grid looks
-// through the units (a thread each) for those in which the FP32 launch met one.
+// Lane-dense kernel (gx_dense.cuh): the entries that FP32 leaves to FP64, of many
+// classes in one launch.  There are few of them (twelve atoms: none of 11.5 M FP32
+// entries), so a small grid looks through the units, a thread each, for those in
+// which the FP32 launch met one.
 #include <algorithm>
 
 #include "gx_dense.cuh"
@@ -21,17 +22,23 @@ __global__ void __launch_bounds__(32 * dense::kWarps) wide_kernel(const __grid_c
     constexpr int THREADS = 32 * dense::kWarps;
     __shared__ int4 queue[64];
     __shared__ long long hits[THREADS];
-    __shared__ int nhit;
+    __shared__ int nhit, wide[kMaxWide];
+    if (threadIdx.x < (unsigned)list.n) wide[threadIdx.x] = *list.cls[threadIdx.x].wide;
+    __syncthreads();
     for (int c = 0; c < list.n; ++c) {
+        const int w = wide[c];
+        if (w == 0) continue;
         const QuartetClass& qc = list.cls[c];
-        if (*qc.wide == 0) continue;
-        const long long items = (long long)qc.ngroup * qc.nchunk;
+        // items: (unit, share of its components), of all units or of the only one
+        const long long first = w > 0 ? (long long)(w - 1) * qc.nchunk : 0;
+        const long long items = w > 0 ? qc.nchunk : (long long)qc.ngroup * qc.nchunk;
         for (long long i0 = blockIdx.x; i0 < items; i0 += (long long)THREADS * gridDim.x) {
             if (threadIdx.x == 0) nhit = 0;
             __syncthreads();
             const long long i = i0 + (long long)threadIdx.x * gridDim.x;
             // (any order: they write disjoint elements)
-            if (i < items && (!qc.unit_start32 || qc.unit_start32[i / qc.nchunk] < 0)) hits[atomicAdd(&nhit, 1)] = i;
+            if (i < items && (w > 0 || !qc.unit_start32 || qc.unit_start32[i / qc.nchunk] < 0))
+                hits[atomicAdd(&nhit, 1)] = first + i;
             __syncthreads();
             const int n = nhit;
             for (int k = 0; k < n; ++k) {

@@ -145,7 +145,7 @@ struct QuartetClass {
     unsigned long long* counters;  // [0] FP64, [1] FP32 primitive quartets evaluated (may be null)
     const int* unit_start32;  // lane-dense kernel: the same for the FP32 entries (bit 31 of a start: the unit
     const int* unit_count32;  //    has entries that FP32 left to FP64)
-    int* wide;                // 1: the class has such entries (null: it can have none)
+    int* wide;                // units with such entries: 0 none, u + 1 unit u alone, -1 several (null: can have none)
 };
 
 // Work units of a plan's small and lane-dense classes with many tasks
