@@ -850,10 +850,12 @@ void* unit_arrays(gx::UnitPlan& u, DeviceBuffer& mem, size_t tail, cudaStream_t 
 // whole task and should not spill into a batch of its own.  A plan that has
 // fewer than three units per SM at that size (the column evaluations of a
 // Cholesky factorisation, one or two atoms) is bound by the time of one unit,
-// and a short batch repeats its entries over the lanes: down to 8 entries.  Two
-// atoms' factorisation 19.8 -> 18.8 ms (16 entries: 19.7, 4: 18.7), their s/p
-// shells in a field 73 -> 48 us; at four units per SM the 98 classes of an s-f
-// atom took 309 us instead of 290.  In the small classes (L <= 2) a unit is one
+// and a short batch repeats its entries over the lanes: down to 8 entries (two
+// atoms' s/p shells in a field 73 -> 57 us; at four units per SM the 98 classes of an s-f
+// atom took 309 us instead of 290).  A column evaluation that is replayed goes by
+// the column plan's own size: with all of them cut to 8 entries the columns of
+// twelve atoms' factorisation took 167 ms instead of 140, of six 46 instead of 42.
+// In the small classes (L <= 2) a unit is one
 // warp's work, not a block's, so they go on halving until there are 64 units
 // per SM: at eight a warp walked up to 256 entries alone while the rest of a
 // five-atom molecule had finished.  Classes with few tasks have no entry in the
@@ -4212,6 +4214,8 @@ void cholesky_core(gx_context* ctx, gx_basis* b, const double* Bf, const double*
                         sp.order = pd.order;
                         sp.stable = pd.stable;
                         sp.ntask = pd.ntask;
+                        sp.primitive_quartets = pd.primitive_quartets;  // (sets the units and shared launches)
+                        sp.model_flops = pd.model_flops;
                         sp.spread_parts = pd.spread_parts;
                         sp.base.range = pd.base.range;
                         sp.tasks.reserve(pd.tasks.bytes);
