@@ -335,36 +335,68 @@ __device__ __forceinline__ int segments(WarpBuffers<NOUT>& w, const QuartetClass
 
 // Adds the buffered values of every shell quartet's lanes to its block in
 // stream order: the result does not depend on how the stream was cut into
-// batches.  kReal: the imaginary parts are zero.
+// batches.  kReal: the imaginary parts are zero.  A lane takes the real or the
+// imaginary part of an element, or a quarter of a long run: a batch of a deep
+// contraction has few elements, and its sums, one lane after 32 entries, were two
+// of the 13 us of a batch of (ss|ss).
 enum AddMode { kReal, kComplex, kFP32 };
 template <int LA, int LB, int LC, int LD, AddMode MODE>
 __device__ __forceinline__ void add_runs(double2* out, const WarpBuffers<nc(LA) * nc(LB) * nc(LC) * nc(LD)>& w, int nseg,
                                          int lane) {
     constexpr int NCD = nc(LC) * nc(LD), NOUT = nc(LA) * nc(LB) * NCD, NCB = nc(LB), NCDD = nc(LD);
-    for (int it = lane; it < nseg * NOUT; it += 32) {
-        const int s = it / NOUT, o = it - s * NOUT;
+    constexpr int PARTS = MODE == kReal ? 1 : 2;
+    auto element = [&](int s, int o, int part) {
         const int ab = o / NCD, cd = o - ab * NCD;
         const int4 st = w.seg_st[s];
-        double2* p = out + w.seg_off[s] + (long long)(ab / NCB) * st.x + (long long)(ab % NCB) * st.y +
-                     (long long)(cd / NCDD) * st.z + (long long)(cd % NCDD) * st.w;
-        const double2* v = w.v + o * 33;
-        const int flags = w.seg_lane[s], l0 = flags & 255, l1 = w.seg_lane[s + 1] & 255;
-        const bool store = flags & kStore;
-        if constexpr (MODE == kReal) {
-            const double old = store ? 0.0 : p->x;
-            const double sum = add_by_runs(old, flags, l0, l1, [&](int k) { return v[k].x; });
-            if (store)
-                *p = c2(sum, 0.0);
-            else
-                p->x = sum;
-        } else if constexpr (MODE == kComplex) {
-            const double2 old = store ? c2(0.0, 0.0) : *p;
-            *p = add_by_runs(old, flags, l0, l1, [&](int k) { return v[k]; });
-        } else {
-            // (FP32 values: their passes cut the stream where the Boys paths part)
-            double2 sum = *p;
-            for (int l = l0; l < l1; ++l) sum = cadd(sum, v[l]);
+        return reinterpret_cast<double*>(out + w.seg_off[s] + (long long)(ab / NCB) * st.x + (long long)(ab % NCB) * st.y +
+                                         (long long)(cd / NCDD) * st.z + (long long)(cd % NCDD) * st.w) +
+               part;
+    };
+    auto put = [&](double* p, bool store, double sum) {
+        if (MODE == kReal && store)
+            *reinterpret_cast<double2*>(p) = c2(sum, 0.0);
+        else
             *p = sum;
+    };
+    int first = 0;
+    if (MODE != kFP32 && nseg > 0 && (w.seg_lane[0] & kLongRuns)) {
+        first = 1;
+        const bool store = w.seg_lane[0] & kStore;
+        const int l1 = w.seg_lane[1] & 255, quarter = lane & 3, l0 = 8 * quarter;
+        for (int i0 = 0; i0 < NOUT * PARTS; i0 += 8) {
+            const int i = i0 + lane / 4, o = i / PARTS, part = i - o * PARTS;
+            const bool valid = i < NOUT * PARTS;
+            const double* v = reinterpret_cast<const double*>(w.v + (valid ? o : 0) * 33) + (valid ? part : 0);
+            double sum = 0.0;
+            if (valid && l0 < l1) {
+                sum = v[2 * l0];
+                for (int k = l0 + 1; k < l0 + 8 && k < l1; ++k) sum += v[2 * k];
+            }
+#pragma unroll
+            for (int j = 1; j < 4; ++j) {
+                const double other = __shfl_down_sync(0xffffffffu, sum, j);
+                if (quarter == 0 && 8 * j < l1) sum += other;
+            }
+            if (valid && quarter == 0) {
+                double* p = element(0, o, part);
+                put(p, store, store ? sum : *p + sum);
+            }
+        }
+    }
+    for (int it = lane; it < (nseg - first) * NOUT * PARTS; it += 32) {
+        const int s = it / (NOUT * PARTS), i = it - s * (NOUT * PARTS), o = i / PARTS, part = i - o * PARTS;
+        double* p = element(first + s, o, part);
+        const double* v = reinterpret_cast<const double*>(w.v + o * 33) + part;
+        const int flags = w.seg_lane[first + s], l0 = flags & 255, l1 = w.seg_lane[first + s + 1] & 255;
+        if constexpr (MODE == kFP32) {
+            // (FP32 values: their passes cut the stream where the Boys paths part)
+            double sum = *p;
+            for (int l = l0; l < l1; ++l) sum += v[2 * l];
+            *p = sum;
+        } else {
+            const bool store = flags & kStore;
+            const double old = store ? 0.0 : *p;
+            put(p, store, add_by_runs(old, flags, l0, l1, [&](int k) { return v[2 * k]; }));
         }
     }
 }

@@ -137,7 +137,8 @@ __device__ __forceinline__ void cut_units(const EriDev& d, const QuartetClass& q
 // after the other, so that the rounding of a deep contraction grows with the
 // number of runs; batches never split a run, so the sums do not depend on how
 // the stream is cut into batches.  Runs of 8 cost a batch two lanes on average;
-// a task of 256 entries or more has room for runs of 32.
+// a task of 256 entries or more has room for runs of 32, which start at lane 0 and
+// are four sums of 8.
 __device__ __forceinline__ int run_length(int survivors) { return survivors >= 256 ? 32 : 8; }
 
 // The surviving primitive quartets of the tasks t0 .. t1 - 1 in stream order
@@ -291,10 +292,14 @@ __device__ __forceinline__ T add_by_runs(T sum, int flags, int l0, int l1, Get&&
     const int run = flags & kSingle ? 1 : (flags & kLongRuns ? 32 : 8);
     bool fresh = flags & kStore;
     for (int l = l0; l < l1; l += run) {
-        T part = v(l);
         const int end = l + run < l1 ? l + run : l1;
-        for (int k = l + 1; k < end; ++k) part = plus(part, v(k));
-        sum = fresh ? part : plus(sum, part);
+        T whole{};
+        for (int l8 = l; l8 < end; l8 += 8) {
+            T part = v(l8);
+            for (int k = l8 + 1; k < l8 + 8 && k < end; ++k) part = plus(part, v(k));
+            whole = l8 == l ? part : plus(whole, part);
+        }
+        sum = fresh ? whole : plus(sum, whole);
         fresh = false;
     }
     return sum;
