@@ -1227,9 +1227,11 @@ gx::QuartetClass unit_class(gx_context* ctx, const PlanData& plan, size_t ci, un
     if (qc.L >= gx::kWideOrder) qc.wide = plan.units.wide + ci;
     qc.bra = ctx->pair_class(k[0], k[1]).dev();
     qc.ket = ctx->pair_class(k[2], k[3]).dev();
-    // few entries: the blocks of a unit share its components (about one in
-    // four primitive quartets of a small plan survives)
-    const int units = (int)(pc.primitive_quartets / 128) + 1, fill = std::max(ctx->sm_count, 1);
+    // few units: the blocks of a unit share its components (about one in four
+    // primitive quartets of a small plan survives, and a unit is at least a task:
+    // 21 (dd|dd) of six primitives a shell in a field took 41 ms with a block each,
+    // 12 with their components shared)
+    const int units = (int)std::min<int64_t>(pc.primitive_quartets / 128 + 1, (int64_t)pc.count), fill = std::max(ctx->sm_count, 1);
     qc.nchunk = gx::dense_chunks(k[0], k[1], k[2], k[3], (fill + units - 1) / units, pc.primitive_quartets <= 32);
     return qc;
 }
