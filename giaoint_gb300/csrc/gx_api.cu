@@ -687,6 +687,7 @@ struct PlanData {
     std::vector<int> task_kk;       // per task (class order): Kab << 16 | Kcd, for regrouping
     std::vector<uint8_t> task_site; // per task: 2 when the bra shells share a centre, + 1 when the ket shells do
     std::vector<int> task_part;     // per task: its part (request) of a packed plan; empty for one part
+    bool one_site = false;          // every part's shells are on one centre
     bool stable = false;            // launch configuration independent of the plan's size (see launch_class)
     std::vector<ClassConf> defconf; // per class: the configuration used before any tuning
     std::vector<int> order;         // launch order: largest model work first, so the longest
@@ -855,6 +856,11 @@ void* unit_arrays(gx::UnitPlan& u, DeviceBuffer& mem, size_t tail, cudaStream_t 
 // atom took 309 us instead of 290).  A column evaluation that is replayed goes by
 // the column plan's own size: with all of them cut to 8 entries the columns of
 // twelve atoms' factorisation took 167 ms instead of 140, of six 46 instead of 42.
+// A plan of fewer than three primitive quartets per SM goes on down to one entry,
+// because the kinds of pairs in a unit (see Stream) are batches one after the other:
+// 27 uncontracted (dd|dd) in a field took 0.47 ms in two units, 0.13 in one each.
+// On one centre there is one kind, and more units are more tables (a 140-function
+// atom's columns took 42 ms instead of 29).
 // In the small classes (L <= 2) a unit is one
 // warp's work, not a block's, so they go on halving until there are 64 units
 // per SM: at eight a warp walked up to 256 entries alone while the rest of a
@@ -882,6 +888,9 @@ void make_units(gx_context* ctx, PlanData& plan) {
             int entries = 256;
             while (entries > 32 && all / entries < full) entries /= 2;
             while (entries > 8 && entries <= 32 && plan_all / entries < 3 * (int64_t)std::max(ctx->sm_count, 1))
+                entries /= 2;
+            while (entries > 1 && entries <= 8 && !plan.one_site && plan_all < 3 * (int64_t)std::max(ctx->sm_count, 1) &&
+                   plan_all / entries < std::max(ctx->sm_count, 1))
                 entries /= 2;
             const int64_t mean = pc.primitive_quartets / std::max<int64_t>((int64_t)pc.count, 1);
             const int64_t target = 64 * (entries - std::min<int64_t>(entries / 16, mean / 4));
@@ -979,6 +988,7 @@ void build_plan_parts(gx_context* ctx, const std::vector<PlanPart>& parts, PlanD
         codes.push_back(kv.first);
     }
     const int nsc = (int)codes.size();
+    plan.one_site = std::all_of(parts.begin(), parts.end(), [](const PlanPart& p) { return p.b->one_site; });
     std::vector<std::vector<int>> part_code(parts.size()), part_site(parts.size());
     for (size_t pi = 0; pi < parts.size(); ++pi) {
         const gx_basis* b = parts[pi].b;
@@ -4215,6 +4225,7 @@ void cholesky_core(gx_context* ctx, gx_basis* b, const double* Bf, const double*
                         sp.defconf = pd.defconf;
                         sp.order = pd.order;
                         sp.stable = pd.stable;
+                        sp.one_site = pd.one_site;
                         sp.ntask = pd.ntask;
                         sp.primitive_quartets = pd.primitive_quartets;  // (sets the units and shared launches)
                         sp.model_flops = pd.model_flops;

@@ -276,13 +276,15 @@ __device__ __forceinline__ void reduce_out(const Out& o, const RT* vb, int ab0, 
     }
 }
 
-// Second transform and sums of a component group, slice by slice.
+// Second transform and sums of a component group, slice by slice (only: the
+// slices of one warp, when the block's warps share the group; -1: all).
 template <int LA, int LB, typename RT, typename EP, int... S>
 __device__ __forceinline__ void slices(const Out& o, const RT* W, RT* vb, const EP* Eb, bool bra_real, int c,
-                                       std::integer_sequence<int, S...>) {
+                                       int only, std::integer_sequence<int, S...>) {
     constexpr int SL = slice_of(nc(LA) * nc(LB));
     (
         [&] {
+            if (sizeof...(S) > 1 && !std::is_same_v<RT, float2> && only >= 0 && S % kWarps != only) return;
             if constexpr (std::is_same_v<RT, double>) {
                 bra<LA, LB, S * SL, double, RT>(vb + o.lane, W, Eb, std::make_integer_sequence<int, SL>{});
             } else if constexpr (std::is_same_v<RT, double2>) {
@@ -303,7 +305,10 @@ __device__ __forceinline__ void slices(const Out& o, const RT* W, RT* vb, const 
 }
 
 // The component groups of one batch: sets of o.parts consecutive groups, dealt
-// out to the block's warps; each lane set takes one group of a set.
+// out to the block's warps; each lane set takes one group of a set.  When one
+// set holds all of them, the warps share the slices of the second transform
+// instead (each forms W): of the latency of a short batch, which is all that a
+// plan of a few quartets waits for, that is a third with d shells.
 template <int LA, int LB, typename RT, typename EP>
 __device__ __forceinline__ void transforms(const Out& o, const RT* R, RT* vb, const int* hsum, const int* kh,
                                            const int2* kb, const EP* Ek, const EP* Eb, bool ket_real, bool bra_real,
@@ -311,7 +316,11 @@ __device__ __forceinline__ void transforms(const Out& o, const RT* R, RT* vb, co
     constexpr int NH = hc(LA + LB), NAB = nc(LA) * nc(LB), CG = group_of(NAB);
     const RT* col = R + (o.lane & (o.width - 1));
     const int set = o.lane / o.width;
-    for (int c1 = o.cbegin + warp * o.parts * CG; c1 < o.cend; c1 += kWarps * o.parts * CG) {
+    constexpr int NS = NAB / slice_of(NAB);
+    // (FP32 transforms are short beside the rest of a batch)
+    constexpr bool SHARED = NS > 1 && !std::is_same_v<RT, float2>;
+    const bool share = SHARED && o.cend - o.cbegin <= o.parts * CG;
+    for (int c1 = o.cbegin + (share ? 0 : warp * o.parts * CG); c1 < o.cend; c1 += kWarps * o.parts * CG) {
         const int cg = min(CG, o.cend - c1);
         for (int u = 0; u < cg; ++u) {
             // (a set beyond the last component repeats it; it is not added)
@@ -327,8 +336,8 @@ __device__ __forceinline__ void transforms(const Out& o, const RT* R, RT* vb, co
             } else {
                 ket<NH, float2, RT>(W, col, Ek + box.x, kh + box.x, box.y, hsum);
             }
-            slices<LA, LB, RT>(o, W, vb + u * NAB * 33, Eb, bra_real, c1,
-                               std::make_integer_sequence<int, NAB / slice_of(NAB)>{});
+            slices<LA, LB, RT>(o, W, vb + u * NAB * 33, Eb, bra_real, c1, SHARED && share ? warp : -1,
+                               std::make_integer_sequence<int, NS>{});
         }
         if constexpr (CG > 1) {
             __syncwarp();
