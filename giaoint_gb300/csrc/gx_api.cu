@@ -1153,8 +1153,8 @@ void build_plan_parts(gx_context* ctx, const std::vector<PlanPart>& parts, PlanD
     }
     plan.ntask = T;
     plan.stable = ctx->stable_launch;
-    // (and a flag per class behind them, see UnitPlan)
-    plan.tasks.reserve(sizeof(gx::Task) * std::max<int64_t>(T, 1) + sizeof(int) * bkeys.size());
+    // (and the classes' `wide` words behind them, see UnitPlan)
+    plan.tasks.reserve(sizeof(gx::Task) * std::max<int64_t>(T, 1) + sizeof(int) * gx::kWideWords * bkeys.size());
     if (T) GX_CUDA(cudaMemcpyAsync(plan.tasks.ptr, all.get(), sizeof(gx::Task) * T, cudaMemcpyHostToDevice, ctx->stream));
     plan.defconf.resize(plan.classes.size());
     for (size_t ci = 0; ci < plan.classes.size(); ++ci) plan.defconf[ci] = default_conf(plan.classes[ci].key);
@@ -1234,7 +1234,7 @@ gx::QuartetClass unit_class(gx_context* ctx, const PlanData& plan, size_t ci, un
     }
     qc.nchunk = 1;
     if (gx::small_class(k[0], k[1], k[2], k[3])) return qc;
-    if (qc.L >= gx::kWideOrder) qc.wide = plan.units.wide + ci;
+    if (qc.L >= gx::kWideOrder) qc.wide = plan.units.wide + ci * gx::kWideWords;
     qc.bra = ctx->pair_class(k[0], k[1]).dev();
     qc.ket = ctx->pair_class(k[2], k[3]).dev();
     // few units: the blocks of a unit share its components (about one in four
@@ -4715,7 +4715,7 @@ void plan_enqueue(gx_eri_plan* plan, const double* B, const double* O, int preci
         GX_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
         try {
             pd.units.wide = static_cast<int*>(
-                unit_arrays(pd.units, *mem, std::max<size_t>(pd.classes.size(), 1) * sizeof(int), ctx->stream));
+                unit_arrays(pd.units, *mem, pd.classes.size() * gx::kWideWords * sizeof(int) + 1, ctx->stream));
         } catch (...) {
             cudaThreadExchangeStreamCaptureMode(&mode);
             pd.units = own;

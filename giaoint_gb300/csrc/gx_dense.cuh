@@ -450,7 +450,8 @@ struct ClassList {
 };
 
 // Unit `unit` of a class; share_of: which of the nchunk blocks that share it;
-// queue: 64 entries of shared memory (kDenseWide).
+// queue: 64 entries of shared memory (kDenseWide, where `unit` is a task in
+// classes without unit arrays).
 template <int LA, int LB, DenseMode MODE>
 __device__ __forceinline__ void dense_block(const EriDev& d, const QuartetClass& qc, int unit, int share_of,
                                             int4* queue = nullptr) {
@@ -478,13 +479,16 @@ __device__ __forceinline__ void dense_block(const EriDev& d, const QuartetClass&
     int* seg_lane = reinterpret_cast<int*>(base + lay.seg_lane);
     int* info = reinterpret_cast<int*>(base + lay.info);  // entries, segments, real sides
     // (set by the FP32 launch, which follows the FP64 one)
-    if (MODE == kDenseF64 && qc.wide && unit == 0 && share_of == 0 && threadIdx.x == 0) *qc.wide = 0;
+    if (MODE == kDenseF64 && qc.wide && unit == 0 && share_of == 0 && threadIdx.x < kWideWords) qc.wide[threadIdx.x] = 0;
     // the unit's tasks (entries past the last unit lie beyond the class)
     const int* start = MODE == kDenseF64 ? qc.unit_start : qc.unit_start32;
     int t0, t1;
     if (start) {
         t0 = start[unit] & 0x7fffffff;
         t1 = min(start[unit + 1] & 0x7fffffff, qc.ntask);
+    } else if (WIDE) {
+        t0 = unit;
+        t1 = unit + 1;
     } else {
         __shared__ int bounds[2];
         __shared__ long long sums[kWarps];
@@ -531,7 +535,7 @@ __device__ __forceinline__ void dense_block(const EriDev& d, const QuartetClass&
                        MODE == kDenseF64 ? 3.4e38f : d.fp32_cut, MODE == kDenseF64 ? qc.unit_count : qc.unit_count32,
                        reinterpret_cast<Walk*>(base + lay.walk));
     WideEntries wide;
-    unsigned skipped = 0;  // FP32: lanes that met an entry left to FP64
+    bool skipped = false;  // FP32: the lane met an entry left to FP64
     __syncthreads();
     for (;;) {
         if (leader) {
@@ -571,7 +575,10 @@ __device__ __forceinline__ void dense_block(const EriDev& d, const QuartetClass&
                 bool mine = active;
                 if constexpr (F32) {
                     if (L >= kWideOrder && seeds_exceed_fp32(pp, ip, iq, L)) mine = false;
-                    skipped |= active && !mine;
+                    if (active && !mine) {
+                        skipped = true;
+                        if (!start && share_of == 0) atomicOr(&qc.wide[1 + task / 32], 1 << (task & 31));
+                    }
                 }
                 const double p = pp.p[ip], q = pp.p[iq];
                 const double rs = rsqrt(p + q);
@@ -705,8 +712,7 @@ __device__ __forceinline__ void dense_block(const EriDev& d, const QuartetClass&
     }
     if constexpr (F32) {
         if (leader && __any_sync(0xffffffffu, skipped) && lane == 0) {
-            const int old = atomicCAS(qc.wide, 0, unit + 1);
-            if (old != 0 && old != unit + 1) *qc.wide = -1;
+            *qc.wide = 1;
             if (start) const_cast<int*>(start)[unit] = t0 | (int)0x80000000;
         }
     }

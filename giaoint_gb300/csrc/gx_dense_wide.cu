@@ -1,7 +1,7 @@
 // Lane-dense kernel (gx_dense.cuh): the entries that FP32 leaves to FP64, of many
 // classes in one launch.  There are few of them (twelve atoms: none of 11.5 M FP32
-// entries), so a small grid looks through the units, a thread each, for those in
-// which the FP32 launch met one.
+// entries), so a small grid looks through the units (the tasks of classes without
+// unit arrays), a thread each, for those in which the FP32 launch met one.
 #include <algorithm>
 
 #include "gx_dense.cuh"
@@ -26,19 +26,18 @@ __global__ void __launch_bounds__(32 * dense::kWarps) wide_kernel(const __grid_c
     if (threadIdx.x < (unsigned)list.n) wide[threadIdx.x] = *list.cls[threadIdx.x].wide;
     __syncthreads();
     for (int c = 0; c < list.n; ++c) {
-        const int w = wide[c];
-        if (w == 0) continue;
+        if (wide[c] == 0) continue;
         const QuartetClass& qc = list.cls[c];
-        // items: (unit, share of its components), of all units or of the only one
-        const long long first = w > 0 ? (long long)(w - 1) * qc.nchunk : 0;
-        const long long items = w > 0 ? qc.nchunk : (long long)qc.ngroup * qc.nchunk;
+        // items: (unit or task, share of its components)
+        const long long items = (long long)(qc.unit_start32 ? qc.ngroup : qc.ntask) * qc.nchunk;
         for (long long i0 = blockIdx.x; i0 < items; i0 += (long long)THREADS * gridDim.x) {
             if (threadIdx.x == 0) nhit = 0;
             __syncthreads();
             const long long i = i0 + (long long)threadIdx.x * gridDim.x;
             // (any order: they write disjoint elements)
-            if (i < items && (w > 0 || !qc.unit_start32 || qc.unit_start32[i / qc.nchunk] < 0))
-                hits[atomicAdd(&nhit, 1)] = first + i;
+            const int u = (int)(i / qc.nchunk);
+            if (i < items && (qc.unit_start32 ? qc.unit_start32[u] < 0 : qc.wide[1 + u / 32] >> (u & 31) & 1))
+                hits[atomicAdd(&nhit, 1)] = i;
             __syncthreads();
             const int n = nhit;
             for (int k = 0; k < n; ++k) {
@@ -75,7 +74,7 @@ cudaError_t launch_wide(const EriDev& d, const std::vector<std::pair<int, Quarte
             // and the launch is the end of its plan)
             const int nchunk = dense_chunks(qc.bra.la, qc.bra.lb, qc.ket.la, qc.ket.lb, 8, true);
             list.cls[list.n++].nchunk = nchunk;
-            units += (long long)qc.ngroup * nchunk;
+            units += (long long)(qc.unit_start32 ? qc.ngroup : qc.ntask) * nchunk;
             smem = std::max(smem, dense_smem(pair, qc, d.all_real ? 8 : 16));
         }
         if (list.n == 0) continue;

@@ -145,7 +145,8 @@ struct QuartetClass {
     unsigned long long* counters;  // [0] FP64, [1] FP32 primitive quartets evaluated (may be null)
     const int* unit_start32;  // lane-dense kernel: the same for the FP32 entries (bit 31 of a start: the unit
     const int* unit_count32;  //    has entries that FP32 left to FP64)
-    int* wide;                // units with such entries: 0 none, u + 1 unit u alone, -1 several (null: can have none)
+    int* wide;                // [kWideWords] whether the class has such entries, and without unit arrays a bit for
+                              //    each task that has (null: it can have none)
 };
 
 // Work units of a plan's small and lane-dense classes with many tasks
@@ -168,7 +169,7 @@ struct UnitPlan {
     long long* tile;            // [tiles] weight prefix of the tiles
     int* start;                 // [nunit]
     unsigned* done;             // blocks finished (0 between executions)
-    int* wide;                  // [classes of the plan] see QuartetClass
+    int* wide;                  // [classes of the plan * kWideWords] see QuartetClass
 };
 
 struct EriDev {
@@ -307,6 +308,7 @@ int dense_chunks(int la, int lb, int lc, int ld, int want, bool single);
 // FP64 (classes of order kWideOrder and up).
 enum DenseMode { kDenseF64, kDenseF32, kDenseWide };
 constexpr int kWideOrder = 5;
+constexpr int kWideWords = 1 + kUnitMinTasks / 32;
 long long unit_tiles(long long ntask);
 cudaError_t launch_units(const UnitPlan& u, const Task* tasks, const EriDev& d, cudaStream_t s);
 // A dense class oriented for its template pair (LA, LB): returns LA * 4 + LB.
