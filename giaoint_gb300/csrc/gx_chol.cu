@@ -158,16 +158,12 @@ __device__ RedKey block_reduce(RedKey r) {
     return r;
 }
 
-// Blocks of the reductions over N entries, at most as many as one block merges,
-// and their threads: an entry each, in blocks of 128 (of 1,000 entries every
-// warp then has a sub-partition to itself) until those run out at 32,768.
-// Beyond, 256: at 50,625 entries the 1,583 updates of a factorisation took
-// 479.3 ms, with 128 threads and a second pass in some blocks 480.3.
-constexpr int RED_BLOCKS = 256;
-int red_threads(long long N) { return N <= 128 * RED_BLOCKS ? 128 : 256; }
+// Blocks of the reductions over N entries, at most as many as one block merges:
+// an entry a thread, in blocks of 128 (of 1,000 entries every warp then has a
+// sub-partition to itself).
+constexpr int RED_BLOCKS = 256, RED_THREADS = 128;
 int red_blocks(long long N) {
-    const int threads = red_threads(N);
-    return (int)std::max<long long>(1, std::min<long long>((N + threads - 1) / threads, RED_BLOCKS));
+    return (int)std::max<long long>(1, std::min<long long>((N + RED_THREADS - 1) / RED_THREADS, RED_BLOCKS));
 }
 
 __global__ void chol_scan_kernel(const double* res, long long N, RedKey* partial) {
@@ -188,7 +184,7 @@ __global__ void chol_final_kernel(const RedKey* partial, int np, Red* out) {
 }
 
 cudaError_t launch_chol_scan(const double* res, long long N, void* partial, void* out, cudaStream_t s) {
-    chol_scan_kernel<<<red_blocks(N), red_threads(N), 0, s>>>(res, N, static_cast<RedKey*>(partial));
+    chol_scan_kernel<<<red_blocks(N), RED_THREADS, 0, s>>>(res, N, static_cast<RedKey*>(partial));
     chol_final_kernel<<<1, 256, 0, s>>>(static_cast<const RedKey*>(partial), red_blocks(N), static_cast<Red*>(out));
     return cudaGetLastError();
 }
@@ -244,10 +240,12 @@ __device__ __forceinline__ double2 conj_mul_sub(double2 acc, double2 a, double2 
 // What a thread of the factor update sums: a column entry, or with HALVES the
 // real or imaginary part of one.  The rows of a few thousand entries come from
 // the L2 cache, and an entry's four dependent-pair FMAs per complex row, 31 ns
-// each for a warp alone on its sub-partition, are the time of the update: two
-// threads halve it (1,000 entries at rank 400, eight chunks: @@ us for one,
-// @@ for two) with the same operations in the same order.  Long columns, bound
-// by memory, keep whole entries.
+// each for a warp alone on its sub-partition, are most of the time of the update:
+// two threads share them, with the same operations in the same order (the 223
+// updates of two atoms in a field, 900 entries, 5.66 -> 5.36 ms, the 348 of
+// three, 2,025 entries, 8.87 -> 8.45 ms, each twice within 0.02; one atom, 225
+// entries, and six, 8,100, are the same either way).  Long columns, bound by
+// memory, keep whole entries.
 template <typename T, bool HALVES>
 struct Entry {
     using Acc = std::conditional_t<HALVES, double, T>;
@@ -423,11 +421,11 @@ cudaError_t launch_chol_step(bool real, const void* L, long long ld, int rank, l
     }
     chol_scale_kernel<<<1, 1, 0, s>>>(res, piv, scale);
     if (real)
-        chol_update_kernel<double><<<red_blocks(N), red_threads(N), 0, s>>>(static_cast<const double*>(work), n, piv,
+        chol_update_kernel<double><<<red_blocks(N), RED_THREADS, 0, s>>>(static_cast<const double*>(work), n, piv,
                                                                          scale, static_cast<double*>(Lrow), res,
                                                                          static_cast<RedKey*>(partial));
     else
-        chol_update_kernel<double2><<<red_blocks(N), red_threads(N), 0, s>>>(static_cast<const double2*>(work), n, piv,
+        chol_update_kernel<double2><<<red_blocks(N), RED_THREADS, 0, s>>>(static_cast<const double2*>(work), n, piv,
                                                                           scale, static_cast<double2*>(Lrow), res,
                                                                           static_cast<RedKey*>(partial));
     chol_final_kernel<<<1, 256, 0, s>>>(static_cast<const RedKey*>(partial), red_blocks(N), static_cast<Red*>(out));
@@ -582,7 +580,7 @@ cudaError_t launch_chol_chain(bool real, void* L, long long N, int n, int rank_h
         if (real) {
             chain_gemv_split_kernel<double, false><<<grid, 128, 0, s>>>(static_cast<const double*>(L), N, st, nchunks,
                                                                         static_cast<double*>(gemv_partials), N);
-            chain_update_kernel<double><<<red_blocks(N), red_threads(N), 0, s>>>(
+            chain_update_kernel<double><<<red_blocks(N), RED_THREADS, 0, s>>>(
                 st, static_cast<const double*>(pool), static_cast<const double*>(gemv_partials), nchunks, n,
                 static_cast<double*>(L), res, static_cast<RedKey*>(partial), red, slot_of, log, tol, psd, select_next);
         } else {
@@ -590,7 +588,7 @@ cudaError_t launch_chol_chain(bool real, void* L, long long N, int n, int rank_h
             auto* gemv = halves ? chain_gemv_split_kernel<double2, true> : chain_gemv_split_kernel<double2, false>;
             gemv<<<halves ? dim3(2 * blocks, nchunks) : grid, 128, 0, s>>>(
                 static_cast<const double2*>(L), N, st, nchunks, static_cast<double2*>(gemv_partials), N);
-            chain_update_kernel<double2><<<red_blocks(N), red_threads(N), 0, s>>>(
+            chain_update_kernel<double2><<<red_blocks(N), RED_THREADS, 0, s>>>(
                 st, static_cast<const double2*>(pool), static_cast<const double2*>(gemv_partials), nchunks, n,
                 static_cast<double2*>(L), res, static_cast<RedKey*>(partial), red, slot_of, log, tol, psd, select_next);
         }
