@@ -785,7 +785,9 @@ def run_gpu(args):
         f64, f32 = ctypes.c_double(), ctypes.c_double()
         nat.check(lib.gx_eri_plan_counts(plan, ctypes.byref(n64), ctypes.byref(n32), ctypes.byref(f64),
                                          ctypes.byref(f32)))
-        return ms, clock_info, (n64.value, n32.value, f64.value, f32.value)
+        launches = ctypes.c_int()
+        nat.check(lib.gx_eri_plan_info(plan, None, None, None, ctypes.byref(launches)))
+        return ms, clock_info, (n64.value, n32.value, f64.value, f32.value, launches.value)
 
     if args.profile_e2e:
         # three host-output calls through the C ABI into page-locked memory,
@@ -1006,9 +1008,9 @@ def run_gpu(args):
                                         "no FP64/FP32 CUDA-core peak",
                          "peak32": peak32.value},
             "parity": parity,
-            # one kernel per (la, lb, lc, ld) class per step; the pair records
-            # are computed once per field, before the timed steps
-            "gpu_launches": int(lib.gx_eri_plan_class_count(plan)) * args.steps,
+            # kernels of a step as the plan enqueues (and replays) them; the pair
+            # records are computed once per field, before the timed steps
+            "gpu_launches": (cnt_mx if headline_mixed else cnt64)[4] * args.steps,
             "autotune": {str({0: "fp64", 1: "mixed", 2: "fp64_exact"}[k]): v for k, v in tuning.items()} or None,
             "graph_replays": int(lib.gx_eri_plan_graph_replays(plan)),
             "clocks": clock_info,

@@ -1380,10 +1380,13 @@ void launch_class(gx_context* ctx, gx::EriDev dev, const PlanData& plan, size_t 
     }
 }
 
-// One launch of a plan: its classes, and the function that enqueues it.
+// One launch of a plan: its classes, the function that enqueues it, and its
+// kernels (a lane-dense launch has a second one in mixed precision, and a third
+// one for what that leaves to FP64).
 struct PlanLaunch {
     std::vector<size_t> classes;
     std::function<void(cudaStream_t)> enqueue;
+    int kernels = 1;
 };
 
 // The launches of one plan (`dev` and `plan` outlive them).  Small and lane-dense classes with few primitive
@@ -1396,6 +1399,11 @@ struct PlanLaunch {
 // of three atoms took 29.1 ms instead of 27.7).
 constexpr int64_t kSharedLaunch = 4096, kSharedPlan = 65536;
 
+// The class may have entries that FP32 leaves to FP64.
+bool wide_order(const PlanClass& pc) {
+    return pc.key[0] + pc.key[1] + pc.key[2] + pc.key[3] >= gx::kWideOrder;
+}
+
 // wide: see launch_dense_classes.
 std::vector<PlanLaunch> plan_launches(gx_context* ctx, const gx::EriDev& dev, const PlanData& plan, int precision,
                                       unsigned long long* counters, bool wide) {
@@ -1403,6 +1411,13 @@ std::vector<PlanLaunch> plan_launches(gx_context* ctx, const gx::EriDev& dev, co
     const auto& tuned = plan.tuned[precision];
     const GroupSet& gs = tuned.valid ? tuned.groups : plan.base;
     const size_t nc = plan.classes.size();
+    const bool mixed = dev.fp32_cut > 0.0f;
+    auto own_kernels = [&](size_t ci) {
+        const PlanClass& pc = plan.classes[ci];
+        const bool dense = !gx::small_class(pc.key[0], pc.key[1], pc.key[2], pc.key[3]) &&
+                           runs_dense(plan, pc, tuned.valid ? tuned.conf[ci] : plan.defconf[ci], dev.all_real);
+        return dense && mixed ? 2 + (wide && wide_order(pc) ? 1 : 0) : 1;
+    };
     std::map<int, std::vector<size_t>> shared;  // by (order and) template pair; small classes at -1
     std::vector<size_t> own;
     for (size_t oi = 0; oi < nc; ++oi) {
@@ -1424,6 +1439,8 @@ std::vector<PlanLaunch> plan_launches(gx_context* ctx, const gx::EriDev& dev, co
     for (auto it = shared.rbegin(); it != shared.rend(); ++it) {
         const int pair = it->first < 0 ? -1 : it->first % 16;
         const std::vector<size_t> cs = it->second;
+        const bool high = std::any_of(cs.begin(), cs.end(), [&](size_t ci) { return wide_order(plan.classes[ci]); });
+        const int lists = pair < 0 ? 1 : gx::dense_lists(cs.size());
         out.push_back({cs, [=, &dev, &plan](cudaStream_t s) {
             std::vector<gx::QuartetClass> classes;
             std::vector<int> keys;
@@ -1438,14 +1455,14 @@ std::vector<PlanLaunch> plan_launches(gx_context* ctx, const gx::EriDev& dev, co
                 GX_CUDA(gx::launch_small_list(dev, keys, classes, s));
             else
                 launch_dense_classes(ctx, pair, dev, classes, s, true);
-        }});
+        }, pair >= 0 && mixed ? 2 * lists + (high ? gx::wide_lists(cs.size()) : 0) : lists});
     }
     for (size_t ci : own)
         out.push_back({{ci}, [=, &dev, &plan, &tuned, &gs](cudaStream_t s) {
             launch_class(ctx, dev, plan, ci, tuned.valid ? tuned.conf[ci] : plan.defconf[ci],
                          gs.dev.as<int2>() + gs.range[ci].first, (int)gs.range[ci].second, counters, s, nullptr,
                          nullptr, nullptr, wide);
-        }});
+        }, own_kernels(ci)});
     return out;
 }
 
@@ -1454,14 +1471,15 @@ std::vector<PlanLaunch> plan_launches(gx_context* ctx, const gx::EriDev& dev, co
 // cost a field of five atoms 0.3 ms of 3.8).  The shared launches are followed by
 // theirs, which then run beside the rest of the plan: a unit of (dd|dd) takes 0.2
 // ms, most of it latency.
-void launch_wide_classes(gx_context* ctx, const gx::EriDev& dev, const PlanData& plan, int precision,
-                         unsigned long long* counters, cudaStream_t s) {
-    if (!(dev.fp32_cut > 0.0f)) return;
+// Returns the launches.
+int launch_wide_classes(gx_context* ctx, const gx::EriDev& dev, const PlanData& plan, int precision,
+                        unsigned long long* counters, cudaStream_t s) {
+    if (!(dev.fp32_cut > 0.0f)) return 0;
     const auto& tuned = plan.tuned[precision];
     std::vector<std::pair<int, gx::QuartetClass>> list;
     for (size_t ci = 0; ci < plan.classes.size(); ++ci) {
         const auto& k = plan.classes[ci].key;
-        if (k[0] + k[1] + k[2] + k[3] < gx::kWideOrder ||
+        if (!wide_order(plan.classes[ci]) ||
             plan.classes[ci].primitive_quartets <= kSharedLaunch ||
             !runs_dense(plan, plan.classes[ci], tuned.valid ? tuned.conf[ci] : plan.defconf[ci], dev.all_real))
             continue;
@@ -1470,6 +1488,7 @@ void launch_wide_classes(gx_context* ctx, const gx::EriDev& dev, const PlanData&
         list.push_back({pair, qc});
     }
     GX_CUDA(gx::launch_wide(dev, list, ctx->sm_count, s));
+    return gx::wide_lists(list.size());
 }
 
 // Enqueue the pair records for (B, O) and every class launch without a wait.
@@ -1489,7 +1508,8 @@ int execute_plan(gx_context* ctx, gx_basis* b, const double* B, const double* O,
     return enqueue_plan(ctx, dev, plan, precision, counters, accumulate, host_mapped);
 }
 
-// Enqueue every class launch of `plan` for the evaluation view `dev`.
+// Enqueue every class launch of `plan` for the evaluation view `dev`; returns the
+// kernels enqueued (without host copies).
 int enqueue_plan(gx_context* ctx, const gx::EriDev& dev, const PlanData& plan, int precision,
                  unsigned long long* counters, bool accumulate, void* host_mapped) {
     cudaStream_t s = ctx->stream;
@@ -1558,9 +1578,11 @@ int enqueue_plan(gx_context* ctx, const gx::EriDev& dev, const PlanData& plan, i
             GX_CUDA(cudaEventRecord(ctx->aux_done[k], ctx->aux[k]));
             GX_CUDA(cudaStreamWaitEvent(s, ctx->aux_done[k], 0));
         }
-    if (!host_mapped) launch_wide_classes(ctx, dev, plan, precision, counters, s);
+    int kernels = (dev.fp32_cut > 0.0f ? plan.units.ntask : plan.units.ntask64) > 0 ? 2 : 0;
+    for (const PlanLaunch& l : launches) kernels += l.kernels;
+    if (!host_mapped) kernels += launch_wide_classes(ctx, dev, plan, precision, counters, s);
     join_copies();
-    return 1 + (int)launches.size();
+    return kernels;
 }
 
 // Enqueue several plans (each with its own evaluation view and counters,
@@ -4600,6 +4622,7 @@ extern "C" int gx_cholesky_last_stats(gx_context* ctx, gx_cholesky_stats* out) {
 struct PlanGraph {
     cudaGraphExec_t exec = nullptr;
     std::array<uintptr_t, 9> key{}, pending{};
+    int kernels = 0;  // in the graph
     bool disabled = false;
     void reset() {
         if (exec) cudaGraphExecDestroy(exec);
@@ -4615,7 +4638,7 @@ struct gx_eri_plan {
     gx_basis* basis;
     PlanData data;
     int64_t total = 0;
-    int last_launches = 0;
+    int last_launches = 0;  // kernels of the last execution
     PlanGraph graph;
     // The last execution that was not captured by the caller: the next one, on
     // whichever stream, follows it (both write the unit arrays).  One that the
@@ -4680,7 +4703,16 @@ int gx_eri_plan_info(const gx_eri_plan* plan, int64_t* tasks, int64_t* primitive
         if (tasks) *tasks = plan->data.ntask;
         if (primitive_quartets) *primitive_quartets = plan->data.primitive_quartets;
         if (model_flops) *model_flops = plan->data.model_flops;
-        if (launches) *launches = 1 + (int)plan->data.classes.size();
+        if (launches) {
+            std::lock_guard<std::mutex> lock(plan->ctx->mu);
+            *launches = plan->last_launches;
+            if (*launches == 0) {  // (not executed yet: what FP64 in a field takes)
+                gx::EriDev dev{};
+                *launches = plan->data.units.ntask64 > 0 ? 2 : 0;
+                for (const PlanLaunch& l : plan_launches(plan->ctx, dev, plan->data, GX_PRECISION_FP64, nullptr, false))
+                    *launches += l.kernels;
+            }
+        }
     });
 }
 
@@ -4737,7 +4769,7 @@ void plan_enqueue(gx_eri_plan* plan, const double* B, const double* O, int preci
     if (capturable && g.exec && g.key == key) {
         GX_CUDA(cudaGraphLaunch(g.exec, ctx->stream));
         ++plan->graph_replays;
-        plan->last_launches = 1 + (int)pd.classes.size();
+        plan->last_launches = g.kernels;
         return;
     }
     if (capturable && g.pending == key) {
@@ -4760,6 +4792,7 @@ void plan_enqueue(gx_eri_plan* plan, const double* B, const double* O, int preci
         if (graph) cudaGraphDestroy(graph);
         if (e == cudaSuccess) {
             g.key = key;
+            g.kernels = plan->last_launches;
             GX_CUDA(cudaGraphLaunch(g.exec, ctx->stream));
             ++plan->graph_replays;
             return;
@@ -4867,7 +4900,9 @@ int gx_eri_plan_profile(gx_eri_plan* plan, const double* B, const double* O, int
             o.per_group = used.per_group;
             o.warps_per_block = wpb[ci];
             o.batch = b1[ci];
-            o.groups = (int64_t)gs.range[ci].second;
+            const bool units = gx::small_class(pc.key[0], pc.key[1], pc.key[2], pc.key[3]) ||
+                               runs_dense(pd, pc, used, dev.all_real);
+            o.groups = units ? pd.unit_grid[ci] : (int64_t)gs.range[ci].second;
             o.kt = tiles[3 * ci];
             o.ct = tiles[3 * ci + 1];
             o.min_blocks = tiles[3 * ci + 2];

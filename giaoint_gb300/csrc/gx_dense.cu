@@ -94,6 +94,8 @@ int dense_orient(int la, int lb, int lc, int ld, QuartetClass& qc) {
     return la * 4 + lb;
 }
 
+int dense_lists(size_t n) { return (int)((n + dense::kMaxClasses - 1) / dense::kMaxClasses); }
+
 int dense_smem(int pair, const QuartetClass& qc, int word) {
     return smem_bytes(pair / 4, pair % 4, qc.ket.la, qc.ket.lb, word);
 }

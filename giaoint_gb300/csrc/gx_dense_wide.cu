@@ -58,6 +58,8 @@ __global__ void __launch_bounds__(32 * dense::kWarps) wide_kernel(const __grid_c
 
 }  // namespace
 
+int wide_lists(size_t n) { return (int)((n + kMaxWide - 1) / kMaxWide); }
+
 cudaError_t launch_wide(const EriDev& d, const std::vector<std::pair<int, QuartetClass>>& classes, int sms,
                         cudaStream_t s) {
     static PerDevice limit;

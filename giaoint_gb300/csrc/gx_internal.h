@@ -315,6 +315,9 @@ cudaError_t launch_units(const UnitPlan& u, const Task* tasks, const EriDev& d, 
 int dense_orient(int la, int lb, int lc, int ld, QuartetClass& qc);
 // Classes of one template pair in as few launches as hold them.
 cudaError_t launch_dense(int pair, const EriDev& d, const std::vector<QuartetClass>& classes, bool f32, cudaStream_t s);
+// Launches that a list of n classes of one pair takes there, and in launch_wide.
+int dense_lists(size_t n);
+int wide_lists(size_t n);
 // Shared memory of a block (qc oriented for `pair`; word: bytes of a table entry).
 int dense_smem(int pair, const QuartetClass& qc, int word);
 // The entries that FP32 left to FP64, of classes of any template pair (given

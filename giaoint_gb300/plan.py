@@ -57,14 +57,21 @@ class EriPlan:
         nat.check(lib.gx_eri_plan_create(self._ctx.handle, basis._device(self._ctx), nat.u32ptr(self.quartets),
                                          len(self.quartets), nat.i64ptr(self.offsets), ctypes.byref(handle)))
         self._handle = handle
-        tasks, prims = ctypes.c_int64(), ctypes.c_int64()
-        flops, launches = ctypes.c_double(), ctypes.c_int()
-        nat.check(lib.gx_eri_plan_info(handle, ctypes.byref(tasks), ctypes.byref(prims), ctypes.byref(flops),
-                                       ctypes.byref(launches)))
+        tasks, prims, flops = ctypes.c_int64(), ctypes.c_int64(), ctypes.c_double()
+        nat.check(lib.gx_eri_plan_info(handle, ctypes.byref(tasks), ctypes.byref(prims), ctypes.byref(flops), None))
         self.tasks = tasks.value
         self.primitive_quartets = prims.value
         self.model_flops = flops.value
-        self.launches = launches.value
+        self._launches = 0
+
+    @property
+    def launches(self) -> int:
+        """Kernel launches of the last execution (before the first: of one in FP64 in a field)."""
+        if self._handle:
+            n = ctypes.c_int()
+            nat.check(nat.lib().gx_eri_plan_info(self._handle, None, None, None, ctypes.byref(n)))
+            self._launches = n.value
+        return self._launches
 
     @property
     def total(self) -> int:
@@ -146,6 +153,7 @@ class EriPlan:
 
     def close(self) -> None:
         if getattr(self, "_handle", None):
+            self._launches = self.launches
             nat.lib().gx_eri_plan_destroy(self._handle)
             self._handle = None
 

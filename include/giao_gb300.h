@@ -404,7 +404,8 @@ typedef struct gx_eri_plan gx_eri_plan;
 int gx_eri_plan_create(gx_context* ctx, gx_basis* basis, const uint32_t* quartets, int64_t nq, int64_t* offsets,
                        gx_eri_plan** out);
 /* tasks (segmented quartets), primitive quartets, FP64 FLOP-model total and
- * kernel launches per execution. */
+ * kernel launches of the last execution (before the first one: of one in FP64
+ * in a field; the pair records of a new field are four more). */
 int gx_eri_plan_info(const gx_eri_plan* plan, int64_t* tasks, int64_t* primitive_quartets, double* model_flops,
                      int* launches);
 /* Enqueue the evaluation for field (B, O) into device memory out_device
@@ -418,7 +419,7 @@ int gx_eri_plan_counts(gx_eri_plan* plan, int64_t* fp64_quartets, int64_t* fp32_
                        double* fp32_flops);
 void gx_eri_plan_destroy(gx_eri_plan* plan);
 
-/* Number of (la, lb, lc, ld) classes (one kernel launch each). */
+/* Number of (la, lb, lc, ld) classes. */
 int gx_eri_plan_class_count(const gx_eri_plan* plan);
 /* Executions served by replaying the plan's CUDA graph so far (a plan is
  * captured on its second execution with the same stream, output, precision
@@ -436,7 +437,7 @@ typedef struct gx_class_profile {
     float ms;                      /* event-timed kernel duration */
     int per_group;                 /* launch configuration: primitive quartets per warp unit (0 = default) */
     int warps_per_block, batch;    /* generic kernel: warps per block, phase-1 batch */
-    int64_t groups;                /* warp work units */
+    int64_t groups;                /* work units (small and lane-dense classes: before screening) */
     int kt, ct;                    /* generic kernel: ket-transform rows and bra-transform components per lane */
     int min_blocks;                /* generic kernel: register-budget variant (resident blocks) */
     int stream;                    /* generic kernel: 1 = per-entry recurrences (stream mode) */
