@@ -690,6 +690,37 @@ def run_reference(args):
     print(json.dumps(line), flush=True)
 
 
+# What the printed line holds of each leg (a line of all of it has 24 KB, which
+# no longer fits the logs that keep the end of a run's output).
+LEG_KEYS = {
+    "run": None, "clocks": None, "parity": None, "config": None,
+    "fp64_exact": ("ms_per_step", "eris_per_s"),
+    "fp64": ("ms_per_step", "eris_per_s", "max_abs_error_vs_fp64_exact"),
+    "mixed": ("ms_per_step", "eris_per_s", "max_abs_error_vs_fp64_exact", "speedup_vs_fp64", "speedup_vs_fp64_exact"),
+    "roofline": ("bound", "unit", "achieved", "peak", "frac"),
+    "e2e": ("value", "unit", "h2d_bytes_per_step", "d2h_bytes_per_step", "seconds_per_step", "cold_call_seconds", "api"),
+    "cpu_baseline": ("value", "unit", "cores", "kind"),
+    "cholesky": ("seconds", "rank", "max_residual", "speedup_vs_cpu_port"),
+    "field_sweep": ("fields", "fp64_ms_total", "mixed_ms_total", "speedup_mixed_vs_fp64", "max_abs_err_mixed_vs_fp64"),
+    "full_tensor": ("ms_per_call_p50", "ms_per_call_min"),
+    "center_derivatives": ("seconds_device", "components_per_s", "seconds_host_output"),
+    "serving": ("requests", "completed", "refused_memory", "p50_ms", "p99_ms", "requests_per_s"),
+}
+
+
+def summary(line):
+    out = {}
+    for key, value in line.items():
+        if key not in LEG_KEYS:
+            if not isinstance(value, (dict, list)):
+                out[key] = value
+        elif LEG_KEYS[key] is None or not isinstance(value, dict):
+            out[key] = value
+        else:
+            out[key] = {k: value[k] for k in LEG_KEYS[key] if k in value}
+    return out
+
+
 def run_gpu(args):
     import torch
 
@@ -1022,7 +1053,8 @@ def run_gpu(args):
             "center_derivatives": derivatives,
             "serving": serving,
         }
-        print(json.dumps(line), flush=True)
+        print(json.dumps(line), file=sys.stderr, flush=True)  # everything, legs and fields one by one
+        print(json.dumps(summary(line)), flush=True)
     lib.gx_eri_plan_destroy(plan)
     if world > 1:
         torch.distributed.destroy_process_group()
