@@ -399,6 +399,7 @@ struct gx_basis {
     // segmented shells: shell s, contraction x -> seg_first[s] + x
     int nseg = 0;
     bool one_site = true;  // all shells on one centre
+    int max_pairs = 0;     // primitive pairs of the deepest shell pair
     std::vector<int> seg_first, seg_l, seg_nprim, seg_primoff, seg_raw, seg_orig;
     std::vector<double> seg_center, seg_exps, seg_coefs;
     DeviceBuffer mem;  // one allocation, and the views of its parts
@@ -485,6 +486,7 @@ void build_segments(gx_basis* b) {
                 words.push_back(b->ctx->pair_class(b->seg_l[a], b->seg_l[bb]).Etot);
             }
             const int64_t count = (int64_t)b->seg_nprim[a] * b->seg_nprim[bb];
+            b->max_pairs = (int)std::max<int64_t>(b->max_pairs, std::min<int64_t>(count, INT32_MAX));
             b->sp_off[k] = (int)npp;
             sp_class[k] = ci;
             sp_E[k] = b->Etotal;
@@ -602,7 +604,8 @@ FieldPairs& field_pairs(gx_basis* b, const double* B, const double* O) {
                                        b->d_classes.as<gx::PairClassDev>(), fp.p.as<double>(), fp.Pr.as<double>(),
                                        fp.Pi.as<double>(), fp.F.as<double2>(), b->d_Eoff.as<long long>(),
                                        fp.Epool.as<double2>(), fp.Epool32.as<float2>(), fp.bound.as<double>(),
-                                       fp.g32.as<float4>(), fp.order.as<int>(), fp.sbound.as<float>(), dev,
+                                       fp.g32.as<float4>(), fp.order.as<int>(), fp.sbound.as<float>(),
+                                       b->max_pairs, dev,
                                        b->ctx->stream));
     fp.written.record(b->ctx->stream);
     fp.valid = true;

@@ -211,7 +211,7 @@ cudaError_t launch_pair_precompute(const BasisDev& basis, const double* B, const
                                    const int* pp_b, const int* pp_pa, const int* pp_pb, const int* pp_class,
                                    const PairClassDev* classes, double* p, double* Pr, double* Pi, double2* F,
                                    const long long* Eoff, double2* Epool, float2* Epool32, double* bound, float4* g32,
-                                   int* order, float* sbound, const EriDev& dev, cudaStream_t s);
+                                   int* order, float* sbound, int max_pairs, const EriDev& dev, cudaStream_t s);
 size_t quartet_smem_bytes(const QuartetClass& qc, int warps_per_block, bool mixed);
 cudaError_t launch_quartets(const EriDev& dev, const QuartetClass& qc, int warps_per_block, int grid,
                             cudaStream_t s);

@@ -671,21 +671,33 @@ __global__ void __launch_bounds__(32 * kBoundWarps) pair_bound_kernel(BasisDev b
 }
 
 // The primitive pairs of every shell pair by decreasing factor (equal ones in
-// record order): the rank of a pair is the number of pairs before it.
-__global__ void pair_order_kernel(BasisDev bs, const double* bound, int* order, float* sbound) {
-    const int sp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+// record order): the rank of a pair is the number of pairs before it.  The factors
+// are not negative, so that they compare as integers (an FP64 comparison occupies
+// the sub-partition for 64 cycles).  A warp takes a shell pair, a block of its own
+// one with more than kWarpPairs primitive pairs, whose comparisons are their
+// square (records and nuclear attraction of two s shells of 50 primitives 2.2 ms,
+// 16 with a warp and FP64 comparisons for every shell pair; of 257, 0.27 and 12 s).
+constexpr int kWarpPairs = 256;
+
+template <bool BLOCK>
+__global__ void __launch_bounds__(BLOCK ? 1024 : 128) pair_order_kernel(BasisDev bs, const double* bound, int* order,
+                                                                        float* sbound) {
+    const int sp = BLOCK ? blockIdx.x : blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (sp >= bs.ns * bs.ns) return;
     const int a = sp / bs.ns, b = sp - a * bs.ns;
     const int first = bs.sp_off[sp], count = bs.nprim[a] * bs.nprim[b];
-    for (int x = threadIdx.x & 31; x < count; x += 32) {
-        const double v = bound[first + x];
+    if (BLOCK != (count > kWarpPairs)) return;
+    const long long* keys = reinterpret_cast<const long long*>(bound + first);
+    for (int x = BLOCK ? threadIdx.x : threadIdx.x & 31; x < count; x += BLOCK ? blockDim.x : 32) {
+        const long long v = keys[x];
         int rank = 0;
+#pragma unroll 4
         for (int y = 0; y < count; ++y) {
-            const double w = bound[first + y];
+            const long long w = keys[y];
             rank += w > v || (w == v && y < x);
         }
         order[first + rank] = first + x;
-        sbound[first + rank] = (float)fmin(v, 3.0e38);
+        sbound[first + rank] = (float)fmin(__longlong_as_double(v), 3.0e38);
     }
 }
 
@@ -733,7 +745,7 @@ cudaError_t launch_pair_precompute(const BasisDev& basis, const double* B, const
                                    const int* pp_b, const int* pp_pa, const int* pp_pb, const int* pp_class,
                                    const PairClassDev* classes, double* p, double* Pr, double* Pi, double2* F,
                                    const long long* Eoff, double2* Epool, float2* Epool32, double* bound, float4* g32,
-                                   int* order, float* sbound, const EriDev& dev, cudaStream_t s) {
+                                   int* order, float* sbound, int max_pairs, const EriDev& dev, cudaStream_t s) {
     if (npp <= 0) return cudaSuccess;
     const double3 Bv = make_double3(B[0], B[1], B[2]), Ov = make_double3(O[0], O[1], O[2]);
     const unsigned warps = (unsigned)((npp + kPairWarps - 1) / kPairWarps);
@@ -744,7 +756,8 @@ cudaError_t launch_pair_precompute(const BasisDev& basis, const double* B, const
     pair_bound_kernel<<<(unsigned)((npp + kBoundWarps - 1) / kBoundWarps), 32 * kBoundWarps, 0, s>>>(basis, dev, npp, pp_a, pp_b, pp_pa, pp_pb, pp_class, classes,
                                                         bound);
     const unsigned pairs = (unsigned)basis.ns * (unsigned)basis.ns;
-    pair_order_kernel<<<(pairs + 3) / 4, 128, 0, s>>>(basis, bound, order, sbound);
+    pair_order_kernel<false><<<(pairs + 3) / 4, 128, 0, s>>>(basis, bound, order, sbound);
+    if (max_pairs > kWarpPairs) pair_order_kernel<true><<<pairs, 1024, 0, s>>>(basis, bound, order, sbound);
     return cudaGetLastError();
 }
 
