@@ -310,7 +310,7 @@ struct WarpBuffers {
     long long seg_off[32];
     int4 seg_st[32];
     int seg_lane[36];  // first lane and flags of each segment, and the end
-    int2 queue[64];    // task, bra pair << 16 | ket pair
+    int2 queue[64];    // task, bra pair * ket pairs of the task + ket pair
     Walk walk;
 };
 
@@ -535,13 +535,15 @@ __device__ __forceinline__ void small_block(const EriDev& d, const QuartetClass&
                 const int n = stream.next(lane, task, rank, pq);
                 more = n > 0;
                 bool mine = lane < n;
+                int at = 0;
                 if (mine) {
                     const Task* tg = qc.tasks + task;
+                    at = pq.x * (d.basis.nprim[tg->sc] * d.basis.nprim[tg->sd]) + pq.y;
                     mine = (pass == 0) ==
                            boys_asymptotic32(pp, pp.order[tg->pab + pq.x], pp.order[tg->pcd + pq.y], L);
                 }
                 const unsigned m = __ballot_sync(0xffffffffu, mine);
-                if (mine) w.queue[waiting + __popc(m & ((1u << lane) - 1u))] = make_int2(task, pq.x << 16 | pq.y);
+                if (mine) w.queue[waiting + __popc(m & ((1u << lane) - 1u))] = make_int2(task, at);
                 waiting += __popc(m);
             }
             __syncwarp();
@@ -555,7 +557,8 @@ __device__ __forceinline__ void small_block(const EriDev& d, const QuartetClass&
             const int nseg = segments<NOUT>(w, qc, en.x, 0, nb, lane);
             if (lane < nb) {
                 const Task* tg = qc.tasks + en.x;
-                const int ip = pp.order[tg->pab + (int)((unsigned)en.y >> 16)], iq = pp.order[tg->pcd + (en.y & 0xffff)];
+                const int Kcd = d.basis.nprim[tg->sc] * d.basis.nprim[tg->sd], P = en.y / Kcd;
+                const int ip = pp.order[tg->pab + P], iq = pp.order[tg->pcd + en.y - P * Kcd];
                 const double p = pp.p[ip], q = pp.p[iq];
                 const double2 X[3] = {c2(pp.Pr[3 * ip] - pp.Pr[3 * iq], pp.Pi[3 * ip] - pp.Pi[3 * iq]),
                                       c2(pp.Pr[3 * ip + 1] - pp.Pr[3 * iq + 1], pp.Pi[3 * ip + 1] - pp.Pi[3 * iq + 1]),

@@ -191,3 +191,26 @@ def test_pair_records_of_deep_contractions_stay_cheap():
                               field=gi.MagneticField((0.1, 0.01 * k, 0.0)))
         best = min(best, time.perf_counter() - start)
     assert best <= 0.2, best
+
+
+def test_mixed_precision_of_very_deep_contractions():
+    """An (ss|ss) of 66,049 bra pairs whose FP32 entries wait in a queue: every entry keeps its own pair (a sum of
+    FP32 values, all entries in the FP32 range: 66,049 roundings of 6e-8 of at most the largest entry, and the FP32
+    recurrence of a few more)."""
+    from giaoint_gb300.plan import EriPlan
+
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(4)
+    deep = [gi.Shell((0.1 * k, 0.0, 0.0), 0, np.exp(rng.uniform(-1.0, 6.0, 257)), rng.uniform(0.1, 1.0, 257))
+            for k in range(2)]
+    basis = gi.Basis(deep + [gi.Shell((0.0, 0.2, 0.0), 0, [0.7], [1.0]), gi.Shell((0.0, 0.0, 0.3), 0, [1.1], [1.0])])
+    plan = EriPlan(basis, [(0, 1, 2, 3), (2, 3, 1, 0)])
+    out = torch.empty(plan.total, dtype=torch.complex128, device="cuda:0")
+    field = gi.MagneticField((0.1, -0.1, 0.05))
+    plan.execute(out, field, precision="fp64_exact")
+    plan.synchronize()
+    exact = out.cpu().numpy()
+    plan.execute(out, field, precision="mixed", mixed_cutoff=1.0e30)
+    plan.synchronize()
+    assert plan.counts()["fp32_quartets"] > 2 * 65536
+    assert np.abs(out.cpu().numpy() - exact).max() <= 1e-6 * np.abs(exact).max()
