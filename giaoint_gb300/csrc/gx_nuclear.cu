@@ -86,88 +86,90 @@ __device__ __forceinline__ void nuclear_block(const NuclearArgs& a, int sa, int 
     const BasisDev& bs = a.bs;
     const PairData& pp = a.pp;
     const int L = pc.la + pc.lb, NL = herm_count(L);
-    const int p0 = bs.sp_off[sa * bs.ns + sb];
-    const int total = bs.nprim[sa] * bs.nprim[sb] * a.nnuc;
+    const int pairs = bs.nprim[sa] * bs.nprim[sb], group = max(1, (1 << 30) / max(1, a.nnuc));  // (32-bit indices)
     const double scale = -6.283185307179586 / 5.914967172795613;  // -2 pi / sqrt(2 pi^{5/2})
-    for (int first = 0; first < total; first += 32) {
-        const int nb = min(32, total - first);
-        const int it = first + min(lane, nb - 1);
-        const int ip = p0 + it / a.nnuc, c = it - (it / a.nnuc) * a.nnuc;
-        const double p = pp.p[ip];
-        double x[3];
-        for (int k = 0; k < 3; ++k) x[k] = pp.Pr[3 * ip + k] - a.center[3 * c + k];
-        const double z = a.charge[c] * scale;
-        if constexpr (REAL) {
-            const double t = p * (x[0] * x[0] + x[1] * x[1] + x[2] * x[2]);
-            double Sh[kDenseOrder + 1], e0;
-            if (const int rc = boys_eval_real(t, L, a.boys, Sh, e0)) {
-                report(a.status, rc, blockIdx.x, L, t, 0.0);
-                e0 = 0.0;
-                for (int k = 0; k <= L; ++k) Sh[k] = 0.0;
-            }
-            double s = e0 * z;
-            for (int k = 0; k <= L; ++k) {
-                Sh[k] *= s;
-                s *= -2.0 * p;
-            }
-            column_rec<double>(L, Sh, x, R + lane, a.herm_xyz);
-        } else {
-            const double2 X[3] = {c2(x[0], pp.Pi[3 * ip]), c2(x[1], pp.Pi[3 * ip + 1]), c2(x[2], pp.Pi[3 * ip + 2])};
-            const double tre = p * (X[0].x * X[0].x + X[1].x * X[1].x + X[2].x * X[2].x -
-                                    (X[0].y * X[0].y + X[1].y * X[1].y + X[2].y * X[2].y));
-            const double tim = 2.0 * p * (X[0].x * X[0].y + X[1].x * X[1].y + X[2].x * X[2].y);
-            double2 Sh[kDenseOrder + 1], e0;
-            if (const int rc = boys_eval(tre, tim, L, a.boys, a.gl, Sh, e0)) {
-                report(a.status, rc, blockIdx.x, L, tre, tim);
-                e0 = c2(0.0, 0.0);
-                for (int k = 0; k <= L; ++k) Sh[k] = c2(0.0, 0.0);
-            }
-            double2 s = cscale(e0, z);
-            for (int k = 0; k <= L; ++k) {
-                Sh[k] = cmul(s, Sh[k]);
-                s = cscale(s, -2.0 * p);
-            }
-            column_rec<double2>(L, Sh, X, R + lane, a.herm_xyz);
-        }
-        __syncwarp();
-        // rows summed over the nuclei of each primitive pair; the sum of the
-        // batch's j-th pair goes to column j, which has been read by then
-        const int k0 = first / a.nnuc, k1 = (first + nb - 1) / a.nnuc;
-        for (int row = lane; row < NL; row += 32) {
-            T* r = R + 33 * row;
-            int l = 0;
-            for (int k = k0; k <= k1; ++k) {
-                const int end = min(nb, (k + 1) * a.nnuc - first);
-                T sum = r[l++];
-                for (; l < end; ++l) sum = nadd(sum, r[l]);
-                r[k - k0] = sum;
-            }
-        }
-        __syncwarp();
-        for (int ab = lane; ab < pc.nab; ab += 32) {
-            const int bo = pc.boxoff[ab], bd = pc.boxdim[ab];
-            const int nbox = (bd & 255) * ((bd >> 8) & 255) * ((bd >> 16) & 255);
-            double2 sum = acc[ab];
-            for (int k = k0; k <= k1; ++k) {
-                const double2* E = pp.Epool + pp.Eoff[p0 + k] + bo;
-                const double2 F = pp.F[p0 + k];
-                T v{};
-                for (int e = 0; e < nbox; ++e) {
-                    const uint32_t ke = pc.ent[bo + e];
-                    const T rv = R[33 * herm_index(ke & 255, (ke >> 8) & 255, (ke >> 16) & 255) + (k - k0)];
-                    if constexpr (REAL)
-                        v = fma(__ldg(&E[e].x), rv, v);
-                    else
-                        v = cmac(v, __ldg(&E[e]), rv);
+    for (int g0 = 0; g0 < pairs; g0 += group) {
+        const int p0 = bs.sp_off[sa * bs.ns + sb] + g0, total = min(group, pairs - g0) * a.nnuc;
+        for (int first = 0; first < total; first += 32) {
+            const int nb = min(32, total - first);
+            const int it = first + min(lane, nb - 1);
+            const int ip = p0 + it / a.nnuc, c = it - (it / a.nnuc) * a.nnuc;
+            const double p = pp.p[ip];
+            double x[3];
+            for (int k = 0; k < 3; ++k) x[k] = pp.Pr[3 * ip + k] - a.center[3 * c + k];
+            const double z = a.charge[c] * scale;
+            if constexpr (REAL) {
+                const double t = p * (x[0] * x[0] + x[1] * x[1] + x[2] * x[2]);
+                double Sh[kDenseOrder + 1], e0;
+                if (const int rc = boys_eval_real(t, L, a.boys, Sh, e0)) {
+                    report(a.status, rc, blockIdx.x, L, t, 0.0);
+                    e0 = 0.0;
+                    for (int k = 0; k <= L; ++k) Sh[k] = 0.0;
                 }
-                if constexpr (REAL)
-                    sum.x = fma(F.x, v, sum.x);
-                else
-                    sum = cmac(sum, F, v);
+                double s = e0 * z;
+                for (int k = 0; k <= L; ++k) {
+                    Sh[k] *= s;
+                    s *= -2.0 * p;
+                }
+                column_rec<double>(L, Sh, x, R + lane, a.herm_xyz);
+            } else {
+                const double2 X[3] = {c2(x[0], pp.Pi[3 * ip]), c2(x[1], pp.Pi[3 * ip + 1]), c2(x[2], pp.Pi[3 * ip + 2])};
+                const double tre = p * (X[0].x * X[0].x + X[1].x * X[1].x + X[2].x * X[2].x -
+                                        (X[0].y * X[0].y + X[1].y * X[1].y + X[2].y * X[2].y));
+                const double tim = 2.0 * p * (X[0].x * X[0].y + X[1].x * X[1].y + X[2].x * X[2].y);
+                double2 Sh[kDenseOrder + 1], e0;
+                if (const int rc = boys_eval(tre, tim, L, a.boys, a.gl, Sh, e0)) {
+                    report(a.status, rc, blockIdx.x, L, tre, tim);
+                    e0 = c2(0.0, 0.0);
+                    for (int k = 0; k <= L; ++k) Sh[k] = c2(0.0, 0.0);
+                }
+                double2 s = cscale(e0, z);
+                for (int k = 0; k <= L; ++k) {
+                    Sh[k] = cmul(s, Sh[k]);
+                    s = cscale(s, -2.0 * p);
+                }
+                column_rec<double2>(L, Sh, X, R + lane, a.herm_xyz);
             }
-            acc[ab] = sum;
+            __syncwarp();
+            // rows summed over the nuclei of each primitive pair; the sum of the
+            // batch's j-th pair goes to column j, which has been read by then
+            const int k0 = first / a.nnuc, k1 = (first + nb - 1) / a.nnuc;
+            for (int row = lane; row < NL; row += 32) {
+                T* r = R + 33 * row;
+                int l = 0;
+                for (int k = k0; k <= k1; ++k) {
+                    const int end = min(nb, (k + 1) * a.nnuc - first);
+                    T sum = r[l++];
+                    for (; l < end; ++l) sum = nadd(sum, r[l]);
+                    r[k - k0] = sum;
+                }
+            }
+            __syncwarp();
+            for (int ab = lane; ab < pc.nab; ab += 32) {
+                const int bo = pc.boxoff[ab], bd = pc.boxdim[ab];
+                const int nbox = (bd & 255) * ((bd >> 8) & 255) * ((bd >> 16) & 255);
+                double2 sum = acc[ab];
+                for (int k = k0; k <= k1; ++k) {
+                    const double2* E = pp.Epool + pp.Eoff[p0 + k] + bo;
+                    const double2 F = pp.F[p0 + k];
+                    T v{};
+                    for (int e = 0; e < nbox; ++e) {
+                        const uint32_t ke = pc.ent[bo + e];
+                        const T rv = R[33 * herm_index(ke & 255, (ke >> 8) & 255, (ke >> 16) & 255) + (k - k0)];
+                        if constexpr (REAL)
+                            v = fma(__ldg(&E[e].x), rv, v);
+                        else
+                            v = cmac(v, __ldg(&E[e]), rv);
+                    }
+                    if constexpr (REAL)
+                        sum.x = fma(F.x, v, sum.x);
+                    else
+                        sum = cmac(sum, F, v);
+                }
+                acc[ab] = sum;
+            }
+            __syncwarp();  // the next batch overwrites the table
         }
-        __syncwarp();  // the next batch overwrites the table
     }
 }
 
