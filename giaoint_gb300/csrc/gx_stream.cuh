@@ -200,6 +200,10 @@ struct Stream {
                     else
                         cnt = counts[chunk + lane];
                 }
+                if (__any_sync(0xffffffffu, cnt > 1 << 25)) {  // (the sum of 32 might not fit)
+                    if (lane > 0) cnt = 0;
+                    next_task = chunk + 1;
+                }
                 incl = cnt;
 #pragma unroll
                 for (int off = 1; off < 32; off <<= 1) {
