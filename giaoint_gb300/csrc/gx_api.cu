@@ -4153,20 +4153,16 @@ void cholesky_core(gx_context* ctx, gx_basis* b, const double* Bf, const double*
                     std::vector<int> flip;
                     int64_t off = 0;
                     // (x y | sb sa), or (sb sa | x y) when (x, y) has the
-                    // higher angular momentum and at least as many primitive
-                    // pairs: the kernels spread the ket components of a shell
-                    // quartet over warps, so the wide pair goes to the ket (a
-                    // low-L pivot against high-L bra pairs otherwise leaves a
-                    // few warps on the long tasks), but they contract each
-                    // bra primitive pair once over all its ket primitive
-                    // pairs, so a contracted pivot pair stays in the ket (on
-                    // the 12-atom molecule, flipping against contracted s
-                    // pivots made the column evaluations 18% slower)
+                    // higher angular momentum: the class-generic kernel
+                    // spreads the ket components of a shell quartet over
+                    // warps, so the wide pair goes to the ket (the 140-function
+                    // atom's columns 29.1 ms, 32.9 without; s/p/d molecules,
+                    // whose classes the lane-dense kernel orients itself, are
+                    // the same either way)
                     const int lpiv = b->l[sa] + b->l[sb];
-                    const int kpiv = b->nprim[sa] * b->nprim[sb];
                     for (int x = 0; x < ns; ++x)
                         for (int y = real ? x : 0; y < ns; ++y) {
-                            const bool fl = b->l[x] + b->l[y] > lpiv && b->nprim[x] * b->nprim[y] >= kpiv;
+                            const bool fl = b->l[x] + b->l[y] > lpiv;
                             if (fl)
                                 req.push_back({(uint32_t)sb, (uint32_t)sa, (uint32_t)x, (uint32_t)y, off});
                             else
