@@ -160,7 +160,7 @@ struct Stream {
     // The last entry handed out, when its task goes on and the walk to it was a long
     // one: the next entry is sought from there (from the task's start every batch of
     // a deep contraction walked over all its bra pairs: one (ss|ss) of 20 primitives
-    // a shell, 1.6e5 entries, 141 instead of 37.6 ms).  In shared memory: held in
+    // a shell, 1.6e5 entries, 141 instead of 29.5 ms).  In shared memory: held in
     // registers it cost the (pp| template an occupancy step, 1% of twelve atoms.
     Walk* walk;
 

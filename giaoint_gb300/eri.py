@@ -10,8 +10,8 @@ Two keyword arguments are additions: ``precision`` and ``mixed_cutoff``.
 product is below 1e-18 (they move no result by more than ~1e-15);
 ``"fp64_exact"`` evaluates every primitive quartet as the reference does;
 ``"mixed"`` evaluates primitive quartets with Schwarz product below
-``mixed_cutoff`` in FP32 (FP64 Boys values, FP64 final summation) and skips
-those below 1e-15.
+``mixed_cutoff`` in FP32 (FP64 Boys values outside the asymptotic sector, FP64
+final summation) and skips those below 1e-15.
 """
 
 from __future__ import annotations

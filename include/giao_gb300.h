@@ -405,7 +405,7 @@ int gx_eri_plan_create(gx_context* ctx, gx_basis* basis, const uint32_t* quartet
                        gx_eri_plan** out);
 /* tasks (segmented quartets), primitive quartets, FP64 FLOP-model total and
  * kernel launches of the last execution (before the first one: of one in FP64
- * in a field; the pair records of a new field are four more). */
+ * in a field; the pair records of a new field are four or five more). */
 int gx_eri_plan_info(const gx_eri_plan* plan, int64_t* tasks, int64_t* primitive_quartets, double* model_flops,
                      int* launches);
 /* Enqueue the evaluation for field (B, O) into device memory out_device
