@@ -85,24 +85,32 @@ bool capturing(cudaStream_t s) {
 struct StreamMark {
     cudaEvent_t ev = nullptr;
     cudaStream_t stream = nullptr;
-    bool set = false;
+    bool set = false, late = false;
     StreamMark() = default;
     StreamMark(const StreamMark&) = delete;
     StreamMark& operator=(const StreamMark&) = delete;
     ~StreamMark() {
         if (ev) cudaEventDestroy(ev);
     }
-    void record(cudaStream_t s) {
-        if (!ev) GX_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-        GX_CUDA(cudaEventRecord(ev, s));
+    // lasting: s lives as long as the mark (the context's own stream), so that the
+    // event can wait until another stream asks (it costs a new basis 10 us)
+    void record(cudaStream_t s, bool lasting) {
+        if (!lasting) record_event(s);
         stream = s;
         set = true;
+        late = lasting;
+    }
+    void record_event(cudaStream_t s) {
+        if (!ev) GX_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+        GX_CUDA(cudaEventRecord(ev, s));
     }
     // Work enqueued on s from here on follows the mark.  (The per-thread default
     // stream is another stream in every thread.)  A stream that is being captured
     // cannot wait for an event outside its graph: the host waits.
-    void follow(cudaStream_t s) const {
+    void follow(cudaStream_t s) {
         if (!set || (s == stream && s != cudaStreamPerThread)) return;
+        if (late) record_event(stream);
+        late = false;
         if (!capturing(s)) {
             GX_CUDA(cudaStreamWaitEvent(s, ev, 0));
             return;
@@ -607,7 +615,7 @@ FieldPairs& field_pairs(gx_basis* b, const double* B, const double* O) {
                                        fp.g32.as<float4>(), fp.order.as<int>(), fp.sbound.as<float>(),
                                        b->max_pairs, dev,
                                        b->ctx->stream));
-    fp.written.record(b->ctx->stream);
+    fp.written.record(b->ctx->stream, b->ctx->stream == b->ctx->own_stream);
     fp.valid = true;
     return fp;
 }
@@ -4826,10 +4834,10 @@ int gx_eri_plan_execute(gx_eri_plan* plan, const double* B, const double* O, int
         try {
             plan_enqueue(plan, B, O, precision, mixed_cutoff, static_cast<double2*>(out_device));
         } catch (...) {
-            plan->done->record(ctx->stream);
+            plan->done->record(ctx->stream, ctx->stream == ctx->own_stream);
             throw;
         }
-        plan->done->record(ctx->stream);
+        plan->done->record(ctx->stream, ctx->stream == ctx->own_stream);
     });
 }
 

@@ -69,7 +69,7 @@ struct NuclearArgs {
     const uint32_t* herm_xyz;
     const PairClassDev* classes;
     const int* pp_class;
-    int nnuc;
+    int nnuc, group;  // nuclei; primitive pairs at a time (their entries are counted in 32 bits)
     const double* charge;
     const double* center;
     const long long* seg_ao;
@@ -86,10 +86,10 @@ __device__ __forceinline__ void nuclear_block(const NuclearArgs& a, int sa, int 
     const BasisDev& bs = a.bs;
     const PairData& pp = a.pp;
     const int L = pc.la + pc.lb, NL = herm_count(L);
-    const int pairs = bs.nprim[sa] * bs.nprim[sb], group = max(1, (1 << 30) / max(1, a.nnuc));  // (32-bit indices)
+    const int pairs = bs.nprim[sa] * bs.nprim[sb];
     const double scale = -6.283185307179586 / 5.914967172795613;  // -2 pi / sqrt(2 pi^{5/2})
-    for (int g0 = 0; g0 < pairs; g0 += group) {
-        const int p0 = bs.sp_off[sa * bs.ns + sb] + g0, total = min(group, pairs - g0) * a.nnuc;
+    for (int g0 = 0; g0 < pairs; g0 += a.group) {
+        const int p0 = bs.sp_off[sa * bs.ns + sb] + g0, total = min(a.group, pairs - g0) * a.nnuc;
         for (int first = 0; first < total; first += 32) {
             const int nb = min(32, total - first);
             const int it = first + min(lane, nb - 1);
@@ -310,7 +310,9 @@ cudaError_t launch_nuclear(const BasisDev& bs, const PairData& pp, const BoysTab
     const long long blocks = (long long)bs.ns * bs.ns;
     if (blocks == 0) return cudaSuccess;
     // pairs by order, so that the low ones do not carry the shared memory of the highest
-    const NuclearArgs args{bs, pp, boys, gl, herm_xyz, classes, pp_class, nnuc, charge, center, seg_ao, n, out, status};
+    const int group = std::max(1, (1 << 30) / std::max(1, nnuc));
+    const NuclearArgs args{bs,     pp,    boys,   gl,     herm_xyz, classes, pp_class, nnuc,
+                           group, charge, center, seg_ao, n,        out,     status};
     const int steps[] = {-1, 2, 4, 6, kDenseOrder};
     for (int k = 0; k < 4 && steps[k] < max_pair_L; ++k) {
         const int hi = steps[k + 1];
